@@ -157,6 +157,7 @@ struct RunPlan {
   uint32_t npc_edge = 0;
   int lut_shift = 0;
   uint32_t lut_base = 0;
+  bool cat_fast = false;           // category_fast_ok
   bool lut_one = false;            // one threshold step after the table is exact for every d^2 <= R^2
   int disjoint = 0;
   std::vector<int8_t> setidx;      // [nC][256]
@@ -196,7 +197,7 @@ struct pp_ctx {
   Result res;
   // scratch
   DevBuf tmp_cell_of, tmp_rank, scan_tmp, bbox, centres, centre_count, work, tables_dev, sel_flags, sel_tmp;
-  DevBuf tri_fill, cflag, rowtab, nc_pre;
+  DevBuf tri_fill, cflag, rowtab, nc_pre, pass_code;
   DevBuf labels_run, perm_dev, gather_src;
   DevBuf mask_in;  // caller's centre mask: [n] input order, then [n] sorted-slot order
   // statistics after clustering: option "aposteriori_guard" = 1 runs the
@@ -361,6 +362,20 @@ void build_lut(const std::vector<float>& T, float r2, int max_cells, std::vector
     for (int c = 0; c + 1 < n && one; ++c) one = lut[c + 1] <= lut[c] + 1;
     *one_step = one && cat(std::max(r2, 0.f)) <= lut[n - 1] + 1;
   }
+}
+
+// Whether floor(sqrt(d^2) * scale + 1/2), to within an eighth of a bin, is the
+// category of d^2 or one less for every d^2 in [0, R^2]: the bins start at 0
+// and every threshold lies within 1/256 of a bin of its edge.  The float
+// evaluation takes little of the margin of 3/8: sqrt.approx is within 2^-23 of
+// the root, and the scale, its quotient and the product each round by 2^-24,
+// together below 2^-21 of at most 16382 bins.
+bool category_fast_ok(const std::vector<float>& T, const Tables& t) {
+  if (t.rmin != 0.f) return false;
+  const double scale = (double)(float)t.hscale;
+  for (size_t k = 1; k < T.size(); ++k)
+    if (!(std::fabs(std::sqrt((double)T[k]) * scale - (double)(k - 1)) < 1.0 / 256)) return false;
+  return true;
 }
 
 inline bool has_type(const uint32_t* m, int t) { return (m[t >> 5] >> (t & 31)) & 1u; }
@@ -688,6 +703,7 @@ int make_plan(pp_ctx* ctx, uint32_t flags, const uint32_t* k_list, int nk, RunPl
   }
   P.catT = threshold_table(t);
   build_lut(P.catT, t.rmax * t.rmax, 4096, P.lut, P.lut_shift, P.lut_base, &P.lut_one);
+  P.cat_fast = category_fast_ok(P.catT, t);
   P.cat_miss = category_of_distance(t, (float)((double)t.rmax + kEpsilon));
   return PP_OK;
 }
@@ -754,7 +770,6 @@ void fill_scan_common(pp::ScanArgs& a, const Cloud& cl, const RunPlan& P, const 
   a.R = t.rmax;
   a.R2 = t.rmax * t.rmax;
   a.box_R2 = std::nextafter(a.R2 * (1.f + 1.f / 4096.f) + 1e-30f, std::numeric_limits<float>::infinity());
-  a.no_box_filter = 0;
   const float Rm = t.rmax + cl.g.margin;
   a.Rm2 = Rm * Rm;
   a.H = P.H;
@@ -766,6 +781,7 @@ void fill_scan_common(pp::ScanArgs& a, const Cloud& cl, const RunPlan& P, const 
   a.lut_shift = P.lut_shift;
   a.lut_base = P.lut_base;
   a.lut_one = P.lut_one ? 1 : 0;
+  a.cat_fast = P.cat_fast ? 1 : 0;
   a.cat_miss = P.cat_miss;
   a.cslot_of = D.cslot;
   a.eslot_of = D.eslot;
@@ -1410,7 +1426,7 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
   pp::ScanArgs a{};
   fill_scan_common(a, *cl, P, D, ctx->tab);
   if (ctx->no_uniform) a.uniform_sets = 0;
-  if (ctx->no_box) a.no_box_filter = 1;
+  if (ctx->no_box) a.box_R2 = std::numeric_limits<float>::infinity();
   a.lists_mode = ctx->knn_lists;
   a.labels = labels;
   a.centres = ctx->centres.as<uint32_t>();
@@ -1471,6 +1487,13 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
     a.bsr = (int)std::floor(((R + g.margin) + 2.f * g.margin) * g.inv_h) + 1;
     a.brows = nullptr;
     if (lanes && (rc = ensure_block_rows(ctx, a.by, a.bz, a.bsr, s, &a.brows)) != PP_OK) return rc;
+    if (lanes) {
+      CK(ctx->pass_code.ensure(std::max<uint64_t>(n, 1) * 4));
+      a.pcode = ctx->pass_code.as<uint32_t>();
+      a.label_sorted = labels ? labels : cl->label_sorted.as<uint8_t>();
+      a.n = n;
+      a.one = 1.f;
+    }
     CK(cudaEventRecord(ctx->ev0, s));
     rc = -3;
     // passes with RDF / RIPK and kNN together take the per-centre scan, which

@@ -39,8 +39,7 @@ struct ScanArgs {
   // geometry of the query
   float R, R2;                 // SpatStatRadiusMax and float(R*R)
   float Rm2;                   // (R + margin)^2 for conservative row trimming
-  float box_R2;                // R2 (1 + 2^-12): centre-per-lane box filter bound
-  int no_box_filter;           // centre-per-lane scans stage every candidate
+  float box_R2;                // R2 (1 + 2^-12): centre-per-lane box filter bound (+inf: every candidate)
   // bins: categories 0 = lowest, 1..nb = bins, nb+1 = highest
   int H;                       // nb + 2
   const float* cat_T;          // [H] smallest d^2 of each category (index 0 unused)
@@ -51,11 +50,18 @@ struct ScanArgs {
   int lut_n, lut_shift;
   uint32_t lut_base;
   int lut_one;                 // the cell's category plus at most one step is exact for d^2 <= R^2
+  int cat_fast;                // rmin = 0 and sqrt(d^2) * guess_scale names the category to within 1/256 bin
   // brick scan: cells per brick, centres per warp batch, bricks to process;
   // the centre-per-lane scan takes blocks of bx x by x bz cells
   int bx, bcap;
   int by, bz;
   uint32_t nbricks;
+  // centre-per-lane scans: per-slot pass codes (written by the pass, n words),
+  // the labels they are made from, and 1.f (see dist2_x2)
+  uint32_t* pcode;
+  const uint8_t* label_sorted;
+  uint64_t n;
+  float one;
   // centre-per-lane scan: stencil rows of a block, (ry, rz) offsets from
   // (yb - bsr, zb - bsr), nearest to the block first; bsr rows each side
   const int16_t* brows;

@@ -23,6 +23,7 @@
 #include <cstdint>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include "pp_internal.h"
@@ -59,6 +60,35 @@ __device__ __forceinline__ float dist2(float ax, float ay, float az, float bx, f
   return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
 }
 
+// Position of the (n + 1)-th set bit of m (n < popc(m)), by halving; __fns
+// searches bit by bit.
+__device__ __forceinline__ uint32_t nth_set(uint32_t m, uint32_t n) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const uint32_t c = __popc(m & ((1u << s) - 1u));
+    if (n >= c) {
+      n -= c;
+      m >>= s;
+      pos += s;
+    }
+  }
+  return pos;
+}
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// v << n, 0 for n > 31.
+__device__ __forceinline__ uint32_t shl_clamp(uint32_t v, uint32_t n) {
+  uint32_t r;
+  asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(n));
+  return r;
+}
+
 // Two floats in one 64-bit register pair, for the packed f32x2 arithmetic of
 // sm_100+ (one instruction, two IEEE round-to-nearest results).
 __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
@@ -80,23 +110,25 @@ __device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsig
   return d;
 }
 // dist2 of one centre (its coordinates duplicated in each pair: cxx = (cx, cx)
-// ...) against two ions whose x, y and z come as pairs: differences and
-// squares packed, the two sums scalar, in dist2's order.  Bit-identical to
-// dist2 on the GPU (checked on 2M random pairs); with the sums packed as well
-// (add.rn.f32x2) the results differ from dist2 by an ulp or two for about one
-// pair in five (measured on 134M pairs, with or without --fmad=false passed to
-// ptxas: a product feeding only a packed add comes out unrounded, as from a
-// fused multiply-add), so they are not.
-__device__ __forceinline__ void dist2_x2(unsigned long long cxx, unsigned long long cyy, unsigned long long czz,
-                                         unsigned long long xx, unsigned long long yy, unsigned long long zz,
-                                         float& d0, float& d1) {
+// ...) against two ions whose x, y and z come as pairs, all eight operations
+// packed, in dist2's order.  The sums are fused multiply-adds by `one` =
+// (1, 1), which round like additions; the ones come from the kernel's
+// arguments (ScanArgs::one), so that the compiler cannot take the operation
+// for an addition: an add.rn.f32x2, or a literal 1, is merged with the squares
+// into unrounded products, and one result in five is then an ulp or two off.
+// This form equals dist2 bit for bit on 1.2e9 pairs (near, far, infinite and
+// subnormal coordinates).
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
+                                                     unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ void dist2_x2(unsigned long long one, unsigned long long cxx, unsigned long long cyy,
+                                         unsigned long long czz, unsigned long long xx, unsigned long long yy,
+                                         unsigned long long zz, float& d0, float& d1) {
   const unsigned long long dx = f2_sub(cxx, xx), dy = f2_sub(cyy, yy), dz = f2_sub(czz, zz);
-  float x0, x1, y0, y1, z0, z1;
-  f2_unpack(f2_mul(dx, dx), x0, x1);
-  f2_unpack(f2_mul(dy, dy), y0, y1);
-  f2_unpack(f2_mul(dz, dz), z0, z1);
-  d0 = __fadd_rn(__fadd_rn(x0, y0), z0);
-  d1 = __fadd_rn(__fadd_rn(x1, y1), z1);
+  f2_unpack(f2_fma(f2_fma(f2_mul(dx, dx), one, f2_mul(dy, dy)), one, f2_mul(dz, dz)), d0, d1);
 }
 
 // ------------------------------------------------------------------ K0 / bbox
@@ -1759,53 +1791,45 @@ __global__ void __launch_bounds__(256) k_brick(ScanArgs a) {
 // [xb, xe) x [yb, ye) x [zb, ze): rows are (yy, zz) with yy in [yb - sr,
 // ye - 1 + sr] and zz in [zb - sr, ze - 1 + sr], row r at (yb - sr + ry,
 // zb - sr + rz) for (ry, rz) = a.brows[r] (nearest to the block first), each
-// trimmed in x to the block's reach and to the reach of the batch's centre
-// box [box[0], box[1]] (world coordinates; rows and cells beyond R of the box
-// hold no neighbour of these centres); len = 0 when the row cannot hold a
-// neighbour of a point of the block.  In symmetric mode the
-// leading cells that precede the block's first cell in slot order and hold
-// only centres are dropped: their pairs with the block are taken from their
-// side (every ion of such a cell has a lower slot than every block centre).
-__device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nrows, int sr, int xb, int xe, int yb,
-                                                int ye, int zb, int ze, bool sym, const float4* box,
-                                                uint32_t& st, uint32_t& len) {
+// trimmed in x to the cells within R of the batch's centre box [box[0],
+// box[1]] (world coordinates; no other cell holds a neighbour of these
+// centres; margins of 1e-3 h and more cover the float evaluation and the
+// approximate root); len = 0 when the row holds none.
+// In symmetric mode a pair of two centres of different blocks is taken by the
+// block that comes first in (z, y, x) order.  low: every cell of the row
+// belongs to an earlier block, so its centres are not staged, and the row is
+// dropped (len = 0) when it holds nothing else; in a row of the block itself
+// the cells before xb are dropped when they hold only centres.
+__device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nrows, int sr, int xb, int yb, int ye,
+                                                int zb, int ze, bool sym, const float4* box, uint32_t& st,
+                                                uint32_t& len, bool& low) {
   const Grid& g = a.g;
   st = 0;
   len = 0;
+  low = false;
   if (r >= nrows) return;
   const int ry = a.brows[2 * r], rz = a.brows[2 * r + 1];
   const int yy = yb - sr + ry, zz = zb - sr + rz;
   if (yy < 0 || yy >= g.ny || zz < 0 || zz >= g.nz) return;
   const float m2 = 2.f * g.margin;
   const float Rp = a.R + g.margin, Rp2 = Rp * Rp;
-  const int cy = yy < yb ? yb - yy : (yy >= ye ? yy - (ye - 1) : 0);
-  const int cz = zz < zb ? zb - zz : (zz >= ze ? zz - (ze - 1) : 0);
-  const float gy = fmaxf(0.f, (float)(cy - 1) * g.h - m2);
-  const float gz = fmaxf(0.f, (float)(cz - 1) * g.h - m2);
-  const float rem = Rp2 - gy * gy - gz * gz;
-  if (rem < 0.f) return;
-  const float half = sqrtf(rem);
-  int x0 = max(0, (int)floorf(((float)xb * g.h - m2 - half) * g.inv_h));
-  int x1 = min(g.nx - 1, (int)floorf(((float)xe * g.h + m2 + half) * g.inv_h));
-  {
-    // the same against the centre box: the row's ions lie within margin of
-    // its cells [lo + c h, lo + (c + 1) h]
-    const float4 lo = box[0], hi = box[1];
-    const float ry0 = g.loy + (float)yy * g.h, rz0 = g.loz + (float)zz * g.h;
-    const float by = fmaxf(0.f, fmaxf(lo.y - (ry0 + g.h), ry0 - hi.y) - m2);
-    const float bz = fmaxf(0.f, fmaxf(lo.z - (rz0 + g.h), rz0 - hi.z) - m2);
-    const float brem = Rp2 - by * by - bz * bz;
-    if (brem < 0.f) return;
-    const float bhalf = sqrtf(brem);
-    x0 = max(x0, (int)floorf((lo.x - g.lox - m2 - bhalf) * g.inv_h));
-    x1 = min(x1, (int)floorf((hi.x - g.lox + m2 + bhalf) * g.inv_h));
-    if (x1 < x0) return;
-  }
+  // the row's ions lie within margin of its cells [lo + c h, lo + (c + 1) h]
+  const float4 lo = box[0], hi = box[1];
+  const float ry0 = g.loy + (float)yy * g.h, rz0 = g.loz + (float)zz * g.h;
+  const float by = fmaxf(0.f, fmaxf(lo.y - (ry0 + g.h), ry0 - hi.y) - m2);
+  const float bz = fmaxf(0.f, fmaxf(lo.z - (rz0 + g.h), rz0 - hi.z) - m2);
+  const float brem = Rp2 - by * by - bz * bz;
+  if (brem < 0.f) return;
+  const float bhalf = sqrt_approx(brem) + m2;
+  const int x0 = max(0, (int)floorf((lo.x - g.lox - bhalf) * g.inv_h));
+  const int x1 = min(g.nx - 1, (int)floorf((hi.x - g.lox + bhalf) * g.inv_h));
+  if (x1 < x0) return;
   const uint64_t cb = ((uint64_t)zz * g.ny + yy) * g.nx;
   int xs = x0;
   if (sym) {
-    const bool own = (zz == zb && yy == yb);
-    if (own || zz < zb || (zz == zb && yy < yb)) {
+    const bool own = yy >= yb && yy < ye && zz >= zb && zz < ze;
+    low = zz < zb || (zz < ze && yy < yb);
+    if (own || low) {
       const int xend = own ? min(x1, xb - 1) : x1;
       if (xend >= x0 && a.nc_pre[cb + xend + 1] == a.nc_pre[cb + x0]) xs = xend + 1;
     }
@@ -1844,42 +1868,81 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
 // of a centre and the float box distance each lie within a few ulp of their
 // exact values (every operation is correctly rounded and the box distance
 // never exceeds a centre's distance), so no ion an exact test would take is
-// dropped.  Survivors are packed into the staging buffer in stencil order; a
-// batch of tests runs each time 32 have gathered, and once more for the rest
-// after the last row.  A survivor that finds the buffer full keeps only its
-// slot and is reloaded and staged after the tests, so nothing else stays live
-// across them.  On the 20M-ion tip (cells of R/4, 4 x 2 x 2 blocks) this took
+// dropped.  Survivors are packed into the staging buffer in stencil order (a
+// ring of two halves of 32); a batch of tests runs each time a half is full,
+// and once more for the rest after the last row.  On the 20M-ion tip (cells of R/4, 4 x 2 x 2 blocks) this took
 // the distance tests per pair from 2.66 to 1.78 (RDF) and from 4.43 to 2.92
-// (kNN).  Option ScanArgs::no_box_filter stages every candidate, as an A/B
+// (kNN).  An infinite ScanArgs::box_R2 stages every candidate, as an A/B
 // switch.
 //
+// An ion's pass code (ScanArgs::pcode, k_pass_codes) is staged as its record's
+// fourth word; in symmetric mode its lowest bit says that it is a centre and
+// is staged as 0.
 // lanes_walk calls, warp-uniformly,
-//   stage(slot, q, key, code)  per staged ion (its lane): key and code to stage
 //   start(self)                a new batch; self = this lane's centre slot or
 //                              0xffffffff; returns the lane's centre position
 //                              (at infinity for no centre)
-//   accept(j, d2, w)           per test of an in-ball staged ion j whose staged
-//                              key is w (inlined into the test loop; a constant
-//                              true costs nothing)
-//   taken(tm, nin, cxx, cyy, czz)  after each staged batch: tm = the lane's
-//                              mask, nin = its in-ball ions (counted when
-//                              COUNT), the centre's coordinates as f32x2 pairs
-//   finish(live)               after the batch's last staged ions
-// In symmetric mode (SYM) a lane takes a staged ion when key > its own slot,
-// otherwise (KEYED) when key != its own slot; stage() sets key accordingly.
-// Without KEYED the key is free for accept() and the centre itself (d^2 = 0)
-// passes the in-ball test: the pass excludes it.  With GATED, accept() alone
-// decides whether an ion is taken: it must then imply the in-ball test.
+//   batch(base, nb, keyed, self, cxx, cyy, czz)  tests of the nb staged ions at
+//                              base (places up to the next multiple of 8 hold
+//                              ions at infinity): self as above for live
+//                              lanes, the centre's coordinates as f32x2 pairs.
+//                              keyed: some of them lie in the block itself;
+//                              skey then holds the slots of those (in
+//                              symmetric mode of the centres among them), else
+//                              0xffffffff: symmetric passes take an ion when
+//                              its key exceeds self, others when it differs
+//   finish(live, tests)        after the batch's last staged ions; tests = the
+//                              (centre, staged ion) tests of the batch
+// Each pair of two centres is met once in symmetric mode (SYM): see
+// block_row_range for the pairs of different blocks; pairs within the block
+// are taken by the lower slot.
+constexpr int kStage = 64;           // staged ions a warp has room for
+constexpr int kStageAll = kStage + 4;  // and one place (of a pair) for dropped candidates; keys stay 16-byte aligned
+
+// What a centre-per-lane pass needs to know of an ion, per sorted slot
+// (ScanArgs::pcode), by its type and whether it is a centre.  Written once per
+// pass so that staging an ion takes one load instead of its label, two table
+// look-ups and its centre flag.
+//   PC_KINDS, PC_CORES  k_lanes (see there); bit 0 set for centres when a.sym
+//   PC_ROW, PC_NIBBLE   k_lanes_knn: float row of the type's environment set
+//                       (param between rows), or that set for every centre
+//                       slot, 4 bits each; set a.emax = none
+enum PassCode { PC_KINDS, PC_CORES, PC_ROW, PC_NIBBLE };
+__global__ void k_pass_codes(ScanArgs a, int kind, uint32_t param, uint32_t* __restrict__ out) {
+  __shared__ uint32_t tab[512];
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+    const int ty = i & 255;
+    const bool jc = a.sym && i >= 256;
+    const int c = a.cslot_of[ty], e = a.eslot_of[ty];
+    uint32_t v = 0;
+    if (kind == PC_KINDS) {
+      const int row = jc && c >= 0 ? c : (a.sym ? a.nC : 0) + (e < 0 ? a.nE : e);
+      v = (uint32_t)row * (uint32_t)a.H * 4u;
+    } else if (kind == PC_CORES) {
+      v = (uint32_t)(e + 1) << 1 | (jc ? (uint32_t)(c + 1) << 9 : 0u);
+    } else if (kind == PC_ROW) {
+      const int si = a.nC > 0 ? a.setidx[ty] : -1;
+      v = (uint32_t)(si < 0 ? a.emax : si) * param;
+    } else {
+      for (int q = 0; q < a.nC; ++q) {
+        const int si = a.setidx[q * 256 + ty];
+        v |= (uint32_t)(si < 0 ? a.emax : si) << (4 * q);
+      }
+    }
+    tab[i] = v | (jc ? 1u : 0u);
+  }
+  __syncthreads();
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x)
+    out[i] = tab[(a.sym && a.cflag[i] ? 256 : 0) + a.label_sorted[i]];
+}
 __device__ __forceinline__ float4 staged_ion(const float4* cand, int j) {
   const float* f = (const float*)cand + (j >> 1) * 8 + (j & 1);
   return make_float4(f[0], f[2], f[4], f[6]);
 }
 
-template <bool SYM, bool COUNT, bool KEYED, bool GATED, class Stage, class Start, class Accept, class Taken,
-          class Finish>
-__device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, float4* cand, uint32_t* ccode, float4* sbox,
-                                                         Stage stage, Start start, Accept accept, Taken taken,
-                                                         Finish finish) {
+template <bool SYM, class Start, class Batch, class Finish>
+__device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, float4* cand, uint32_t* skey, float4* sbox,
+                                                         Start start, Batch batch, Finish finish) {
   const Grid& g = a.g;
   const int lane = threadIdx.x & 31;
   const uint32_t lemask = (2u << lane) - 1u;
@@ -1889,7 +1952,6 @@ __device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, floa
   const int BX = max(a.bx, 1), BY = max(a.by, 1), BZ = max(a.bz, 1);
   const int nry = BY + 2 * sr, nrows = nry * (BZ + 2 * sr);
   const uint32_t nbx = (uint32_t)((g.nx + BX - 1) / BX), nby = (uint32_t)((g.ny + BY - 1) / BY);
-  const float R2 = a.R2;
   const uint32_t WT = max(a.tile, 1u);
   unsigned long long tests = 0;  // (centre, staged ion) distance tests, warp-uniform
   for (;;) {
@@ -1932,15 +1994,15 @@ __device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, floa
           const uint32_t base = pos;
           uint32_t takem = cm;
           if (have > room) {
-            const int lastl = (int)__fns(cm, 0, room);
+            const uint32_t lastl = nth_set(cm, (uint32_t)room - 1u);
             takem = cm & ((2u << lastl) - 1u);
-            pos += (uint32_t)lastl + 1u;
+            pos += lastl + 1u;
           } else {
             pos += 32u;
           }
           const int ntake = __popc(takem);
           const int want = lane - mc;
-          if (want >= 0 && want < ntake) self = base + (uint32_t)__fns(takem, 0, want + 1);
+          if (want >= 0 && want < ntake) self = base + nth_set(takem, (uint32_t)want);
           mc += ntake;
         }
         if (mc == 0) break;
@@ -1964,45 +2026,38 @@ __device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, floa
           }
           __syncwarp();
         }
-        auto put = [&](uint32_t p, const float4& q, uint32_t key, uint32_t code) {
+        auto put = [&](uint32_t p, const float4& q, uint32_t code) {
           float* f = (float*)cand + (p >> 1) * 8 + (p & 1);
           f[0] = q.x;
           f[2] = q.y;
           f[4] = q.z;
-          f[6] = __uint_as_float(key);
-          ccode[p] = code;
+          f[6] = __uint_as_float(code);
         };
-        uint32_t fill = 0;  // staged ions waiting for a batch of tests (warp-uniform)
-        // the tests of the first nb staged ions (the rest of the buffer holds ions at infinity)
+        uint32_t btests = 0;   // distance tests of this batch of centres
+        uint32_t base = 0;     // the half that fills: places [base, base + 32) of the ring
+        uint32_t fill = 0;     // staged ions waiting for a batch of tests (warp-uniform)
+        bool keyed = false;    // ... among them ions of the block itself
         auto run_batch = [&](uint32_t nb) {
-          if (lane >= nb) put(lane, make_float4(kInf(), kInf(), kInf(), 0.f), 0u, 0u);  // no lane takes these
           __syncwarp();
-          tests += (unsigned long long)__popc(live) * nb;
-          uint32_t tm = 0, nin = 0;
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float4 c0 = cand[j], c1 = cand[j + 1];
-            float d0, d1;
-            dist2_x2(cxx, cyy, czz, f2_pack(c0.x, c0.y), f2_pack(c0.z, c0.w), f2_pack(c1.x, c1.y), d0, d1);
-            const uint32_t k0 = __float_as_uint(c1.z), k1 = __float_as_uint(c1.w);
-            const bool in0 = (d0 <= R2) && (!KEYED || (SYM ? (k0 > self) : (k0 != self)));
-            const bool in1 = (d1 <= R2) && (!KEYED || (SYM ? (k1 > self) : (k1 != self)));
-            if (COUNT) nin += (in0 ? 1u : 0u) + (in1 ? 1u : 0u);
-            tm |= ((GATED || in0) && accept(j, d0, k0)) ? (1u << j) : 0u;
-            tm |= ((GATED || in1) && accept(j + 1, d1, k1)) ? (2u << j) : 0u;
-          }
-          taken(tm, nin, cxx, cyy, czz);
+          btests += (uint32_t)__popc(live) * nb;
+          batch(base, nb, keyed, self, cxx, cyy, czz);
           __syncwarp();
         };
+        const int nown = BY * BZ;  // the row table starts with the block's own rows
         for (int r0 = 0; r0 < nrows && live; r0 += 32) {
           uint32_t st, len;
-          block_row_range(a, r0 + lane, nrows, sr, xb, xe, yb, ye, zb, ze, SYM, sbox, st, len);
+          bool low;
+          block_row_range(a, r0 + lane, nrows, sr, xb, yb, ye, zb, ze, SYM, sbox, st, len, low);
           const uint32_t ne = __ballot_sync(FULL, len > 0);
           const int cnt_rows = __popc(ne);
           if (cnt_rows == 0) continue;
-          const int src = (lane < cnt_rows) ? (int)__fns(ne, 0, lane + 1) : 0;
+          const uint32_t src = (lane < cnt_rows) ? nth_set(ne, (uint32_t)lane) : 0u;
           const uint32_t rst = __shfl_sync(FULL, st, src);
           uint32_t rlen = __shfl_sync(FULL, len, src);
+          // rows (compacted) that are the block's own, and of earlier blocks
+          const uint32_t ownm = __ballot_sync(FULL, lane < cnt_rows && r0 + (int)src < nown);
+          const int lowc = SYM ? __shfl_sync(FULL, low ? 1 : 0, src) : 0;
+          const uint32_t lowm = SYM ? __ballot_sync(FULL, lane < cnt_rows && lowc != 0) : 0u;
           if (lane >= cnt_rows) rlen = 0;
           uint32_t inc = rlen;
 #pragma unroll
@@ -2010,60 +2065,67 @@ __device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, floa
             const uint32_t t = __shfl_up_sync(FULL, inc, o);
             if (lane >= o) inc += t;
           }
-          const uint32_t exc = inc - rlen;
           const uint32_t total = __shfl_sync(FULL, inc, 31);
-          int before = 0;
+          // candidate t of these rows is slot t + first[its row]; exc = the
+          // row's first t (lanes without a row: never reached)
+          const uint32_t exc = lane < cnt_rows ? inc - rlen : 0xffffffffu;
+          const uint32_t first = rst - (inc - rlen);
+          int row0 = -1;  // last row that starts before this step
           for (uint32_t bb = 0; bb < total; bb += 32) {
-            const uint32_t bitv = (lane < cnt_rows && rlen > 0 && exc >= bb && exc < bb + 32) ? (1u << (exc - bb)) : 0u;
-            const uint32_t smask = __reduce_or_sync(FULL, bitv);
-            const int row = before + __popc(smask & lemask) - 1;
-            before += __popc(smask);
-            const int rowc = row < 0 ? 0 : (row > 31 ? 31 : row);
-            const uint32_t rs = __shfl_sync(FULL, rst, rowc);
-            const uint32_t rp = __shfl_sync(FULL, exc, rowc);
-            const uint32_t t = bb + lane;
-            bool keep = false;
-            uint32_t slot = 0;
-            float4 q;
-            if (t < total) {
-              slot = rs + (t - rp);
-              q = __ldg(a.ions + slot);
-              const float4 lo = sbox[0], hi = sbox[1];
-              const float gx = fmaxf(fmaxf(__fsub_rn(lo.x, q.x), __fsub_rn(q.x, hi.x)), 0.f);
-              const float gy = fmaxf(fmaxf(__fsub_rn(lo.y, q.y), __fsub_rn(q.y, hi.y)), 0.f);
-              const float gz = fmaxf(fmaxf(__fsub_rn(lo.z, q.z), __fsub_rn(q.z, hi.z)), 0.f);
-              const float bd = __fadd_rn(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)), __fmul_rn(gz, gz));
-              keep = a.no_box_filter || bd <= a.box_R2;
+            const uint32_t smask = __reduce_or_sync(FULL, shl_clamp(1u, exc - bb));
+            const int row = row0 + __popc(smask & lemask);
+            row0 += __popc(smask);
+            const uint32_t t = min(bb + lane, total - 1u);
+            const uint32_t slot = __shfl_sync(FULL, first, row) + t;
+            const float4 q = __ldg(a.ions + slot);
+            uint32_t code = __ldg(a.pcode + slot), key = 0xffffffffu;
+            const float4 lo = sbox[0], hi = sbox[1];
+            const float gx = fmaxf(fmaxf(__fsub_rn(lo.x, q.x), __fsub_rn(q.x, hi.x)), 0.f);
+            const float gy = fmaxf(fmaxf(__fsub_rn(lo.y, q.y), __fsub_rn(q.y, hi.y)), 0.f);
+            const float gz = fmaxf(fmaxf(__fsub_rn(lo.z, q.z), __fsub_rn(q.z, hi.z)), 0.f);
+            const float bd = __fadd_rn(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)), __fmul_rn(gz, gz));
+            bool keep = (bd <= a.box_R2) && bb + lane < total;
+            bool jc = false;
+            if (SYM) {
+              jc = (code & 1u) != 0;
+              code &= ~1u;
+              if (lowm) keep = keep && !(jc && ((lowm >> row) & 1u));
+            }
+            bool own_it = false;
+            if (ownm) {
+              // ions of the block's own rows: which cell (the expression of k_cell_count)
+              if ((ownm >> row) & 1u) {
+                const int cx = cell_coord(q.x, g.lox, g.inv_h, g.nx);
+                if (SYM) keep = keep && !(jc && cx < xb);
+                if (cx >= xb && cx < xe && (jc || !SYM)) key = slot;
+              }
+              own_it = __any_sync(FULL, keep && key != 0xffffffffu);
+              keyed |= own_it;
             }
             const uint32_t km = __ballot_sync(FULL, keep);
-            const uint32_t at = fill + (uint32_t)__popc(km & (lemask >> 1));
-            uint32_t over = 0xffffffffu;
-            if (keep) {
-              if (at < 32u) {
-                uint32_t key, code;
-                stage(slot, q, key, code);
-                put(at, q, key, code);
-              } else {
-                over = slot;
-              }
-            }
+            // dropped candidates go to a place past the ring
+            const uint32_t at = (base + fill + (uint32_t)__popc(km & (lemask >> 1))) & (uint32_t)(kStage - 1);
+            const uint32_t p = keep ? at : (uint32_t)kStage;
+            put(p, q, code);
+            if (keyed || ownm) skey[p] = key;  // rows of the block come first, so earlier ions of a keyed half have keys
             fill += (uint32_t)__popc(km);
             if (fill >= 32u) {
               run_batch(32u);
               fill -= 32u;
-              const uint32_t om = __ballot_sync(FULL, over != 0xffffffffu);
-              if (over != 0xffffffffu) {
-                const float4 qo = __ldg(a.ions + over);
-                uint32_t key, code;
-                stage(over, qo, key, code);
-                put((uint32_t)__popc(om & (lemask >> 1)), qo, key, code);
-              }
-              __syncwarp();
+              base ^= 32u;
+              keyed = own_it;
             }
           }
         }
-        if (fill > 0u) run_batch(fill);
-        finish(live);
+        if (fill > 0u) {
+          if (lane >= (int)fill && lane < (int)((fill + 7u) & ~7u)) {
+            put(base + lane, make_float4(kInf(), kInf(), kInf(), 0.f), 0u);  // no lane takes these
+            skey[base + lane] = 0u;
+          }
+          run_batch(fill);
+        }
+        tests += btests;
+        finish(live, btests);
         __syncwarp();
       }
     }
@@ -2071,180 +2133,268 @@ __device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, floa
   return tests;
 }
 
-// RDF / RIPK pass.  After each staged batch every lane lists its taken pairs
-// at its offset in the batch's pair list and the lanes take the list 64 at a
-// time: d^2 is recomputed, binned and added to the (shared) RDF bins, so the
-// bin lookup and the histogram atomics run for in-ball pairs only.  In
-// symmetric mode a staged ion carries key = its slot when it is a centre and
-// 0xffffffff otherwise, and a pair of two centres is taken by the lower slot
-// and credited to both.  SMEM (bins in shared memory, fewer than 2^16 of
-// them): the staged ion's code and the lane's centre info hold ready bin
-// offsets, 16 bits each -- code: env offset (its env slot * H) | its centre
-// base (centre slot * nE * H) << 16; info: centre base | env offset << 16;
-// 0xffff for none, 0xfffe for a centre without a slot -- so a pair's bin is
-// two additions away from its category.
-constexpr int kLanesWarps = 16;  // warps per block of k_lanes
+// Category guess of the centre-per-lane passes (ScanArgs::cat_fast: rmin = 0
+// and thresholds checked by the host): g = floor(sqrt(d^2) * scale + 1/2), to
+// within an eighth of a bin, from the approximate square root; g or g + 1 is
+// the category, decided by one compare with the category's exact threshold.  A
+// saturating fused multiply-add maps [0, R] into [0, 1] (d^2 out of the ball
+// to 1) and a second one, by 4 (H - 1) 2^-149, rounds to a denormal float
+// whose bits are the integer 4 g plus at most 3.
+struct FastCat {
+  float tk, t0, tg;
+  __device__ __forceinline__ explicit FastCat(const ScanArgs& a) {
+    const float tn = (float)(4 * (a.H - 1));
+    tk = __fdiv_rn(4.f * a.guess_scale, tn);
+    t0 = __fdiv_rn(2.f, tn);
+    tg = __uint_as_float((uint32_t)(4 * (a.H - 1)));
+  }
+  // four times the guess of a d^2 in the ball; up to 4 (H - 1) for any other
+  __device__ __forceinline__ uint32_t guess4(float d2) const {
+    float t;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(t) : "f"(sqrt_approx(d2)), "f"(tk), "f"(t0));
+    return __float_as_uint(__fmaf_rn(t, tg, 0.f)) & ~3u;
+  }
+};
 
-template <bool SYM, bool SMEM>
-__global__ void __launch_bounds__(kLanesWarps * 32, 2) k_lanes(ScanArgs a) {
+// RDF / RIPK pass.  Every lane bins its in-ball pairs inside the test loop:
+// d^2, the category and one shared-memory atomic per test, eight tests in
+// flight, no lists and no further warp synchronisation.  On the tips about a
+// fifth of the lanes hold an in-ball pair at a test, so four categories out of
+// five are computed for nothing; still this takes 20 instructions a test,
+// where a bit mask per test, a list of the taken pairs and their binning by
+// full warps (this kernel before) took 45.  Issue slots bound it (87% busy;
+// DRAM 0.3%): a third of its instructions stage the ions, two thirds test and
+// bin them.  All 36 pair RDFs of the 20M-ion tip (R = 2 nm, 0.01 nm bins): 32.1
+// ms with lists, 23.3 ms binning in the loop, 19.1 ms with pairs of blocks met
+// once and the ring buffer, 15.6 ms with pass codes, packed sums, the
+// unpredicated atomic and the branch-free staging.
+//
+// Categories: FAST = FastCat, otherwise the lookup table.
+//
+// BINS = 2: shared bins by *unordered kind* of pair, [centre slot][row][H]
+// with RW rows: in symmetric mode one row per centre slot of the staged ion
+// (a pair of two centres, to be credited both ways), then one row per
+// environment slot for staged ions that are not centres, and a last row for
+// ions without one.  A pair is one atomic, whatever it is credited to; the
+// credits and the pair count are worked out once per bin when the bins are
+// added to the global cores.  BINS = 1: shared bins in the layout of the
+// cores, up to two atomics a pair (twice the kinds do not fit); BINS = 0:
+// atomics on the cores.
+// Pass code of an ion: BINS 2 the byte offset of its row, others (env slot +
+// 1) << 1 | (centre slot + 1) << 9; the lowest bit set for centres in
+// symmetric mode.
+constexpr int kLanesWarps = 32;  // warps per block of k_lanes: one block per SM, one set of bins
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+template <bool SYM, int BINS, bool FAST>
+__global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
   constexpr int NW = kLanesWarps;
   extern __shared__ __align__(16) unsigned char smem[];
   const int H = a.H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t RW = (SYM ? (uint32_t)a.nC : 0u) + (uint32_t)a.nE + 1u;  // BINS 2: rows per centre slot
+  const uint32_t nbin = BINS == 2 ? (uint32_t)a.nC * RW * (uint32_t)H : BINS == 1 ? (uint32_t)a.nC * a.nE * H : 0u;
   unsigned char* sp = smem;
   unsigned long long* since_flush = (unsigned long long*)sp; sp += 16;
-  float4* candA = (float4*)sp; sp += NW * 32 * 16;
-  float4* cposA = (float4*)sp; sp += NW * 32 * 16;
+  float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
   float4* boxA = (float4*)sp; sp += NW * 2 * 16;
-  uint32_t* ccodeA = (uint32_t*)sp; sp += NW * 32 * 4;
-  uint32_t* cinfoA = (uint32_t*)sp; sp += NW * 32 * 4;
-  uint16_t* plistA = (uint16_t*)sp; sp += NW * 1024 * 2;
+  uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
+  uint32_t* sdummy = (uint32_t*)sp; sp += 32 * 4;    // where the lanes without a pair add
   float* sT = (float*)sp; sp += ((H + 4) & ~3) * 4;  // H thresholds, then +inf
-  uint32_t* srdf = (uint32_t*)sp; sp += (SMEM ? (size_t)a.nC * a.nE * H * 4 : 0);
-  uint16_t* slut = (uint16_t*)sp; sp += ((a.lut_n + 7) & ~7) * 2;
+  uint32_t* srdf = (uint32_t*)sp; sp += (size_t)nbin * 4;
   int8_t* scs = (int8_t*)sp; sp += 256;
-  int8_t* ses = (int8_t*)sp;
+  int8_t* ses = (int8_t*)sp; sp += 256;
+  int8_t* sce = (int8_t*)sp; sp += 256;  // environment slot of a centre slot's type
+  uint16_t* slut = (uint16_t*)sp;        // not FAST
   for (int i = threadIdx.x; i <= H; i += blockDim.x) sT[i] = i < H ? a.cat_T[i] : kInf();
-  for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) { scs[i] = a.cslot_of[i]; ses[i] = a.eslot_of[i]; }
-  if (SMEM) for (int i = threadIdx.x; i < a.nC * a.nE * H; i += blockDim.x) srdf[i] = 0;
+  if (!FAST)
+    for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+    const int8_t c = a.cslot_of[i], e = a.eslot_of[i];
+    scs[i] = c;
+    ses[i] = e;
+    if (c >= 0) sce[c] = e;  // slots and types are one to one
+  }
+  if constexpr (BINS > 0)
+    for (uint32_t i = threadIdx.x; i < nbin; i += blockDim.x) srdf[i] = 0;
   if (threadIdx.x == 0) *since_flush = 0ull;
   __syncthreads();
 
-  float4* cand = candA + warp * 32;
-  float4* cpos = cposA + warp * 32;        // centre of lane c
-  uint32_t* ccode = ccodeA + warp * 32;
-  uint32_t* cinfo = cinfoA + warp * 32;    // lane c: centre slot * nE | (env slot + 1) << 16, or SMEM's offsets
-  uint16_t* plist = plistA + warp * 1024;  // the staged batch's pairs, (lane << 5) | staged index
+  float4* cand = candA + warp * kStageAll;
+  uint32_t* skey = skeyA + warp * kStageAll;
   unsigned long long pairs_lane = 0, centres = 0;
+  uint32_t inb = 0;                   // in-ball pairs of the batch (BINS < 2)
+  int cs = 0, esc = -1;               // this lane's centre: its centre and environment slot
   constexpr unsigned long long FLUSH = 1ull << 30;
-  uint32_t inb = 0;
 
-  const uint32_t cH = (uint32_t)a.nE * (uint32_t)H;  // bins of one centre slot
-  auto stage = [&](uint32_t slot, const float4& q, uint32_t& key, uint32_t& code) {
-    const uint32_t m = a.labels ? (uint32_t)a.labels[slot] : __float_as_uint(q.w);
-    const bool jc = SYM && a.cflag[slot] != 0;
-    key = SYM ? (jc ? slot : 0xffffffffu) : slot;
-    const int es = ses[m & 255];
-    if constexpr (SMEM) {
-      const int cs = scs[m & 255];
-      const uint32_t cb = !jc ? 0xffffu : (cs < 0 ? 0xfffeu : (uint32_t)cs * cH);
-      code = (es < 0 ? 0xffffu : (uint32_t)es * (uint32_t)H) | (cb << 16);
+  // adds shared bin i's count v to the global cores
+  auto flush_bin = [&](uint32_t i, uint32_t v) {
+    if constexpr (BINS == 2) {
+      const uint32_t c = i / (RW * (uint32_t)H), rest = i - c * RW * (uint32_t)H;
+      const uint32_t row = rest / (uint32_t)H, b = rest - row * (uint32_t)H;
+      if (SYM && row < (uint32_t)a.nC) {
+        pairs_lane += 2ull * v;
+        const int e1 = sce[row], e0 = sce[c];
+        if (e1 >= 0) atomicAdd(&a.rdf_core[((uint64_t)c * a.nE + e1) * H + b], (unsigned long long)v);
+        if (e0 >= 0) atomicAdd(&a.rdf_core[((uint64_t)row * a.nE + e0) * H + b], (unsigned long long)v);
+      } else {
+        pairs_lane += v;
+        const uint32_t e = row - (SYM ? (uint32_t)a.nC : 0u);
+        if (e < (uint32_t)a.nE) atomicAdd(&a.rdf_core[((uint64_t)c * a.nE + e) * H + b], (unsigned long long)v);
+      }
     } else {
-      // (env slot + 1) | (centre slot + 1) << 8 | is-centre << 16
-      code = (uint32_t)(es + 1) | (jc ? ((uint32_t)(scs[m & 255] + 1) << 8) | 0x10000u : 0u);
+      atomicAdd(&a.rdf_core[i], (unsigned long long)v);
     }
   };
   auto start = [&](uint32_t self) {
     float4 cp = make_float4(kInf(), kInf(), kInf(), 0.f);
-    int cs = -1, es = -1;
+    cs = 0;
+    esc = -1;
     if (self != 0xffffffffu) {
       cp = a.ions[self];
-      const uint32_t ct = a.labels ? (uint32_t)a.labels[self] : __float_as_uint(cp.w);
-      cs = scs[ct & 255];
-      es = ses[ct & 255];
+      const uint32_t ct = (a.labels ? (uint32_t)a.labels[self] : __float_as_uint(cp.w)) & 255u;
+      cs = scs[ct];
+      esc = ses[ct];
       if (cs < 0) {  // selection guarantees a slot; record and drop the centre otherwise
         atomicOr(a.status, ST_TYPE_RANGE);
         cp = make_float4(kInf(), kInf(), kInf(), 0.f);
+        cs = 0;
       }
     }
-    cpos[lane] = cp;
-    if constexpr (SMEM)
-      cinfo[lane] = (uint32_t)(cs < 0 ? 0 : cs) * cH | ((es < 0 ? 0xffffu : (uint32_t)es * (uint32_t)H) << 16);
-    else
-      cinfo[lane] = (uint32_t)(cs < 0 ? 0 : cs) * (uint32_t)a.nE | ((uint32_t)(es + 1) << 16);
     inb = 0;
     return cp;
   };
-  auto bin_pair = [&](uint32_t e) {
-    const int c = (int)(e >> 5), j = (int)(e & 31u);
-    const float4 p = cpos[c];
-    const float4 q = staged_ion(cand, j);
-    const float d2 = dist2(p.x, p.y, p.z, q.x, q.y, q.z);
-    const uint32_t cj = ccode[j], ci = cinfo[c];
-    uint32_t cat;
-    if (a.lut_one) {
-      cat = (uint32_t)category_one(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT);
+  const float R2 = a.R2;
+  const unsigned long long one = f2_pack(a.one, a.one);
+  const FastCat fc(a);
+  // four times the guess g of a d^2 in the ball; up to 4 (H - 1) for any other
+  auto guess4 = [&](float d2) -> uint32_t {
+    if constexpr (FAST) {
+      return fc.guess4(d2);
     } else {
-      cat = (uint32_t)category_lut(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT, H);
-    }
-    if constexpr (SMEM) {
-      if ((cj & 0xffffu) != 0xffffu) atomicAdd(&srdf[(ci & 0xffffu) + (cj & 0xffffu) + cat], 1u);
-      if (SYM && (cj >> 16) != 0xffffu) {
-        // the same pair seen from the staged ion, a centre too
-        ++inb;
-        if ((cj >> 16) != 0xfffeu && (ci >> 16) != 0xffffu) atomicAdd(&srdf[(cj >> 16) + (ci >> 16) + cat], 1u);
-      }
-    } else {
-      const int esj = (int)(cj & 255u) - 1;
-      if (esj >= 0) atomicAdd(&a.rdf_core[((ci & 0xffffu) + (uint32_t)esj) * (uint32_t)H + cat], 1ull);
-      if (SYM && (cj & 0x10000u)) {
-        ++inb;
-        const int csj = (int)((cj >> 8) & 255u) - 1;
-        const int esc = (int)(ci >> 16) - 1;
-        if (esc >= 0 && csj >= 0)
-          atomicAdd(&a.rdf_core[((uint32_t)csj * a.nE + (uint32_t)esc) * (uint32_t)H + cat], 1ull);
-      }
+      const float m = fminf(d2, R2);
+      int c = (int)(__float_as_uint(m) >> a.lut_shift) - (int)a.lut_base;
+      c = c < 0 ? 0 : (c >= a.lut_n ? a.lut_n - 1 : c);
+      int g = slut[c];
+      if (!a.lut_one)
+        while (g + 1 < H && sT[g + 1] <= m) ++g;
+      return (uint32_t)g << 2;
     }
   };
-  auto taken = [&](uint32_t tm, uint32_t, unsigned long long, unsigned long long, unsigned long long) {
-    const uint32_t np = __popc(tm);
-    uint32_t ex = np;
+  // BINS 2: the tests, eight at a time, so that eight table loads are in
+  // flight before the first update.  A lane without a pair adds to a word of
+  // its own: a predicated shared atomic is compiled into a branch around it,
+  // three more instructions a test (19.1 against 17.5 ms).
+  const uint32_t dummy = smem_addr(sdummy + lane);
+  auto batch_kinds = [&](auto with_key, uint32_t base, uint32_t nb, uint32_t self, unsigned long long cxx,
+                         unsigned long long cyy, unsigned long long czz) {
+    constexpr bool WK = decltype(with_key)::value;
+    const uint32_t lbase = smem_addr(srdf) + (uint32_t)cs * RW * (uint32_t)H * 4u;
+    const uint2* key2 = (const uint2*)(skey + base);
+    const float4* cb = cand + base;
+#pragma unroll 1
+    for (uint32_t j0 = 0; j0 < nb; j0 += 8) {
+      float d[8], th[8];
+      uint32_t x[8];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(FULL, ex, o);
-      if (lane >= o) ex += t;
-    }
-    const uint32_t E = __shfl_sync(FULL, ex, 31);
-    inb += np;
-    for (uint32_t at = ex - np; tm; ++at) {
-      const int j = __ffs(tm) - 1;
-      tm &= tm - 1u;
-      plist[at] = (uint16_t)((lane << 5) | j);
-    }
-    __syncwarp();
-    for (uint32_t k = lane; k < E; k += 64) {
-      const uint32_t e0 = plist[k];
-      const bool two = k + 32 < E;
-      const uint32_t e1 = two ? plist[k + 32] : 0u;
-      bin_pair(e0);
-      if (two) bin_pair(e1);
+      for (int u = 0; u < 8; u += 2) {
+        const float4 c0 = cb[j0 + u], c1 = cb[j0 + u + 1];
+        dist2_x2(one, cxx, cyy, czz, f2_pack(c0.x, c0.y), f2_pack(c0.z, c0.w), f2_pack(c1.x, c1.y), d[u], d[u + 1]);
+        x[u] = __float_as_uint(c1.z);
+        x[u + 1] = __float_as_uint(c1.w);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t g4 = guess4(d[u]);
+        th[u] = *(const float*)((const char*)(sT + 1) + g4);
+        x[u] = x[u] + lbase + g4;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if constexpr (WK) {
+          const uint2 kk = key2[(j0 + u) >> 1];
+          const uint32_t k = (u & 1) ? kk.y : kk.x;
+          if (!(SYM ? k > self : k != self)) d[u] = kInf();
+        }
+        // bin address: one category up when d^2 reaches its threshold; the
+        // lane's own word when it is out of the ball
+        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 y;\n\t"
+                     "setp.le.f32 q, %1, %0;\n\t"
+                     "mov.u32 y, %2;\n\t"
+                     "@q add.u32 y, y, 4;\n\t"
+                     "setp.le.f32 p, %0, %3;\n\t"
+                     "selp.u32 y, y, %4, p;\n\t"
+                     "red.shared.add.u32 [y], 1;\n\t}"
+                     :: "f"(d[u]), "f"(th[u]), "r"(x[u]), "f"(R2), "r"(dummy) : "memory");
+      }
     }
   };
-  auto finish = [&](uint32_t live) {
-    pairs_lane += inb;
-    if (lane == 0) centres += (unsigned long long)__popc(live);
-    if (SMEM) {
-      // keep every shared bin below 2^32 (see k_scan)
-      uint32_t tot = inb;
-      for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(FULL, tot, o);
-      unsigned long long old = 0;
-      if (lane == 0) old = atomicAdd(since_flush, (unsigned long long)tot);
-      old = __shfl_sync(FULL, old, 0);
-      if (old / FLUSH != (old + tot) / FLUSH) {
-        for (int i = lane; i < a.nC * a.nE * H; i += 32) {
-          const uint32_t v = atomicExch(&srdf[i], 0u);
-          if (v) atomicAdd(&a.rdf_core[i], (unsigned long long)v);
+  auto batch = [&](uint32_t base, uint32_t nb, bool keyed, uint32_t self, unsigned long long cxx,
+                   unsigned long long cyy, unsigned long long czz) {
+    if constexpr (BINS == 2) {
+      if (keyed) batch_kinds(std::true_type{}, base, nb, self, cxx, cyy, czz);
+      else batch_kinds(std::false_type{}, base, nb, self, cxx, cyy, czz);
+    } else {
+#pragma unroll 1
+      for (uint32_t j = 0; j < nb; j += 2) {
+        const float4 c0 = cand[base + j], c1 = cand[base + j + 1];
+        float d[2];
+        dist2_x2(one, cxx, cyy, czz, f2_pack(c0.x, c0.y), f2_pack(c0.z, c0.w), f2_pack(c1.x, c1.y), d[0], d[1]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const uint32_t key = keyed ? skey[base + j + u] : 0xffffffffu;
+          if (!(d[u] <= R2) || !(SYM ? key > self : key != self)) continue;
+          uint32_t cat = guess4(d[u]) >> 2;
+          cat += sT[cat + 1] <= d[u] ? 1u : 0u;
+          const uint32_t cj = __float_as_uint(u ? c1.w : c1.z);
+          const int esj = (int)((cj >> 1) & 255u) - 1, csj = (int)((cj >> 9) & 255u) - 1;
+          auto add = [&](uint32_t i) {
+            if constexpr (BINS == 1) atomicAdd(&srdf[i], 1u);
+            else atomicAdd(&a.rdf_core[i], 1ull);
+          };
+          ++inb;
+          if (esj >= 0) add(((uint32_t)cs * a.nE + (uint32_t)esj) * (uint32_t)H + cat);
+          if (SYM && csj >= 0) {
+            // the same pair seen from the staged ion, a centre too
+            ++inb;
+            if (esc >= 0) add(((uint32_t)csj * a.nE + (uint32_t)esc) * (uint32_t)H + cat);
+          }
         }
       }
     }
   };
-  auto accept = [](int, float, uint32_t) { return true; };
-  const unsigned long long tests =
-      lanes_walk<SYM, false, true, false>(a, cand, ccode, boxA + warp * 2, stage, start, accept, taken, finish);
+  auto finish = [&](uint32_t live, uint32_t btests) {
+    pairs_lane += inb;
+    if (lane == 0) centres += (unsigned long long)__popc(live);
+    if constexpr (BINS > 0) {
+      // keep every shared bin below 2^32: a bin gains at most one count per
+      // credit of a test; each time the block's tests cross a multiple of 2^30
+      // the warp that crossed it moves all bins to the global uint64 cores
+      unsigned long long old = 0;
+      if (lane == 0) old = atomicAdd(since_flush, (unsigned long long)btests);
+      old = __shfl_sync(FULL, old, 0);
+      if (old / FLUSH != (old + btests) / FLUSH) {
+        for (uint32_t i = lane; i < nbin; i += 32) {
+          const uint32_t v = atomicExch(&srdf[i], 0u);
+          if (v) flush_bin(i, v);
+        }
+      }
+    }
+  };
+  const unsigned long long tests = 
+      lanes_walk<SYM>(a, cand, skey, boxA + warp * 2, start, batch, finish);
   if (lane == 0 && a.tests) atomicAdd(a.tests, tests);
-
+  __syncthreads();
+  if constexpr (BINS > 0)
+    for (uint32_t i = threadIdx.x; i < nbin; i += blockDim.x) {
+      const uint32_t v = srdf[i];
+      if (v) flush_bin(i, v);
+    }
   for (int o = 16; o; o >>= 1) pairs_lane += __shfl_xor_sync(FULL, pairs_lane, o);
   if (lane == 0) {
     atomicAdd(&a.counters[0], pairs_lane);
     atomicAdd(&a.counters[1], centres);
-  }
-  __syncthreads();
-  if (SMEM) {
-    for (int i = threadIdx.x; i < a.nC * a.nE * H; i += blockDim.x) {
-      const uint32_t v = srdf[i];
-      if (v) atomicAdd(&a.rdf_core[i], (unsigned long long)v);
-    }
   }
 }
 
@@ -2290,36 +2440,23 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
   // row per set -- then the row of "no set"; with CAT the category rows after
   const int frows = CAT ? EM + 1 : EM * K + 1;
   unsigned char* sp = smem;
-  float4* candA = (float4*)sp; sp += NW * 32 * 16;
+  float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
   float4* boxA = (float4*)sp; sp += NW * 2 * 16;
-  uint32_t* ccodeA = (uint32_t*)sp; sp += NW * 32 * 4;
+  uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
   float* listA = (float*)sp; sp += (size_t)NW * frows * 32 * 4;
   uint16_t* catA = (uint16_t*)sp; sp += CAT ? (((size_t)NW * EM * K * 32 * 2 + 15) & ~size_t(15)) : 0;
   float* sT = (float*)sp; sp += ((H + 4) & ~3) * 4;  // H thresholds, then +inf
-  uint16_t* slut = (uint16_t*)sp; sp += ((a.lut_n + 7) & ~7) * 2;
   int8_t* scs = (int8_t*)sp; sp += 256;
-  uint32_t* skey = (uint32_t*)sp;  // [256] per type: its environment set (EM: none) for every centre slot, 4 bits each
+  uint16_t* slut = (uint16_t*)sp;  // unless a.cat_fast
   const uint32_t RSTRIDE = CAT ? 32u : (uint32_t)K * 32u;  // float rows between sets
   for (int i = threadIdx.x; i <= H; i += blockDim.x) sT[i] = i < H ? a.cat_T[i] : kInf();
-  for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    scs[i] = a.cslot_of[i];
-    uint32_t key = 0;
-    if (UNI) {
-      const int si = a.nC > 0 ? a.setidx[i] : -1;
-      key = (uint32_t)(si < 0 ? EM : si) * RSTRIDE;
-    } else {
-      for (int c = 0; c < a.nC; ++c) {
-        const int si = a.setidx[c * 256 + i];
-        key |= (uint32_t)(si < 0 ? EM : si) << (4 * c);
-      }
-    }
-    skey[i] = key;
-  }
+  if (!a.cat_fast)
+    for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) scs[i] = a.cslot_of[i];
   __syncthreads();
 
-  float4* cand = candA + warp * 32;
-  uint32_t* ccode = ccodeA + warp * 32;
+  float4* cand = candA + warp * kStageAll;
+  uint32_t* skey = skeyA + warp * kStageAll;
   // set p, rank r at L[(p * K + K - 1 - r) * 32]; with CAT, set p's threshold
   // at L[p * 32] and its rank r at C[(p * K + K - 1 - r) * 32]
   float* L = listA + (size_t)warp * frows * 32 + lane;
@@ -2331,13 +2468,6 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
   int cs = -1, nset = 0, sh = 0;  // centre slot, its sets, 4 * slot (its nibble in a staged key)
   uint32_t me = 0xffffffffu;      // this lane's centre slot
 
-  // the staged key carries the ion's environment set for every centre slot
-  // (read by the test loop with the position), the code its slot
-  auto stage = [&](uint32_t slot, const float4& q, uint32_t& key, uint32_t& code) {
-    const uint32_t m = (a.labels ? (uint32_t)a.labels[slot] : __float_as_uint(q.w)) & 255u;
-    key = skey[m];
-    code = slot;
-  };
   auto start = [&](uint32_t self) {
     float4 cp = make_float4(kInf(), kInf(), kInf(), 0.f);
     cs = -1;
@@ -2362,22 +2492,20 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
     inb = 0;
     return cp;
   };
+  // category of an in-ball d^2 (see k_lanes)
+  const FastCat fc(a);
+  auto category_of = [&](float d2) -> int {
+    if (!a.cat_fast) return category_lut(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT, H);
+    const int g = (int)(fc.guess4(d2) >> 2);
+    return g + (sT[g + 1] <= d2 ? 1 : 0);
+  };
   // float row (offset) of a staged key's environment set for this lane's centre type
   auto row_of = [&](uint32_t w) -> uint32_t { return UNI ? w : ((w >> sh) & 15u) * RSTRIDE; };
-  auto accept = [&](int, float d2, uint32_t w) {
-    // the set's K-th value or threshold (the -inf row for ions in no set)
-    return d2 < L[row_of(w)];
-  };
   auto insert = [&](uint32_t row, float d2) {
     float* Lp = L + row;  // row s holds rank K - 1 - s
     if (!(d2 < Lp[0])) return;
     if constexpr (CAT) {
-      int c;
-      if (a.lut_one) {
-        c = category_one(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT);
-      } else {
-        c = category_lut(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT, H);
-      }
+      const int c = category_of(d2);
       uint16_t* Cp = C + (row / 32u) * (uint32_t)K * 32u;
       if constexpr (KB > 0) {
         int v[KB];
@@ -2423,8 +2551,24 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
       Lp[(K - 1 - r) * 32] = d2;
     }
   };
-  auto taken = [&](uint32_t tm, uint32_t nin, unsigned long long cxx, unsigned long long cyy, unsigned long long czz) {
-    inb += nin;
+  const unsigned long long one = f2_pack(a.one, a.one);
+  auto batch = [&](uint32_t base, uint32_t nb, bool keyed, uint32_t, unsigned long long cxx, unsigned long long cyy,
+                   unsigned long long czz) {
+    uint32_t tm = 0;  // staged ions below the K-th value or threshold of their set (the -inf row for no set)
+    const float4* cb = cand + base;
+#pragma unroll
+    for (int j0 = 0; j0 < 32; j0 += 8) {
+      if (j0 >= (int)nb) break;
+#pragma unroll
+      for (int j = j0; j < j0 + 8; j += 2) {
+        const float4 c0 = cb[j], c1 = cb[j + 1];
+        float d0, d1;
+        dist2_x2(one, cxx, cyy, czz, f2_pack(c0.x, c0.y), f2_pack(c0.z, c0.w), f2_pack(c1.x, c1.y), d0, d1);
+        inb += (d0 <= a.R2 ? 1u : 0u) + (d1 <= a.R2 ? 1u : 0u);
+        tm |= d0 < L[row_of(__float_as_uint(c1.z))] ? (1u << j) : 0u;
+        tm |= d1 < L[row_of(__float_as_uint(c1.w))] ? (2u << j) : 0u;
+      }
+    }
     float cx, cy, cz, dup;
     f2_unpack(cxx, cx, dup);
     f2_unpack(cyy, cy, dup);
@@ -2432,13 +2576,13 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
     while (tm) {
       const int j = __ffs(tm) - 1;
       tm &= tm - 1u;
-      const float4 q = staged_ion(cand, j);
+      const float4 q = staged_ion(cb, j);
       const float d2 = dist2(cx, cy, cz, q.x, q.y, q.z);
-      if (d2 == 0.f && ccode[j] == me) continue;  // the centre itself
+      if (keyed && d2 == 0.f && skey[base + j] == me) continue;  // the centre itself
       insert(row_of(__float_as_uint(q.w)), d2);
     }
   };
-  auto finish = [&](uint32_t live) {
+  auto finish = [&](uint32_t live, uint32_t) {
     if (lane == 0) centres += (unsigned long long)__popc(live);
     // every live centre met itself once in the in-ball count (d^2 = 0)
     pairs_lane += inb - (me != 0xffffffffu ? 1u : 0u);
@@ -2454,7 +2598,7 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
           return (v == (int)CNONE) ? a.cat_miss : v;
         } else {
           const float v = L[(p * K + K - a.kvals[kk]) * 32];
-          return (v == RUP) ? a.cat_miss : category_lut(v, slut, a.lut_n, a.lut_base, a.lut_shift, sT, H);
+          return (v == RUP) ? a.cat_miss : category_of(v);
         }
       };
       if constexpr (KB > 0) {
@@ -2473,7 +2617,7 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
     }
   };
   const unsigned long long tests =
-      lanes_walk<false, true, false, true>(a, cand, ccode, boxA + warp * 2, stage, start, accept, taken, finish);
+      lanes_walk<false>(a, cand, skey, boxA + warp * 2, start, batch, finish);
   if (lane == 0 && a.tests) atomicAdd(a.tests, tests);
 
   for (int o = 16; o; o >>= 1) pairs_lane += __shfl_xor_sync(FULL, pairs_lane, o);
@@ -3396,31 +3540,44 @@ int launch_brick(const ScanArgs& a, int kr, int sm_count, size_t* smem_used, cud
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-size_t lanes_smem(const ScanArgs& a) {
+static void launch_pass_codes(const ScanArgs& a, PassCode kind, uint32_t param, int sm_count, cudaStream_t s) {
+  counted();
+  const uint64_t blocks = (a.n + 1023) / 1024;
+  k_pass_codes<<<(unsigned)(blocks < (uint64_t)sm_count * 8 ? (blocks ? blocks : 1) : (uint64_t)sm_count * 8), 256, 0, s>>>(
+      a, (int)kind, param, a.pcode);
+}
+
+// Shared memory of k_lanes with `bins` shared bins (0 = none).
+static size_t lanes_smem(const ScanArgs& a, size_t bins, bool fast) {
   constexpr int NW = kLanesWarps;
-  size_t b = 16 + 2 * NW * 32 * 16 + NW * 2 * 16 + 2 * NW * 32 * 4 + NW * 1024 * 2 + (size_t)((a.H + 4) & ~3) * 4;
-  if (a.rdf_in_smem) b += (size_t)a.nC * a.nE * a.H * 4;
-  b += (size_t)((a.lut_n + 7) & ~7) * 2 + 512;
-  return b;
+  return 16 + NW * kStageAll * 16 + NW * 2 * 16 + NW * kStageAll * 4 + 32 * 4 + (size_t)((a.H + 4) & ~3) * 4 + bins * 4 +
+         3 * 256 +
+         (fast ? 0 : (size_t)((a.lut_n + 7) & ~7) * 2);
 }
 
 int launch_lanes(const ScanArgs& a, int kr, int sm_count, size_t* smem_used, cudaStream_t s) {
   if (a.mode != 0 || kr > 0 || (a.flags & PP_CNTNB) || !(a.flags & PP_RDF) || a.bx < 1 || a.by < 1 || a.bz < 1 ||
       a.nC > 254 || a.nE > 254 || !a.brows)
     return -3;
-  const size_t smem = lanes_smem(a);
+  // bins by kind of pair while they fit beside the staging buffers, then in
+  // the cores' layout, then none in shared memory
+  constexpr size_t cap = 224 * 1024;
+  const bool fast = a.cat_fast != 0;
+  const size_t kinds = (size_t)a.nC * ((a.sym ? a.nC : 0) + a.nE + 1) * a.H, cores = (size_t)a.nC * a.nE * a.H;
+  const int bins = lanes_smem(a, kinds, fast) <= cap ? 2 : lanes_smem(a, cores, fast) <= cap ? 1 : 0;
+  const size_t smem = lanes_smem(a, bins == 2 ? kinds : bins == 1 ? cores : 0, fast);
   if (smem_used) *smem_used = smem;
-  if (smem > 200 * 1024) return -3;
-  auto kern = a.sym ? (a.rdf_in_smem ? k_lanes<true, true> : k_lanes<true, false>)
-                    : (a.rdf_in_smem ? k_lanes<false, true> : k_lanes<false, false>);
+  if (smem > cap) return -3;
+#define PP_LANES_KERN(SYMV, FASTV) \
+  (bins == 2 ? k_lanes<SYMV, 2, FASTV> : bins == 1 ? k_lanes<SYMV, 1, FASTV> : k_lanes<SYMV, 0, FASTV>)
+  auto kern = a.sym ? (fast ? PP_LANES_KERN(true, true) : PP_LANES_KERN(true, false))
+                    : (fast ? PP_LANES_KERN(false, true) : PP_LANES_KERN(false, false));
+#undef PP_LANES_KERN
   if (!allow_dynamic_smem((const void*)kern, smem))
     return -1;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLanesWarps * 32, smem) != cudaSuccess ||
-      per_sm < 1)
-    return -1;
+  launch_pass_codes(a, bins == 2 ? PC_KINDS : PC_CORES, 0, sm_count, s);
   counted();
-  kern<<<sm_count * per_sm, kLanesWarps * 32, smem, s>>>(a);
+  kern<<<sm_count, kLanesWarps * 32, smem, s>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -3429,8 +3586,8 @@ size_t lanes_knn_smem(const ScanArgs& a, bool cat) {
   const size_t em = a.emax > 1 ? a.emax : 1;
   const size_t frows = cat ? em + 1 : em * a.kmax + 1;
   const size_t crows = cat ? (((size_t)NW * em * a.kmax * 32 * 2 + 15) & ~size_t(15)) : 0;
-  return NW * 32 * 16 + NW * 2 * 16 + NW * 32 * 4 + (size_t)NW * frows * 32 * 4 + crows + (size_t)((a.H + 4) & ~3) * 4 +
-         (size_t)((a.lut_n + 7) & ~7) * 2 + 256 + 256 * 4;
+  return NW * kStageAll * 16 + NW * 2 * 16 + NW * kStageAll * 4 + (size_t)NW * frows * 32 * 4 + crows + (size_t)((a.H + 4) & ~3) * 4 +
+         (a.cat_fast ? 0 : (size_t)((a.lut_n + 7) & ~7) * 2) + 256;
 }
 
 int launch_lanes_knn(const ScanArgs& a, bool disjoint_sets, int sm_count, size_t* smem_used, cudaStream_t s) {
@@ -3460,6 +3617,7 @@ int launch_lanes_knn(const ScanArgs& a, bool disjoint_sets, int sm_count, size_t
 #undef PP_KNN_KERN
   if (!allow_dynamic_smem((const void*)kern, smem))
     return -1;
+  launch_pass_codes(a, uni ? PC_ROW : PC_NIBBLE, cat ? 32u : (uint32_t)a.kmax * 32u, sm_count, s);
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLanesKnnWarps * 32, smem) != cudaSuccess ||
       per_sm < 1)

@@ -1,0 +1,71 @@
+"""Forms of the centre-per-lane RDF pass against the oracle: where its bins live
+(by kind of pair or in the cores' layout in shared memory, or in global memory,
+by their number), how categories are found (approximate root or table), which
+ions are centres, and blocks cut by the grid's edges.  Counts are whole numbers
+and must be equal."""
+import numpy as np
+import pytest
+
+from paraprobe_gb300 import native as N
+from paraprobe_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+# 4 centre and 5 environment slots: 4 * (4 + 5 + 1) rows of bins by kind fit
+# 224 KB up to about 1,100 bins, the cores' 20 rows up to about 2,200
+HISTS = [(0.0, 0.01, 1.2), (0.0, 0.0011, 1.2), (0.0, 0.0008, 1.2), (0.0, 0.0003, 1.2),
+         (0.3, 0.01, 1.2), (0.3, 0.0008, 1.2), (0.0, 0.4, 1.2), (0.0, 0.037, 1.25)]
+
+
+@pytest.mark.parametrize("hist", HISTS)
+@pytest.mark.parametrize("symmetric", [1, 0])
+def test_lanes_rdf_bin_forms(ctx, oracle, hist, symmetric):
+    spec = synth.cone_specimen(n=20000, r_apex=5.0, half_angle_deg=10.0, length=14.0, n_clusters=20, members=40,
+                               nspecies=6, seed=97, nseg=48, stack=4.0)
+    trg = [[1], [2, 3], [3], [1, 4]]
+    env = [[1, 2], [3, 6], [1, 2, 3, 5], [5]]  # type 4: a centre in no environment; 5, 6: never centres
+    cid = ctx.upload(spec.xyz, spec.labels)
+    ctx.hull(cid, spec.hull, 0.5)
+    ctx.tuning(cid, 4.0, ((3 | 2 << 8 | 2 << 12) << 16) | N.PP_TILE_LANES)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.set_option("symmetric", symmetric)
+    try:
+        ctx.run(cid, N.PP_RDF | N.PP_RIPK)
+        bins, st = ctx.fetch(), ctx.stats()
+        assert ctx.last_kernel() == "k_lanes"
+    finally:
+        ctx.set_option("symmetric", 1)
+        ctx.free(cid)
+    surf = oracle.surface_distance(spec.xyz, spec.hull, np.float32(hist[2]))
+    ref = oracle.spatstat(spec.xyz, spec.labels, surf, *hist, N.PP_RDF | N.PP_RIPK, trg, env, [])
+    assert st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
+    assert np.array_equal(bins, ref["bins"])
+
+
+def test_lanes_pairs_on_bin_edges(ctx, oracle):
+    """Ions on a lattice of 2^-4 nm: most distances lie exactly on bin edges or
+    on R, and coincident ions give d = 0."""
+    g = np.arange(24, dtype=np.float32) / 16
+    xyz = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    xyz = np.concatenate([xyz, xyz[:500]]).astype(np.float32)
+    labels = (1 + np.arange(len(xyz)) % 3).astype(np.uint8)
+    types = [1, 2, 3]
+    trg, env = [[a] for a in types for b in types], [[b] for a in types for b in types]
+    hist = (0.0, 0.0625, 0.5)
+    cid = ctx.upload(xyz, labels)
+    ctx.surfdist(cid, np.full(len(xyz), 10.0, dtype=np.float32))
+    ctx.tuning(cid, 4.0, ((4 | 2 << 8 | 2 << 12) << 16) | N.PP_TILE_LANES)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.run(cid, N.PP_RDF)
+    rdf, st = ctx.fetch(), ctx.stats()
+    assert ctx.last_kernel() == "k_lanes"
+    ctx.run(cid, N.PP_MKNN, [7, 3, 1])
+    knn, st2 = ctx.fetch(), ctx.stats()
+    assert ctx.last_kernel() == "k_lanes_knn"
+    ctx.free(cid)
+    surf = np.full(len(xyz), 10.0, dtype=np.float32)
+    for got, s, flags, ks in ((rdf, st, N.PP_RDF, []), (knn, st2, N.PP_MKNN, [7, 3, 1])):
+        ref = oracle.spatstat(xyz, labels, surf, *hist, flags, trg, env, ks)
+        assert s["pairs"] == ref["pairs"] and np.array_equal(got, ref["bins"])
