@@ -258,6 +258,11 @@ int pp_fetch_npcorr(pp_ctx* ctx, uint32_t* counts, uint64_t cap, uint64_t* edge)
  *                       while they fit two blocks per SM, bin categories
  *                       beyond (default); 1 = distances; 2 = categories.
  *                       Results are identical either way.
+ *   "knn_walks"         the kNN centre-per-lane scan walks dense sets only as
+ *                       far as their k-th neighbours lie and the other sets'
+ *                       ions apart: 0 = where that is faster (default), 1 =
+ *                       never, 2 = wherever the sets allow.  Results are
+ *                       identical either way.
  *   "box_filter"        the centre-per-lane scans test only ions within R of
  *                       the bounding box of a batch's centres (default 1);
  *                       0 tests every ion of the block's stencil rows.

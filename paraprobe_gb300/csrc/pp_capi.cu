@@ -198,6 +198,7 @@ struct pp_ctx {
   // scratch
   DevBuf tmp_cell_of, tmp_rank, scan_tmp, bbox, centres, centre_count, work, tables_dev, sel_flags, sel_tmp;
   DevBuf tri_fill, cflag, rowtab, nc_pre, pass_code;
+  DevBuf type_counts, sp_start, sp_ions, sp_slot;  // kNN passes in two walks
   DevBuf labels_run, perm_dev, gather_src;
   DevBuf mask_in;  // caller's centre mask: [n] input order, then [n] sorted-slot order
   // statistics after clustering: option "aposteriori_guard" = 1 runs the
@@ -230,6 +231,7 @@ struct pp_ctx {
   bool no_lanes = false;  // option "lanes" = 0: RDF passes take the per-centre or brick scan
   bool no_uniform = false;  // option "uniform_sets" = 0: the kNN lane scan decodes sets per centre slot
   bool no_box = false;      // option "box_filter" = 0: the lane scans stage every candidate of the cell rows
+  int knn_walks = 0;        // option "knn_walks": 0 automatic, 1 one walk, 2 two walks where the sets allow
   int knn_lists = 0;        // option "knn_lists": 0 automatic, 1 d^2 lists, 2 category lists
   DevBuf brows;           // stencil rows of a cell block, nearest first (centre-per-lane scan)
   int brows_key[3] = {-1, -1, -1};
@@ -1348,8 +1350,10 @@ int ensure_block_rows(pp_ctx* ctx, int by, int bz, int sr, cudaStream_t s, const
 
 // Select the centres of a plain run into ctx->centres (cell order); returns
 // their number.  Synchronises the stream once to learn the count.
+// type_counts (256 words, nullable) receives the ions of each type.
 int select_centres(pp_ctx* ctx, Cloud& cl, const uint8_t* labels, const float* surf, const int8_t* cslot, float R,
-                   uint32_t* ncent, cudaStream_t s, const uint8_t* extra_slot_mask = nullptr) {
+                   uint32_t* ncent, cudaStream_t s, const uint8_t* extra_slot_mask = nullptr,
+                   unsigned long long* type_counts = nullptr) {
   const uint64_t n = cl.n;
   CK(ctx->centres.ensure(std::max<uint64_t>(n, 1) * 4));
   CK(ctx->centre_count.ensure(8));
@@ -1361,9 +1365,165 @@ int select_centres(pp_ctx* ctx, Cloud& cl, const uint8_t* labels, const float* s
                             extra_slot_mask, ctx->sel_flags.as<uint32_t>(), ctx->sel_tmp.as<uint32_t>(), tmp_elems * 2,
                             ctx->centres.as<uint32_t>(), ctx->centre_count.as<uint32_t>(), ctx->cflag.as<uint8_t>(), s);
   CK(cudaGetLastError());
+  if (type_counts) {
+    CK(ctx->type_counts.ensure(256 * 8));
+    CK(cudaMemsetAsync(ctx->type_counts.p, 0, 256 * 8, s));
+    pp::launch_type_count(labels ? labels : cl.label_sorted.as<uint8_t>(), n, ctx->type_counts.as<unsigned long long>(),
+                          ctx->sm_count, s);
+    CK(cudaMemcpyAsync(type_counts, ctx->type_counts.p, 256 * 8, cudaMemcpyDeviceToHost, s));
+  }
   CK(cudaMemcpyAsync(ncent, ctx->centre_count.p, 4, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   return PP_OK;
+}
+
+// Ions per nm^3 inside the specimen: the mean m of a grid cell from the share
+// of cells that hold any, n / occupied = m / (1 - exp(-m)).
+double ion_density(const Cloud& cl) {
+  if (!cl.occupied || !cl.n) return 0.0;
+  const double per = (double)cl.n / (double)cl.occupied;
+  double m = per;
+  for (int i = 0; i < 30; ++i) m = per * (1.0 - std::exp(-m));
+  const double h = cl.g.h;
+  return m > 1e-3 ? m / (h * h * h) : 0.0;
+}
+
+// First radius of a set of `share` of the ions, for orders up to k: it holds
+// k + 4.5 sqrt(k) + 2 of the set's ions on average, so that hardly a centre has
+// fewer than k.
+double near_radius(double rho, double share, int k) {
+  return std::cbrt((k + 4.5 * std::sqrt((double)k) + 2.0) / (4.18879 * rho * share));
+}
+constexpr double kNearDenseR = 0.6;  // dense: first radius up to this share of R
+
+// Whether two walks can pay for a kNN pass: some set may be dense, and the
+// in-ball pairs make up for the preparation (pass codes, type counts, the
+// sparse list, two or three more kernels: 40 to 80 us).  Measured on tips of
+// 50k to 1M ions, R = 2 nm, k = 4 and 10: with the pairs counted by the pass's
+// RDF part 983 -> 817 us from 1e7 pairs on; with a count of their own even at
+// 9e7 (1108 / 1152 us) and 1775 -> 1442 us at 3.3e8.
+bool near_pays(const pp_ctx* ctx, const Cloud& cl, float R, int kmax, uint64_t centres, bool count) {
+  const double rho = ion_density(cl);
+  if (ctx->knn_walks == 1 || !(rho > 0.0) || near_radius(rho, 1.0, kmax) > kNearDenseR * R) return false;
+  return ctx->knn_walks == 2 || (double)centres * rho * 4.18879 * R * R * R >= (count ? 1.5e8 : 1e7);
+}
+
+// Dense sets of a kNN pass in two walks (k_lanes_near) for a block of a.bx x
+// a.by x a.bz cells, from the ions of each type; fills ScanArgs::near_* and
+// returns whether the pass is worth it (sparse = ions of the other sets).
+bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long long* type_counts, pp::ScanArgs& a,
+               uint64_t* sparse) {
+  const uint64_t n = cl.n;
+  if (!a.uniform_sets || !P.disjoint || P.kmax < 1 || P.kmax > 20 || P.emax > 15 || !cl.occupied || !n) return false;
+  const double h = cl.g.h, rho = ion_density(cl);
+  if (!(rho > 0.0)) return false;
+  std::vector<uint64_t> ions(16, 0);
+  for (int ty = 0; ty < 256; ++ty) {
+    const int p = P.setidx[ty];
+    if (p >= 0) ions[p] += type_counts[ty];
+  }
+  std::vector<std::pair<double, int>> dense;
+  for (int p = 0; p < P.emax; ++p) {
+    if (!ions[p]) continue;
+    const double r = near_radius(rho, (double)ions[p] / (double)n, P.kmax);
+    if (r <= kNearDenseR * R) dense.push_back({r, p});
+  }
+  if (dense.empty()) return false;
+  std::sort(dense.begin(), dense.end());
+  if (dense.size() > (size_t)pp::kNearMax) dense.resize(pp::kNearMax);
+  // ions around a block's box within r
+  const double bx = a.bx * h, by = a.by * h, bz = a.bz * h;
+  auto around = [&](double r) {
+    return bx * by * bz + 2.0 * r * (bx * by + by * bz + bz * bx) + 3.14159 * r * r * (bx + by + bz) + 4.18879 * r * r * r;
+  };
+  std::memset(a.near_map, 0, sizeof a.near_map);
+  a.near_n = (int)dense.size();
+  double walk = 0.0;
+  uint64_t in_dense = 0, in_sets = 0;
+  for (int p = 0; p < 16; ++p) in_sets += ions[p];
+  for (int d = 0; d < a.near_n; ++d) {
+    const int p = dense[d].second;
+    a.near_map[p] = (int8_t)~d;
+    a.near_set[d] = p;
+    a.near_r[d] = (float)dense[d].first;
+    walk += around(dense[d].first);
+    in_dense += ions[p];
+    // stencil rows (nearest first) that reach within the radius: up to the
+    // largest squared gap, in cells, of a row with a point that near
+    const double rr = dense[d].first + 4.0 * cl.g.margin;
+    const int sr = a.bsr;
+    int G = 0;
+    for (int gz = 0; gz <= sr; ++gz)
+      for (int gy = 0; gy <= sr; ++gy) {
+        const double y = std::max(gy - 1, 0) * h, z = std::max(gz - 1, 0) * h;
+        if (y * y + z * z <= rr * rr) G = std::max(G, gy * gy + gz * gz);
+      }
+    int rows = 0;
+    const int ny = a.by + 2 * sr, nz = a.bz + 2 * sr;
+    auto gap = [sr](int r, int b) { return r < sr ? sr - r : (r >= sr + b ? r - (sr + b - 1) : 0); };
+    for (int rz = 0; rz < nz; ++rz)
+      for (int ry = 0; ry < ny; ++ry) {
+        const int gy = gap(ry, a.by), gz = gap(rz, a.bz);
+        rows += gy * gy + gz * gz <= G;
+      }
+    a.near_rows[d] = rows;
+  }
+  a.near_sp = 0;
+  for (int p = 0; p < P.emax; ++p)
+    if (a.near_map[p] >= 0) a.near_map[p] = (int8_t)a.near_sp++;
+  *sparse = in_sets - in_dense;
+  // the sparse list's grid: the cloud's, coarsened to cells of about R / 2
+  const Grid& g = cl.g;
+  const int f = std::max(1, (int)std::lround(0.5 * R / h));
+  Grid sg = g;
+  sg.h = (float)(h * f);
+  sg.inv_h = (float)(1.0 / (h * f));
+  sg.nx = (g.nx + f - 1) / f;
+  sg.ny = (g.ny + f - 1) / f;
+  sg.nz = (g.nz + f - 1) / f;
+  sg.ncells = (uint64_t)sg.nx * sg.ny * sg.nz;
+  a.sp_g = sg;
+  a.near_hot = 0;
+  for (int c = 1; c < P.nC; ++c)
+    if (type_counts[P.ctype[c]] > type_counts[P.ctype[a.near_hot]]) a.near_hot = c;
+  walk += around(R) * (double)*sparse / (double)n;
+  if (walk > 0.5 * around(R)) return false;
+  // the dense sets' shared histograms end at the first radius
+  const float d2 = a.near_r[a.near_n - 1] * a.near_r[a.near_n - 1];
+  a.near_hd = (int)(std::upper_bound(P.catT.begin() + 1, P.catT.end(), d2) - P.catT.begin());
+  return true;
+}
+
+// The kNN part of a pass in two walks (k_lanes_near) where near_plan finds it
+// worth it, else -3.  count: the pass has no other part that counts its in-ball
+// pairs, so they are counted by a symmetric walk of their own first (needs
+// ctx->nc_pre); the two take the work counters a.work[0] and [1].
+int run_near(pp_ctx* ctx, Cloud& cl, const RunPlan& P, const unsigned long long* type_counts, float R,
+             const pp::ScanArgs& a0, bool count, size_t* smem, cudaStream_t s) {
+  pp::ScanArgs a = a0;
+  uint64_t sparse = 0;
+  if (!near_pays(ctx, cl, R, P.kmax, (uint64_t)a.ncentres * std::max<uint32_t>(a.sample_stride, 1), count)) return -3;
+  if (!near_plan(cl, P, R, type_counts, a, &sparse)) return -3;
+  const uint64_t sp_words = a.sp_g.ncells + 1;
+  CK(ctx->sp_start.ensure(sp_words * 8));  // starts, then cursors
+  CK(ctx->sp_ions.ensure(std::max<uint64_t>(sparse, 1) * 16));
+  CK(ctx->sp_slot.ensure(std::max<uint64_t>(sparse, 1) * 4));
+  const uint64_t tmp_elems = sp_words / 2048 + 64;
+  CK(ctx->scan_tmp.ensure(tmp_elems * 8 * 2));
+  if (count) {
+    pp::ScanArgs ac = a;
+    ac.sym = ctx->no_sym ? 0 : 1;
+    ac.nc_pre = ctx->nc_pre.as<uint32_t>();
+    const int rc = pp::launch_lanes_count(ac, ctx->sm_count, s);
+    if (rc) return rc;
+    a.work = a0.work + 1;
+    a.counters = (unsigned long long*)(ctx->work.as<unsigned char>() + 16);  // counted already
+  }
+  const int rc = pp::launch_lanes_near(a, ctx->sm_count, ctx->sp_start.as<uint32_t>(),
+                                       ctx->sp_start.as<uint32_t>() + sp_words, ctx->sp_ions.as<float4>(),
+                                       ctx->sp_slot.as<uint32_t>(), (uint32_t)sparse, ctx->scan_tmp.as<uint32_t>(),
+                                       tmp_elems * 4, smem, s);
+  return count && rc == -3 ? -1 : rc;  // the pairs were counted
 }
 
 // One pass of compute_generic_spatstat3 on the device.  centre_limit > 0
@@ -1409,7 +1569,12 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
     mask_slot = m_in + n;
   }
   uint32_t ncent = 0;
-  if ((rc = select_centres(ctx, *cl, labels, surf, D.cslot, R, &ncent, s, mask_slot))) return rc;
+  const bool near_ok = P.kr == 1 && P.kmax <= 20 && P.disjoint && !ctx->no_lanes &&
+                       !(flags & (PP_CNTNB | PP_NPCORR)) && near_pays(ctx, *cl, R, P.kmax, n, !(flags & (PP_RDF | PP_RIPK)));
+  std::vector<unsigned long long> type_counts(near_ok ? 256 : 0);
+  if ((rc = select_centres(ctx, *cl, labels, surf, D.cslot, R, &ncent, s, mask_slot,
+                           near_ok ? type_counts.data() : nullptr)))
+    return rc;
   ctx->last_centres_all = ncent;
   // a tuning sample: every stride-th centre (or brick) over the whole cloud
   uint32_t stride = 1;
@@ -1461,7 +1626,7 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
   // to both (the counts are the same as the per-centre ball scan's)
   a.sym = ((P.kr == 0 || split) && !(flags & PP_CNTNB) && (a.flags & PP_RDF) && !ctx->no_sym) ? 1 : 0;
   a.cflag = ctx->cflag.as<uint8_t>();
-  if (a.sym) {
+  if (a.sym || near_ok) {
     CK(ctx->nc_pre.ensure((cl->g.ncells + 1) * 4));
     const uint64_t tmp_elems = (cl->g.ncells + 1) / 2048 + 64;
     CK(ctx->scan_tmp.ensure(tmp_elems * 8 * 2));
@@ -1519,7 +1684,8 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
           ak.counters = (unsigned long long*)(ctx->work.as<unsigned char>() + 16);
           ak.nbricks = (uint32_t)nb;
           ak.tile = 4;
-          rc = pp::launch_lanes_knn(ak, P.disjoint != 0, ctx->sm_count, &smem, s);
+          rc = near_ok ? run_near(ctx, *cl, P, type_counts.data(), R, ak, false, &smem, s) : -3;
+          if (rc == -3) rc = pp::launch_lanes_knn(ak, P.disjoint != 0, ctx->sm_count, &smem, s);
           ctx->last_kind = 4;
           if (rc == -3) {  // overlapping sets, or lists too large for shared memory
             ak.tile = a.tile;
@@ -1554,7 +1720,8 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
         a.nbricks = (uint32_t)nb;
         const uint32_t keep = a.tile;
         a.tile = 4;  // blocks per warp work item
-        rc = pp::launch_lanes_knn(a, P.disjoint != 0, ctx->sm_count, &smem, s);
+        rc = near_ok ? run_near(ctx, *cl, P, type_counts.data(), R, a, true, &smem, s) : -3;
+        if (rc == -3) rc = pp::launch_lanes_knn(a, P.disjoint != 0, ctx->sm_count, &smem, s);
         if (rc == 0) ctx->last_kind = 3;
         a.tile = keep;
       }
@@ -1955,6 +2122,11 @@ int pp_set_option(pp_ctx* ctx, const char* name, int value) {
   if (std::strcmp(name, "knn_lists") == 0) {
     if (value < 0 || value > 2) return fail(ctx, PP_ERR_INVALID, "knn_lists must be 0, 1 or 2");
     ctx->knn_lists = value;
+    return PP_OK;
+  }
+  if (std::strcmp(name, "knn_walks") == 0) {
+    if (value < 0 || value > 2) return fail(ctx, PP_ERR_INVALID, "knn_walks must be 0, 1 or 2");
+    ctx->knn_walks = value;
     return PP_OK;
   }
   if (std::strcmp(name, "npcorr_order") == 0) {

@@ -15,6 +15,8 @@ enum StatusBits : int {
   ST_TYPE_RANGE = 8,       // a type id had no slot where one was required
 };
 
+constexpr int kNearMax = 4;  // dense environment sets of a kNN pass in two walks
+
 // Uniform cell grid over a cloud's bounding box.  Cells are stored x-fastest
 // (cell = (z * ny + y) * nx + x) so the cells of one (y, z) row are
 // contiguous: a row of the stencil is one contiguous run of ions.
@@ -62,6 +64,22 @@ struct ScanArgs {
   const uint8_t* label_sorted;
   uint64_t n;
   float one;
+  // kNN passes in two walks (k_lanes_near): the dense sets, each with the
+  // radius its k-th neighbours are looked for in first and the stencil rows
+  // within it; near_map[set] = row of a sparse set's list, or ~(index) of a
+  // dense set; the ions of sparse sets as a list of their own in cell order
+  int near_n, near_sp;           // dense and sparse sets
+  int8_t near_map[16];
+  int near_set[kNearMax];
+  float near_r[kNearMax];
+  int near_rows[kNearMax];
+  int near_hot;                  // centre slot of most ions: its bins are kept in shared memory
+  int near_hd;                   // bins of its dense sets' shared histograms
+  int near_hs;                   // its sparse sets' bins are shared too
+  Grid sp_g;                     // the list's grid, coarser than g
+  const float4* sp_ions;
+  const uint32_t* sp_start;      // sp_g.ncells + 1
+  const uint32_t* sp_slot;
   // centre-per-lane scan: stencil rows of a block, (ry, rz) offsets from
   // (yb - bsr, zb - bsr), nearest to the block first; bsr rows each side
   const int16_t* brows;
@@ -259,6 +277,15 @@ void launch_count_occupied(const uint32_t* cell_start, uint64_t ncells, unsigned
 // every type in at most one environment set of each centre type
 // (ScanArgs::setidx valid); -3 = not applicable
 int launch_lanes_knn(const ScanArgs& a, bool disjoint_sets, int sm_count, size_t* smem_used, cudaStream_t s);
+// kNN-only passes in two walks (ScanArgs::near_*); -3 = not applicable.
+// sp_start, sp_cursor: sp_g.ncells + 1 words each; sp_tmp: exclusive-scan
+// scratch for as many; sp_cap: ions sp_ions / sp_slot have room for
+int launch_lanes_near(const ScanArgs& a, int sm_count, uint32_t* sp_start, uint32_t* sp_cursor, float4* sp_ions,
+                      uint32_t* sp_slot, uint32_t sp_cap, uint32_t* sp_tmp, uint64_t sp_tmp_elems, size_t* smem_used,
+                      cudaStream_t s);
+// the in-ball pairs (ScanArgs::counters) of a pass that need not bin them
+int launch_lanes_count(const ScanArgs& a, int sm_count, cudaStream_t s);
+void launch_type_count(const uint8_t* labels, uint64_t n, unsigned long long* out, int sm_count, cudaStream_t s);
 int launch_apply(const ApplyArgs& a, int sm_count, cudaStream_t s);
 // Batched kNN in two phases, 32 realisations per warp (one per lane).
 // Walk: per (centre, realisation) the category of the k-th member of every

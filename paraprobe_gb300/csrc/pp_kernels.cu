@@ -20,6 +20,7 @@
 // src/PARAPROBE_Histogram.h:97-117), so no double arithmetic runs per pair.
 
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <mutex>
@@ -583,6 +584,53 @@ __global__ void k_nc_count(const uint32_t* __restrict__ cell_start, uint64_t nce
       for (uint32_t j = cell_start[c]; j < cell_start[c + 1]; ++j) k += cflag[j] ? 0u : 1u;
     out[c] = k;
   }
+}
+
+// Sparse ions (pass code below `lim`) per cell of a grid of their own, and,
+// with the exclusive prefix of those counts in `cursor`, their records:
+// position, pass code in the fourth word, and their slots.
+__global__ void k_sparse_count(const float4* __restrict__ ions, uint64_t n, const uint32_t* __restrict__ code,
+                               uint32_t lim, Grid g, uint32_t* __restrict__ counts) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    if (code[i] >= lim) continue;
+    const float4 q = ions[i];
+    const uint32_t c = ((uint32_t)cell_coord(q.z, g.loz, g.inv_h, g.nz) * (uint32_t)g.ny +
+                        (uint32_t)cell_coord(q.y, g.loy, g.inv_h, g.ny)) * (uint32_t)g.nx +
+                       (uint32_t)cell_coord(q.x, g.lox, g.inv_h, g.nx);
+    atomicAdd(&counts[c], 1u);
+  }
+}
+__global__ void k_sparse_fill(const float4* __restrict__ ions, uint64_t n, const uint32_t* __restrict__ code,
+                              uint32_t lim, Grid g, uint32_t* __restrict__ cursor, uint32_t cap,
+                              float4* __restrict__ out, uint32_t* __restrict__ out_slot, int* status) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t k = code[i];
+    if (k >= lim) continue;
+    float4 q = ions[i];
+    const uint32_t c = ((uint32_t)cell_coord(q.z, g.loz, g.inv_h, g.nz) * (uint32_t)g.ny +
+                        (uint32_t)cell_coord(q.y, g.loy, g.inv_h, g.ny)) * (uint32_t)g.nx +
+                       (uint32_t)cell_coord(q.x, g.lox, g.inv_h, g.nx);
+    const uint32_t at = atomicAdd(&cursor[c], 1u);
+    if (at >= cap) {  // cannot happen: the host sized the list from the same labels
+      atomicOr(status, ST_BAD_SLOT);
+      continue;
+    }
+    q.w = __uint_as_float(k);
+    out[at] = q;
+    out_slot[at] = (uint32_t)i;
+  }
+}
+
+// Ions of each type id (256 counts, zeroed by the caller).
+__global__ void k_type_count(const uint8_t* __restrict__ labels, uint64_t n, unsigned long long* __restrict__ out) {
+  __shared__ uint32_t h[256];
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
+  __syncthreads();
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    atomicAdd(&h[labels[i]], 1u);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 256; i += blockDim.x)
+    if (h[i]) atomicAdd(&out[i], (unsigned long long)h[i]);
 }
 
 // Triangle binning for the hull distance: every cell of tg that a triangle's
@@ -1789,10 +1837,10 @@ __global__ void __launch_bounds__(256) k_brick(ScanArgs a) {
 
 // Ion range [st, st + len) of row r of the stencil of the cell block
 // [xb, xe) x [yb, ye) x [zb, ze): rows are (yy, zz) with yy in [yb - sr,
-// ye - 1 + sr] and zz in [zb - sr, ze - 1 + sr], row r at (yb - sr + ry,
-// zb - sr + rz) for (ry, rz) = a.brows[r] (nearest to the block first), each
-// trimmed in x to the cells within R of the batch's centre box [box[0],
-// box[1]] (world coordinates; no other cell holds a neighbour of these
+// ye - 1 + sr] and zz in [zb - sr, ze - 1 + sr] (sr = a.bsr), row r at (yb - sr
+// + ry, zb - sr + rz) for (ry, rz) = a.brows[r] (nearest to the block first),
+// each trimmed in x to the cells within R of the batch's centre box [box[0],
+// box[1]] (world coordinates; no other cell holds an ion within R of these
 // centres; margins of 1e-3 h and more cover the float evaluation and the
 // approximate root); len = 0 when the row holds none.
 // In symmetric mode a pair of two centres of different blocks is taken by the
@@ -1800,10 +1848,30 @@ __global__ void __launch_bounds__(256) k_brick(ScanArgs a) {
 // belongs to an earlier block, so its centres are not staged, and the row is
 // dropped (len = 0) when it holds nothing else; in a row of the block itself
 // the cells before xb are dropped when they hold only centres.
-__device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nrows, int sr, int xb, int yb, int ye,
-                                                int zb, int ze, bool sym, const float4* box, uint32_t& st,
-                                                uint32_t& len, bool& low) {
+struct LaneBlock {
+  int xb, xe, yb, ye, zb, ze;
+};
+// Cells [x0, x1] of grid row (yy, zz) within R of the box; false for none.
+__device__ __forceinline__ bool row_box_range(const Grid& g, float R, int yy, int zz, const float4* box, int& x0,
+                                              int& x1) {
+  const float m2 = 2.f * g.margin;
+  const float Rp = R + g.margin, Rp2 = Rp * Rp;
+  // the row's ions lie within margin of its cells [lo + c h, lo + (c + 1) h]
+  const float4 lo = box[0], hi = box[1];
+  const float ry0 = g.loy + (float)yy * g.h, rz0 = g.loz + (float)zz * g.h;
+  const float by = fmaxf(0.f, fmaxf(lo.y - (ry0 + g.h), ry0 - hi.y) - m2);
+  const float bz = fmaxf(0.f, fmaxf(lo.z - (rz0 + g.h), rz0 - hi.z) - m2);
+  const float brem = Rp2 - by * by - bz * bz;
+  if (brem < 0.f) return false;
+  const float bhalf = sqrt_approx(brem) + m2;
+  x0 = max(0, (int)floorf((lo.x - g.lox - bhalf) * g.inv_h));
+  x1 = min(g.nx - 1, (int)floorf((hi.x - g.lox + bhalf) * g.inv_h));
+  return x0 <= x1;
+}
+__device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nrows, float R, const LaneBlock& b, bool sym, const float4* box,
+                                                uint32_t& st, uint32_t& len, bool& low) {
   const Grid& g = a.g;
+  const int sr = a.bsr, xb = b.xb, yb = b.yb, ye = b.ye, zb = b.zb, ze = b.ze;
   st = 0;
   len = 0;
   low = false;
@@ -1811,19 +1879,8 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
   const int ry = a.brows[2 * r], rz = a.brows[2 * r + 1];
   const int yy = yb - sr + ry, zz = zb - sr + rz;
   if (yy < 0 || yy >= g.ny || zz < 0 || zz >= g.nz) return;
-  const float m2 = 2.f * g.margin;
-  const float Rp = a.R + g.margin, Rp2 = Rp * Rp;
-  // the row's ions lie within margin of its cells [lo + c h, lo + (c + 1) h]
-  const float4 lo = box[0], hi = box[1];
-  const float ry0 = g.loy + (float)yy * g.h, rz0 = g.loz + (float)zz * g.h;
-  const float by = fmaxf(0.f, fmaxf(lo.y - (ry0 + g.h), ry0 - hi.y) - m2);
-  const float bz = fmaxf(0.f, fmaxf(lo.z - (rz0 + g.h), rz0 - hi.z) - m2);
-  const float brem = Rp2 - by * by - bz * bz;
-  if (brem < 0.f) return;
-  const float bhalf = sqrt_approx(brem) + m2;
-  const int x0 = max(0, (int)floorf((lo.x - g.lox - bhalf) * g.inv_h));
-  const int x1 = min(g.nx - 1, (int)floorf((hi.x - g.lox + bhalf) * g.inv_h));
-  if (x1 < x0) return;
+  int x0, x1;
+  if (!row_box_range(g, R, yy, zz, box, x0, x1)) return;
   const uint64_t cb = ((uint64_t)zz * g.ny + yy) * g.nx;
   int xs = x0;
   if (sym) {
@@ -1878,24 +1935,27 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
 // An ion's pass code (ScanArgs::pcode, k_pass_codes) is staged as its record's
 // fourth word; in symmetric mode its lowest bit says that it is a centre and
 // is staged as 0.
-// lanes_walk calls, warp-uniformly,
+// lanes_blocks fetches work and calls, warp-uniformly,
 //   start(self)                a new batch; self = this lane's centre slot or
 //                              0xffffffff; returns the lane's centre position
 //                              (at infinity for no centre)
-//   batch(base, nb, keyed, self, cxx, cyy, czz)  tests of the nb staged ions at
-//                              base (places up to the next multiple of 8 hold
-//                              ions at infinity): self as above for live
-//                              lanes, the centre's coordinates as f32x2 pairs.
-//                              keyed: some of them lie in the block itself;
-//                              skey then holds the slots of those (in
-//                              symmetric mode of the centres among them), else
-//                              0xffffffff: symmetric passes take an ion when
-//                              its key exceeds self, others when it differs
-//   finish(live, tests)        after the batch's last staged ions; tests = the
-//                              (centre, staged ion) tests of the batch
-// Each pair of two centres is met once in symmetric mode (SYM): see
-// block_row_range for the pairs of different blocks; pairs within the block
-// are taken by the lower slot.
+//   body(batch)                the batch's pass over the ions around it
+// stage_rows walks the rows and cells within R of the batch's box, stages the
+// ions whose box distance squared is at most `bound` and calls
+//   run(base, nb, keyed)       tests of the nb staged ions at base (places up
+//                              to the next multiple of 8 hold ions at
+//                              infinity).  keyed: some of them lie in the
+//                              block itself; skey then holds the slots of
+//                              those (in symmetric mode of the centres among
+//                              them), else 0xffffffff: symmetric passes take
+//                              an ion when its key exceeds the lane's centre
+//                              slot, others when it differs
+// and returns how many ions it staged.  Each pair of two centres is met once
+// in symmetric mode (SYM): see block_row_range for the pairs of different
+// blocks; pairs within the block are taken by the lower slot.  MATCH: only
+// ions with pass code `match` are staged.  SPARSE: the ions of the sparse list
+// (ScanArgs::sp_*, codes in the records) on its own grid instead of all; skey
+// then holds every staged ion's slot, and nrows is not used.
 constexpr int kStage = 64;           // staged ions a warp has room for
 constexpr int kStageAll = kStage + 4;  // and one place (of a pair) for dropped candidates; keys stay 16-byte aligned
 
@@ -1907,7 +1967,10 @@ constexpr int kStageAll = kStage + 4;  // and one place (of a pair) for dropped 
 //   PC_ROW, PC_NIBBLE   k_lanes_knn: float row of the type's environment set
 //                       (param between rows), or that set for every centre
 //                       slot, 4 bits each; set a.emax = none
-enum PassCode { PC_KINDS, PC_CORES, PC_ROW, PC_NIBBLE };
+//   PC_NEAR             k_lanes_near: ScanArgs::near_map of the type's set
+//   PC_COUNT            k_lanes counting pairs: twice the pairs a neighbour is
+enum PassCode { PC_KINDS, PC_CORES, PC_ROW, PC_NIBBLE, PC_NEAR, PC_COUNT };
+constexpr uint32_t kNearDense = 0x80000000u, kNearNone = 0xffffffffu;
 __global__ void k_pass_codes(ScanArgs a, int kind, uint32_t param, uint32_t* __restrict__ out) {
   __shared__ uint32_t tab[512];
   for (int i = threadIdx.x; i < 512; i += blockDim.x) {
@@ -1923,6 +1986,11 @@ __global__ void k_pass_codes(ScanArgs a, int kind, uint32_t param, uint32_t* __r
     } else if (kind == PC_ROW) {
       const int si = a.nC > 0 ? a.setidx[ty] : -1;
       v = (uint32_t)(si < 0 ? a.emax : si) * param;
+    } else if (kind == PC_NEAR) {
+      const int si = a.nC > 0 ? a.setidx[ty] : -1;
+      v = si < 0 ? kNearNone : a.near_map[si] < 0 ? kNearDense | (uint32_t)(~a.near_map[si]) : (uint32_t)a.near_map[si] * param;
+    } else if (kind == PC_COUNT) {
+      v = jc ? 4u : 2u;
     } else {
       for (int q = 0; q < a.nC; ++q) {
         const int si = a.setidx[q * 256 + ty];
@@ -1940,20 +2008,151 @@ __device__ __forceinline__ float4 staged_ion(const float4* cand, int j) {
   return make_float4(f[0], f[2], f[4], f[6]);
 }
 
-template <bool SYM, class Start, class Batch, class Finish>
-__device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, float4* cand, uint32_t* skey, float4* sbox,
-                                                         Start start, Batch batch, Finish finish) {
-  const Grid& g = a.g;
+struct LaneBatch : LaneBlock {
+  uint32_t self;  // this lane's centre slot, 0xffffffff for none
+  uint32_t live;  // lanes with a centre
+  unsigned long long cxx, cyy, czz;  // its coordinates, each twice
+};
+
+template <bool SYM, bool MATCH, bool SPARSE, class Run>
+__device__ __forceinline__ uint32_t stage_rows(const ScanArgs& a, const LaneBatch& B, int nrows, float R, float bound,
+                                               uint32_t match, float4* cand, uint32_t* skey, const float4* sbox,
+                                               Run run) {
+  const Grid& g = SPARSE ? a.sp_g : a.g;
   const int lane = threadIdx.x & 31;
   const uint32_t lemask = (2u << lane) - 1u;
-  // rows up to sr cells away (in y or z) from the block can hold a neighbour
-  // (sr = floor((R + 3 margin) / h) + 1, computed by the host with the row table)
-  const int sr = a.bsr;
+  const float4* __restrict__ ions = SPARSE ? a.sp_ions : a.ions;
+  int sy0 = 0, sz0 = 0, sny = 1;  // SPARSE: the grid rows around the box
+  if constexpr (SPARSE) {
+    const float4 lo = sbox[0], hi = sbox[1];
+    const float ext = R + 2.f * g.margin;
+    sy0 = max(0, (int)floorf((lo.y - ext - g.loy) * g.inv_h));
+    sz0 = max(0, (int)floorf((lo.z - ext - g.loz) * g.inv_h));
+    sny = max(0, min(g.ny - 1, (int)floorf((hi.y + ext - g.loy) * g.inv_h)) - sy0 + 1);
+    nrows = sny * max(0, min(g.nz - 1, (int)floorf((hi.z + ext - g.loz) * g.inv_h)) - sz0 + 1);
+  }
+  auto put = [&](uint32_t p, const float4& q, uint32_t code) {
+    float* f = (float*)cand + (p >> 1) * 8 + (p & 1);
+    f[0] = q.x;
+    f[2] = q.y;
+    f[4] = q.z;
+    f[6] = __uint_as_float(code);
+  };
+  uint32_t base = 0;    // the half that fills: places [base, base + 32) of the ring
+  uint32_t fill = 0;    // staged ions waiting for a batch of tests (warp-uniform)
+  uint32_t staged = 0;
+  bool keyed = false;   // ions of the block itself wait
+  const int nown = max(a.by, 1) * max(a.bz, 1);  // the row table starts with the block's own rows
+  for (int r0 = 0; r0 < nrows; r0 += 32) {
+    uint32_t st, len;
+    bool low;
+    if constexpr (SPARSE) {
+      st = len = 0;
+      low = false;
+      const int r = r0 + lane, rz = r / sny;
+      int x0, x1;
+      if (r < nrows && row_box_range(g, R, sy0 + r - rz * sny, sz0 + rz, sbox, x0, x1)) {
+        const uint32_t cb = (uint32_t)((sz0 + rz) * g.ny + sy0 + r - rz * sny) * (uint32_t)g.nx;
+        st = a.sp_start[cb + x0];
+        len = a.sp_start[cb + x1 + 1] - st;
+      }
+    } else {
+      block_row_range(a, r0 + lane, nrows, R, B, SYM, sbox, st, len, low);
+    }
+    const uint32_t ne = __ballot_sync(FULL, len > 0);
+    const int cnt_rows = __popc(ne);
+    if (cnt_rows == 0) continue;
+    const uint32_t src = (lane < cnt_rows) ? nth_set(ne, (uint32_t)lane) : 0u;
+    const uint32_t rst = __shfl_sync(FULL, st, src);
+    uint32_t rlen = __shfl_sync(FULL, len, src);
+    // rows (compacted) that are the block's own, and of earlier blocks
+    const uint32_t ownm = SPARSE ? 0u : __ballot_sync(FULL, lane < cnt_rows && r0 + (int)src < nown);
+    const int lowc = SYM ? __shfl_sync(FULL, low ? 1 : 0, src) : 0;
+    const uint32_t lowm = SYM ? __ballot_sync(FULL, lane < cnt_rows && lowc != 0) : 0u;
+    if (lane >= cnt_rows) rlen = 0;
+    uint32_t inc = rlen;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(FULL, inc, o);
+      if (lane >= o) inc += t;
+    }
+    const uint32_t total = __shfl_sync(FULL, inc, 31);
+    // candidate t of these rows is slot t + first[its row]; exc = the
+    // row's first t (lanes without a row: never reached)
+    const uint32_t exc = lane < cnt_rows ? inc - rlen : 0xffffffffu;
+    const uint32_t first = rst - (inc - rlen);
+    int row0 = -1;  // last row that starts before this step
+    for (uint32_t bb = 0; bb < total; bb += 32) {
+      const uint32_t smask = __reduce_or_sync(FULL, shl_clamp(1u, exc - bb));
+      const int row = row0 + __popc(smask & lemask);
+      row0 += __popc(smask);
+      const uint32_t t = min(bb + lane, total - 1u);
+      const uint32_t slot = __shfl_sync(FULL, first, row) + t;
+      const float4 q = __ldg(ions + slot);
+      uint32_t code = SPARSE ? __float_as_uint(q.w) : __ldg(a.pcode + slot), key = 0xffffffffu;
+      const float4 lo = sbox[0], hi = sbox[1];
+      const float gx = fmaxf(fmaxf(__fsub_rn(lo.x, q.x), __fsub_rn(q.x, hi.x)), 0.f);
+      const float gy = fmaxf(fmaxf(__fsub_rn(lo.y, q.y), __fsub_rn(q.y, hi.y)), 0.f);
+      const float gz = fmaxf(fmaxf(__fsub_rn(lo.z, q.z), __fsub_rn(q.z, hi.z)), 0.f);
+      const float bd = __fadd_rn(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)), __fmul_rn(gz, gz));
+      bool keep = (bd <= bound) && bb + lane < total;
+      if (MATCH) keep = keep && code == match;
+      bool jc = false;
+      if (SYM) {
+        jc = (code & 1u) != 0;
+        code &= ~1u;
+        if (lowm) keep = keep && !(jc && ((lowm >> row) & 1u));
+      }
+      bool own_it = false;
+      if (ownm) {
+        // ions of the block's own rows: which cell (the expression of k_cell_count)
+        if ((ownm >> row) & 1u) {
+          const int cx = cell_coord(q.x, g.lox, g.inv_h, g.nx);
+          if (SYM) keep = keep && !(jc && cx < B.xb);
+          if (cx >= B.xb && cx < B.xe && (jc || !SYM)) key = slot;
+        }
+        own_it = __any_sync(FULL, keep && key != 0xffffffffu);
+        keyed |= own_it;
+      }
+      const uint32_t km = __ballot_sync(FULL, keep);
+      // dropped candidates go to a place past the ring
+      const uint32_t at = (base + fill + (uint32_t)__popc(km & (lemask >> 1))) & (uint32_t)(kStage - 1);
+      const uint32_t p = keep ? at : (uint32_t)kStage;
+      put(p, q, code);
+      if (SPARSE) skey[p] = a.sp_slot[slot];
+      else if (keyed || ownm) skey[p] = key;  // rows of the block come first, so earlier ions of a keyed half have keys
+      fill += (uint32_t)__popc(km);
+      if (fill >= 32u) {
+        __syncwarp();
+        run(base, 32u, keyed);
+        __syncwarp();
+        staged += 32u;
+        fill -= 32u;
+        base ^= 32u;
+        keyed = own_it;
+      }
+    }
+  }
+  if (fill > 0u) {
+    if (lane >= (int)fill && lane < (int)((fill + 7u) & ~7u)) {
+      put(base + lane, make_float4(kInf(), kInf(), kInf(), 0.f), 0u);  // no lane takes these
+      skey[base + lane] = 0u;
+    }
+    __syncwarp();
+    run(base, fill, keyed);
+    __syncwarp();
+    staged += fill;
+  }
+  return staged;
+}
+
+template <class Start, class Body>
+__device__ __forceinline__ void lanes_blocks(const ScanArgs& a, float4* sbox, Start start, Body body) {
+  const Grid& g = a.g;
+  const int lane = threadIdx.x & 31;
   const int BX = max(a.bx, 1), BY = max(a.by, 1), BZ = max(a.bz, 1);
-  const int nry = BY + 2 * sr, nrows = nry * (BZ + 2 * sr);
   const uint32_t nbx = (uint32_t)((g.nx + BX - 1) / BX), nby = (uint32_t)((g.ny + BY - 1) / BY);
   const uint32_t WT = max(a.tile, 1u);
-  unsigned long long tests = 0;  // (centre, staged ion) distance tests, warp-uniform
   for (;;) {
     uint32_t w0 = 0;
     if (lane == 0) w0 = atomicAdd(a.work, WT);
@@ -2010,7 +2209,6 @@ __device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, floa
         const bool lv = cp.x != kInf();
         const uint32_t live = __ballot_sync(FULL, lv);
         if (live) self = lv ? self : 0xffffffffu;
-        const unsigned long long cxx = f2_pack(cp.x, cp.x), cyy = f2_pack(cp.y, cp.y), czz = f2_pack(cp.z, cp.z);
         {
           // the live centres' bounding box (order-preserving keys: min and max
           // are exact), kept in shared memory: sbox[0] low, sbox[1] high corner
@@ -2026,111 +2224,20 @@ __device__ __forceinline__ unsigned long long lanes_walk(const ScanArgs& a, floa
           }
           __syncwarp();
         }
-        auto put = [&](uint32_t p, const float4& q, uint32_t code) {
-          float* f = (float*)cand + (p >> 1) * 8 + (p & 1);
-          f[0] = q.x;
-          f[2] = q.y;
-          f[4] = q.z;
-          f[6] = __uint_as_float(code);
-        };
-        uint32_t btests = 0;   // distance tests of this batch of centres
-        uint32_t base = 0;     // the half that fills: places [base, base + 32) of the ring
-        uint32_t fill = 0;     // staged ions waiting for a batch of tests (warp-uniform)
-        bool keyed = false;    // ... among them ions of the block itself
-        auto run_batch = [&](uint32_t nb) {
-          __syncwarp();
-          btests += (uint32_t)__popc(live) * nb;
-          batch(base, nb, keyed, self, cxx, cyy, czz);
-          __syncwarp();
-        };
-        const int nown = BY * BZ;  // the row table starts with the block's own rows
-        for (int r0 = 0; r0 < nrows && live; r0 += 32) {
-          uint32_t st, len;
-          bool low;
-          block_row_range(a, r0 + lane, nrows, sr, xb, yb, ye, zb, ze, SYM, sbox, st, len, low);
-          const uint32_t ne = __ballot_sync(FULL, len > 0);
-          const int cnt_rows = __popc(ne);
-          if (cnt_rows == 0) continue;
-          const uint32_t src = (lane < cnt_rows) ? nth_set(ne, (uint32_t)lane) : 0u;
-          const uint32_t rst = __shfl_sync(FULL, st, src);
-          uint32_t rlen = __shfl_sync(FULL, len, src);
-          // rows (compacted) that are the block's own, and of earlier blocks
-          const uint32_t ownm = __ballot_sync(FULL, lane < cnt_rows && r0 + (int)src < nown);
-          const int lowc = SYM ? __shfl_sync(FULL, low ? 1 : 0, src) : 0;
-          const uint32_t lowm = SYM ? __ballot_sync(FULL, lane < cnt_rows && lowc != 0) : 0u;
-          if (lane >= cnt_rows) rlen = 0;
-          uint32_t inc = rlen;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(FULL, inc, o);
-            if (lane >= o) inc += t;
-          }
-          const uint32_t total = __shfl_sync(FULL, inc, 31);
-          // candidate t of these rows is slot t + first[its row]; exc = the
-          // row's first t (lanes without a row: never reached)
-          const uint32_t exc = lane < cnt_rows ? inc - rlen : 0xffffffffu;
-          const uint32_t first = rst - (inc - rlen);
-          int row0 = -1;  // last row that starts before this step
-          for (uint32_t bb = 0; bb < total; bb += 32) {
-            const uint32_t smask = __reduce_or_sync(FULL, shl_clamp(1u, exc - bb));
-            const int row = row0 + __popc(smask & lemask);
-            row0 += __popc(smask);
-            const uint32_t t = min(bb + lane, total - 1u);
-            const uint32_t slot = __shfl_sync(FULL, first, row) + t;
-            const float4 q = __ldg(a.ions + slot);
-            uint32_t code = __ldg(a.pcode + slot), key = 0xffffffffu;
-            const float4 lo = sbox[0], hi = sbox[1];
-            const float gx = fmaxf(fmaxf(__fsub_rn(lo.x, q.x), __fsub_rn(q.x, hi.x)), 0.f);
-            const float gy = fmaxf(fmaxf(__fsub_rn(lo.y, q.y), __fsub_rn(q.y, hi.y)), 0.f);
-            const float gz = fmaxf(fmaxf(__fsub_rn(lo.z, q.z), __fsub_rn(q.z, hi.z)), 0.f);
-            const float bd = __fadd_rn(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)), __fmul_rn(gz, gz));
-            bool keep = (bd <= a.box_R2) && bb + lane < total;
-            bool jc = false;
-            if (SYM) {
-              jc = (code & 1u) != 0;
-              code &= ~1u;
-              if (lowm) keep = keep && !(jc && ((lowm >> row) & 1u));
-            }
-            bool own_it = false;
-            if (ownm) {
-              // ions of the block's own rows: which cell (the expression of k_cell_count)
-              if ((ownm >> row) & 1u) {
-                const int cx = cell_coord(q.x, g.lox, g.inv_h, g.nx);
-                if (SYM) keep = keep && !(jc && cx < xb);
-                if (cx >= xb && cx < xe && (jc || !SYM)) key = slot;
-              }
-              own_it = __any_sync(FULL, keep && key != 0xffffffffu);
-              keyed |= own_it;
-            }
-            const uint32_t km = __ballot_sync(FULL, keep);
-            // dropped candidates go to a place past the ring
-            const uint32_t at = (base + fill + (uint32_t)__popc(km & (lemask >> 1))) & (uint32_t)(kStage - 1);
-            const uint32_t p = keep ? at : (uint32_t)kStage;
-            put(p, q, code);
-            if (keyed || ownm) skey[p] = key;  // rows of the block come first, so earlier ions of a keyed half have keys
-            fill += (uint32_t)__popc(km);
-            if (fill >= 32u) {
-              run_batch(32u);
-              fill -= 32u;
-              base ^= 32u;
-              keyed = own_it;
-            }
-          }
+        if (live) {
+          LaneBatch B;
+          B.xb = xb; B.xe = xe; B.yb = yb; B.ye = ye; B.zb = zb; B.ze = ze;
+          B.self = self;
+          B.live = live;
+          B.cxx = f2_pack(cp.x, cp.x);
+          B.cyy = f2_pack(cp.y, cp.y);
+          B.czz = f2_pack(cp.z, cp.z);
+          body(B);
         }
-        if (fill > 0u) {
-          if (lane >= (int)fill && lane < (int)((fill + 7u) & ~7u)) {
-            put(base + lane, make_float4(kInf(), kInf(), kInf(), 0.f), 0u);  // no lane takes these
-            skey[base + lane] = 0u;
-          }
-          run_batch(fill);
-        }
-        tests += btests;
-        finish(live, btests);
         __syncwarp();
       }
     }
   }
-  return tests;
 }
 
 // Category guess of the centre-per-lane passes (ScanArgs::cat_fast: rmin = 0
@@ -2178,8 +2285,9 @@ struct FastCat {
 // ions without one.  A pair is one atomic, whatever it is credited to; the
 // credits and the pair count are worked out once per bin when the bins are
 // added to the global cores.  BINS = 1: shared bins in the layout of the
-// cores, up to two atomics a pair (twice the kinds do not fit); BINS = 0:
-// atomics on the cores.
+// cores, up to two atomics a pair (where the kinds do not fit); BINS = 0:
+// atomics on the cores; BINS = 3: no bins, the pass counts the in-ball pairs
+// of a kNN pass whose own walk does not meet them all (k_lanes_near).
 // Pass code of an ion: BINS 2 the byte offset of its row, others (env slot +
 // 1) << 1 | (centre slot + 1) << 9; the lowest bit set for centres in
 // symmetric mode.
@@ -2216,7 +2324,7 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
     ses[i] = e;
     if (c >= 0) sce[c] = e;  // slots and types are one to one
   }
-  if constexpr (BINS > 0)
+  if constexpr (BINS == 1 || BINS == 2)
     for (uint32_t i = threadIdx.x; i < nbin; i += blockDim.x) srdf[i] = 0;
   if (threadIdx.x == 0) *since_flush = 0ull;
   __syncthreads();
@@ -2330,11 +2438,39 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
       }
     }
   };
+  // BINS 3: only the number of in-ball pairs; the pass codes are twice the
+  // pairs one counts for
+  auto batch_count = [&](auto with_key, uint32_t base, uint32_t nb, uint32_t self, unsigned long long cxx,
+                         unsigned long long cyy, unsigned long long czz) {
+    constexpr bool WK = decltype(with_key)::value;
+    const uint2* key2 = (const uint2*)(skey + base);
+    const float4* cb = cand + base;
+#pragma unroll 1
+    for (uint32_t j0 = 0; j0 < nb; j0 += 8) {
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        const float4 c0 = cb[j0 + u], c1 = cb[j0 + u + 1];
+        float d0, d1;
+        dist2_x2(one, cxx, cyy, czz, f2_pack(c0.x, c0.y), f2_pack(c0.z, c0.w), f2_pack(c1.x, c1.y), d0, d1);
+        bool in0 = d0 <= R2, in1 = d1 <= R2;
+        if constexpr (WK) {
+          const uint2 kk = key2[(j0 + u) >> 1];
+          in0 = in0 && (SYM ? kk.x > self : kk.x != self);
+          in1 = in1 && (SYM ? kk.y > self : kk.y != self);
+        }
+        inb += in0 ? __float_as_uint(c1.z) : 0u;
+        inb += in1 ? __float_as_uint(c1.w) : 0u;
+      }
+    }
+  };
   auto batch = [&](uint32_t base, uint32_t nb, bool keyed, uint32_t self, unsigned long long cxx,
                    unsigned long long cyy, unsigned long long czz) {
     if constexpr (BINS == 2) {
       if (keyed) batch_kinds(std::true_type{}, base, nb, self, cxx, cyy, czz);
       else batch_kinds(std::false_type{}, base, nb, self, cxx, cyy, czz);
+    } else if constexpr (BINS == 3) {
+      if (keyed) batch_count(std::true_type{}, base, nb, self, cxx, cyy, czz);
+      else batch_count(std::false_type{}, base, nb, self, cxx, cyy, czz);
     } else {
 #pragma unroll 1
       for (uint32_t j = 0; j < nb; j += 2) {
@@ -2365,9 +2501,9 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
     }
   };
   auto finish = [&](uint32_t live, uint32_t btests) {
-    pairs_lane += inb;
+    pairs_lane += BINS == 3 ? inb >> 1 : inb;
     if (lane == 0) centres += (unsigned long long)__popc(live);
-    if constexpr (BINS > 0) {
+    if constexpr (BINS == 1 || BINS == 2) {
       // keep every shared bin below 2^32: a bin gains at most one count per
       // credit of a test; each time the block's tests cross a multiple of 2^30
       // the warp that crossed it moves all bins to the global uint64 cores
@@ -2382,11 +2518,21 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
       }
     }
   };
-  const unsigned long long tests = 
-      lanes_walk<SYM>(a, cand, skey, boxA + warp * 2, start, batch, finish);
+  unsigned long long tests = 0;  // (centre, staged ion) distance tests, warp-uniform
+  const float4* sbox = boxA + warp * 2;
+  const int nrows = (max(a.by, 1) + 2 * a.bsr) * (max(a.bz, 1) + 2 * a.bsr);
+  lanes_blocks(a, boxA + warp * 2, start, [&](const LaneBatch& B) {
+    const uint32_t staged = stage_rows<SYM, false, false>(
+        a, B, nrows, a.R, a.box_R2, 0u, cand, skey, sbox, [&](uint32_t base, uint32_t nb, bool keyed) {
+          batch(base, nb, keyed, B.self, B.cxx, B.cyy, B.czz);
+        });
+    const uint32_t btests = (uint32_t)__popc(B.live) * staged;
+    tests += btests;
+    finish(B.live, btests);
+  });
   if (lane == 0 && a.tests) atomicAdd(a.tests, tests);
   __syncthreads();
-  if constexpr (BINS > 0)
+  if constexpr (BINS == 1 || BINS == 2)
     for (uint32_t i = threadIdx.x; i < nbin; i += blockDim.x) {
       const uint32_t v = srdf[i];
       if (v) flush_bin(i, v);
@@ -2582,7 +2728,7 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
       insert(row_of(__float_as_uint(q.w)), d2);
     }
   };
-  auto finish = [&](uint32_t live, uint32_t) {
+  auto finish = [&](uint32_t live) {
     if (lane == 0) centres += (unsigned long long)__popc(live);
     // every live centre met itself once in the in-ball count (d^2 = 0)
     pairs_lane += inb - (me != 0xffffffffu ? 1u : 0u);
@@ -2616,8 +2762,17 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
       }
     }
   };
-  const unsigned long long tests =
-      lanes_walk<false>(a, cand, skey, boxA + warp * 2, start, batch, finish);
+  unsigned long long tests = 0;  // (centre, staged ion) distance tests, warp-uniform
+  const float4* sbox = boxA + warp * 2;
+  const int nrows = (max(a.by, 1) + 2 * a.bsr) * (max(a.bz, 1) + 2 * a.bsr);
+  lanes_blocks(a, boxA + warp * 2, start, [&](const LaneBatch& B) {
+    const uint32_t staged = stage_rows<false, false, false>(
+        a, B, nrows, a.R, a.box_R2, 0u, cand, skey, sbox, [&](uint32_t base, uint32_t nb, bool keyed) {
+          batch(base, nb, keyed, B.self, B.cxx, B.cyy, B.czz);
+        });
+    tests += (unsigned long long)__popc(B.live) * staged;
+    finish(B.live);
+  });
   if (lane == 0 && a.tests) atomicAdd(a.tests, tests);
 
   for (int o = 16; o; o >>= 1) pairs_lane += __shfl_xor_sync(FULL, pairs_lane, o);
@@ -2625,6 +2780,396 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
     atomicAdd(&a.counters[0], pairs_lane);
     atomicAdd(&a.counters[1], centres);
   }
+}
+
+// kNN passes in two walks, for uniform disjoint sets of which some are dense
+// (the matrix of an alloy): a dense set's k-th neighbours lie well within R, so
+// the ions of that set are walked within a radius r first chosen by the host
+// from the set's mean density (near_r, k_lanes_near), and only the ions of the
+// other, sparse sets -- a list of their own, a few per cent of the ions --
+// within R (k_lanes_sparse).  On the 20M-ion tip (k <= 10, R = 2 nm) a batch of
+// centres meets 0.29k ions instead of 1.3k.  Two kernels, not one with both
+// walks: together they miss the instruction cache (5.9 of 12.7 cycles per
+// instruction).  In-ball pairs are not counted by either (see run_near).
+//
+// Bins: most centres are of one type (near_hot), and adding its categories to
+// the cores in global memory took longer than finding them.  They are counted
+// in shared memory, a dense set's below near_hd in 32 bits each, a sparse set's
+// in 16 bits each, moved to the cores every 2^15 centres of the block; the
+// other centres' go to the cores.  Missing neighbours, most of the sparse
+// sets' orders, are counted once per set and centre, by the orders found.
+constexpr int kNearWarps = 24;  // most warps of a block; one block per SM
+
+// Rows (of 32 lanes) of a dense set's buffer: about 2 K and what eight tests add.
+__host__ __device__ constexpr int near_cap(int KB) { return 2 * KB + 28; }
+
+// The parts the two kernels share: tables in shared memory, categories, and
+// the counts of found orders.
+struct NearCommon {
+  const ScanArgs& a;
+  float* sT;
+  uint32_t* sfound;  // [centre slot][set][orders found]
+  int8_t* scs;
+  uint16_t* slut;
+  FastCat fc;
+  __device__ __forceinline__ NearCommon(const ScanArgs& a_, unsigned char*& sp) : a(a_), fc(a_) {
+    const int H = a.H;
+    sT = (float*)sp; sp += ((H + 4) & ~3) * 4;  // H thresholds, then +inf
+    const uint32_t nfound = (uint32_t)a.nC * a.emax * (a.nkI + 1);
+    sfound = (uint32_t*)sp; sp += (size_t)nfound * 4;
+    scs = (int8_t*)sp; sp += 256;
+    slut = (uint16_t*)sp;  // unless a.cat_fast
+    for (int i = threadIdx.x; i <= H; i += blockDim.x) sT[i] = i < H ? a.cat_T[i] : kInf();
+    for (uint32_t i = threadIdx.x; i < nfound; i += blockDim.x) sfound[i] = 0;
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) scs[i] = a.cslot_of[i];
+    if (!a.cat_fast)
+      for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
+  }
+  __device__ __forceinline__ int category_of(float d2) const {
+    if (!a.cat_fast) return category_lut(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT, a.H);
+    const int g = (int)(fc.guess4(d2) >> 2);
+    return g + (sT[g + 1] <= d2 ? 1 : 0);
+  }
+  __device__ __forceinline__ float4 start(uint32_t self, int& cs) const {
+    float4 cp = make_float4(kInf(), kInf(), kInf(), 0.f);
+    cs = -1;
+    if (self != 0xffffffffu) {
+      cp = a.ions[self];
+      const uint32_t ct = a.labels ? (uint32_t)a.labels[self] : __float_as_uint(cp.w);
+      cs = scs[ct & 255];
+      if (cs < 0) {  // selection guarantees a slot; record and drop the centre otherwise
+        atomicOr(a.status, ST_TYPE_RANGE);
+        cp = make_float4(kInf(), kInf(), kInf(), 0.f);
+      }
+    }
+    return cp;
+  }
+  __device__ __forceinline__ unsigned long long* core(int cs, int p) const {
+    return a.knn_core + ((uint64_t)cs * a.nS + a.set_list[cs * 32 + p]) * a.nkI * a.H;
+  }
+  __device__ __forceinline__ void found(int cs, int p, int orders) const {
+    if (orders < a.nkI) atomicAdd(&sfound[((uint32_t)cs * a.emax + p) * (a.nkI + 1) + orders], 1u);
+  }
+  // the missing orders' counts (after a block barrier)
+  __device__ __forceinline__ void flush_found() const {
+    if (a.cat_miss < 0) return;
+    const uint32_t nfound = (uint32_t)a.nC * a.emax * (a.nkI + 1);
+    for (uint32_t i = threadIdx.x; i < nfound; i += blockDim.x) {
+      const uint32_t v = sfound[i];
+      if (!v) continue;
+      const uint32_t f = i % (a.nkI + 1), p = (i / (a.nkI + 1)) % a.emax, c = i / (a.nkI + 1) / a.emax;
+      for (int kk = f; kk < a.nkI; ++kk)  // found the first f orders: the rest are missing
+        atomicAdd(&core(c, p)[(uint64_t)kk * a.H + a.cat_miss], (unsigned long long)v);
+    }
+  }
+};
+static size_t near_common_smem(const ScanArgs& a) {
+  return (size_t)((a.H + 4) & ~3) * 4 + (size_t)a.nC * a.emax * (a.nkI + 1) * 4 + 256 +
+         (a.cat_fast ? 0 : (size_t)((a.lut_n + 7) & ~7) * 2);
+}
+
+// The K <= KB smallest of the cnt values L[i * 32] of each lane, ascending
+// (+inf: none), in v[KB - K .. KB): the places before hold -inf, so that the
+// K-th smallest is always v[KB - 1] and the array stays in registers.
+template <int KB>
+__device__ __forceinline__ void near_smallest(const float* L, int cnt, int K, float (&v)[KB]) {
+#pragma unroll
+  for (int q = 0; q < KB; ++q) v[q] = q < KB - K ? -kInf() : kInf();
+  const int most = (int)__reduce_max_sync(FULL, (uint32_t)cnt);
+  for (int i = 0; i < most; ++i) {
+    const float x = i < cnt ? L[i * 32] : kInf();
+#pragma unroll
+    for (int q = KB - 1; q > 0; --q) v[q] = fminf(v[q], fmaxf(v[q - 1], x));
+    v[0] = fminf(v[0], x);
+  }
+}
+
+// Dense sets, one at a time.  A lane appends every d^2 below r^2 to a buffer
+// of its own in shared memory (an unordered column, no insertion in the test
+// loop), shrinks it to the K smallest if it fills, and takes the K smallest
+// once at the end with a min/max network in registers.  If at least K ions lie
+// within r these are its neighbours; the lanes of the others walk again with
+// 1.5 r, up to R (every ion within r of a lane's centre is within r of the
+// batch's box).
+template <int KB>
+__global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_near(ScanArgs a) {
+  constexpr int CAP = near_cap(KB);
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int H = a.H, K = a.kmax, HD = a.near_hd, nkI = a.nkI;
+  const int NW = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned char* sp = smem;
+  float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
+  float4* boxA = (float4*)sp; sp += NW * 2 * 16;
+  uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
+  float* listA = (float*)sp; sp += (size_t)NW * CAP * 32 * 4;
+  const uint32_t nhist = (uint32_t)a.near_n * nkI * HD;  // the hot centre slot's [set][order][HD]
+  uint32_t* shist = (uint32_t*)sp; sp += (size_t)nhist * 4;
+  for (uint32_t i = threadIdx.x; i < nhist; i += blockDim.x) shist[i] = 0;
+  const NearCommon nc(a, sp);
+  __syncthreads();
+  float4* cand = candA + warp * kStageAll;
+  uint32_t* skey = skeyA + warp * kStageAll;
+  float* L = listA + (size_t)warp * CAP * 32 + lane;
+  const float RUP = (a.R2 >= 0.f && a.R2 < kInf()) ? __uint_as_float(__float_as_uint(a.R2) + 1u) : kInf();
+  unsigned long long centres = 0, tests = 0;
+  int cs = -1;
+  const unsigned long long one = f2_pack(a.one, a.one);
+  const float4* sbox = boxA + warp * 2;
+  const int nrows = (max(a.by, 1) + 2 * a.bsr) * (max(a.bz, 1) + 2 * a.bsr);
+  const uint32_t buf = smem_addr(L);
+
+  lanes_blocks(a, boxA + warp * 2, [&](uint32_t self) { return nc.start(self, cs); }, [&](const LaneBatch& B) {
+    if (lane == 0) centres += (unsigned long long)__popc(B.live);
+    for (int dn = 0; dn < a.near_n; ++dn) {
+      bool need = cs >= 0;
+      float r = a.near_r[dn];
+      int rows = a.near_rows[dn];
+      for (;;) {
+        const bool full = !(r < a.R);
+        const float r2 = __fmul_rn(r, r);
+        float thr = !need ? -kInf() : full ? RUP : r2;
+        uint32_t at = buf;  // where this lane's next value goes
+        const uint32_t staged = stage_rows<false, true, false>(
+            a, B, rows, full ? a.R : r, full ? a.box_R2 : r2 * (1.f + 1.f / 4096.f), kNearDense | (uint32_t)dn, cand,
+            skey, sbox, [&](uint32_t base, uint32_t nb, bool keyed) {
+              const float4* cb = cand + base;
+#pragma unroll 1
+              for (uint32_t j0 = 0; j0 < nb; j0 += 8) {
+                float d[8];
+#pragma unroll
+                for (int u = 0; u < 8; u += 2) {
+                  const float4 c0 = cb[j0 + u];
+                  const float2 c1 = *(const float2*)&cb[j0 + u + 1];
+                  dist2_x2(one, B.cxx, B.cyy, B.czz, f2_pack(c0.x, c0.y), f2_pack(c0.z, c0.w), f2_pack(c1.x, c1.y),
+                           d[u], d[u + 1]);
+                }
+                if (keyed) {  // not the centre itself
+                  const uint4* k4 = (const uint4*)(skey + base + j0);
+                  const uint4 k0 = k4[0], k1 = k4[1];
+                  const uint32_t kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+#pragma unroll
+                  for (int u = 0; u < 8; ++u)
+                    if (kk[u] == B.self) d[u] = kInf();
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                  asm volatile("{\n\t.reg .pred p;\n\t"
+                               "setp.lt.f32 p, %1, %2;\n\t"
+                               "@p st.shared.f32 [%0], %1;\n\t"
+                               "@p add.u32 %0, %0, 128;\n\t}"
+                               : "+r"(at) : "f"(d[u]), "f"(thr) : "memory");
+                if (__any_sync(FULL, at > buf + (uint32_t)(CAP - 8) * 128u)) {
+                  // full: keep the K smallest and take only smaller ones from here on
+                  float w[KB];
+                  const int cnt = (int)((at - buf) >> 7);
+                  near_smallest<KB>(L, cnt, K, w);
+#pragma unroll
+                  for (int q = 0; q < KB; ++q)
+                    if (q >= KB - K && q < KB - K + cnt) L[(q - (KB - K)) * 32] = w[q];
+                  at = buf + (uint32_t)min(cnt, K) * 128u;
+                  thr = fminf(thr, w[KB - 1]);
+                }
+              }
+            });
+        tests += (unsigned long long)__popc(B.live) * staged;
+        const int cnt = (int)((at - buf) >> 7);
+        float v[KB];
+        near_smallest<KB>(L, cnt, K, v);
+        const bool done = need && (full || v[KB - 1] < kInf());
+        if (done) {
+          // through the lane's column, so that the loop over orders is not unrolled
+#pragma unroll
+          for (int q = 0; q < KB; ++q)
+            if (q >= KB - K) L[(q - (KB - K)) * 32] = v[q];
+          const int p = a.near_set[dn], hd = cs == a.near_hot ? HD : 0;
+          unsigned long long* core = nc.core(cs, p);
+          uint32_t* h = shist + (uint32_t)dn * nkI * HD;
+          int kk = 0;
+          for (; kk < nkI; ++kk) {
+            const int k = a.kvals[kk];
+            if (k > cnt) break;
+            const int cat = nc.category_of(L[(k - 1) * 32]);
+            if (cat < hd) atomicAdd(&h[(uint32_t)kk * HD + cat], 1u);
+            else atomicAdd(&core[(uint64_t)kk * H + cat], 1ull);
+          }
+          nc.found(cs, p, kk);
+        }
+        need = need && !done;
+        __syncwarp();
+        if (!__any_sync(FULL, need)) break;
+        r *= 1.5f;
+        if (r > 0.8f * a.R) r = a.R;
+        rows = nrows;
+      }
+    }
+  });
+
+  if (lane == 0) {
+    atomicAdd(&a.counters[1], centres);
+    if (a.tests) atomicAdd(a.tests, tests);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nhist; i += blockDim.x) {
+    const uint32_t v = shist[i];
+    if (!v) continue;
+    const uint32_t b = i % HD, kk = (i / HD) % nkI, dn = i / HD / nkI;
+    atomicAdd(&nc.core(a.near_hot, a.near_set[dn])[(uint64_t)kk * H + b], (unsigned long long)v);
+  }
+  nc.flush_found();
+}
+
+// Sparse sets together: threshold test and sorted insertion as in k_lanes_knn
+// (CAT: the lists hold categories), over the sparse list.
+template <int KB, bool CAT>
+__global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_sparse(ScanArgs a) {
+  constexpr uint32_t CNONE = 0xffffu;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int H = a.H, K = a.kmax, SPN = a.near_sp, nkI = a.nkI;
+  const int NW = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int frows = CAT ? SPN : SPN * K, lrows = frows + (CAT ? (SPN * K + 1) / 2 : 0);
+  unsigned char* sp = smem;
+  float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
+  float4* boxA = (float4*)sp; sp += NW * 2 * 16;
+  uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
+  float* listA = (float*)sp; sp += (size_t)NW * lrows * 32 * 4;
+  // the hot centre slot's bins [set][order][H], halfwords; centres taken
+  const uint32_t nhalf = a.near_hs ? ((uint32_t)SPN * nkI * H + 1) / 2 : 0u;
+  uint32_t* sflush = (uint32_t*)sp; sp += 16;
+  uint32_t* shalf = (uint32_t*)sp; sp += (size_t)nhalf * 4;
+  for (uint32_t i = threadIdx.x; i < nhalf; i += blockDim.x) shalf[i] = 0;
+  if (threadIdx.x == 0) *sflush = 0;
+  const NearCommon nc(a, sp);
+  __syncthreads();
+  float4* cand = candA + warp * kStageAll;
+  uint32_t* skey = skeyA + warp * kStageAll;
+  float* L = listA + (size_t)warp * lrows * 32 + lane;
+  uint16_t* C = (uint16_t*)(listA + (size_t)warp * lrows * 32 + frows * 32) + lane;
+  const float RUP = (a.R2 >= 0.f && a.R2 < kInf()) ? __uint_as_float(__float_as_uint(a.R2) + 1u) : kInf();
+  unsigned long long tests = 0;
+  int cs = -1;
+  const unsigned long long one = f2_pack(a.one, a.one);
+  const float4* sbox = boxA + warp * 2;
+
+  // moves the halfword bins to the cores; word i holds bins 2 i and 2 i + 1
+  auto flush_half = [&](int from, int step) {
+    for (uint32_t i = from; i < nhalf; i += step) {
+      const uint32_t v = atomicExch(&shalf[i], 0u);
+      for (int u = 0; u < 2; ++u) {
+        const uint32_t cnt = u ? v >> 16 : v & 0xffffu;
+        if (!cnt) continue;
+        const uint32_t j = 2 * i + u, b = j % (uint32_t)H, kk = (j / (uint32_t)H) % nkI, m = j / (uint32_t)H / nkI;
+        int p = 0;
+        while (p < a.emax && a.near_map[p] != (int)m) ++p;
+        atomicAdd(&nc.core(a.near_hot, p)[(uint64_t)kk * H + b], (unsigned long long)cnt);
+      }
+    }
+  };
+  lanes_blocks(a, boxA + warp * 2, [&](uint32_t self) { return nc.start(self, cs); }, [&](const LaneBatch& B) {
+    if constexpr (CAT) {
+      for (int p = 0; p < SPN; ++p) L[p * 32] = RUP;
+      for (int e = 0; e < SPN * K; ++e) C[e * 32] = (uint16_t)CNONE;
+    } else {
+      for (int e = 0; e < SPN * K; ++e) L[e * 32] = RUP;
+    }
+    float cx, cy, cz, dup;
+    f2_unpack(B.cxx, cx, dup);
+    f2_unpack(B.cyy, cy, dup);
+    f2_unpack(B.czz, cz, dup);
+    // sorted insertion, largest first (see k_lanes_knn)
+    auto insert = [&](uint32_t row, float d2) {
+      float* Lp = L + row;
+      if (!(d2 < Lp[0])) return;
+      if constexpr (CAT) {
+        const int c = nc.category_of(d2);
+        uint16_t* Cp = C + (row / 32u) * (uint32_t)K * 32u;
+        int v[KB];
+#pragma unroll
+        for (int q = 0; q < KB; ++q) v[q] = (q < K) ? (int)Cp[q * 32] : -1;
+#pragma unroll
+        for (int q = 0; q < KB; ++q)
+          if (q < K) v[q] = min(v[q], max(q + 1 < KB ? v[q + 1 < KB ? q + 1 : q] : -1, c));
+#pragma unroll
+        for (int q = 0; q < KB; ++q)
+          if (q < K) Cp[q * 32] = (uint16_t)v[q];
+        Lp[0] = (v[0] == (int)CNONE) ? RUP : nc.sT[v[0]];
+      } else {
+        float v[KB];
+#pragma unroll
+        for (int q = 0; q < KB; ++q) v[q] = (q < K) ? Lp[q * 32] : -kInf();
+#pragma unroll
+        for (int q = 0; q < KB; ++q)
+          if (q < K) Lp[q * 32] = fminf(v[q], fmaxf(q + 1 < KB ? v[q + 1 < KB ? q + 1 : q] : -kInf(), d2));
+      }
+    };
+    const uint32_t staged = stage_rows<false, false, true>(
+        a, B, 0, a.R, a.box_R2, 0u, cand, skey, sbox, [&](uint32_t base, uint32_t nb, bool) {
+          const float4* cb = cand + base;
+          uint32_t tm = 0;
+#pragma unroll 1
+          for (uint32_t j0 = 0; j0 < nb; j0 += 8) {
+            uint32_t m8 = 0;
+#pragma unroll
+            for (int u = 0; u < 8; u += 2) {
+              const float4 c0 = cb[j0 + u], c1 = cb[j0 + u + 1];
+              float d0, d1;
+              dist2_x2(one, B.cxx, B.cyy, B.czz, f2_pack(c0.x, c0.y), f2_pack(c0.z, c0.w), f2_pack(c1.x, c1.y), d0, d1);
+              m8 |= d0 < L[__float_as_uint(c1.z)] ? (1u << u) : 0u;
+              m8 |= d1 < L[__float_as_uint(c1.w)] ? (2u << u) : 0u;
+            }
+            tm |= m8 << j0;
+          }
+          while (tm) {
+            const int j = __ffs(tm) - 1;
+            tm &= tm - 1u;
+            const float4 q = staged_ion(cb, j);
+            if (skey[base + j] == B.self) continue;  // the centre itself
+            insert(__float_as_uint(q.w), dist2(cx, cy, cz, q.x, q.y, q.z));
+          }
+        });
+    tests += (unsigned long long)__popc(B.live) * staged;
+    const int nset = cs >= 0 ? a.nsets[cs] : 0;
+    const bool hot = a.near_hs && cs == a.near_hot;
+    for (int p = 0; p < nset; ++p) {
+      const int m = a.near_map[p];
+      if (m < 0) continue;
+      unsigned long long* core = nc.core(cs, p);
+      int kk = 0;
+      for (; kk < nkI; ++kk) {  // orders ascend: the first one missing ends them
+        const int row = m * K + K - a.kvals[kk];
+        int cat;
+        if constexpr (CAT) {
+          cat = C[row * 32];
+          if (cat == (int)CNONE) break;
+        } else {
+          const float v = L[row * 32];
+          if (v == RUP) break;
+          cat = nc.category_of(v);
+        }
+        if (hot) {
+          const uint32_t i = ((uint32_t)m * nkI + kk) * H + cat;
+          atomicAdd(&shalf[i >> 1], (i & 1u) ? 0x10000u : 1u);
+        } else {
+          atomicAdd(&core[(uint64_t)kk * H + cat], 1ull);
+        }
+      }
+      nc.found(cs, p, kk);
+    }
+    if (a.near_hs) {
+      // a halfword gains at most one count a centre: empty them before 2^16
+      const uint32_t n = (uint32_t)__popc(B.live);
+      uint32_t old = 0;
+      if (lane == 0) old = atomicAdd(sflush, n);
+      old = __shfl_sync(FULL, old, 0);
+      if ((old >> 15) != ((old + n) >> 15)) flush_half(lane, 32);
+    }
+    __syncwarp();
+  });
+  if (lane == 0 && a.tests) atomicAdd(a.tests, tests);
+  __syncthreads();
+  flush_half(threadIdx.x, blockDim.x);
+  nc.flush_found();
 }
 
 // --------------------------------------------------------------- K5 batched
@@ -3578,6 +4123,87 @@ int launch_lanes(const ScanArgs& a, int kr, int sm_count, size_t* smem_used, cud
   launch_pass_codes(a, bins == 2 ? PC_KINDS : PC_CORES, 0, sm_count, s);
   counted();
   kern<<<sm_count, kLanesWarps * 32, smem, s>>>(a);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_lanes_count(const ScanArgs& a, int sm_count, cudaStream_t s) {
+  if (a.mode != 0 || a.bx < 1 || a.by < 1 || a.bz < 1 || !a.brows) return -3;
+  const size_t smem = lanes_smem(a, 0, true);
+  if (smem > 224 * 1024) return -3;
+  auto kern = a.sym ? k_lanes<true, 3, true> : k_lanes<false, 3, true>;
+  if (!allow_dynamic_smem((const void*)kern, smem)) return -1;
+  launch_pass_codes(a, PC_COUNT, 0, sm_count, s);
+  counted();
+  kern<<<sm_count, kLanesWarps * 32, smem, s>>>(a);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+void launch_type_count(const uint8_t* labels, uint64_t n, unsigned long long* out, int sm_count, cudaStream_t s) {
+  counted();
+  const uint64_t blocks = (n + 4095) / 4096;
+  k_type_count<<<(unsigned)(blocks < (uint64_t)sm_count * 4 ? (blocks ? blocks : 1) : (uint64_t)sm_count * 4), 256, 0, s>>>(
+      labels, n, out);
+}
+
+int launch_lanes_near(const ScanArgs& a0, int sm_count, uint32_t* sp_start, uint32_t* sp_cursor, float4* sp_ions,
+                      uint32_t* sp_slot, uint32_t sp_cap, uint32_t* sp_tmp, uint64_t sp_tmp_elems, size_t* smem_used,
+                      cudaStream_t s) {
+  ScanArgs a = a0;
+  if (a.mode != 0 || (a.flags & (PP_CNTNB | PP_RDF)) || !a.uniform_sets || a.kmax < 1 || a.kmax > 20 || a.bx < 1 ||
+      a.by < 1 || a.bz < 1 || !a.brows || a.nC > 127 || a.emax > 15 || a.near_n < 1 || a.near_n > kNearMax)
+    return -3;
+  const int KB = a.kmax <= 8 ? 8 : a.kmax <= 10 ? 10 : a.kmax <= 16 ? 16 : 20;
+  const size_t cap = 224 * 1024, common = near_common_smem(a), stage = (size_t)kStageAll * 20 + 32;
+  // the hot centre type's shared bins while they leave the warps room
+  a.near_hs = a.near_sp > 0 && ((size_t)a.near_sp * a.nkI * a.H + 1) / 2 * 4 <= 90 * 1024 ? 1 : 0;
+  if ((size_t)a.near_n * a.nkI * a.near_hd * 4 > 64 * 1024) a.near_hd = 0;
+  const size_t fix_d = common + (size_t)a.near_n * a.nkI * a.near_hd * 4;
+  const size_t fix_s = common + 16 + (a.near_hs ? ((size_t)a.near_sp * a.nkI * a.H + 1) / 2 * 4 : 0);
+  auto sparse_warp = [&](bool cat) {
+    const int frows = cat ? a.near_sp : a.near_sp * a.kmax;
+    return stage + (size_t)(frows + (cat ? (a.near_sp * a.kmax + 1) / 2 : 0)) * 128;
+  };
+  auto warps = [&](size_t fix, size_t each) {
+    return fix >= cap ? 0 : (int)std::min<size_t>(kNearWarps, (cap - fix) / each);
+  };
+  // category lists for the sparse sets where distances would leave fewer than
+  // 16 warps
+  const bool cat = a.lists_mode == 2 || (a.lists_mode == 0 && warps(fix_s, sparse_warp(false)) < 16 &&
+                                         warps(fix_s, sparse_warp(true)) > warps(fix_s, sparse_warp(false)));
+  const size_t dense_warp = stage + (size_t)near_cap(KB) * 128;
+  const int wd = warps(fix_d, dense_warp), ws = a.near_sp > 0 ? warps(fix_s, sparse_warp(cat)) : 4;
+  if (wd < 4 || ws < 4 || (cat && a.H > 65535)) return -3;
+  const size_t smem_d = fix_d + dense_warp * wd, smem_s = fix_s + sparse_warp(cat) * ws;
+  if (smem_used) *smem_used = std::max(smem_d, smem_s);
+  launch_pass_codes(a, PC_NEAR, cat ? 32u : (uint32_t)a.kmax * 32u, sm_count, s);
+  if (a.near_sp > 0) {
+    const uint64_t cells = a.sp_g.ncells;
+    if (cudaMemsetAsync(sp_start, 0, (cells + 1) * 4, s) != cudaSuccess) return -1;
+    counted();
+    k_sparse_count<<<grid_for(a.n, 256), 256, 0, s>>>(a.ions, a.n, a.pcode, kNearDense, a.sp_g, sp_start);
+    excl_scan<uint32_t>(sp_start, cells + 1, sp_tmp, sp_tmp_elems, s);
+    if (cudaMemcpyAsync(sp_cursor, sp_start, (cells + 1) * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return -1;
+    counted();
+    k_sparse_fill<<<grid_for(a.n, 256), 256, 0, s>>>(a.ions, a.n, a.pcode, kNearDense, a.sp_g, sp_cursor, sp_cap, sp_ions,
+                                                     sp_slot, a.status);
+  }
+  a.sp_start = sp_start;
+  a.sp_ions = sp_ions;
+  a.sp_slot = sp_slot;
+  auto dense = KB == 8 ? k_lanes_near<8> : KB == 10 ? k_lanes_near<10> : KB == 16 ? k_lanes_near<16> : k_lanes_near<20>;
+  if (!allow_dynamic_smem((const void*)dense, smem_d)) return -1;
+  counted();
+  dense<<<sm_count, wd * 32, smem_d, s>>>(a);
+  if (a.near_sp > 0) {
+    auto sparse = KB == 8    ? (cat ? k_lanes_sparse<8, true> : k_lanes_sparse<8, false>)
+                  : KB == 10 ? (cat ? k_lanes_sparse<10, true> : k_lanes_sparse<10, false>)
+                  : KB == 16 ? (cat ? k_lanes_sparse<16, true> : k_lanes_sparse<16, false>)
+                             : (cat ? k_lanes_sparse<20, true> : k_lanes_sparse<20, false>);
+    if (!allow_dynamic_smem((const void*)sparse, smem_s)) return -1;
+    a.work = a.work + 1;
+    counted();
+    sparse<<<sm_count, ws * 32, smem_s, s>>>(a);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -69,3 +69,48 @@ def test_lanes_pairs_on_bin_edges(ctx, oracle):
     for got, s, flags, ks in ((rdf, st, N.PP_RDF, []), (knn, st2, N.PP_MKNN, [7, 3, 1])):
         ref = oracle.spatstat(xyz, labels, surf, *hist, flags, trg, env, ks)
         assert s["pairs"] == ref["pairs"] and np.array_equal(got, ref["bins"])
+
+
+@pytest.mark.parametrize("ks", [[1], [8, 3], [9, 1], [10, 5, 1], [16, 2], [20, 19, 1]])
+@pytest.mark.parametrize("fractions", [(0.97, 0.02, 0.01), (0.5, 0.45, 0.05), (0.999, 0.001, 0.0)])
+@pytest.mark.parametrize("lists,rmin", [(0, 0.0), (2, 0.0), (0, 0.05)])
+def test_knn_in_two_walks(ctx, oracle, ks, fractions, lists, rmin):
+    """Dense sets within a first radius, sparse sets from their own list: every
+    list size class, one or two dense sets, sets without ions, both list forms,
+    table categories; clusters and a hole make centres that need more than the
+    first radius; coincident ions and masked centres."""
+    spec = synth.cylinder_specimen(n=24000, radius=3.0, height=18.0, fractions=fractions, seed=7 + len(ks), nseg=48,
+                                   stack=4.0)
+    xyz = spec.xyz.copy()
+    inside = np.linalg.norm(xyz - np.array([0, 0, 9.0], dtype=np.float32), axis=1) < 1.1
+    keep = ~inside | (np.arange(len(xyz)) % 40 == 0)  # a nearly empty ball: few neighbours within the first radius
+    xyz, labels = xyz[keep], spec.labels[keep]
+    xyz[:200] = xyz[200:400]
+    types = [1, 2, 3]
+    trg, env = [[a] for a in types for b in types], [[b] for a in types for b in types]
+    hist = (rmin, 0.01, 1.5)
+    n = len(xyz)
+    mask = (np.arange(n) % 7 != 0).astype(np.uint8)
+    cid = ctx.upload(xyz, labels)
+    ctx.surfdist(cid, np.where(np.arange(n) % 11 == 0, 1.0, 10.0).astype(np.float32))
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.set_option("knn_lists", lists)
+    ctx.set_option("knn_walks", 2)
+    try:
+        ctx.run(cid, N.PP_MKNN, ks)
+        got, st, kernel = ctx.fetch(), ctx.stats(), ctx.last_kernel()
+        ctx.run(cid, N.PP_MKNN, ks, centre_mask=mask)
+        part, stp = ctx.fetch(), ctx.stats()
+        ctx.run(cid, N.PP_MKNN, ks, centre_mask=1 - mask)
+        rest, str_ = ctx.fetch(), ctx.stats()
+    finally:
+        ctx.set_option("knn_lists", 0)
+        ctx.set_option("knn_walks", 0)
+        ctx.free(cid)
+    assert kernel == "k_lanes_knn"
+    surf = np.where(np.arange(n) % 11 == 0, 1.0, 10.0).astype(np.float32)
+    ref = oracle.spatstat(xyz, labels, surf, *hist, N.PP_MKNN, trg, env, ks)
+    assert st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
+    assert np.array_equal(got, ref["bins"])
+    assert np.array_equal(part + rest, got) and stp["pairs"] + str_["pairs"] == st["pairs"]
