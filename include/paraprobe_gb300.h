@@ -189,13 +189,11 @@ int pp_run_aposteriori(pp_ctx* ctx, int cloud, const uint8_t* clustered, uint32_
 /* Project-written autotuner: times the pass on about `sample` centres
  * (0 = 200000; at least 8192 per SM, so that every kernel form fills the GPU)
  * for cell edges R/2 .. R/5 -- for passes the centre-per-lane
- * scan takes, at the default cell block of that edge (about a warp of
- * centres) and two fixed shapes; for other passes with the per-centre scan at
- * block tiles of 32, 128 and 512 centres and with the brick scan at bricks of
- * 4, 8 and 16 cells, and for passes with RDF / RIPK and kNN together (no
- * CNTNB or NPCORR) of dense centres also as two centre-per-lane passes at
- * those cell blocks -- keeps the fastest for this
- * cloud and rebuilds its cell grid.  best_tile comes back in the
+ * scans take, at two fixed cell blocks (for passes with RDF / RIPK and kNN
+ * together also at the default block of that edge, about a warp of centres);
+ * for other passes with the per-centre scan at block tiles of 32, 128 and 512
+ * centres and with the brick scan at bricks of 4, 8 and 16 cells -- keeps the
+ * fastest for this cloud and rebuilds its cell grid.  best_tile comes back in the
  * pp_cloud_tuning encoding.  Uses the current tasks and histogram settings;
  * results of the trial runs are discarded.  Has no counterpart in the
  * reference (its KD-tree has no tuning). */
@@ -208,15 +206,16 @@ int pp_autotune(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_list, 
  * for passes without CNTNB whose kNN, if any, has k <= 32 and disjoint
  * environment sets; other passes use the per-centre scan);
  * ((bx | by << 8 | bz << 12) << 16) | PP_TILE_LANES with bx in 1..64 and by,
- * bz in 0..15 (0 = 1) = blocks of bx x by x bz cells for the centre-per-lane
- * scan that RDF / RIPK passes without CNTNB take (one centre per lane, the
- * block's stencil ions staged in shared memory; default 4 x 2 x 2), leaving
- * the other code as it was.  With a cell block set this way, a pass with
- * RDF / RIPK and kNN together (no CNTNB or NPCORR) runs as two passes: the
- * RDF / RIPK part on the centre-per-lane scan, then the kNN part on the
- * centre-per-lane kNN scan (the per-centre scan for overlapping environment
- * sets or lists too large for shared memory).  Results do not depend on the
- * tuning. */
+ * bz in 0..15 (0 = 1) = blocks of by x bz cells across, as long as hold a
+ * warp of centres (bx: nominal), for the centre-per-lane scans of passes
+ * without CNTNB (one centre per lane, the block's stencil ions staged in
+ * shared memory; by default about a warp of centres, twice as long as wide),
+ * leaving the other code as it was.  A pass with RDF / RIPK and kNN together
+ * (no CNTNB or NPCORR) runs as two passes: the RDF / RIPK part on the
+ * centre-per-lane scan, then the kNN part on the centre-per-lane kNN scan;
+ * with a cell block set this way also where no kNN lane scan applies
+ * (overlapping environment sets or lists too large for shared memory), the kNN
+ * part then on the per-centre scan.  Results do not depend on the tuning. */
 int pp_cloud_tuning(pp_ctx* ctx, int cloud, float cell_ratio, uint32_t tile);
 
 /* FP64 audit of the current tasks and histogram settings on up to
@@ -335,9 +334,7 @@ int pp_last_kernel_ms(pp_ctx* ctx, float* ms);
  * RIPK and kNN run as two passes (see pp_cloud_tuning).  The centre-per-lane
  * scans take passes of dense centres (at least 0.35 per non-empty cell, or a
  * block shape set with pp_cloud_tuning) without CNTNB or NPCORR, kNN only with
- * disjoint environment sets; a pass with both RDF / RIPK and kNN takes the
- * per-centre scan unless a block shape is set.  No counterpart in the
- * reference. */
+ * disjoint environment sets.  No counterpart in the reference. */
 int pp_last_kernel(pp_ctx* ctx, const char** name);
 /* Candidate distance tests (centre, candidate) the last pp_run evaluated --
  * an implementation figure beside the in-ball pairs of pp_run_stats (their

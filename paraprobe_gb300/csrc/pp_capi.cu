@@ -460,19 +460,52 @@ int build_grid(pp_ctx* ctx, Cloud& cl, float R, cudaStream_t s) {
   return PP_OK;
 }
 
-// Default cell block of the centre-per-lane scans: about 24 centres (a warp's
-// worth) at the mean number of centres per non-empty cell, twice as long in x
-// as in y and z.  Returns false when centres are too sparse for a block to
-// fill a warp without streaming far more ions than the centres' balls hold
-// (fewer than 0.35 centres per non-empty cell); such passes take the
-// per-centre scan.
+// Ions per nm^3 inside the specimen: the mean m of a grid cell from the share
+// of cells that hold any, n / occupied = m / (1 - exp(-m)).
+double ion_density(const Cloud& cl) {
+  if (!cl.occupied || !cl.n) return 0.0;
+  const double per = (double)cl.n / (double)cl.occupied;
+  double m = per;
+  for (int i = 0; i < 30; ++i) m = per * (1.0 - std::exp(-m));
+  const double h = cl.g.h;
+  return m > 1e-3 ? m / (h * h * h) : 0.0;
+}
+
+// Default cell block of the centre-per-lane scans: about 28 centres (most of a
+// warp) at their mean density, twice as long in x as in y and z.  Returns false
+// when centres are too sparse for a block to fill a warp without streaming far
+// more ions than the centres' balls hold (fewer than 0.35 centres per non-empty
+// cell); such passes take the per-centre scan.
 bool default_block(const Cloud& cl, uint64_t ncent, int* bx, int* by, int* bz) {
   const double per_cell = cl.occupied ? (double)ncent / (double)cl.occupied : 0.0;
   if (per_cell < 0.35) return false;
-  const double cells = std::max(1.0, 24.0 / per_cell);
+  const double h = cl.g.h, mean = ion_density(cl) * h * h * h * (double)ncent / (double)cl.n;
+  const double cells = std::max(1.0, 28.0 / std::max(mean, 1e-3));
   const int side = (int)std::lround(std::cbrt(cells / 2.0));
   *by = *bz = std::min(15, std::max(1, side));
   *bx = (int)std::min(64L, std::max(1L, std::lround(cells / ((double)*by * *bz))));
+  return true;
+}
+
+// Work items of the centre-per-lane scans: chunks of columns of blocks, as long
+// as leaves every warp of the device (32 an SM) 8 of them that hold ions, since
+// the last block of a chunk is cut short; but no shorter than holds 10 centres,
+// unless not every warp would have one then.  False when they cannot be counted
+// in 32 bits.
+bool lane_items(const pp_ctx* ctx, const Cloud& cl, uint64_t ncent, pp::ScanArgs& a) {
+  const Grid& g = cl.g;
+  const uint64_t cols = (((uint64_t)g.ny + a.by - 1) / a.by) * (((uint64_t)g.nz + a.bz - 1) / a.bz);
+  const double h = g.h, density = ion_density(cl);
+  const double column = density * h * h * h * a.by * a.bz * (double)ncent / (double)cl.n;  // centres per cell of length
+  const double held = density > 0.0 ? (double)cl.n / (density * h * h * h * (double)g.ncells) : 1.0;
+  auto items = [&](int ch) { return cols * (((uint64_t)g.nx + ch - 1) / ch); };
+  const double warps = 32.0 * ctx->sm_count;
+  a.chunk = 64;
+  while (a.chunk > 1 && held * (double)items(a.chunk) < (column * a.chunk > 20.0 ? 8.0 * warps : warps)) a.chunk /= 2;
+  uint64_t nb = items(a.chunk);
+  if (nb >= (1ull << 32)) return false;
+  if (a.sample_stride > 1) nb = std::max<uint64_t>(1, nb / a.sample_stride);
+  a.nbricks = (uint32_t)nb;
   return true;
 }
 
@@ -1350,10 +1383,8 @@ int ensure_block_rows(pp_ctx* ctx, int by, int bz, int sr, cudaStream_t s, const
 
 // Select the centres of a plain run into ctx->centres (cell order); returns
 // their number.  Synchronises the stream once to learn the count.
-// type_counts (256 words, nullable) receives the ions of each type.
 int select_centres(pp_ctx* ctx, Cloud& cl, const uint8_t* labels, const float* surf, const int8_t* cslot, float R,
-                   uint32_t* ncent, cudaStream_t s, const uint8_t* extra_slot_mask = nullptr,
-                   unsigned long long* type_counts = nullptr) {
+                   uint32_t* ncent, cudaStream_t s, const uint8_t* extra_slot_mask = nullptr) {
   const uint64_t n = cl.n;
   CK(ctx->centres.ensure(std::max<uint64_t>(n, 1) * 4));
   CK(ctx->centre_count.ensure(8));
@@ -1365,27 +1396,9 @@ int select_centres(pp_ctx* ctx, Cloud& cl, const uint8_t* labels, const float* s
                             extra_slot_mask, ctx->sel_flags.as<uint32_t>(), ctx->sel_tmp.as<uint32_t>(), tmp_elems * 2,
                             ctx->centres.as<uint32_t>(), ctx->centre_count.as<uint32_t>(), ctx->cflag.as<uint8_t>(), s);
   CK(cudaGetLastError());
-  if (type_counts) {
-    CK(ctx->type_counts.ensure(256 * 8));
-    CK(cudaMemsetAsync(ctx->type_counts.p, 0, 256 * 8, s));
-    pp::launch_type_count(labels ? labels : cl.label_sorted.as<uint8_t>(), n, ctx->type_counts.as<unsigned long long>(),
-                          ctx->sm_count, s);
-    CK(cudaMemcpyAsync(type_counts, ctx->type_counts.p, 256 * 8, cudaMemcpyDeviceToHost, s));
-  }
   CK(cudaMemcpyAsync(ncent, ctx->centre_count.p, 4, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   return PP_OK;
-}
-
-// Ions per nm^3 inside the specimen: the mean m of a grid cell from the share
-// of cells that hold any, n / occupied = m / (1 - exp(-m)).
-double ion_density(const Cloud& cl) {
-  if (!cl.occupied || !cl.n) return 0.0;
-  const double per = (double)cl.n / (double)cl.occupied;
-  double m = per;
-  for (int i = 0; i < 30; ++i) m = per * (1.0 - std::exp(-m));
-  const double h = cl.g.h;
-  return m > 1e-3 ? m / (h * h * h) : 0.0;
 }
 
 // First radius of a set of `share` of the ions, for orders up to k: it holds
@@ -1496,13 +1509,12 @@ bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long l
 
 // The kNN part of a pass in two walks (k_lanes_near) where near_plan finds it
 // worth it, else -3.  count: the pass has no other part that counts its in-ball
-// pairs, so they are counted by a symmetric walk of their own first (needs
-// ctx->nc_pre); the two take the work counters a.work[0] and [1].
+// pairs, so they are counted by a symmetric walk of their own first; the
+// kernels take the work counters from a.work on, one each.
 int run_near(pp_ctx* ctx, Cloud& cl, const RunPlan& P, const unsigned long long* type_counts, float R,
              const pp::ScanArgs& a0, bool count, size_t* smem, cudaStream_t s) {
   pp::ScanArgs a = a0;
   uint64_t sparse = 0;
-  if (!near_pays(ctx, cl, R, P.kmax, (uint64_t)a.ncentres * std::max<uint32_t>(a.sample_stride, 1), count)) return -3;
   if (!near_plan(cl, P, R, type_counts, a, &sparse)) return -3;
   const uint64_t sp_words = a.sp_g.ncells + 1;
   CK(ctx->sp_start.ensure(sp_words * 8));  // starts, then cursors
@@ -1513,7 +1525,6 @@ int run_near(pp_ctx* ctx, Cloud& cl, const RunPlan& P, const unsigned long long*
   if (count) {
     pp::ScanArgs ac = a;
     ac.sym = ctx->no_sym ? 0 : 1;
-    ac.nc_pre = ctx->nc_pre.as<uint32_t>();
     const int rc = pp::launch_lanes_count(ac, ctx->sm_count, s);
     if (rc) return rc;
     a.work = a0.work + 1;
@@ -1569,12 +1580,7 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
     mask_slot = m_in + n;
   }
   uint32_t ncent = 0;
-  const bool near_ok = P.kr == 1 && P.kmax <= 20 && P.disjoint && !ctx->no_lanes &&
-                       !(flags & (PP_CNTNB | PP_NPCORR)) && near_pays(ctx, *cl, R, P.kmax, n, !(flags & (PP_RDF | PP_RIPK)));
-  std::vector<unsigned long long> type_counts(near_ok ? 256 : 0);
-  if ((rc = select_centres(ctx, *cl, labels, surf, D.cslot, R, &ncent, s, mask_slot,
-                           near_ok ? type_counts.data() : nullptr)))
-    return rc;
+  if ((rc = select_centres(ctx, *cl, labels, surf, D.cslot, R, &ncent, s, mask_slot))) return rc;
   ctx->last_centres_all = ncent;
   // a tuning sample: every stride-th centre (or brick) over the whole cloud
   uint32_t stride = 1;
@@ -1612,42 +1618,63 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
   a.mode = 0;
   a.sample_stride = stride;
   a.rdf_in_smem = ((a.flags & PP_RDF) && (size_t)P.nC * P.nE * P.H * 4 <= 96 * 1024) ? 1 : 0;
-  // a cell block set by tuning applies to every pass; one set by
-  // pp_cloud_prepare only to passes of dense centres
+  // centre-per-lane scans: the cell block.  One set by tuning applies to every
+  // pass; one set by pp_cloud_prepare only to passes of dense centres, which
+  // have a default block otherwise.
+  const Grid& g = cl->g;
+  const bool rows_fit = (int)std::floor((R + 3.f * g.margin) * g.inv_h) + 1 <= 7;
+  const bool both = P.kr > 0 && (a.flags & PP_RDF);
   int dbx = 0, dby = 0, dbz = 0;
-  const bool block_ok = cl->lanes_bx != 0 &&
-                        (!cl->lanes_auto || default_block(*cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1),
-                                                          &dbx, &dby, &dbz));
-  // RDF / RIPK and kNN in one pass on a cloud tuned to a centre-per-lane cell
-  // block: two centre-per-lane passes, RDF / RIPK then kNN
-  const bool split = P.kr > 0 && (a.flags & PP_RDF) && block_ok && !ctx->no_lanes &&
-                     !(flags & (PP_CNTNB | PP_NPCORR));
+  const bool dense = default_block(*cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), &dbx, &dby, &dbz);
+  const bool block_ok = cl->lanes_bx != 0 && (!cl->lanes_auto || dense);
+  bool lanes = rows_fit && !ctx->no_lanes && !(flags & (PP_CNTNB | PP_NPCORR)) && (block_ok || dense);
+  // RDF / RIPK and kNN in one pass run as two centre-per-lane passes, RDF /
+  // RIPK then kNN: the per-centre scan, which serves both from one candidate
+  // stream, takes 2291 us against 1884 on a 1M-ion tip at R = 1 nm (56 ions a
+  // ball, k <= 10), 5530 against 1578 at R = 2 nm, and 481 against 303 at 20k
+  // ions.  It keeps the passes whose kNN no lane scan takes (overlapping sets,
+  // more than 8 centre types) and those of too few centres to give the lanes of
+  // two passes work (2191 against 2698 us at 3.3k centres of 1000 neighbours),
+  // unless the cloud is tuned to a block.
+  const bool split = both && lanes &&
+                     (block_ok || (P.disjoint && P.nC <= 8 && P.emax <= 15 && P.kmax <= 64 &&
+                                   (uint64_t)ncent * std::max<uint32_t>(stride, 1) >= 4096));
+  if (both && !split) lanes = false;
+  // kNN in two walks: needs the ions of each type of this run's labels
+  const bool near_ok = lanes && P.kr == 1 && P.kmax <= 20 && P.disjoint &&
+                       near_pays(ctx, *cl, R, P.kmax, (uint64_t)ncent * std::max<uint32_t>(stride, 1), !both);
+  std::vector<unsigned long long> type_counts(near_ok ? 256 : 0);
+  if (near_ok) {
+    CK(ctx->type_counts.ensure(256 * 8));
+    CK(cudaMemsetAsync(ctx->type_counts.p, 0, 256 * 8, s));
+    pp::launch_type_count(labels ? labels : cl->label_sorted.as<uint8_t>(), n, ctx->type_counts.as<unsigned long long>(),
+                          ctx->sm_count, s);
+    CK(cudaMemcpyAsync(type_counts.data(), ctx->type_counts.p, 256 * 8, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+  }
   // RDF / RIPK alone: each pair of two centres is computed once and credited
   // to both (the counts are the same as the per-centre ball scan's)
   a.sym = ((P.kr == 0 || split) && !(flags & PP_CNTNB) && (a.flags & PP_RDF) && !ctx->no_sym) ? 1 : 0;
   a.cflag = ctx->cflag.as<uint8_t>();
-  if (a.sym || near_ok) {
-    CK(ctx->nc_pre.ensure((cl->g.ncells + 1) * 4));
-    const uint64_t tmp_elems = (cl->g.ncells + 1) / 2048 + 64;
-    CK(ctx->scan_tmp.ensure(tmp_elems * 8 * 2));
-    pp::launch_nc_prefix(cl->cell_start.as<uint32_t>(), cl->g.ncells, a.cflag, ctx->nc_pre.as<uint32_t>(),
-                         ctx->scan_tmp.as<uint32_t>(), tmp_elems * 4, s);
-    a.nc_pre = ctx->nc_pre.as<uint32_t>();
-  }
   ctx->ev_recorded = false;
   if (ncent > 0) {
     size_t smem = 0;
-    const Grid& g = cl->g;
-    const bool rows_fit = (int)std::floor((R + 3.f * g.margin) * g.inv_h) + 1 <= 7;
-    // centre-per-lane scans: cell block and its stencil rows
-    bool lanes = rows_fit && !ctx->no_lanes && !(flags & (PP_CNTNB | PP_NPCORR)) &&
-                 (split || !(P.kr > 0 && (a.flags & PP_RDF)));
     if (lanes && block_ok) {
       a.bx = (int)cl->lanes_bx;
       a.by = (int)std::max<uint32_t>(cl->lanes_by, 1);
       a.bz = (int)std::max<uint32_t>(cl->lanes_bz, 1);
     } else if (lanes) {
-      lanes = default_block(*cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), &a.bx, &a.by, &a.bz);
+      a.bx = dbx;
+      a.by = dby;
+      a.bz = dbz;
+    }
+    if (lanes || a.sym) {  // prefix of the non-centre ions per cell
+      CK(ctx->nc_pre.ensure((g.ncells + 1) * 4));
+      const uint64_t tmp_elems = (g.ncells + 1) / 2048 + 64;
+      CK(ctx->scan_tmp.ensure(tmp_elems * 8 * 2));
+      pp::launch_nc_prefix(cl->cell_start.as<uint32_t>(), g.ncells, a.cflag, ctx->nc_pre.as<uint32_t>(),
+                           ctx->scan_tmp.as<uint32_t>(), tmp_elems * 4, s);
+      a.nc_pre = ctx->nc_pre.as<uint32_t>();
     }
     a.bsr = (int)std::floor(((R + g.margin) + 2.f * g.margin) * g.inv_h) + 1;
     a.brows = nullptr;
@@ -1661,20 +1688,11 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
     }
     CK(cudaEventRecord(ctx->ev0, s));
     rc = -3;
-    // passes with RDF / RIPK and kNN together take the per-centre scan, which
-    // serves both from one candidate stream, unless the cloud is tuned to a
-    // cell block (the autotuner times both): then the RDF / RIPK part and the
-    // kNN part run as two centre-per-lane passes, the second on a fresh work
-    // counter and with its pair and centre counts dropped (the first counted
-    // them)
+    // RDF / RIPK and kNN: the second pass on fresh work counters and with its
+    // pair and centre counts dropped (the first counted them)
     if (rc == -3 && a.brows && split) {
-      const uint64_t nb_x = ((uint64_t)g.nx + a.bx - 1) / a.bx, nb_y = ((uint64_t)g.ny + a.by - 1) / a.by;
-      uint64_t nb = nb_x * nb_y * (((uint64_t)g.nz + a.bz - 1) / a.bz);
-      if (stride > 1) nb = std::max<uint64_t>(1, nb / stride);
-      if (nb < (1ull << 32)) {
+      if (lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a)) {
         pp::ScanArgs ar = a;
-        ar.nbricks = (uint32_t)nb;
-        ar.tile = 4;
         rc = pp::launch_lanes(ar, 0, ctx->sm_count, &smem, s);
         if (rc == 0) {
           pp::ScanArgs ak = a;
@@ -1682,13 +1700,10 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
           ak.sym = 0;
           ak.work = a.work + 1;
           ak.counters = (unsigned long long*)(ctx->work.as<unsigned char>() + 16);
-          ak.nbricks = (uint32_t)nb;
-          ak.tile = 4;
           rc = near_ok ? run_near(ctx, *cl, P, type_counts.data(), R, ak, false, &smem, s) : -3;
           if (rc == -3) rc = pp::launch_lanes_knn(ak, P.disjoint != 0, ctx->sm_count, &smem, s);
           ctx->last_kind = 4;
           if (rc == -3) {  // overlapping sets, or lists too large for shared memory
-            ak.tile = a.tile;
             rc = pp::launch_scan(ak, P.kr, P.emax, ctx->sm_count, &smem, s);
             ctx->last_kind = 5;
           }
@@ -1697,34 +1712,14 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
       }
     }
     if (P.kr > 0) a.sym = 0;  // the per-centre scans need every centre's whole ball
-    if (rc == -3 && a.brows && P.kr == 0 && (a.flags & PP_RDF)) {
-      const uint64_t nb_x = ((uint64_t)g.nx + a.bx - 1) / a.bx, nb_y = ((uint64_t)g.ny + a.by - 1) / a.by;
-      uint64_t nb = nb_x * nb_y * (((uint64_t)g.nz + a.bz - 1) / a.bz);
-      if (stride > 1) nb = std::max<uint64_t>(1, nb / stride);
-      if (nb < (1ull << 32)) {
-        a.nbricks = (uint32_t)nb;
-        const uint32_t keep = a.tile;
-        a.tile = 4;  // bricks per warp work item
-        rc = pp::launch_lanes(a, P.kr, ctx->sm_count, &smem, s);
-        if (rc == 0) ctx->last_kind = 2;
-        a.tile = keep;
-      }
+    if (rc == -3 && a.brows && P.kr == 0 && (a.flags & PP_RDF) && lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a)) {
+      rc = pp::launch_lanes(a, P.kr, ctx->sm_count, &smem, s);
+      if (rc == 0) ctx->last_kind = 2;
     }
-    // kNN-only passes (with RDF in the same pass every in-ball pair would be
-    // walked per lane; the per-centre scan does that pass better)
-    if (rc == -3 && a.brows && P.kr > 0 && !(a.flags & PP_RDF)) {
-      const uint64_t nb_x = ((uint64_t)g.nx + a.bx - 1) / a.bx, nb_y = ((uint64_t)g.ny + a.by - 1) / a.by;
-      uint64_t nb = nb_x * nb_y * (((uint64_t)g.nz + a.bz - 1) / a.bz);
-      if (stride > 1) nb = std::max<uint64_t>(1, nb / stride);
-      if (nb < (1ull << 32)) {
-        a.nbricks = (uint32_t)nb;
-        const uint32_t keep = a.tile;
-        a.tile = 4;  // blocks per warp work item
-        rc = near_ok ? run_near(ctx, *cl, P, type_counts.data(), R, a, true, &smem, s) : -3;
-        if (rc == -3) rc = pp::launch_lanes_knn(a, P.disjoint != 0, ctx->sm_count, &smem, s);
-        if (rc == 0) ctx->last_kind = 3;
-        a.tile = keep;
-      }
+    if (rc == -3 && a.brows && P.kr > 0 && !(a.flags & PP_RDF) && lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a)) {
+      rc = near_ok ? run_near(ctx, *cl, P, type_counts.data(), R, a, true, &smem, s) : -3;
+      if (rc == -3) rc = pp::launch_lanes_knn(a, P.disjoint != 0, ctx->sm_count, &smem, s);
+      if (rc == 0) ctx->last_kind = 3;
     }
     if (rc == -3 && cl->brick && rows_fit) {
       a.bx = (int)(cl->brick >> 16);
@@ -1953,7 +1948,7 @@ int pp_autotune(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_list, 
   // passes the centre-per-lane scan takes: cell blocks of about 2 x 1 x 1 R/2
   // (a few tens of centres at atom-probe densities) for each cell edge
   const uint32_t lanes_tiles[4][2] = {{lanes_code(2, 1, 1), lanes_code(2, 2, 1)},
-                                      {lanes_code(3, 2, 2), lanes_code(2, 2, 2)},
+                                      {lanes_code(3, 2, 2), lanes_code(4, 2, 1)},
                                       {lanes_code(4, 2, 2), lanes_code(4, 3, 3)},
                                       {lanes_code(5, 3, 3), lanes_code(4, 4, 4)}};
   // other passes: per-centre tiles, then brick codes (cells per brick << 16 | batch)
@@ -1977,10 +1972,7 @@ int pp_autotune(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_list, 
       cl->lanes_bx = cl->lanes_by = cl->lanes_bz = 0;
     }
   };
-  // RDF / RIPK with kNN in one pass: the per-centre scan's tiles and the two
-  // centre-per-lane passes a cell block gives
-  const bool combined = (flags & (PP_RDF | PP_RIPK)) && (flags & (PP_1NN | PP_MKNN)) &&
-                        !(flags & (PP_CNTNB | PP_NPCORR)) && !ctx->no_lanes;
+  const bool combined = (flags & (PP_RDF | PP_RIPK)) && (flags & (PP_1NN | PP_MKNN));
   float bestr = keep_ratio, bestms = 1e30f;
   uint32_t bestt = 0;
   int rc = PP_OK;
@@ -1997,13 +1989,13 @@ int pp_autotune(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_list, 
     // passes too, the default block won on the tuning sample but lost on the
     // whole 20M-ion tip, so they keep the two shapes.)
     int dbx = 0, dby = 0, dbz = 0;
-    const bool dense = combined && default_block(*cl, ctx->last_centres_all, &dbx, &dby, &dbz);
+    const bool dense = lanes && combined && default_block(*cl, ctx->last_centres_all, &dbx, &dby, &dbz);
     uint32_t tiles[sizeof scan_tiles / sizeof scan_tiles[0] + 3];
     int ntiles = 0;
-    if (!lanes)
+    if (!lanes) {
       for (uint32_t t : scan_tiles) tiles[ntiles++] = t;
-    if (lanes || dense) {
-      const uint32_t dcode = (!lanes && dense) ? lanes_code((uint32_t)dbx, (uint32_t)dby, (uint32_t)dbz) : 0u;
+    } else {
+      const uint32_t dcode = dense ? lanes_code((uint32_t)dbx, (uint32_t)dby, (uint32_t)dbz) : 0u;
       if (dcode && dcode != lanes_tiles[ri][0] && dcode != lanes_tiles[ri][1]) tiles[ntiles++] = dcode;
       tiles[ntiles++] = lanes_tiles[ri][0];
       tiles[ntiles++] = lanes_tiles[ri][1];

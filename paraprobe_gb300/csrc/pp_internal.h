@@ -54,10 +54,12 @@ struct ScanArgs {
   int lut_one;                 // the cell's category plus at most one step is exact for d^2 <= R^2
   int cat_fast;                // rmin = 0 and sqrt(d^2) * guess_scale names the category to within 1/256 bin
   // brick scan: cells per brick, centres per warp batch, bricks to process;
-  // the centre-per-lane scan takes blocks of bx x by x bz cells
+  // the centre-per-lane scans take blocks of by x bz cells across (bx: their
+  // nominal length), from nbricks chunks of `chunk` cells of a column of blocks
   int bx, bcap;
   int by, bz;
   uint32_t nbricks;
+  int chunk;
   // centre-per-lane scans: per-slot pass codes (written by the pass, n words),
   // the labels they are made from, and 1.f (see dist2_x2)
   uint32_t* pcode;

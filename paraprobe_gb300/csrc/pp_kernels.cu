@@ -1864,8 +1864,8 @@ __device__ __forceinline__ bool row_box_range(const Grid& g, float R, int yy, in
   const float brem = Rp2 - by * by - bz * bz;
   if (brem < 0.f) return false;
   const float bhalf = sqrt_approx(brem) + m2;
-  x0 = max(0, (int)floorf((lo.x - g.lox - bhalf) * g.inv_h));
-  x1 = min(g.nx - 1, (int)floorf((hi.x - g.lox + bhalf) * g.inv_h));
+  x0 = max(0, __float2int_rd((lo.x - g.lox - bhalf) * g.inv_h));
+  x1 = min(g.nx - 1, __float2int_rd((hi.x - g.lox + bhalf) * g.inv_h));
   return x0 <= x1;
 }
 __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nrows, float R, const LaneBlock& b, bool sym, const float4* box,
@@ -1876,12 +1876,12 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
   len = 0;
   low = false;
   if (r >= nrows) return;
-  const int ry = a.brows[2 * r], rz = a.brows[2 * r + 1];
-  const int yy = yb - sr + ry, zz = zb - sr + rz;
+  const short2 ro = ((const short2*)a.brows)[r];
+  const int yy = yb - sr + ro.x, zz = zb - sr + ro.y;
   if (yy < 0 || yy >= g.ny || zz < 0 || zz >= g.nz) return;
   int x0, x1;
   if (!row_box_range(g, R, yy, zz, box, x0, x1)) return;
-  const uint64_t cb = ((uint64_t)zz * g.ny + yy) * g.nx;
+  const uint32_t cb = ((uint32_t)zz * (uint32_t)g.ny + (uint32_t)yy) * (uint32_t)g.nx;  // fewer than 2^32 cells
   int xs = x0;
   if (sym) {
     const bool own = yy >= yb && yy < ye && zz >= zb && zz < ze;
@@ -1899,7 +1899,9 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
 
 // ----------------------------------------------- K3'' centre-per-lane blocks
 // Passes with one centre per lane.  A warp takes up to 32 centres of a block
-// of bx x by x bz cells (rows of the block in slot order) and streams the
+// of by x bz cells across and as many along x, up to 32, as hold no more (rows
+// of the block in slot order; this fills 28 of 32 lanes on the tips, where
+// blocks of fixed length filled 24) and streams the
 // block's stencil rows through a per-warp staging buffer, 32 ions at a time;
 // every lane then tests the 32 staged ions against its own centre and keeps a
 // 32-bit mask of the ions it takes.  A test is half a broadcast shared load,
@@ -1913,8 +1915,7 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
 // cells a side) keeps the staged region close to the union of the centres'
 // balls.  The pair set and d^2 expression are those of k_scan; what is done
 // with the taken pairs is up to the pass (k_lanes: RDF / RIPK bins,
-// k_lanes_knn: kNN lists).  Warps fetch blocks `tile` at a time
-// from the global work counter, without block barriers.
+// k_lanes_knn: kNN lists).
 //
 // Box filter: the cell rows hold, beside the centres' neighbours, every ion
 // within reach of any point of the cell block.  Each batch of centres takes
@@ -1935,7 +1936,8 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
 // An ion's pass code (ScanArgs::pcode, k_pass_codes) is staged as its record's
 // fourth word; in symmetric mode its lowest bit says that it is a centre and
 // is staged as 0.
-// lanes_blocks fetches work and calls, warp-uniformly,
+// Warps fetch chunks of `chunk` cells of a column of blocks from the global
+// work counter, without block barriers.  lanes_blocks calls, warp-uniformly,
 //   start(self)                a new batch; self = this lane's centre slot or
 //                              0xffffffff; returns the lane's centre position
 //                              (at infinity for no centre)
@@ -2147,93 +2149,99 @@ __device__ __forceinline__ uint32_t stage_rows(const ScanArgs& a, const LaneBatc
 }
 
 template <class Start, class Body>
-__device__ __forceinline__ void lanes_blocks(const ScanArgs& a, float4* sbox, Start start, Body body) {
+__device__ __forceinline__ void lanes_blocks(const ScanArgs& a, float4* sbox, uint32_t* queue, Start start, Body body) {
   const Grid& g = a.g;
   const int lane = threadIdx.x & 31;
-  const int BX = max(a.bx, 1), BY = max(a.by, 1), BZ = max(a.bz, 1);
-  const uint32_t nbx = (uint32_t)((g.nx + BX - 1) / BX), nby = (uint32_t)((g.ny + BY - 1) / BY);
-  const uint32_t WT = max(a.tile, 1u);
+  const uint32_t ltmask = (1u << lane) - 1u;
+  const int BY = max(a.by, 1), BZ = max(a.bz, 1), CH = a.chunk;
+  const uint32_t nch = (uint32_t)((g.nx + CH - 1) / CH), nby = (uint32_t)((g.ny + BY - 1) / BY);
   for (;;) {
-    uint32_t w0 = 0;
-    if (lane == 0) w0 = atomicAdd(a.work, WT);
-    w0 = __shfl_sync(FULL, w0, 0);
-    if (w0 >= a.nbricks) break;
-    const uint32_t wend = min(w0 + WT, a.nbricks);
-    for (uint32_t wb = w0; wb < wend; ++wb) {
-      const uint32_t b = (a.sample_stride > 1) ? wb * a.sample_stride : wb;
-      const uint32_t bz_i = b / (nbx * nby), rest = b - bz_i * (nbx * nby);
-      const uint32_t by_i = rest / nbx, bx_i = rest - by_i * nbx;
-      const int xb = (int)bx_i * BX, yb = (int)by_i * BY, zb = (int)bz_i * BZ;
-      const int xe = min(xb + BX, g.nx), ye = min(yb + BY, g.ny), ze = min(zb + BZ, g.nz);
-      const int nseg = (ye - yb) * (ze - zb);
-      // centres: the block's row segments [cell_start(row, xb), cell_start(row, xe)) in slot order
-      int seg = 0;
-      uint32_t pos = 0, s1 = 0;
-      {
-        const uint64_t hrow = ((uint64_t)zb * g.ny + yb) * g.nx;
-        pos = a.cell_start[hrow + xb];
-        s1 = a.cell_start[hrow + xe];
+    uint32_t w = 0;
+    if (lane == 0) w = atomicAdd(a.work, 1u);
+    w = __shfl_sync(FULL, w, 0);
+    if (w >= a.nbricks) break;
+    if (a.sample_stride > 1) w *= a.sample_stride;
+    const uint32_t col = w / nch, bz_i = col / nby;
+    LaneBatch B;
+    B.yb = (int)(col - bz_i * nby) * BY;
+    B.zb = (int)bz_i * BZ;
+    B.ye = min(B.yb + BY, g.ny);
+    B.ze = min(B.zb + BZ, g.nz);
+    const int X1 = min((int)(w - col * nch) * CH + CH, g.nx);
+    for (B.xb = (int)(w - col * nch) * CH; B.xb < X1; B.xb = B.xe) {
+      // the block's length: as many columns, up to 32, as hold at most 32
+      // centres; cum = centres of the columns up to this lane's
+      const int x = min(B.xb + lane, X1 - 1);
+      uint32_t cum = 0;
+      for (int sz = B.zb; sz < B.ze; ++sz)
+        for (int sy = B.yb; sy < B.ye; ++sy) {
+          const uint32_t row = ((uint32_t)sz * (uint32_t)g.ny + (uint32_t)sy) * (uint32_t)g.nx;
+          cum += (a.cell_start[row + x + 1] - a.cell_start[row + B.xb]) - (a.nc_pre[row + x + 1] - a.nc_pre[row + B.xb]);
+        }
+      const uint32_t none = __ballot_sync(FULL, cum == 0u && B.xb + lane < X1);
+      if (none & 1u) {  // skip the empty columns
+        B.xe = B.xb + (none == FULL ? 32 : __ffs(~none) - 1);
+        continue;
       }
+      const int ncol = max(1, __popc(__ballot_sync(FULL, cum <= 32u && B.xb + lane < X1)));
+      B.xe = B.xb + ncol;
+      // centres: the block's row segments [cell_start(row, xb), cell_start(row, xe)) in slot order
+      int sy = B.yb, sz = B.zb;
+      uint32_t pos = 0, s1 = 0, have = 0, head = 0;
+      bool more = true;
       for (;;) {
         // ---- the next batch: lane l takes the l-th next centre of the block
-        int mc = 0;
-        uint32_t self = 0xffffffffu;
-        while (mc < 32) {
+        while (have < 32u && more) {
           if (pos >= s1) {
-            if (++seg >= nseg) break;
-            const int sy = yb + seg % (ye - yb), sz = zb + seg / (ye - yb);
-            const uint64_t hrow = ((uint64_t)sz * g.ny + sy) * g.nx;
-            pos = a.cell_start[hrow + xb];
-            s1 = a.cell_start[hrow + xe];
+            if (sz >= B.ze) {
+              more = false;
+              break;
+            }
+            const uint32_t row = ((uint32_t)sz * (uint32_t)g.ny + (uint32_t)sy) * (uint32_t)g.nx;
+            pos = a.cell_start[row + B.xb];
+            s1 = a.cell_start[row + B.xe];
+            if (++sy == B.ye) {
+              sy = B.yb;
+              ++sz;
+            }
             continue;
           }
           const uint32_t sl = pos + lane;
-          const uint32_t cm = __ballot_sync(FULL, sl < s1 && a.cflag[sl] != 0);
-          const int room = 32 - mc, have = __popc(cm);
-          const uint32_t base = pos;
-          uint32_t takem = cm;
-          if (have > room) {
-            const uint32_t lastl = nth_set(cm, (uint32_t)room - 1u);
-            takem = cm & ((2u << lastl) - 1u);
-            pos += lastl + 1u;
-          } else {
-            pos += 32u;
-          }
-          const int ntake = __popc(takem);
-          const int want = lane - mc;
-          if (want >= 0 && want < ntake) self = base + nth_set(takem, (uint32_t)want);
-          mc += ntake;
+          const bool c = sl < s1 && a.cflag[sl] != 0;
+          const uint32_t cm = __ballot_sync(FULL, c);
+          if (c) queue[(head + have + (uint32_t)__popc(cm & ltmask)) & 63u] = sl;
+          have += (uint32_t)__popc(cm);
+          pos += 32u;
         }
-        if (mc == 0) break;
+        if (have == 0u) break;
+        __syncwarp();
+        const uint32_t self = (uint32_t)lane < have ? queue[(head + lane) & 63u] : 0xffffffffu;
+        const uint32_t take = min(have, 32u);
+        have -= take;
+        head += take;
+        __syncwarp();
         const float4 cp = start(self);
         const bool lv = cp.x != kInf();
-        const uint32_t live = __ballot_sync(FULL, lv);
-        if (live) self = lv ? self : 0xffffffffu;
-        {
-          // the live centres' bounding box (order-preserving keys: min and max
-          // are exact), kept in shared memory: sbox[0] low, sbox[1] high corner
-          const float blx = o2f(__reduce_min_sync(FULL, f2o(lv ? cp.x : kInf())));
-          const float bly = o2f(__reduce_min_sync(FULL, f2o(lv ? cp.y : kInf())));
-          const float blz = o2f(__reduce_min_sync(FULL, f2o(lv ? cp.z : kInf())));
-          const float bhx = o2f(__reduce_max_sync(FULL, f2o(lv ? cp.x : -kInf())));
-          const float bhy = o2f(__reduce_max_sync(FULL, f2o(lv ? cp.y : -kInf())));
-          const float bhz = o2f(__reduce_max_sync(FULL, f2o(lv ? cp.z : -kInf())));
-          if (lane == 0) {
-            sbox[0] = make_float4(blx, bly, blz, 0.f);
-            sbox[1] = make_float4(bhx, bhy, bhz, 0.f);
-          }
-          __syncwarp();
+        B.live = __ballot_sync(FULL, lv);
+        if (B.live == 0u) continue;
+        B.self = lv ? self : 0xffffffffu;
+        B.cxx = f2_pack(cp.x, cp.x);
+        B.cyy = f2_pack(cp.y, cp.y);
+        B.czz = f2_pack(cp.z, cp.z);
+        // the live centres' bounding box (order-preserving keys: min and max
+        // are exact), kept in shared memory: sbox[0] low, sbox[1] high corner
+        const float blx = o2f(__reduce_min_sync(FULL, f2o(lv ? cp.x : kInf())));
+        const float bly = o2f(__reduce_min_sync(FULL, f2o(lv ? cp.y : kInf())));
+        const float blz = o2f(__reduce_min_sync(FULL, f2o(lv ? cp.z : kInf())));
+        const float bhx = o2f(__reduce_max_sync(FULL, f2o(lv ? cp.x : -kInf())));
+        const float bhy = o2f(__reduce_max_sync(FULL, f2o(lv ? cp.y : -kInf())));
+        const float bhz = o2f(__reduce_max_sync(FULL, f2o(lv ? cp.z : -kInf())));
+        if (lane == 0) {
+          sbox[0] = make_float4(blx, bly, blz, 0.f);
+          sbox[1] = make_float4(bhx, bhy, bhz, 0.f);
         }
-        if (live) {
-          LaneBatch B;
-          B.xb = xb; B.xe = xe; B.yb = yb; B.ye = ye; B.zb = zb; B.ze = ze;
-          B.self = self;
-          B.live = live;
-          B.cxx = f2_pack(cp.x, cp.x);
-          B.cyy = f2_pack(cp.y, cp.y);
-          B.czz = f2_pack(cp.z, cp.z);
-          body(B);
-        }
+        __syncwarp();
+        body(B);
         __syncwarp();
       }
     }
@@ -2274,7 +2282,8 @@ struct FastCat {
 // bin them.  All 36 pair RDFs of the 20M-ion tip (R = 2 nm, 0.01 nm bins): 32.1
 // ms with lists, 23.3 ms binning in the loop, 19.1 ms with pairs of blocks met
 // once and the ring buffer, 15.6 ms with pass codes, packed sums, the
-// unpredicated atomic and the branch-free staging.
+// unpredicated atomic and the branch-free staging, 13.2 ms with blocks cut at
+// 32 centres (lanes_blocks).
 //
 // Categories: FAST = FastCat, otherwise the lookup table.
 //
@@ -2308,6 +2317,7 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
   float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
   float4* boxA = (float4*)sp; sp += NW * 2 * 16;
   uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
+  uint32_t* queueA = (uint32_t*)sp; sp += NW * 64 * 4;
   uint32_t* sdummy = (uint32_t*)sp; sp += 32 * 4;    // where the lanes without a pair add
   float* sT = (float*)sp; sp += ((H + 4) & ~3) * 4;  // H thresholds, then +inf
   uint32_t* srdf = (uint32_t*)sp; sp += (size_t)nbin * 4;
@@ -2521,7 +2531,7 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
   unsigned long long tests = 0;  // (centre, staged ion) distance tests, warp-uniform
   const float4* sbox = boxA + warp * 2;
   const int nrows = (max(a.by, 1) + 2 * a.bsr) * (max(a.bz, 1) + 2 * a.bsr);
-  lanes_blocks(a, boxA + warp * 2, start, [&](const LaneBatch& B) {
+  lanes_blocks(a, boxA + warp * 2, queueA + warp * 64, start, [&](const LaneBatch& B) {
     const uint32_t staged = stage_rows<SYM, false, false>(
         a, B, nrows, a.R, a.box_R2, 0u, cand, skey, sbox, [&](uint32_t base, uint32_t nb, bool keyed) {
           batch(base, nb, keyed, B.self, B.cxx, B.cyy, B.czz);
@@ -2544,6 +2554,75 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
   }
 }
 
+constexpr int kKnnWarps = 24;  // most warps of a block of the kNN passes; one block per SM
+
+// What the kNN passes share: tables in shared memory, categories, and the
+// counts of missing neighbours -- most orders of a rare species have none, so
+// they are counted once per set and centre, by the number of orders found,
+// instead of one by one in the cores.
+struct KnnCommon {
+  const ScanArgs& a;
+  float* sT;
+  uint32_t* sfound;  // [centre slot][set][orders found]
+  int8_t* scs;
+  uint16_t* slut;
+  FastCat fc;
+  __device__ __forceinline__ KnnCommon(const ScanArgs& a_, unsigned char*& sp) : a(a_), fc(a_) {
+    const int H = a.H;
+    sT = (float*)sp; sp += ((H + 4) & ~3) * 4;  // H thresholds, then +inf
+    const uint32_t nfound = (uint32_t)a.nC * a.emax * (a.nkI + 1);
+    sfound = (uint32_t*)sp; sp += (size_t)nfound * 4;
+    scs = (int8_t*)sp; sp += 256;
+    slut = (uint16_t*)sp;  // unless a.cat_fast
+    for (int i = threadIdx.x; i <= H; i += blockDim.x) sT[i] = i < H ? a.cat_T[i] : kInf();
+    for (uint32_t i = threadIdx.x; i < nfound; i += blockDim.x) sfound[i] = 0;
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) scs[i] = a.cslot_of[i];
+    if (!a.cat_fast)
+      for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
+  }
+  __device__ __forceinline__ int category_of(float d2) const {
+    if (!a.cat_fast) return category_lut(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT, a.H);
+    const int g = (int)(fc.guess4(d2) >> 2);
+    return g + (sT[g + 1] <= d2 ? 1 : 0);
+  }
+  __device__ __forceinline__ float4 start(uint32_t self, int& cs) const {
+    float4 cp = make_float4(kInf(), kInf(), kInf(), 0.f);
+    cs = -1;
+    if (self != 0xffffffffu) {
+      cp = a.ions[self];
+      const uint32_t ct = a.labels ? (uint32_t)a.labels[self] : __float_as_uint(cp.w);
+      cs = scs[ct & 255];
+      if (cs < 0) {  // selection guarantees a slot; record and drop the centre otherwise
+        atomicOr(a.status, ST_TYPE_RANGE);
+        cp = make_float4(kInf(), kInf(), kInf(), 0.f);
+      }
+    }
+    return cp;
+  }
+  __device__ __forceinline__ unsigned long long* core(int cs, int p) const {
+    return a.knn_core + ((uint64_t)cs * a.nS + a.set_list[cs * 32 + p]) * a.nkI * a.H;
+  }
+  __device__ __forceinline__ void found(int cs, int p, int orders) const {
+    if (orders < a.nkI) atomicAdd(&sfound[((uint32_t)cs * a.emax + p) * (a.nkI + 1) + orders], 1u);
+  }
+  // the missing orders' counts (after a block barrier)
+  __device__ __forceinline__ void flush_found() const {
+    if (a.cat_miss < 0) return;
+    const uint32_t nfound = (uint32_t)a.nC * a.emax * (a.nkI + 1);
+    for (uint32_t i = threadIdx.x; i < nfound; i += blockDim.x) {
+      const uint32_t v = sfound[i];
+      if (!v) continue;
+      const uint32_t f = i % (a.nkI + 1), p = (i / (a.nkI + 1)) % a.emax, c = i / (a.nkI + 1) / a.emax;
+      for (int kk = f; kk < a.nkI; ++kk)  // found the first f orders: the rest are missing
+        atomicAdd(&core(c, p)[(uint64_t)kk * a.H + a.cat_miss], (unsigned long long)v);
+    }
+  }
+};
+static size_t knn_common_smem(const ScanArgs& a) {
+  return (size_t)((a.H + 4) & ~3) * 4 + (size_t)a.nC * a.emax * (a.nkI + 1) * 4 + 256 +
+         (a.cat_fast ? 0 : (size_t)((a.lut_n + 7) & ~7) * 2);
+}
+
 // kNN pass (no RDF in the same pass), every type in at most one environment
 // set of each centre type.  Each lane keeps, in shared memory, the K smallest
 // d^2 of its centre per environment set, largest first (set p, rank r of lane
@@ -2559,7 +2638,6 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
 // are taken.  Taken ions go into the sorted lists.  At the end of the batch
 // the k-th values are binned (a missing neighbour at R + EPSILON), as k_scan
 // does.
-constexpr int kLanesKnnWarps = 8;
 
 // KB > 0: K <= KB, and an insertion loads the whole list at once (KB
 // independent shared loads) instead of walking it; KB = 0: any K.
@@ -2567,8 +2645,8 @@ constexpr int kLanesKnnWarps = 8;
 // usual all-pairs task lists); a staged ion then carries that set's list row
 // as a ready offset instead of one 4-bit set index per centre slot.
 // CAT: the lists hold bin categories (uint16), not d^2 -- half the shared
-// memory, for many sets of large k (8 sets of k = 20 fit two blocks of 8
-// warps per SM instead of one).  The k-th smallest category is the category
+// memory, for many sets of large k (8 sets of k = 20 fit 18 warps per SM
+// instead of 9).  The k-th smallest category is the category
 // of the k-th smallest d^2 (categories rise with d^2), which is all the
 // histogram needs.  Each set keeps, beside its categories, the float test
 // threshold: the smallest d^2 of its K-th category (just above R^2 while the
@@ -2576,11 +2654,11 @@ constexpr int kLanesKnnWarps = 8;
 // K-th one, so the test stays one float compare; a taken ion's category is
 // looked up once, at insertion, and the binning at the end needs none.
 template <int KB, bool UNI, bool CAT>
-__global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a) {
-  constexpr int NW = kLanesKnnWarps;
+__global__ void __launch_bounds__(kKnnWarps * 32, 1) k_lanes_knn(ScanArgs a) {
   constexpr uint32_t CNONE = 0xffffu;  // CAT: an empty list place (above every category)
   extern __shared__ __align__(16) unsigned char smem[];
   const int H = a.H, K = a.kmax, EM = a.emax;
+  const int NW = blockDim.x >> 5;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // per warp: float rows -- the lists (EM * K rows) or, with CAT, one threshold
   // row per set -- then the row of "no set"; with CAT the category rows after
@@ -2589,16 +2667,11 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
   float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
   float4* boxA = (float4*)sp; sp += NW * 2 * 16;
   uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
+  uint32_t* queueA = (uint32_t*)sp; sp += NW * 64 * 4;
   float* listA = (float*)sp; sp += (size_t)NW * frows * 32 * 4;
-  uint16_t* catA = (uint16_t*)sp; sp += CAT ? (((size_t)NW * EM * K * 32 * 2 + 15) & ~size_t(15)) : 0;
-  float* sT = (float*)sp; sp += ((H + 4) & ~3) * 4;  // H thresholds, then +inf
-  int8_t* scs = (int8_t*)sp; sp += 256;
-  uint16_t* slut = (uint16_t*)sp;  // unless a.cat_fast
+  uint16_t* catA = (uint16_t*)sp; sp += CAT ? (size_t)NW * EM * K * 32 * 2 : 0;
   const uint32_t RSTRIDE = CAT ? 32u : (uint32_t)K * 32u;  // float rows between sets
-  for (int i = threadIdx.x; i <= H; i += blockDim.x) sT[i] = i < H ? a.cat_T[i] : kInf();
-  if (!a.cat_fast)
-    for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) scs[i] = a.cslot_of[i];
+  const KnnCommon nc(a, sp);
   __syncthreads();
 
   float4* cand = candA + warp * kStageAll;
@@ -2615,17 +2688,7 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
   uint32_t me = 0xffffffffu;      // this lane's centre slot
 
   auto start = [&](uint32_t self) {
-    float4 cp = make_float4(kInf(), kInf(), kInf(), 0.f);
-    cs = -1;
-    if (self != 0xffffffffu) {
-      cp = a.ions[self];
-      const uint32_t ct = a.labels ? (uint32_t)a.labels[self] : __float_as_uint(cp.w);
-      cs = scs[ct & 255];
-      if (cs < 0) {  // selection guarantees a slot; record and drop the centre otherwise
-        atomicOr(a.status, ST_TYPE_RANGE);
-        cp = make_float4(kInf(), kInf(), kInf(), 0.f);
-      }
-    }
+    const float4 cp = nc.start(self, cs);
     nset = cs >= 0 ? a.nsets[cs] : 0;
     sh = 4 * (cs < 0 ? 0 : cs);
     if constexpr (CAT) {
@@ -2638,20 +2701,13 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
     inb = 0;
     return cp;
   };
-  // category of an in-ball d^2 (see k_lanes)
-  const FastCat fc(a);
-  auto category_of = [&](float d2) -> int {
-    if (!a.cat_fast) return category_lut(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT, H);
-    const int g = (int)(fc.guess4(d2) >> 2);
-    return g + (sT[g + 1] <= d2 ? 1 : 0);
-  };
   // float row (offset) of a staged key's environment set for this lane's centre type
   auto row_of = [&](uint32_t w) -> uint32_t { return UNI ? w : ((w >> sh) & 15u) * RSTRIDE; };
   auto insert = [&](uint32_t row, float d2) {
     float* Lp = L + row;  // row s holds rank K - 1 - s
     if (!(d2 < Lp[0])) return;
     if constexpr (CAT) {
-      const int c = category_of(d2);
+      const int c = nc.category_of(d2);
       uint16_t* Cp = C + (row / 32u) * (uint32_t)K * 32u;
       if constexpr (KB > 0) {
         int v[KB];
@@ -2663,7 +2719,7 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
 #pragma unroll
         for (int s = 0; s < KB; ++s)
           if (s < K) Cp[s * 32] = (uint16_t)v[s];
-        Lp[0] = (v[0] == (int)CNONE) ? RUP : sT[v[0]];
+        Lp[0] = (v[0] == (int)CNONE) ? RUP : nc.sT[v[0]];
       } else {
         int r = K - 1;
         while (r > 0) {
@@ -2674,7 +2730,7 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
         }
         Cp[(K - 1 - r) * 32] = (uint16_t)c;
         const int kth = Cp[0];
-        Lp[0] = (kth == (int)CNONE) ? RUP : sT[kth];
+        Lp[0] = (kth == (int)CNONE) ? RUP : nc.sT[kth];
       }
     } else if constexpr (KB > 0) {
       // the sorted list with d2 in and its largest value out, as a min/max
@@ -2732,40 +2788,30 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
     if (lane == 0) centres += (unsigned long long)__popc(live);
     // every live centre met itself once in the in-ball count (d^2 = 0)
     pairs_lane += inb - (me != 0xffffffffu ? 1u : 0u);
-    // the k-th smallest d^2 (category) of each set -> its bin (or the miss
-    // bin); with KB, a set's categories are found first (independent loads)
-    // and added after
+    // the k-th smallest d^2 (category) of each set -> its bin
     for (int p = 0; p < nset; ++p) {
-      const int Sg = a.set_list[cs * 32 + p];
-      unsigned long long* core = a.knn_core + ((uint64_t)cs * a.nS + Sg) * a.nkI * H;
-      auto cat_of = [&](int kk) {
+      unsigned long long* core = nc.core(cs, p);
+      int kk = 0;
+      for (; kk < a.nkI; ++kk) {  // orders ascend: the first one missing ends them
+        const int row = p * K + K - a.kvals[kk];
+        int cat;
         if constexpr (CAT) {
-          const int v = C[(p * K + K - a.kvals[kk]) * 32];
-          return (v == (int)CNONE) ? a.cat_miss : v;
+          cat = C[row * 32];
+          if (cat == (int)CNONE) break;
         } else {
-          const float v = L[(p * K + K - a.kvals[kk]) * 32];
-          return (v == RUP) ? a.cat_miss : category_of(v);
+          const float v = L[row * 32];
+          if (v == RUP) break;
+          cat = nc.category_of(v);
         }
-      };
-      if constexpr (KB > 0) {
-        int cats[KB];
-#pragma unroll
-        for (int kk = 0; kk < KB; ++kk) cats[kk] = kk < a.nkI ? cat_of(kk) : -1;
-#pragma unroll
-        for (int kk = 0; kk < KB; ++kk)
-          if (cats[kk] >= 0) atomicAdd(&core[(uint64_t)kk * H + cats[kk]], 1ull);
-      } else {
-        for (int kk = 0; kk < a.nkI; ++kk) {
-          const int cat = cat_of(kk);
-          if (cat >= 0) atomicAdd(&core[(uint64_t)kk * H + cat], 1ull);
-        }
+        atomicAdd(&core[(uint64_t)kk * H + cat], 1ull);
       }
+      nc.found(cs, p, kk);
     }
   };
   unsigned long long tests = 0;  // (centre, staged ion) distance tests, warp-uniform
   const float4* sbox = boxA + warp * 2;
   const int nrows = (max(a.by, 1) + 2 * a.bsr) * (max(a.bz, 1) + 2 * a.bsr);
-  lanes_blocks(a, boxA + warp * 2, start, [&](const LaneBatch& B) {
+  lanes_blocks(a, boxA + warp * 2, queueA + warp * 64, start, [&](const LaneBatch& B) {
     const uint32_t staged = stage_rows<false, false, false>(
         a, B, nrows, a.R, a.box_R2, 0u, cand, skey, sbox, [&](uint32_t base, uint32_t nb, bool keyed) {
           batch(base, nb, keyed, B.self, B.cxx, B.cyy, B.czz);
@@ -2780,6 +2826,8 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
     atomicAdd(&a.counters[0], pairs_lane);
     atomicAdd(&a.counters[1], centres);
   }
+  __syncthreads();
+  nc.flush_found();
 }
 
 // kNN passes in two walks, for uniform disjoint sets of which some are dense
@@ -2788,85 +2836,19 @@ __global__ void __launch_bounds__(kLanesKnnWarps * 32, 3) k_lanes_knn(ScanArgs a
 // from the set's mean density (near_r, k_lanes_near), and only the ions of the
 // other, sparse sets -- a list of their own, a few per cent of the ions --
 // within R (k_lanes_sparse).  On the 20M-ion tip (k <= 10, R = 2 nm) a batch of
-// centres meets 0.29k ions instead of 1.3k.  Two kernels, not one with both
-// walks: together they miss the instruction cache (5.9 of 12.7 cycles per
-// instruction).  In-ball pairs are not counted by either (see run_near).
+// centres meets 0.29k ions instead of 1.3k: 5.3 + 4.9 ms where k_lanes_knn
+// takes 28.  Two kernels, not one with both walks: together they miss the
+// instruction cache (5.9 of 12.7 cycles per instruction; 19.0 against 13.5 ms).
+// In-ball pairs are not counted by either (see run_near; 7.5 ms here).
 //
 // Bins: most centres are of one type (near_hot), and adding its categories to
 // the cores in global memory took longer than finding them.  They are counted
 // in shared memory, a dense set's below near_hd in 32 bits each, a sparse set's
 // in 16 bits each, moved to the cores every 2^15 centres of the block; the
-// other centres' go to the cores.  Missing neighbours, most of the sparse
-// sets' orders, are counted once per set and centre, by the orders found.
-constexpr int kNearWarps = 24;  // most warps of a block; one block per SM
+// other centres' go to the cores.
 
 // Rows (of 32 lanes) of a dense set's buffer: about 2 K and what eight tests add.
 __host__ __device__ constexpr int near_cap(int KB) { return 2 * KB + 28; }
-
-// The parts the two kernels share: tables in shared memory, categories, and
-// the counts of found orders.
-struct NearCommon {
-  const ScanArgs& a;
-  float* sT;
-  uint32_t* sfound;  // [centre slot][set][orders found]
-  int8_t* scs;
-  uint16_t* slut;
-  FastCat fc;
-  __device__ __forceinline__ NearCommon(const ScanArgs& a_, unsigned char*& sp) : a(a_), fc(a_) {
-    const int H = a.H;
-    sT = (float*)sp; sp += ((H + 4) & ~3) * 4;  // H thresholds, then +inf
-    const uint32_t nfound = (uint32_t)a.nC * a.emax * (a.nkI + 1);
-    sfound = (uint32_t*)sp; sp += (size_t)nfound * 4;
-    scs = (int8_t*)sp; sp += 256;
-    slut = (uint16_t*)sp;  // unless a.cat_fast
-    for (int i = threadIdx.x; i <= H; i += blockDim.x) sT[i] = i < H ? a.cat_T[i] : kInf();
-    for (uint32_t i = threadIdx.x; i < nfound; i += blockDim.x) sfound[i] = 0;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) scs[i] = a.cslot_of[i];
-    if (!a.cat_fast)
-      for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
-  }
-  __device__ __forceinline__ int category_of(float d2) const {
-    if (!a.cat_fast) return category_lut(d2, slut, a.lut_n, a.lut_base, a.lut_shift, sT, a.H);
-    const int g = (int)(fc.guess4(d2) >> 2);
-    return g + (sT[g + 1] <= d2 ? 1 : 0);
-  }
-  __device__ __forceinline__ float4 start(uint32_t self, int& cs) const {
-    float4 cp = make_float4(kInf(), kInf(), kInf(), 0.f);
-    cs = -1;
-    if (self != 0xffffffffu) {
-      cp = a.ions[self];
-      const uint32_t ct = a.labels ? (uint32_t)a.labels[self] : __float_as_uint(cp.w);
-      cs = scs[ct & 255];
-      if (cs < 0) {  // selection guarantees a slot; record and drop the centre otherwise
-        atomicOr(a.status, ST_TYPE_RANGE);
-        cp = make_float4(kInf(), kInf(), kInf(), 0.f);
-      }
-    }
-    return cp;
-  }
-  __device__ __forceinline__ unsigned long long* core(int cs, int p) const {
-    return a.knn_core + ((uint64_t)cs * a.nS + a.set_list[cs * 32 + p]) * a.nkI * a.H;
-  }
-  __device__ __forceinline__ void found(int cs, int p, int orders) const {
-    if (orders < a.nkI) atomicAdd(&sfound[((uint32_t)cs * a.emax + p) * (a.nkI + 1) + orders], 1u);
-  }
-  // the missing orders' counts (after a block barrier)
-  __device__ __forceinline__ void flush_found() const {
-    if (a.cat_miss < 0) return;
-    const uint32_t nfound = (uint32_t)a.nC * a.emax * (a.nkI + 1);
-    for (uint32_t i = threadIdx.x; i < nfound; i += blockDim.x) {
-      const uint32_t v = sfound[i];
-      if (!v) continue;
-      const uint32_t f = i % (a.nkI + 1), p = (i / (a.nkI + 1)) % a.emax, c = i / (a.nkI + 1) / a.emax;
-      for (int kk = f; kk < a.nkI; ++kk)  // found the first f orders: the rest are missing
-        atomicAdd(&core(c, p)[(uint64_t)kk * a.H + a.cat_miss], (unsigned long long)v);
-    }
-  }
-};
-static size_t near_common_smem(const ScanArgs& a) {
-  return (size_t)((a.H + 4) & ~3) * 4 + (size_t)a.nC * a.emax * (a.nkI + 1) * 4 + 256 +
-         (a.cat_fast ? 0 : (size_t)((a.lut_n + 7) & ~7) * 2);
-}
 
 // The K <= KB smallest of the cnt values L[i * 32] of each lane, ascending
 // (+inf: none), in v[KB - K .. KB): the places before hold -inf, so that the
@@ -2892,7 +2874,7 @@ __device__ __forceinline__ void near_smallest(const float* L, int cnt, int K, fl
 // 1.5 r, up to R (every ion within r of a lane's centre is within r of the
 // batch's box).
 template <int KB>
-__global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_near(ScanArgs a) {
+__global__ void __launch_bounds__(kKnnWarps * 32, 1) k_lanes_near(ScanArgs a) {
   constexpr int CAP = near_cap(KB);
   extern __shared__ __align__(16) unsigned char smem[];
   const int H = a.H, K = a.kmax, HD = a.near_hd, nkI = a.nkI;
@@ -2902,11 +2884,12 @@ __global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_near(ScanArgs a) {
   float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
   float4* boxA = (float4*)sp; sp += NW * 2 * 16;
   uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
+  uint32_t* queueA = (uint32_t*)sp; sp += NW * 64 * 4;
   float* listA = (float*)sp; sp += (size_t)NW * CAP * 32 * 4;
   const uint32_t nhist = (uint32_t)a.near_n * nkI * HD;  // the hot centre slot's [set][order][HD]
   uint32_t* shist = (uint32_t*)sp; sp += (size_t)nhist * 4;
   for (uint32_t i = threadIdx.x; i < nhist; i += blockDim.x) shist[i] = 0;
-  const NearCommon nc(a, sp);
+  const KnnCommon nc(a, sp);
   __syncthreads();
   float4* cand = candA + warp * kStageAll;
   uint32_t* skey = skeyA + warp * kStageAll;
@@ -2919,7 +2902,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_near(ScanArgs a) {
   const int nrows = (max(a.by, 1) + 2 * a.bsr) * (max(a.bz, 1) + 2 * a.bsr);
   const uint32_t buf = smem_addr(L);
 
-  lanes_blocks(a, boxA + warp * 2, [&](uint32_t self) { return nc.start(self, cs); }, [&](const LaneBatch& B) {
+  lanes_blocks(a, boxA + warp * 2, queueA + warp * 64, [&](uint32_t self) { return nc.start(self, cs); }, [&](const LaneBatch& B) {
     if (lane == 0) centres += (unsigned long long)__popc(B.live);
     for (int dn = 0; dn < a.near_n; ++dn) {
       bool need = cs >= 0;
@@ -3022,7 +3005,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_near(ScanArgs a) {
 // Sparse sets together: threshold test and sorted insertion as in k_lanes_knn
 // (CAT: the lists hold categories), over the sparse list.
 template <int KB, bool CAT>
-__global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_sparse(ScanArgs a) {
+__global__ void __launch_bounds__(kKnnWarps * 32, 1) k_lanes_sparse(ScanArgs a) {
   constexpr uint32_t CNONE = 0xffffu;
   extern __shared__ __align__(16) unsigned char smem[];
   const int H = a.H, K = a.kmax, SPN = a.near_sp, nkI = a.nkI;
@@ -3033,6 +3016,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_sparse(ScanArgs a)
   float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
   float4* boxA = (float4*)sp; sp += NW * 2 * 16;
   uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
+  uint32_t* queueA = (uint32_t*)sp; sp += NW * 64 * 4;
   float* listA = (float*)sp; sp += (size_t)NW * lrows * 32 * 4;
   // the hot centre slot's bins [set][order][H], halfwords; centres taken
   const uint32_t nhalf = a.near_hs ? ((uint32_t)SPN * nkI * H + 1) / 2 : 0u;
@@ -3040,7 +3024,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_sparse(ScanArgs a)
   uint32_t* shalf = (uint32_t*)sp; sp += (size_t)nhalf * 4;
   for (uint32_t i = threadIdx.x; i < nhalf; i += blockDim.x) shalf[i] = 0;
   if (threadIdx.x == 0) *sflush = 0;
-  const NearCommon nc(a, sp);
+  const KnnCommon nc(a, sp);
   __syncthreads();
   float4* cand = candA + warp * kStageAll;
   uint32_t* skey = skeyA + warp * kStageAll;
@@ -3066,7 +3050,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 1) k_lanes_sparse(ScanArgs a)
       }
     }
   };
-  lanes_blocks(a, boxA + warp * 2, [&](uint32_t self) { return nc.start(self, cs); }, [&](const LaneBatch& B) {
+  lanes_blocks(a, boxA + warp * 2, queueA + warp * 64, [&](uint32_t self) { return nc.start(self, cs); }, [&](const LaneBatch& B) {
     if constexpr (CAT) {
       for (int p = 0; p < SPN; ++p) L[p * 32] = RUP;
       for (int e = 0; e < SPN * K; ++e) C[e * 32] = (uint16_t)CNONE;
@@ -4095,7 +4079,7 @@ static void launch_pass_codes(const ScanArgs& a, PassCode kind, uint32_t param, 
 // Shared memory of k_lanes with `bins` shared bins (0 = none).
 static size_t lanes_smem(const ScanArgs& a, size_t bins, bool fast) {
   constexpr int NW = kLanesWarps;
-  return 16 + NW * kStageAll * 16 + NW * 2 * 16 + NW * kStageAll * 4 + 32 * 4 + (size_t)((a.H + 4) & ~3) * 4 + bins * 4 +
+  return 16 + NW * kStageAll * 16 + NW * 2 * 16 + NW * (kStageAll + 64) * 4 + 32 * 4 + (size_t)((a.H + 4) & ~3) * 4 + bins * 4 +
          3 * 256 +
          (fast ? 0 : (size_t)((a.lut_n + 7) & ~7) * 2);
 }
@@ -4153,7 +4137,7 @@ int launch_lanes_near(const ScanArgs& a0, int sm_count, uint32_t* sp_start, uint
       a.by < 1 || a.bz < 1 || !a.brows || a.nC > 127 || a.emax > 15 || a.near_n < 1 || a.near_n > kNearMax)
     return -3;
   const int KB = a.kmax <= 8 ? 8 : a.kmax <= 10 ? 10 : a.kmax <= 16 ? 16 : 20;
-  const size_t cap = 224 * 1024, common = near_common_smem(a), stage = (size_t)kStageAll * 20 + 32;
+  const size_t cap = 224 * 1024, common = knn_common_smem(a), stage = (size_t)kStageAll * 20 + 32 + 256;
   // the hot centre type's shared bins while they leave the warps room
   a.near_hs = a.near_sp > 0 && ((size_t)a.near_sp * a.nkI * a.H + 1) / 2 * 4 <= 90 * 1024 ? 1 : 0;
   if ((size_t)a.near_n * a.nkI * a.near_hd * 4 > 64 * 1024) a.near_hd = 0;
@@ -4164,7 +4148,7 @@ int launch_lanes_near(const ScanArgs& a0, int sm_count, uint32_t* sp_start, uint
     return stage + (size_t)(frows + (cat ? (a.near_sp * a.kmax + 1) / 2 : 0)) * 128;
   };
   auto warps = [&](size_t fix, size_t each) {
-    return fix >= cap ? 0 : (int)std::min<size_t>(kNearWarps, (cap - fix) / each);
+    return fix >= cap ? 0 : (int)std::min<size_t>(kKnnWarps, (cap - fix) / each);
   };
   // category lists for the sparse sets where distances would leave fewer than
   // 16 warps
@@ -4207,30 +4191,26 @@ int launch_lanes_near(const ScanArgs& a0, int sm_count, uint32_t* sp_start, uint
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-size_t lanes_knn_smem(const ScanArgs& a, bool cat) {
-  constexpr int NW = kLanesKnnWarps;
-  const size_t em = a.emax > 1 ? a.emax : 1;
-  const size_t frows = cat ? em + 1 : em * a.kmax + 1;
-  const size_t crows = cat ? (((size_t)NW * em * a.kmax * 32 * 2 + 15) & ~size_t(15)) : 0;
-  return NW * kStageAll * 16 + NW * 2 * 16 + NW * kStageAll * 4 + (size_t)NW * frows * 32 * 4 + crows + (size_t)((a.H + 4) & ~3) * 4 +
-         (a.cat_fast ? 0 : (size_t)((a.lut_n + 7) & ~7) * 2) + 256;
-}
-
 int launch_lanes_knn(const ScanArgs& a, bool disjoint_sets, int sm_count, size_t* smem_used, cudaStream_t s) {
-  if (a.mode != 0 || (a.flags & (PP_CNTNB | PP_RDF)) || !disjoint_sets || a.kmax < 1 || a.kmax > 64 || a.bx < 1 ||
-      a.by < 1 || a.bz < 1 || !a.brows || a.nC > 8 || a.emax > 15)  // sets packed 4 bits per centre slot
+  if (a.mode != 0 || (a.flags & (PP_CNTNB | PP_RDF)) || !disjoint_sets || a.kmax < 1 || a.kmax > 64 || a.by < 1 ||
+      a.bz < 1 || !a.brows || a.nC > 8 || a.emax > 15)  // sets packed 4 bits per centre slot
     return -3;
-  // d^2 lists while they leave room for two blocks of 8 warps per SM;
+  // one block per SM of as many warps as fit; d^2 lists while at least 16 do,
   // category lists beyond that (e.g. 8 sets of k = 20: 20.6 KB a warp as d^2,
-  // 11.4 KB as categories); one block per SM for the largest
-  bool cat = a.lists_mode == 2;
-  size_t smem = lanes_knn_smem(a, cat);
-  if (!cat && a.lists_mode == 0 && smem > 110 * 1024 && lanes_knn_smem(a, true) < smem) {
-    cat = true;
-    smem = lanes_knn_smem(a, true);
-  }
+  // 11.4 KB as categories)
+  const size_t cap = 224 * 1024, fix = knn_common_smem(a), em = a.emax > 1 ? a.emax : 1;
+  auto warp_bytes = [&](bool cat) {
+    const size_t rows = cat ? em + 1 : em * a.kmax + 1;
+    return (size_t)kStageAll * 20 + 32 + 256 + rows * 128 + (cat ? em * a.kmax * 64 : 0);
+  };
+  auto warps = [&](bool cat) {
+    return fix >= cap ? 0 : (int)std::min<size_t>(kKnnWarps, (cap - fix) / warp_bytes(cat));
+  };
+  const bool cat = a.lists_mode == 2 || (a.lists_mode == 0 && warps(false) < 16 && warps(true) > warps(false));
+  const int NW = warps(cat);
+  const size_t smem = fix + warp_bytes(cat) * NW;
   if (smem_used) *smem_used = smem;
-  if (smem > 200 * 1024 || (cat && a.H > 65535)) return -3;
+  if (NW < 1 || (cat && a.H > 65535)) return -3;
   const bool uni = a.uniform_sets != 0;
 #define PP_KNN_KERN(KBV) \
   (cat ? (uni ? k_lanes_knn<KBV, true, true> : k_lanes_knn<KBV, false, true>) \
@@ -4244,12 +4224,8 @@ int launch_lanes_knn(const ScanArgs& a, bool disjoint_sets, int sm_count, size_t
   if (!allow_dynamic_smem((const void*)kern, smem))
     return -1;
   launch_pass_codes(a, uni ? PC_ROW : PC_NIBBLE, cat ? 32u : (uint32_t)a.kmax * 32u, sm_count, s);
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLanesKnnWarps * 32, smem) != cudaSuccess ||
-      per_sm < 1)
-    return -1;
   counted();
-  kern<<<sm_count * per_sm, kLanesKnnWarps * 32, smem, s>>>(a);
+  kern<<<sm_count, NW * 32, smem, s>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
