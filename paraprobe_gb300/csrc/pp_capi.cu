@@ -100,7 +100,7 @@ struct Cloud {
   // hull / ion2surf
   // tuning (pp_autotune): cell edge = R / cell_ratio, centres per block tile
   float cell_ratio = 4.0f;
-  uint32_t tile = 128;
+  uint32_t tile = 0;  // 0 = untuned: by the pass's centres
   // brick scan: (cells per brick << 16) | centres per warp batch; 0 = the
   // per-centre scan with `tile` centres per block work item
   uint32_t brick = 0;
@@ -836,7 +836,9 @@ void fill_scan_common(pp::ScanArgs& a, const Cloud& cl, const RunPlan& P, const 
   a.uniform_sets = 1;
   for (int c = 1; c < P.nC && a.uniform_sets; ++c)
     if (std::memcmp(&P.setidx[(size_t)c * 256], &P.setidx[0], 256) != 0) a.uniform_sets = 0;
-  a.tile = std::max<uint32_t>(cl.tile, 1);
+  // centres per block work item of the per-centre scan; untuned, few centres
+  // are spread over the device instead (set by the passes that know them)
+  a.tile = cl.tile ? cl.tile : 128;
   a.rowtab = D.rowtab;
   a.sym = 0;
 }
@@ -1602,6 +1604,9 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
   a.labels = labels;
   a.centres = ctx->centres.as<uint32_t>();
   a.ncentres = ncent;
+  // at least 8 work items a SM down to a centre per warp: 4k centres in items
+  // of 128 kept 32 of 152 SMs busy
+  if (!cl->tile) a.tile = std::min<uint32_t>(128, std::max<uint32_t>(8, ncent / (8u * (uint32_t)ctx->sm_count)));
   if (no_miss) a.cat_miss = -1;
   a.flags = flags & (PP_RDF | PP_RIPK | PP_CNTNB);
   if (flags & PP_RIPK) a.flags |= PP_RDF;
@@ -3053,7 +3058,7 @@ void run_multi(pp_ctx* w, const std::vector<ServerRequest*>& qs, cudaStream_t s)
     m.counters = counters;
     m.rdf_words = (uint32_t)rdf_words;
     m.lists = lists;
-    m.tile = 32;
+    m.tile = std::min<uint32_t>(32, std::max<uint32_t>(4, m.ncentres / (8u * (uint32_t)w->sm_count)));  // a warp each, at least
     m.work = w->work.as<uint32_t>();
     size_t smem = 0;
     const int rc = pp::launch_multi(m, w->sm_count, &smem, s);
