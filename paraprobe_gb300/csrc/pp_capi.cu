@@ -200,6 +200,8 @@ struct pp_ctx {
   DevBuf tri_fill, cflag, rowtab, nc_pre, pass_code;
   DevBuf type_counts, sp_start, sp_ions, sp_slot;  // kNN passes in two walks
   DevBuf labels_run, perm_dev, gather_src;
+  DevBuf neigh;    // pp_neighbors: count and records
+  PinBuf neigh_stage;
   DevBuf mask_in;  // caller's centre mask: [n] input order, then [n] sorted-slot order
   // statistics after clustering: option "aposteriori_guard" = 1 runs the
   // reference's guard loop as written (see pp_run_aposteriori)
@@ -2242,29 +2244,32 @@ int pp_neighbors(pp_ctx* ctx, int cloud, uint64_t ion, float r, uint64_t* ids, f
   CK(cudaSetDevice(ctx->device));
   int rc = ensure_grid(ctx, *cl, r, 0);
   if (rc) return rc;
-  uint32_t self = 0;
-  CK(cudaMemcpy(&self, cl->slot_of_id.as<uint32_t>() + ion, 4, cudaMemcpyDeviceToHost));
-  const uint32_t dcap = 1u << 22;
-  DevBuf bs, bd, bc;
-  CK(bs.ensure(dcap * 4));
-  CK(bd.ensure(dcap * 4));
-  CK(bc.ensure(4));
-  CK(cudaMemset(bc.p, 0, 4));
-  pp::launch_neighbors(cl->ions.as<float4>(), cl->cell_start.as<uint32_t>(), cl->g, self, r, nullptr,
-                       bs.as<uint32_t>(), bd.as<float>(), dcap, bc.as<uint32_t>(), 0);
+  // one buffer, kept by the context: the count, then (d^2 bits, input index)
+  // records; the first kHead records come with the count
+  constexpr uint32_t dcap = 1u << 22, kHead = 4095;
+  CK(ctx->neigh.ensure((size_t)(dcap + 1) * 8));
+  CK(ctx->neigh_stage.ensure((size_t)(kHead + 1) * 8));
+  CK(cudaMemsetAsync(ctx->neigh.p, 0, 8, 0));
+  pp::launch_neighbors(cl->ions.as<float4>(), cl->cell_start.as<uint32_t>(), cl->g, cl->slot_of_id.as<uint32_t>(),
+                       cl->id_of_slot.as<uint32_t>(), (uint32_t)ion, r, ctx->neigh.p, dcap, 0);
   CK(cudaGetLastError());
-  uint32_t cnt = 0;
-  CK(cudaMemcpy(&cnt, bc.p, 4, cudaMemcpyDeviceToHost));
+  CK(cudaMemcpyAsync(ctx->neigh_stage.p, ctx->neigh.p, (size_t)(kHead + 1) * 8, cudaMemcpyDeviceToHost, 0));
+  CK(cudaStreamSynchronize(0));
+  struct Rec { uint32_t d2, id; };
+  const Rec* rec = static_cast<const Rec*>(ctx->neigh_stage.p);
+  const uint32_t cnt = rec[0].d2;
   if (cnt > dcap) return fail(ctx, PP_ERR_OVERFLOW, "more than %u neighbours", dcap);
-  std::vector<uint32_t> slots(cnt), id_of(cl->n);
-  std::vector<float> dd(cnt);
-  CK(cudaMemcpy(slots.data(), bs.p, cnt * 4, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(dd.data(), bd.p, cnt * 4, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(id_of.data(), cl->id_of_slot.p, cl->n * 4, cudaMemcpyDeviceToHost));
+  std::vector<Rec> all;
+  if (cnt > kHead) {
+    all.resize((size_t)cnt + 1);
+    CK(cudaMemcpy(all.data(), ctx->neigh.p, ((size_t)cnt + 1) * 8, cudaMemcpyDeviceToHost));
+    rec = all.data();
+  }
   std::vector<std::pair<float, uint64_t>> v(cnt);
   for (uint32_t k = 0; k < cnt; ++k) {
-    const uint32_t idx = id_of[slots[k]];
-    v[k] = {dd[k], cl->ids.empty() ? (uint64_t)idx : (uint64_t)cl->ids[idx]};
+    float d;
+    std::memcpy(&d, &rec[k + 1].d2, 4);
+    v[k] = {d, cl->ids.empty() ? (uint64_t)rec[k + 1].id : (uint64_t)cl->ids[rec[k + 1].id]};
   }
   std::sort(v.begin(), v.end());
   *count = cnt;

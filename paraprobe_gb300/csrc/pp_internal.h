@@ -370,9 +370,8 @@ void launch_perm_mask(const uint8_t* labels_r, const uint32_t* centres, uint32_t
                       const int8_t* cslot_of, uint8_t* centre_ok, cudaStream_t s);
 void launch_exclusive_scan_u64_from_u32(const uint32_t* in, uint64_t n, unsigned long long* out,
                                         unsigned long long* tmp, uint64_t tmp_elems, cudaStream_t s);
-void launch_neighbors(const float4* ions, const uint32_t* cell_start, Grid g, uint32_t self,
-                      float R, const uint32_t* id_of_slot, uint32_t* out_slot, float* out_d2,
-                      uint32_t cap, uint32_t* count, cudaStream_t s);
+void launch_neighbors(const float4* ions, const uint32_t* cell_start, Grid g, const uint32_t* slot_of_id,
+                      const uint32_t* id_of_slot, uint32_t ion, float R, void* out, uint32_t cap, cudaStream_t s);
 
 unsigned long long kernel_launches();
 // FP64 audit of the float distances and bins of the selected centres.
