@@ -272,6 +272,10 @@ int pp_fetch_npcorr(pp_ctx* ctx, uint32_t* counts, uint64_t cap, uint64_t* edge)
  *   "aposteriori_guard" pp_run_aposteriori's guard zone: 0 = every
  *                       unclustered ion within R of a clustered ion (default),
  *                       1 = the reference's guard loop as written (see there).
+ *   "batched_minor"     pp_run_batched counts the pairs and members of the type
+ *                       most ions are of by what is not of it: 0 = never, 1 =
+ *                       where three quarters of the ions are (default), 2 =
+ *                       always.  Results are identical either way.
  *   "batched_pair_cap"  most pairs pp_run_batched holds at once; larger lists
  *                       are built and applied a chunk of centres at a time
  *                       (0 = sized from free device memory, the default). */

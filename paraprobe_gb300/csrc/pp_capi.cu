@@ -215,6 +215,7 @@ struct pp_ctx {
   DevBuf labels_il, ok_il;  // group-major interleaved copies of real_labels / centre_ok
   DevBuf knn_labels, knn_ok, knn_rec, knn_recc;  // 32-realisation kNN: layouts and records
   DevBuf knn_rest_labels, knn_rest_ok;           // the realisations after the last full 32
+  DevBuf minor_masks, minor_sums;                // batched runs of clouds of one common type
   DevBuf maxlist;           // longest pair list (one uint32)
   uint32_t geo_maxlist = 0;
   uint64_t geo_key_version = ~0ull;
@@ -223,6 +224,7 @@ struct pp_ctx {
   uint32_t geo_ncentres = 0;
   uint64_t geo_pairs = 0;
   bool geo_emitted_all = false;  // the pair buffer holds every list (not one chunk's)
+  int batched_minor = 1;         // option "batched_minor": see pp_run_batched
   uint64_t pair_cap_opt = 0;     // option "batched_pair_cap": most pairs held at once (0 = by free memory)
   uint32_t npc_order = 0;        // option "npcorr_order": SpatStatKNNOrder - 1 of the n-point correlations
   DevBuf geo_counters;           // pair counters of the geometry passes
@@ -2128,6 +2130,11 @@ int pp_set_option(pp_ctx* ctx, const char* name, int value) {
     ctx->knn_walks = value;
     return PP_OK;
   }
+  if (std::strcmp(name, "batched_minor") == 0) {
+    if (value < 0 || value > 2) return fail(ctx, PP_ERR_INVALID, "batched_minor must be 0, 1 or 2");
+    ctx->batched_minor = value;
+    return PP_OK;
+  }
   if (std::strcmp(name, "npcorr_order") == 0) {
     if (value < 0 || value > 31) return fail(ctx, PP_ERR_INVALID, "npcorr_order must be in [0, 31]");
     ctx->npc_order = (uint32_t)value;
@@ -2549,8 +2556,63 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
       knn32 = pp::knn32_check(kq) == 0;
       if (knn32) b.flags &= ~PP_MKNN;
     }
+    // clouds of one common type: RDF of the label sets and kNN by what is not
+    // of it (k_minor_walk), where its bins fit.  Its work grows with the share
+    // of the other ions, and at a quarter of them is still the smaller one.
+    const int nlab = nreal - n_rois;
+    bool minor_rdf = false, minor_knn = false;
+    {
+      std::vector<unsigned long long> tc(256);
+      CK(ctx->type_counts.ensure(256 * 8));
+      CK(cudaMemsetAsync(ctx->type_counts.p, 0, 256 * 8, s));
+      pp::launch_type_count(cl->label_sorted.as<uint8_t>(), n, ctx->type_counts.as<unsigned long long>(), ctx->sm_count, s);
+      CK(cudaMemcpyAsync(tc.data(), ctx->type_counts.p, 256 * 8, cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+      const int dom = (int)(std::max_element(tc.begin(), tc.end()) - tc.begin());
+      if (ctx->batched_minor && (ctx->batched_minor == 2 || 4 * tc[dom] >= 3 * n)) {
+        kq.dom = dom;
+        kq.dom_c = P.cslot_of[dom];
+        kq.dom_e = P.eslot_of[dom];
+        kq.nE = P.nE;
+        kq.eslot_of = D.eslot;
+        kq.rdf_core = b.rdf_core;
+        kq.counters = b.counters;
+        kq.nlab = nlab;
+        kq.centres = b.centres;
+        kq.ncentres = nc;
+        kq.pair_off = b.pair_off;
+        kq.pair_slot = b.pair_slot;
+        kq.pair_cat = b.pair_cat;
+        kq.n = n;
+        kq.nreal = nreal;
+        kq.cslot_of = D.cslot;
+        kq.nsets = D.nsets;
+        kq.nC = P.nC;
+        kq.H = P.H;
+        const int want_knn = knn32 && P.disjoint, want_rdf = nlab > 0 && (b.flags & PP_RDF) && !(b.flags & PP_MKNN);
+        for (int form = 0; form < 3 && !minor_rdf && !minor_knn; ++form) {
+          kq.do_rdf = form == 1 ? 0 : want_rdf;
+          kq.do_knn = form == 2 ? 0 : want_knn;
+          if ((kq.do_rdf || kq.do_knn) && pp::minor_warps(kq)) {
+            minor_rdf = kq.do_rdf != 0;
+            minor_knn = kq.do_knn != 0;
+          }
+        }
+        if (!minor_rdf && !minor_knn) kq.do_rdf = kq.do_knn = 0;
+      }
+    }
+    // the fused kernel is left with the regions of interest
+    const uint8_t* RLb = RL;
+    const uint8_t* OKb = OK;
+    int nrb = nreal;
+    if (minor_rdf) {
+      b.rbase = nlab;
+      b.nreal = nrb = n_rois;
+      RLb = RL + (uint64_t)nlab * n;
+      OKb = OK + (uint64_t)nlab * nc;
+    }
     if (pp::apply_configure(b)) return fail(ctx, PP_ERR_UNSUPPORTED, "RDF bins of one realisation exceed shared memory");
-    b.ngroups = (nreal + b.group - 1) / b.group;
+    b.ngroups = std::max(1, (nrb + b.group - 1) / b.group);
     // tile: enough pairs per item to amortise the per-item flush of the
     // shared bins, enough items to balance the persistent blocks, at most
     // 65535 centres (16-bit kNN bins) and fewer than 2^31 pairs (RDF bins)
@@ -2570,8 +2632,10 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
     const uint64_t nrg = (uint64_t)b.ngroups * b.group;
     CK(ctx->labels_il.ensure(std::max<uint64_t>(n, 1) * nrg));
     CK(ctx->ok_il.ensure(std::max<uint64_t>(nc, 1) * nrg));
-    pp::launch_interleave(RL, nreal, n, b.group, ctx->labels_il.as<uint8_t>(), s);
-    pp::launch_interleave(OK, nreal, nc, b.group, ctx->ok_il.as<uint8_t>(), s);
+    if (nrb) {
+      pp::launch_interleave(RLb, nrb, n, b.group, ctx->labels_il.as<uint8_t>(), s);
+      pp::launch_interleave(OKb, nrb, nc, b.group, ctx->ok_il.as<uint8_t>(), s);
+    }
     b.labels = ctx->labels_il.as<uint8_t>();
     b.centre_ok = ctx->ok_il.as<uint8_t>();
     int ng32 = 0;
@@ -2583,10 +2647,11 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
     pp::ApplyArgs bk;
     std::memset(&bk, 0, sizeof bk);
     bool knn_rest = false;
+    const int ngm = minor_knn ? (nreal + 31) / 32 : minor_rdf ? (nlab + 31) / 32 : 0;  // groups of k_minor_walk
     if (knn32) {
       const int rest = nreal % 32;
       ng32 = (nreal + 31) / 32;
-      if (rest > 0 && rest <= 8) {
+      if (rest > 0 && rest <= 8 && !minor_knn) {
         bk = b;
         bk.flags = PP_MKNN;
         bk.count = 0;
@@ -2606,16 +2671,6 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
           bk.centre_ok = ctx->knn_rest_ok.as<uint8_t>();
         }
       }
-      // the realisations of the 32-lane groups (all, or all but the rest)
-      const uint64_t r32 = std::min<uint64_t>((uint64_t)ng32 * 32, (uint64_t)nreal);
-      CK(ctx->knn_labels.ensure(std::max<uint64_t>(n, 1) * 32 * std::max(ng32, 1)));
-      CK(ctx->knn_ok.ensure(std::max<uint64_t>(nc, 1) * 32 * std::max(ng32, 1)));
-      if (r32) {
-        pp::launch_interleave(RL, r32, n, 32, ctx->knn_labels.as<uint8_t>(), s);
-        pp::launch_interleave(OK, r32, nc, 32, ctx->knn_ok.as<uint8_t>(), s);
-      }
-      kq.labels = ctx->knn_labels.as<uint8_t>();
-      kq.centre_ok = ctx->knn_ok.as<uint8_t>();
       // records of one launch: at most 3 GiB
       const uint64_t per_centre = NT * 64 + 32;
       chunk = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(nc, (3ull << 30) / per_centre));
@@ -2623,9 +2678,40 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
       CK(ctx->knn_recc.ensure((uint64_t)chunk * 32));
       kq.rec = ctx->knn_rec.as<uint16_t>();
       kq.rec_c = ctx->knn_recc.as<uint8_t>();
+    }
+    if (ng32 || ngm) {
+      // the realisations of the 32-lane groups (all, or all but the rest)
+      const int ngl = std::max(ng32, ngm);
+      const uint64_t r32 = std::min<uint64_t>((uint64_t)ngl * 32, (uint64_t)nreal);
+      CK(ctx->knn_labels.ensure(std::max<uint64_t>(n, 1) * 32 * ngl));
+      CK(ctx->knn_ok.ensure(std::max<uint64_t>(nc, 1) * 32 * ngl));
+      pp::launch_interleave(RL, r32, n, 32, ctx->knn_labels.as<uint8_t>(), s);
+      pp::launch_interleave(OK, r32, nc, 32, ctx->knn_ok.as<uint8_t>(), s);
+      kq.labels = ctx->knn_labels.as<uint8_t>();
+      kq.centre_ok = ctx->knn_ok.as<uint8_t>();
       kq.work = ctx->work.as<uint32_t>() + 1;
     }
+    uint64_t sums_bytes = 0;
+    if (ngm) {
+      CK(ctx->minor_masks.ensure(std::max<uint64_t>(n, 1) * 4 * ngm));
+      pp::launch_minor_masks(kq.labels, n * (uint64_t)ngm, kq.dom, ctx->minor_masks.as<uint32_t>(), s);
+      kq.minor = ctx->minor_masks.as<uint32_t>();
+      // sums of one call: cleared, filled and read by the graph.  The last
+      // group's lanes may lie past the realisations: rows for whole groups
+      const uint64_t rr = (uint64_t)ngm * 32, H = P.H;
+      const uint64_t nsa = rr * (uint64_t)(P.nC + 1) * H, nso = rr * (uint64_t)P.nC * H;
+      const uint64_t nfound = rr * (uint64_t)P.nC * std::max(P.emax, 1) * (P.kvals.size() + 1);
+      sums_bytes = (nsa + nso + H) * 8 + nfound * 4;
+      CK(ctx->minor_sums.ensure(sums_bytes));
+      kq.sa = ctx->minor_sums.as<unsigned long long>();
+      kq.so = kq.sa + nsa;
+      kq.tcat = kq.so + nso;
+      kq.found = (uint32_t*)(kq.tcat + H);
+      if (!knn32) chunk = nc;
+    }
     auto enqueue = [&](cudaStream_t st) -> int {
+      if (sums_bytes && cudaMemsetAsync(ctx->minor_sums.p, 0, sums_bytes, st) != cudaSuccess)
+        return fail(ctx, PP_ERR_CUDA, "memset failed");
       for (const Chunk& ch : chunks) {
         if (chunked) {
           set_emit_range(ch.c0, ch.c1, ch.p0, ch.p1);
@@ -2639,7 +2725,10 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
         bc.cbase = ch.c0;
         bc.pair_base = ch.p0;
         if (cudaMemsetAsync(ctx->work.p, 0, 8, st) != cudaSuccess) return fail(ctx, PP_ERR_CUDA, "memset failed");
-        if (pp::launch_apply(bc, ctx->sm_count, st)) return fail(ctx, PP_ERR_CUDA, "apply launch failed");
+        if (nrb && pp::launch_apply(bc, ctx->sm_count, st)) return fail(ctx, PP_ERR_CUDA, "apply launch failed");
+        if (minor_rdf &&
+            pp::launch_cat_hist(b.pair_cat, ch.p1 - ch.p0, P.H, kq.tcat, ctx->sm_count, st))
+          return fail(ctx, PP_ERR_CUDA, "pair sum launch failed");
         if (knn_rest) {
           pp::ApplyArgs kc = bk;
           kc.centres = bk.centres + ch.c0;
@@ -2653,14 +2742,21 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
         }
         pp::KnnArgs k = kq;
         k.pair_base = ch.p0;
-        for (int g = 0; g < ng32; ++g) {
+        for (int g = 0; g < std::max(ng32, ngm); ++g) {
           for (uint32_t c0 = ch.c0; c0 < ch.c1; c0 += chunk) {
             k.grp = g;
             k.c0 = c0;
             k.cn = std::min(chunk, ch.c1 - c0);
             k.tile = 4;  // centres per warp work item
-            if (cudaMemsetAsync(k.work, 0, 4, st) != cudaSuccess) return fail(ctx, PP_ERR_CUDA, "memset failed");
-            if (pp::launch_knn_walk(k, ctx->sm_count, st)) return fail(ctx, PP_ERR_CUDA, "kNN walk launch failed");
+            if (g < ngm) {
+              if (cudaMemsetAsync(k.work, 0, 4, st) != cudaSuccess) return fail(ctx, PP_ERR_CUDA, "memset failed");
+              if (pp::launch_minor_walk(k, ctx->sm_count, st)) return fail(ctx, PP_ERR_CUDA, "minor walk launch failed");
+            }
+            if (g >= ng32) continue;
+            if (!minor_knn) {
+              if (cudaMemsetAsync(k.work, 0, 4, st) != cudaSuccess) return fail(ctx, PP_ERR_CUDA, "memset failed");
+              if (pp::launch_knn_walk(k, ctx->sm_count, st)) return fail(ctx, PP_ERR_CUDA, "kNN walk launch failed");
+            }
             const uint32_t nranges = (uint32_t)std::max<uint64_t>(1, (8ull * ctx->sm_count + NT - 1) / NT);
             k.tile = std::max<uint32_t>(1, (k.cn + nranges - 1) / nranges);
             if (cudaMemsetAsync(k.work, 0, 4, st) != cudaSuccess) return fail(ctx, PP_ERR_CUDA, "memset failed");
@@ -2668,6 +2764,7 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
           }
         }
       }
+      if (ngm && pp::launch_minor_fin(kq, st)) return fail(ctx, PP_ERR_CUDA, "minor sums launch failed");
       return PP_OK;
     };
     std::string sig((const char*)&b, sizeof b);
@@ -2675,7 +2772,8 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
     sig.append((const char*)&ea_sig, sizeof ea_sig);
     sig.append((const char*)&bk, sizeof bk);
     sig.append((const char*)chunks.data(), chunks.size() * sizeof(Chunk));
-    const uint64_t extra[5] = {(uint64_t)ng32, chunk, nc, (uint64_t)ctx->sm_count, chunked ? 1u : 0u};
+    const uint64_t extra[8] = {(uint64_t)ng32, chunk, nc, (uint64_t)ctx->sm_count, chunked ? 1u : 0u,
+                               (uint64_t)ngm, (uint64_t)nrb, sums_bytes};
     sig.append((const char*)extra, sizeof extra);
     if (!ctx->apply_exec || sig != ctx->apply_sig) {
       if (!ctx->cap_stream) CK(cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));

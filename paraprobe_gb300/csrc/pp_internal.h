@@ -320,7 +320,25 @@ struct KnnArgs {
   uint32_t tile;                    // centres per walk work item / per bin work item
   int cblk;                         // centre types per bin histogram (set by knn32_check)
   unsigned long long* knn_core;     // [nreal][nC][nS][nkI][H]
+  // k_minor_walk: the type most ions are of, its centre and environment slot
+  // (-1: none), what the walk does, and for RDF the realisations that are whole
+  // label sets (the first nlab)
+  int dom, dom_c, dom_e;
+  int do_rdf, do_knn, nlab, nE;
+  const uint32_t* minor;            // [ngroups][n] bit r: not dom in realisation r of the group
+  const int8_t* eslot_of;
+  unsigned long long* rdf_core;     // [nreal][nC][nE][H]
+  unsigned long long* counters;     // [nreal][2]
+  unsigned long long* sa;           // [nlab][rows + 1][H] lists of the centres that are not dom
+  unsigned long long* so;           // [nlab][nC][H] neighbours without an environment slot
+  unsigned long long* tcat;         // [H] all pairs
+  uint32_t* found;                  // [nreal][nC][nsmax][nkI + 1] centres by orders found
 };
+int minor_warps(const KnnArgs& k);
+int launch_minor_walk(const KnnArgs& k, int sm_count, cudaStream_t s);
+int launch_minor_fin(const KnnArgs& k, cudaStream_t s);
+void launch_minor_masks(const uint8_t* labels, uint64_t total, int dom, uint32_t* out, cudaStream_t s);
+int launch_cat_hist(const uint16_t* cat, uint64_t n, int H, unsigned long long* out, int sm_count, cudaStream_t s);
 // -2 when a warp's records or the bin histogram do not fit shared memory
 int knn32_check(KnnArgs& k);
 int launch_knn_walk(const KnnArgs& k, int sm_count, cudaStream_t s);

@@ -3617,6 +3617,322 @@ __global__ void __launch_bounds__(1024, 1) k_knn_bin(KnnArgs a) {
   }
 }
 
+// --------------------------------------------- K5' batched, one common type
+// Most ions of an alloy are of one type (dom), so of the pairs of a
+// realisation all but a few per cent are told by what they are not.  Per
+// geometry centre and 32 realisations (one per lane) a warp transposes the
+// "is not dom" bits of 32 list entries, one word per ion and 32 realisations
+// (k_minor_masks), so that each lane holds the entries that are not dom in its
+// realisation, and touches only those:
+//   RDF  N(c, t) for t != dom from these entries; A(c), all neighbours of the
+//        centres of type c, for c != dom (few lanes hold such a centre: the
+//        warp adds the list for them); then with T, all pairs by category,
+//        A(dom) = T - sum A(c) and N(c, dom) = A(c) - sum N(c, t): whole
+//        numbers, exactly what counting every pair gives (k_minor_fin).
+//   kNN  the k-th member of dom's set is the k-th zero bit; the other sets
+//        count their entries as k_knn_walk does, which takes every entry.
+// 2M-ion tip, 65 label sets (f = 4% not dom), R = 1.5 nm, 36 pairs, k = 1..8:
+// the whole call 109 -> 59 ms (k_minor_walk 25 ms where k_knn_walk and k_apply
+// took 74).
+// Bins: N(dom, t) as [t][category][realisation] words (lane r hits bank r) and
+// A as [realisation][c][category] in shared memory; the rest, of centres that
+// are not dom and types without a slot, in global memory.
+__global__ void k_minor_masks(const uint8_t* __restrict__ labels, uint64_t total, uint32_t dom,
+                              uint32_t* __restrict__ out) {
+  const uint32_t d4 = dom * 0x01010101u;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint4* p = (const uint4*)(labels + i * 32);
+    const uint4 a = p[0], b = p[1];
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t m = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m |= ((((__vcmpne4(w[k], d4) & 0x01010101u) * 0x01020408u) >> 24) & 0xfu) << (4 * k);
+    out[i] = m;
+  }
+}
+
+// Pairs by category (a range of list entries).
+__global__ void k_cat_hist(const uint16_t* __restrict__ cat, uint64_t n, int H, unsigned long long* __restrict__ out) {
+  extern __shared__ uint32_t hcat[];
+  for (int i = threadIdx.x; i < H; i += blockDim.x) hcat[i] = 0;
+  __syncthreads();
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    atomicAdd(&hcat[cat[i]], 1u);
+  __syncthreads();
+  for (int i = threadIdx.x; i < H; i += blockDim.x)
+    if (hcat[i]) atomicAdd(&out[i], (unsigned long long)hcat[i]);
+}
+
+// 32 x 32 bit transpose across a warp: bit r of lane e -> bit e of lane r.
+__device__ __forceinline__ uint32_t bits_transpose(uint32_t x, int lane) {
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int s = 16; s; s >>= 1, m ^= m << s) {
+    const uint32_t y = __shfl_xor_sync(FULL, x, s);
+    x = (lane & s) ? ((x & ~m) | ((y >> s) & m)) : ((x & m) | ((y << s) & ~m));
+  }
+  return x;
+}
+
+struct MinorLayout {
+  int RN, RA;              // rows: environment slots / centre slots but dom's
+  size_t nset, nmiss, nN, nA;  // bytes of the set table; words of the others
+  __host__ __device__ MinorLayout(const KnnArgs& a) {
+    RN = a.nE - (a.dom_e >= 0 ? 1 : 0);
+    RA = a.nC - (a.dom_c >= 0 ? 1 : 0);
+    nset = a.do_knn ? (size_t)(a.nC + 1) * 256 : 0;
+    nmiss = a.do_knn ? (size_t)a.nsmax * (a.nkI + 1) * 32 : 0;
+    nN = a.do_rdf && a.dom_c >= 0 ? (size_t)RN * a.H * 32 : 0;
+    nA = a.do_rdf ? (size_t)RA * a.H * 32 : 0;
+  }
+  __host__ __device__ size_t warp_bytes(const KnnArgs& a) const {
+    return 128 + 64 + (a.do_knn ? (size_t)a.nsmax * 32 : 0);
+  }
+  __host__ __device__ size_t bytes(const KnnArgs& a, int nwarps) const {
+    return (nmiss + nN + nA) * 4 + 256 * 4 + nset + 3 * 256 + (size_t)a.nC * 4 + nwarps * warp_bytes(a);
+  }
+};
+
+template <bool RDF, bool KNN>
+__global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int H = a.H, nkI = a.nkI, NT = a.nsmax * nkI, kmax = a.kmax;
+  const MinorLayout Lo(a);
+  const int RA = Lo.RA;
+  uint32_t* sMiss = (uint32_t*)smem;             // [set][orders found][32], centres of type dom
+  uint32_t* sN = sMiss + Lo.nmiss;               // [RN][H][32]
+  uint32_t* sA = sN + Lo.nN;                     // [32][RA][H]
+  uint32_t* sKv = sA + Lo.nA;                    // [nkI <= 256] orders
+  int* sNs = (int*)(sKv + 256);                  // [nC]
+  uint32_t* wslotA = (uint32_t*)(sNs + a.nC);    // per warp: the 32 entries' slots ...
+  uint16_t* wcatA = (uint16_t*)(wslotA + nwarps * 32);  // ... and categories
+  uint8_t* sCnt = (uint8_t*)(wcatA + nwarps * 32);      // [nwarps][nsmax][32] members met
+  int8_t* sC = (int8_t*)(sCnt + (KNN ? nwarps * a.nsmax * 32 : 0));
+  int8_t* sE = sC + 256;
+  int8_t* sK = sE + 256;
+  int8_t* sSet = sK + 256;                       // [nC + 1][256]
+  for (uint32_t i = threadIdx.x; i < (uint32_t)(Lo.nmiss + Lo.nN + Lo.nA); i += blockDim.x) sMiss[i] = 0;
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) { sC[i] = a.cslot_of[i]; sE[i] = a.eslot_of[i]; sK[i] = -1; }
+  for (int i = threadIdx.x; i < a.nC; i += blockDim.x) sNs[i] = a.nsets[i];
+  if (KNN)
+    for (int i = threadIdx.x; i < (a.nC + 1) * 256; i += blockDim.x) sSet[i] = i < a.nC * 256 ? a.setidx[i] : (int8_t)-1;
+  __syncthreads();
+  if (KNN)
+    for (int i = threadIdx.x; i < nkI; i += blockDim.x) {
+      sKv[i] = (uint32_t)a.kvals[i];
+      sK[a.kvals[i]] = (int8_t)i;
+    }
+  __syncthreads();
+  uint32_t* wslot = wslotA + warp * 32;
+  uint16_t* wcat = wcatA + warp * 32;
+  uint8_t* cnt = sCnt + warp * a.nsmax * 32 + lane;
+  const uint8_t* lab = a.labels + (uint64_t)a.grp * a.n * 32 + lane;
+  const uint8_t* okp = a.centre_ok + (uint64_t)a.grp * a.ncentres * 32 + lane;
+  const uint32_t* minor = a.minor + (uint64_t)a.grp * a.n;
+  const int real = a.grp * 32 + lane;
+  const bool rdf_lane = RDF && real < a.nlab;
+  unsigned long long pairs = 0, centres = 0;
+  const uint32_t ntiles = (a.cn + a.tile - 1) / a.tile;
+  for (;;) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(a.work, 1u);
+    item = __shfl_sync(FULL, item, 0);
+    if (item >= ntiles) break;
+    const uint32_t l0 = item * a.tile, l1 = min(l0 + a.tile, a.cn);
+    for (uint32_t li = l0; li < l1; ++li) {
+      const uint32_t ci = a.c0 + li;
+      const uint32_t self = a.centres[ci];
+      const uint32_t tc = lab[(uint64_t)self * 32];
+      const int c = (real < a.nreal && okp[(uint64_t)ci * 32] != 0) ? (int)sC[tc] : -1;
+      const unsigned long long o0 = a.pair_off[ci], o1 = a.pair_off[ci + 1];
+      // RDF: the row this lane's centre adds its whole list to (-1: none)
+      int arow = -1;
+      if (RDF && rdf_lane) {
+        if (c >= 0) {
+          pairs += o1 - o0;
+          ++centres;
+          if (c != a.dom_c) arow = c - (a.dom_c >= 0 && c > a.dom_c ? 1 : 0);
+        } else if (a.dom_c >= 0) {
+          arow = RA;
+        }
+      }
+      const uint32_t abits = RDF ? __ballot_sync(FULL, arow >= 0) : 0u;
+      // kNN: sets with fewer than kmax members met; dom's set, its members met
+      // and orders found
+      int nset = 0, unsat = 0, qd = -1, nd = 0, kd = 0;
+      const int row = (c >= 0 ? c : a.nC) * 256;
+      uint16_t* out = nullptr;
+      if (KNN) {
+        nset = c >= 0 ? sNs[c] : 0;
+        unsat = nset;
+        qd = sSet[row + a.dom];
+        for (int q = 0; q < a.nsmax; ++q) cnt[q * 32] = 0;
+        out = a.rec + (uint64_t)li * NT * 32 + lane;
+      }
+      const bool rneed = RDF && rdf_lane && c >= 0;
+      uint32_t nx_slot = 0, nx_cat = 0, nx_m = 0;
+      if (o0 + lane < o1) {
+        nx_slot = a.pair_slot[o0 + lane - a.pair_base];
+        nx_cat = a.pair_cat[o0 + lane - a.pair_base];
+        nx_m = minor[nx_slot];
+      }
+      for (unsigned long long e0 = o0; e0 < o1; e0 += 32) {
+        if (!RDF && !__any_sync(FULL, unsat > 0)) break;
+        const uint32_t my_slot = nx_slot, my_cat = nx_cat;
+        const uint32_t ne = (uint32_t)min(32ull, o1 - e0);
+        const uint32_t valid = ne == 32u ? FULL : (1u << ne) - 1u;
+        const uint32_t w = bits_transpose(nx_m, lane);
+        wslot[lane] = my_slot;
+        wcat[lane] = (uint16_t)my_cat;
+        if (e0 + 32 + lane < o1) {
+          nx_slot = a.pair_slot[e0 + 32 + lane - a.pair_base];
+          nx_cat = a.pair_cat[e0 + 32 + lane - a.pair_base];
+          nx_m = minor[nx_slot];
+        }
+        __syncwarp();
+        if (RDF) {
+          for (uint32_t ab = abits; ab; ab &= ab - 1u) {
+            const int rr = __ffs(ab) - 1;
+            const int ar = __shfl_sync(FULL, arow, rr);
+            if ((uint32_t)lane < ne) {
+              if (ar < RA) atomicAdd(&sA[((uint32_t)rr * RA + ar) * H + my_cat], 1u);
+              else atomicAdd(&a.sa[((uint64_t)(a.grp * 32 + rr) * (RA + 1) + RA) * H + my_cat], 1ull);
+            }
+          }
+        }
+        uint32_t b = (rneed || unsat > 0) ? w & valid : 0u;
+        uint32_t z = ~w & valid;  // members of dom's set
+        while (b) {
+          // two entries at a time: their label loads are in flight together
+          const int j0 = __ffs(b) - 1;
+          b &= b - 1u;
+          const int j1 = b ? __ffs(b) - 1 : -1;
+          b &= b - 1u;  // 0 stays 0
+          uint32_t t2[2];
+          t2[0] = lab[(uint64_t)wslot[j0] << 5];
+          t2[1] = j1 >= 0 ? lab[(uint64_t)wslot[j1] << 5] : 0u;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int j = u ? j1 : j0;
+            if (j < 0) break;
+            const uint32_t t = t2[u], cat = wcat[j];
+            if (rneed) {
+              const int e = sE[t];
+              if (e < 0) {
+                atomicAdd(&a.so[((uint64_t)real * a.nC + c) * H + cat], 1ull);
+              } else if (c == a.dom_c) {
+                atomicAdd(&sN[((uint32_t)(e - (a.dom_e >= 0 && e > a.dom_e ? 1 : 0)) * H + cat) * 32 + lane], 1u);
+              } else {
+                atomicAdd(&a.rdf_core[(((uint64_t)real * a.nC + c) * a.nE + e) * H + cat], 1ull);
+              }
+            }
+            if (KNN) {
+              const int q = sSet[row + t];
+              if (q == qd) {
+                if (q >= 0) z |= 1u << j;  // a set that holds dom too: counted with its entries below
+              } else if (q >= 0) {
+                const int m = cnt[q * 32];
+                if (m < kmax) {
+                  const int kk = sK[m + 1];
+                  if (kk >= 0) out[(q * nkI + kk) * 32] = (uint16_t)cat;
+                  cnt[q * 32] = (uint8_t)(m + 1);
+                  unsat -= (m + 1 == kmax);
+                }
+              }
+            }
+          }
+        }
+        if (KNN && qd >= 0 && nd < kmax) {
+          const int more = __popc(z);
+          while (kd < nkI && (int)sKv[kd] <= nd + more) {
+            out[(qd * nkI + kd) * 32] = wcat[nth_set(z, sKv[kd] - 1u - (uint32_t)nd)];
+            ++kd;
+          }
+          nd += more;
+          unsat -= nd >= kmax;
+        }
+        __syncwarp();
+      }
+      if (KNN) {
+        // the slots not met hold no category; orders found per set
+        for (int q = 0; q < a.nsmax; ++q) {
+          int f = 0;
+          if (q == qd) f = kd;
+          else
+            while (f < nkI && (int)sKv[f] <= (int)cnt[q * 32]) ++f;
+          for (int kk = f; kk < nkI; ++kk) out[(q * nkI + kk) * 32] = (uint16_t)0xffff;
+          if (q < nset && f < nkI) {
+            if (c == a.dom_c) atomicAdd(&sMiss[(q * (nkI + 1) + f) * 32 + lane], 1u);
+            else atomicAdd(&a.found[(((uint64_t)real * a.nC + c) * a.nsmax + q) * (nkI + 1) + f], 1u);
+          }
+        }
+        a.rec_c[(uint64_t)li * 32 + lane] = c >= 0 ? (uint8_t)c : (uint8_t)0xff;
+      }
+    }
+  }
+  if (rdf_lane && centres) {
+    atomicAdd(&a.counters[2 * (uint64_t)real], pairs);
+    atomicAdd(&a.counters[2 * (uint64_t)real + 1], centres);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < (uint32_t)Lo.nN; i += blockDim.x) {
+    const uint32_t v = sN[i];
+    if (!v) continue;
+    const int r = a.grp * 32 + (int)(i & 31u), e = (int)(i / 32 / H), cat = (int)(i / 32 - (uint32_t)e * H);
+    const int es = e + (a.dom_e >= 0 && e >= a.dom_e ? 1 : 0);
+    atomicAdd(&a.rdf_core[(((uint64_t)r * a.nC + a.dom_c) * a.nE + es) * H + cat], (unsigned long long)v);
+  }
+  for (uint32_t i = threadIdx.x; i < (uint32_t)Lo.nA; i += blockDim.x) {
+    const uint32_t v = sA[i];
+    if (!v) continue;
+    const uint32_t rr = i / (uint32_t)(RA * H), rest = i - rr * (uint32_t)(RA * H);
+    atomicAdd(&a.sa[(uint64_t)(a.grp * 32 + rr) * (RA + 1) * H + rest], (unsigned long long)v);
+  }
+  for (uint32_t i = threadIdx.x; i < (uint32_t)Lo.nmiss; i += blockDim.x) {
+    const uint32_t v = sMiss[i];
+    if (!v) continue;
+    const int r = a.grp * 32 + (int)(i & 31u), f = (int)((i >> 5) % (nkI + 1)), q = (int)((i >> 5) / (nkI + 1));
+    atomicAdd(&a.found[(((uint64_t)r * a.nC + a.dom_c) * a.nsmax + q) * (nkI + 1) + f], v);
+  }
+}
+
+// The counts told by what they are not (see above), per realisation, and the
+// missing neighbours.
+__global__ void k_minor_fin(KnnArgs a) {
+  const int H = a.H, r = blockIdx.y;
+  const MinorLayout Lo(a);
+  const int RA = Lo.RA;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nC * H; i += gridDim.x * blockDim.x) {
+    const int c = i / H, cat = i - c * H;
+    if (a.do_rdf && r < a.nlab && a.dom_e >= 0) {
+      const unsigned long long* sa = a.sa + (uint64_t)r * (RA + 1) * H + cat;
+      unsigned long long all;
+      if (c == a.dom_c) {
+        all = a.tcat[cat];
+        for (int q = 0; q <= RA; ++q) all -= sa[(uint64_t)q * H];
+      } else {
+        all = sa[(uint64_t)(c - (a.dom_c >= 0 && c > a.dom_c ? 1 : 0)) * H];
+      }
+      unsigned long long* core = a.rdf_core + ((uint64_t)r * a.nC + c) * a.nE * H + cat;
+      all -= a.so[((uint64_t)r * a.nC + c) * H + cat];
+      for (int e = 0; e < a.nE; ++e)
+        if (e != a.dom_e) all -= core[(uint64_t)e * H];
+      core[(uint64_t)a.dom_e * H] = all;
+    }
+  }
+  if (a.do_knn)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nC * a.nsmax * a.nkI; i += gridDim.x * blockDim.x) {
+      const int kk = i % a.nkI, q = (i / a.nkI) % a.nsmax, c = i / a.nkI / a.nsmax;
+      if (q >= a.nsets[c]) continue;
+      const uint32_t* f = a.found + (((uint64_t)r * a.nC + c) * a.nsmax + q) * (a.nkI + 1);
+      unsigned long long miss = 0;
+      for (int k = 0; k <= kk; ++k) miss += f[k];  // found the first k orders: order kk is missing
+      if (miss)
+        atomicAdd(&a.knn_core[((((uint64_t)r * a.nC + c) * a.nS + a.set_list[c * 32 + q]) * a.nkI + kk) * H + a.cat_miss], miss);
+    }
+}
+
 // Realisation-major byte arrays src[rows][cols] to the group-major layout
 // k_apply reads: dst[((r / G) * cols + c) * G + r % G], rows padded to a
 // multiple of G with zeros.
@@ -4332,6 +4648,47 @@ int launch_knn_walk(const KnnArgs& k, int sm_count, cudaStream_t s) {
     return -1;
   counted();
   kern<<<sm_count * per_sm, w * 32, smem, s>>>(k);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// warps of a k_minor_walk block; 0 = its bins do not fit shared memory
+int minor_warps(const KnnArgs& k) {
+  const MinorLayout L(k);
+  for (int w = 32; w >= 8; w /= 2)
+    if (L.bytes(k, w) <= 224 * 1024) return w;
+  return 0;
+}
+
+int launch_minor_walk(const KnnArgs& k, int sm_count, cudaStream_t s) {
+  const int w = minor_warps(k);
+  if (!w) return -2;
+  const size_t smem = MinorLayout(k).bytes(k, w);
+  auto kern = k.do_rdf ? (k.do_knn ? k_minor_walk<true, true> : k_minor_walk<true, false>) : k_minor_walk<false, true>;
+  if (!allow_dynamic_smem((const void*)kern, smem)) return -1;
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, w * 32, smem) != cudaSuccess || per_sm < 1)
+    return -1;
+  counted();
+  kern<<<sm_count * per_sm, w * 32, smem, s>>>(k);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_minor_fin(const KnnArgs& k, cudaStream_t s) {
+  counted();
+  k_minor_fin<<<dim3(8, (unsigned)k.nreal), 256, 0, s>>>(k);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+void launch_minor_masks(const uint8_t* labels, uint64_t total, int dom, uint32_t* out, cudaStream_t s) {
+  counted();
+  k_minor_masks<<<grid_for(total, 256), 256, 0, s>>>(labels, total, (uint32_t)dom, out);
+}
+
+int launch_cat_hist(const uint16_t* cat, uint64_t n, int H, unsigned long long* out, int sm_count, cudaStream_t s) {
+  const size_t smem = (size_t)H * 4;
+  if (!allow_dynamic_smem((const void*)k_cat_hist, smem)) return -1;
+  counted();
+  k_cat_hist<<<sm_count * 2, 1024, smem, s>>>(cat, n, H, out);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

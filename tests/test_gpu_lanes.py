@@ -114,3 +114,58 @@ def test_knn_in_two_walks(ctx, oracle, ks, fractions, lists, rmin):
     assert st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
     assert np.array_equal(got, ref["bins"])
     assert np.array_equal(part + rest, got) and stp["pairs"] + str_["pairs"] == st["pairs"]
+
+
+TASKS = {
+    "pairs": ([[a] for a in (1, 2, 3) for b in (1, 2, 3)], [[b] for a in (1, 2, 3) for b in (1, 2, 3)]),
+    "common type in a wider set": ([[2], [1]], [[1, 2, 3], [1, 4]]),
+    "common type never a centre": ([[2], [3]], [[1], [1, 2]]),
+    "common type in no set": ([[1], [2, 3]], [[2], [2, 3, 4]]),
+    "overlapping sets": ([[1], [1]], [[1, 2], [2, 3]]),
+}
+
+
+@pytest.mark.parametrize("form", [0, 1, 2])
+@pytest.mark.parametrize("tasks", sorted(TASKS))
+@pytest.mark.parametrize("nsets,rois,cap", [(3, 2, 0), (34, 0, 0), (40, 3, 60000)])
+def test_batched_by_common_type(ctx, oracle, form, tasks, nsets, rois, cap):
+    """Batched realisations counted by what is not of the common type, for sets
+    that hold it, hold it with others or leave it out, types without a slot,
+    label sets that are no shuffles, groups of 32 and their remainders, regions
+    of interest and pair lists in chunks."""
+    spec = synth.cylinder_specimen(n=9000, radius=2.5, height=11.0, fractions=(0.9, 0.05, 0.04, 0.01), seed=17, nseg=32,
+                                   stack=4.0)
+    n = len(spec.xyz)
+    rng = np.random.default_rng(nsets)
+    sets = np.stack([rng.permutation(spec.labels) for _ in range(nsets)])
+    sets[1] = rng.integers(0, 5, n)                 # no common type, and type 0
+    sets[2] = 2                                     # one type only
+    roi = np.stack([[0.3, -0.2, 5.5, 2.2 + 0.4 * q] for q in range(rois)]).astype(np.float32) if rois else None
+    trg, env = TASKS[tasks]
+    hist, ks, flags = (0.0, 0.02, 0.9), [12, 5, 1], N.PP_RDF | N.PP_1NN | N.PP_MKNN
+    d2 = np.where(np.arange(n) % 9 == 0, 0.1, 10.0).astype(np.float32)
+    cid = ctx.upload(spec.xyz, spec.labels)
+    ctx.surfdist(cid, d2)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.set_option("batched_minor", form)
+    ctx.set_option("batched_pair_cap", cap)
+    try:
+        ctx.run_batched(cid, flags, ks, include_original=True, label_sets=sets, rois=roi)
+        got = [ctx.fetch_batched(r) for r in range(ctx.batched_count())]
+        stats = [ctx.batched_stats(r) for r in range(ctx.batched_count())]
+    finally:
+        ctx.set_option("batched_minor", 1)
+        ctx.set_option("batched_pair_cap", 0)
+        ctx.free(cid)
+    assert len(got) == 1 + nsets + rois
+    for r in [0, 1, 2, 3, nsets] + list(range(1 + nsets, 1 + nsets + rois)):
+        lab = spec.labels if r == 0 or r > nsets else sets[r - 1]
+        surf = d2
+        if r > nsets:
+            c = roi[r - 1 - nsets]
+            far = c[3] - np.sqrt(((spec.xyz - c[:3]) ** 2).sum(1, dtype=np.float64)) < hist[2]
+            surf = np.where(far, 0.0, d2).astype(np.float32)
+        ref = oracle.spatstat(spec.xyz, lab.astype(np.uint8), surf, *hist, flags, trg, env, ks)
+        assert stats[r]["centres"] == ref["centres"] and stats[r]["pairs"] == ref["pairs"], r
+        assert np.array_equal(got[r], ref["bins"]), r
