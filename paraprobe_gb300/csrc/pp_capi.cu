@@ -200,6 +200,7 @@ struct pp_ctx {
   DevBuf tri_fill, cflag, rowtab, nc_pre, pass_code;
   DevBuf type_counts, sp_start, sp_ions, sp_slot;  // kNN passes in two walks
   DevBuf labels_run, perm_dev, gather_src;
+  DevBuf vox;      // pp_cloud_inside: sums, ions per voxel, union-find parents
   DevBuf neigh;    // pp_neighbors: count and records
   PinBuf neigh_stage;
   DevBuf mask_in;  // caller's centre mask: [n] input order, then [n] sorted-slot order
@@ -1176,9 +1177,9 @@ int pp_surfdist_upload(pp_ctx* ctx, int cloud, const float* d2) {
 
 // NumberOfIonsInside / VolumeInside of the RDF header: the reference's
 // occupancy grid (vxlizer::rectangular_binning and the steps it calls,
-// src/PARAPROBE_SolverHdl.cpp:5059-5386).  The device bins every ion; the
-// host labels the empty voxels in raster order with the Hoshen-Kopelman rules
-// of src/PARAPROBE_HoshenKopelman.cpp:55-146 -- a voxel joins its labelled -x,
+// src/PARAPROBE_SolverHdl.cpp:5059-5386).  The device bins every ion, labels
+// the empty voxels with the Hoshen-Kopelman rules of
+// src/PARAPROBE_HoshenKopelman.cpp:55-146 -- a voxel joins its labelled -x,
 // -y and -z neighbours, except that with all three labelled only -y and -z are
 // merged, and voxel 0 (label 0) stays unlabelled -- takes the cluster of the
 // guard corner (0, 0, nz - 1) as vacuum (:5196-5270), marks the non-vacuum
@@ -1223,74 +1224,22 @@ int pp_cloud_inside(pp_ctx* ctx, int cloud, float bin_width_min, float bin_width
   const uint64_t nx = nv[0], ny = nv[1], nz = nv[2], nxy = nx * ny, nxyz = nxy * nz;
   if (nx >= 0xffffffffull || ny >= 0xffffffffull || nz >= 0xffffffffull || nxyz >= 0xffffffffull)
     return fail(ctx, PP_ERR_UNSUPPORTED, "the occupancy grid needs 2^32 or more voxels (the reference's limit too)");
-  DevBuf occ_dev;
-  CK(occ_dev.ensure(nxyz * 4));
-  CK(cudaMemsetAsync(occ_dev.p, 0, nxyz * 4, s));
-  CK(ctx->res.status.ensure(4));
-  CK(cudaMemsetAsync(ctx->res.status.p, 0, 4, s));
+  // sums and status, then the ions per voxel and the union-find parents
+  const size_t vox_bytes = 64 + (size_t)nxyz * 8;
+  CK(ctx->vox.ensure(vox_bytes));
+  CK(cudaMemsetAsync(ctx->vox.p, 0, 64 + nxyz * 4, s));
+  unsigned long long* sums = ctx->vox.as<unsigned long long>();
+  uint32_t* occ = ctx->vox.as<uint32_t>() + 16;
   const uint32_t nv32[3] = {(uint32_t)nx, (uint32_t)ny, (uint32_t)nz};
-  pp::launch_voxel_count(cl->xyz.as<float>(), n, lo, w, nv32, occ_dev.as<uint32_t>(), ctx->res.status.as<int>(), s);
-  std::vector<uint32_t> occ(nxyz);
-  int st = 0;
-  CK(cudaMemcpyAsync(occ.data(), occ_dev.p, nxyz * 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&st, ctx->res.status.p, 4, cudaMemcpyDeviceToHost, s));
+  pp::launch_voxel_count(cl->xyz.as<float>(), n, lo, w, nv32, occ, (int*)(sums + 5), s);
+  pp::launch_voxel_classes(occ, nv32, occ + nxyz, (uint32_t*)(sums + 4), sums, s);
+  CK(cudaGetLastError());
+  unsigned long long got[6];
+  CK(cudaMemcpyAsync(got, sums, sizeof got, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  if (st) return fail(ctx, PP_ERR_DEVICE, "an ion fell outside the occupancy grid");
-  // Hoshen-Kopelman clusters of the empty voxels (union-find over voxel ids)
-  std::vector<uint32_t> parent(nxyz);
-  for (uint64_t b = 0; b < nxyz; ++b) parent[b] = (uint32_t)b;
-  auto root = [&](uint32_t a) {
-    while (parent[a] != a) {
-      parent[a] = parent[parent[a]];
-      a = parent[a];
-    }
-    return a;
-  };
-  auto join = [&](uint32_t a, uint32_t b) {
-    a = root(a);
-    b = root(b);
-    if (a != b) parent[a] = b;
-  };
-  auto labelled = [&](uint64_t b) { return b != 0 && occ[b] == 0; };
-  for (uint64_t z = 0; z < nz; ++z)
-    for (uint64_t y = 0; y < ny; ++y)
-      for (uint64_t x = 0; x < nx; ++x) {
-        const uint64_t v = x + y * nx + z * nxy;
-        if (!labelled(v)) continue;
-        const bool lx = x > 0 && labelled(v - 1), ly = y > 0 && labelled(v - nx), lz = z > 0 && labelled(v - nxy);
-        if (lx && ly && lz) {
-          join((uint32_t)(v - nx), (uint32_t)(v - nxy));
-          join((uint32_t)v, (uint32_t)(v - nx));
-          continue;
-        }
-        if (lx) join((uint32_t)v, (uint32_t)(v - 1));
-        if (ly) join((uint32_t)v, (uint32_t)(v - nx));
-        if (lz) join((uint32_t)v, (uint32_t)(v - nxy));
-      }
-  std::vector<uint8_t> cls(nxyz, 0);  // 1 vacuum, 2 surface
-  const uint64_t corner = (nz - 1) * nxy;
-  if (labelled(corner)) {
-    const uint32_t rc = root((uint32_t)corner);
-    for (uint64_t b = 0; b < nxyz; ++b)
-      if (labelled(b) && root((uint32_t)b) == rc) cls[b] = 1;
-  }
-  for (uint64_t z = 1; z + 1 < nz; ++z)
-    for (uint64_t y = 1; y + 1 < ny; ++y)
-      for (uint64_t x = 1; x + 1 < nx; ++x) {
-        if (cls[x + y * nx + z * nxy] != 1) continue;
-        for (int dz = -1; dz <= 1; ++dz)
-          for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) {
-              const uint64_t t = (x + dx) + (y + dy) * nx + (z + dz) * nxy;
-              if ((dx || dy || dz) && cls[t] != 1) cls[t] = 2;
-            }
-      }
-  uint64_t nvac = 0, nsrf = 0, nin = 0, ions_in = 0;
-  for (uint64_t b = 0; b < nxyz; ++b) {
-    if (cls[b] == 1) ++nvac;
-    else if (cls[b] == 2) ++nsrf;
-    else { ++nin; ions_in += occ[b]; }
-  }
+  if (ctx->vox.bytes > ((size_t)256 << 20)) ctx->vox.release();  // a grid this large is not kept
+  if ((uint32_t)got[5]) return fail(ctx, PP_ERR_DEVICE, "an ion fell outside the occupancy grid");
+  const uint64_t nvac = got[0], nsrf = got[1], nin = got[2], ions_in = got[3];
   float vol = (float)nin;
   vol *= w * w * w;
   if (nions_inside) *nions_inside = ions_in;

@@ -169,3 +169,14 @@ def test_batched_by_common_type(ctx, oracle, form, tasks, nsets, rois, cap):
         ref = oracle.spatstat(spec.xyz, lab.astype(np.uint8), surf, *hist, flags, trg, env, ks)
         assert stats[r]["centres"] == ref["centres"] and stats[r]["pairs"] == ref["pairs"], r
         assert np.array_equal(got[r], ref["bins"]), r
+
+
+def test_inside_repeats(ctx):
+    """The occupancy grid's clusters are joined concurrently: the counts of a
+    porous cloud are the same every time."""
+    rng = np.random.default_rng(5)
+    xyz = rng.uniform(0, 30, (9000, 3)).astype(np.float32)
+    cid = ctx.upload(xyz, np.ones(len(xyz), dtype=np.uint8))
+    got = {tuple(sorted(ctx.inside(cid, 1.0, 1.0).items())) for _ in range(40)}
+    ctx.free(cid)
+    assert len(got) == 1
