@@ -571,13 +571,13 @@ int ensure_tri_bins(pp_ctx* ctx, Cloud& cl, float rp, cudaStream_t s) {
   CK(ctx->scan_tmp.ensure(tmp_elems * 8 * 2));
   uint64_t total = 0;
   uint64_t cap = cl.tcell_list.bytes / 4;
-  int brc = pp::launch_tri_bins(cl.tri_box.as<float>(), nt, tg, grow, cl.tcell_start.as<uint32_t>(),
+  int brc = pp::launch_tri_bins(cl.tri_dev.as<float>(), cl.tri_box.as<float>(), nt, tg, grow, cl.tcell_start.as<uint32_t>(),
                                 ctx->tri_fill.as<uint32_t>(), cl.tcell_list.as<uint32_t>(), cap,
                                 ctx->scan_tmp.as<uint32_t>(), tmp_elems * 4, &total, s);
   if (brc == 1) {
     CK(cl.tcell_list.ensure(std::max<uint64_t>(total, 1) * 4));
     cap = cl.tcell_list.bytes / 4;
-    brc = pp::launch_tri_bins(cl.tri_box.as<float>(), nt, tg, grow, cl.tcell_start.as<uint32_t>(),
+    brc = pp::launch_tri_bins(cl.tri_dev.as<float>(), cl.tri_box.as<float>(), nt, tg, grow, cl.tcell_start.as<uint32_t>(),
                               ctx->tri_fill.as<uint32_t>(), cl.tcell_list.as<uint32_t>(), cap,
                               ctx->scan_tmp.as<uint32_t>(), tmp_elems * 4, &total, s);
   }
@@ -624,7 +624,8 @@ int ensure_surface(pp_ctx* ctx, Cloud& cl, float R, cudaStream_t s, const float*
     if (rc) return rc;
     pp::launch_surface_cells(cl.ions.as<float4>(), cl.cell_start.as<uint32_t>(), cl.g, cl.tri_f,
                              cl.tri_box.as<float>(), cl.tri_dev.as<float>(), cl.tcell_start.as<uint32_t>(),
-                             cl.tcell_list.as<uint32_t>(), cl.tg, rp, dst->as<float>(), s);
+                             cl.tcell_list.as<uint32_t>(), cl.tg, rp, cl.tri_slack,
+                             ion_density(cl) * cl.tg.h * cl.tg.h * cl.tg.h, dst->as<float>(), s);
     CK(cudaGetLastError());
   }
   if (!ctx->readonly_clouds) {

@@ -240,10 +240,10 @@ void launch_permute_labels(const uint8_t* label_by_id, const uint32_t* perm, con
                            uint64_t n, uint8_t* dst_by_slot, cudaStream_t s);
 void launch_surface_cells(const float4* ions, const uint32_t* cell_start, Grid g, int f, const float* tri_box,
                           const float* tri, const uint32_t* tcs, const uint32_t* tct, Grid tg, float rprime,
-                          float* surf, cudaStream_t s);
+                          float slack, double ions_per_cell, float* surf, cudaStream_t s);
 // packed caller-order xyz in, ion2surf out in the same order (no cell sort)
 void launch_surface_xyz(const float* xyz, uint64_t n, const float* tbox, const float* tri, const uint32_t* tstart,
-                        const uint32_t* tlist, Grid tg, float rp, float* out, cudaStream_t s);
+                        const uint32_t* tlist, Grid tg, float rp, float slack, float* out, cudaStream_t s);
 void launch_tri_box(const float* tri, uint64_t ntri, float* box, cudaStream_t s);
 // ions per voxel of the occupancy grid (lo = grid origin, nv = voxels per axis)
 void launch_voxel_count(const float* xyz, uint64_t n, const float* lo, float w, const uint32_t* nv, uint32_t* occ,
@@ -268,7 +268,7 @@ void launch_nc_prefix(const uint32_t* cell_start, uint64_t ncells, const uint8_t
 const int8_t* row_table_host(int* entries);
 // Bin triangles (boxes tbox[6 t]) into every cell of tg their box grown by
 // rp + slack reaches; fills tstart (ncells + 1) and tlist (returns the count).
-int launch_tri_bins(const float* tbox, uint64_t ntri, Grid tg, float grow, uint32_t* tstart, uint32_t* tfill,
+int launch_tri_bins(const float* tri, const float* tbox, uint64_t ntri, Grid tg, float grow, uint32_t* tstart, uint32_t* tfill,
                     uint32_t* tlist, uint64_t list_cap, uint32_t* scan_tmp, uint64_t scan_tmp_elems,
                     uint64_t* total_out, cudaStream_t s);
 int launch_scan(const ScanArgs& a, int kr, int emax, int sm_count, size_t* smem_used, cudaStream_t s);

@@ -386,7 +386,9 @@ __device__ float tri_dist2(const float* __restrict__ t, float px, float py, floa
 // triangles whose float AABB overlaps [p - R', p + R'] (touching counts,
 // src/PARAPROBE_AABBTree.cpp:112-124), in the order of the cell's list; every
 // triangle is listed in each hull cell its AABB grown by R' + slack reaches.
-// One warp per hull cell: the hull grid `tg` is the
+// `split` warps per hull cell, each taking every split-th 32 of its ions (few
+// cells hold ions and triangles, and a warp per cell left most of the device
+// waiting for the fullest ones): the hull grid `tg` is the
 // ion grid `g` coarsened f times per axis (same origin), so a hull cell's ions
 // are f x f row segments of consecutive slots.  The warp takes them 32 at a
 // time (rows concatenated); the cell's triangles are staged in shared memory
@@ -397,26 +399,40 @@ __device__ float tri_dist2(const float* __restrict__ t, float px, float py, floa
 // hull cell (its ion cell divided by f) lists every triangle whose box grown
 // by R' + slack reaches it: the two cell computations can only disagree
 // within float rounding of a boundary, which the slack covers.
+//
+// Most of a cell's triangles are far from an ion's nearest one, so each is
+// first measured by its box: nothing of a triangle is nearer than its box, and
+// tri_dist2's closest point lies in the triangle (its barycentric coordinates
+// are clamped) to within the rounding of the coordinates, which `slack` (the
+// host's 1e-3 + 1e-5 of the largest coordinate, 80 ulp and more) covers; so a
+// box grown by slack that is farther than the smallest value so far cannot
+// lower it.  Triangles without area, which may give NaN, are always evaluated
+// (kTriFlat, k_tri_fill).  1M-ion cylinder, 33k triangles:
+// 2.60 -> 0.61 ms (1.65 with the boxes alone and a warp per cell).
+constexpr uint32_t kTriFlat = 0x80000000u;  // list entry: no area, never skipped
 constexpr int kSurfWarps = 8;
+constexpr int kSurfTri = 24;  // words of a staged triangle: grown box, box, vertices (16-byte aligned)
 __global__ void __launch_bounds__(kSurfWarps * 32) k_surface_cells(const float4* __restrict__ ions,
                                                               const uint32_t* __restrict__ cell_start, Grid g, int f,
                                                               const float* __restrict__ tbox,
                                                               const float* __restrict__ tri,
                                                               const uint32_t* __restrict__ tstart,
                                                               const uint32_t* __restrict__ tlist, Grid tg, float rp,
-                                                              float* __restrict__ out) {
-  // per staged triangle: box lo x,y,z, hi x,y,z, the 9 vertex coordinates and
-  // a pad (17 words: conflict-free stores)
-  __shared__ float stri[kSurfWarps][32][17];
+                                                              float slack, int split, float* __restrict__ out) {
+  __shared__ __align__(16) float stri[kSurfWarps][32][kSurfTri];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float (*st)[17] = stri[warp];
+  float (*st)[kSurfTri] = stri[warp];
   const uint32_t lemask = (2u << lane) - 1u;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const float rp2 = __fmul_rn(rp, rp);
-  for (uint64_t tc = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; tc < tg.ncells; tc += nwarps) {
-    const int tx = (int)(tc % (uint64_t)tg.nx);
-    const uint64_t tr = tc / (uint64_t)tg.nx;
-    const int ty = (int)(tr % (uint64_t)tg.ny), tz = (int)(tr / (uint64_t)tg.ny);
+  const uint32_t items = (uint32_t)tg.ncells * (uint32_t)split;  // fewer than 60M cells, at most 16 warps each
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < items; w += nwarps) {
+    const uint32_t tc = w / (uint32_t)split, part = w - tc * (uint32_t)split;
+    uint32_t next = part;  // this warp's next 32-ion step of the cell
+    const uint32_t tr = tc / (uint32_t)tg.nx;
+    const int tx = (int)(tc - tr * (uint32_t)tg.nx);
+    const int tz = (int)(tr / (uint32_t)tg.ny), ty = (int)(tr - (uint32_t)tz * (uint32_t)tg.ny);
+    uint32_t step = 0;
     const uint32_t k0 = tstart[tc], k1 = tstart[tc + 1];
     const int x0 = tx * f, x1 = min(x0 + f, g.nx);
     const int ny = min(f, g.ny - ty * f), nz = min(f, g.nz - tz * f);
@@ -433,7 +449,7 @@ __global__ void __launch_bounds__(kSurfWarps * 32) k_surface_cells(const float4*
       const uint32_t ne = __ballot_sync(FULL, len > 0);
       const int cnt_rows = __popc(ne);
       if (cnt_rows == 0) continue;
-      const int src = lane < cnt_rows ? (int)__fns(ne, 0, lane + 1) : 0;
+      const int src = lane < cnt_rows ? (int)nth_set(ne, (uint32_t)lane) : 0;
       const uint32_t rst = __shfl_sync(FULL, st0, src);
       uint32_t rlen = __shfl_sync(FULL, len, src);
       if (lane >= cnt_rows) rlen = 0;
@@ -452,6 +468,8 @@ __global__ void __launch_bounds__(kSurfWarps * 32) k_surface_cells(const float4*
         const int row = before + __popc(smask & lemask) - 1;
         before += __popc(smask);
         const int rowc = row < 0 ? 0 : (row > 31 ? 31 : row);
+        if (step++ != next) continue;
+        next += (uint32_t)split;
         const uint32_t rs = __shfl_sync(FULL, rst, rowc);
         const uint32_t rpos = __shfl_sync(FULL, exc, rowc);
         const uint32_t t = bb + lane;
@@ -464,19 +482,30 @@ __global__ void __launch_bounds__(kSurfWarps * 32) k_surface_cells(const float4*
         const float hx = __fadd_rn(p.x, rp), hy = __fadd_rn(p.y, rp), hz = __fadd_rn(p.z, rp);
         for (uint32_t kb = k0; kb < k1; kb += 32) {
           if (kb + lane < k1) {
-            const uint32_t tt = tlist[kb + lane];
+            const uint32_t te = tlist[kb + lane], tt = te & ~kTriFlat;
+            const float grow = (te & kTriFlat) ? kInf() : slack;
             const float* b = tbox + 6 * (uint64_t)tt;
             const float* v = tri + 9 * (uint64_t)tt;
 #pragma unroll
-            for (int q = 0; q < 6; ++q) st[lane][q] = b[q];
+            for (int q = 0; q < 3; ++q) {
+              st[lane][q] = b[q] - grow;
+              st[lane][3 + q] = b[3 + q] + grow;
+              st[lane][6 + q] = b[q];
+              st[lane][9 + q] = b[3 + q];
+            }
 #pragma unroll
-            for (int q = 0; q < 9; ++q) st[lane][6 + q] = v[q];
+            for (int q = 0; q < 9; ++q) st[lane][12 + q] = v[q];
           }
           __syncwarp();
           const int m = (int)min(32u, k1 - kb);
           for (int j = 0; j < m; ++j) {
-            const float* b = st[j];
-            if (!have || b[3] < lx || b[0] > hx || b[4] < ly || b[1] > hy || b[5] < lz || b[2] > hz) continue;
+            const float4 ga = *(const float4*)&st[j][0];
+            const float2 gb = *(const float2*)&st[j][4];
+            const float gx = fmaxf(fmaxf(ga.x - p.x, p.x - ga.w), 0.f), gy = fmaxf(fmaxf(ga.y - p.y, p.y - gb.x), 0.f),
+                        gz = fmaxf(fmaxf(ga.z - p.z, p.z - gb.y), 0.f);
+            if (!have || gx * gx + gy * gy + gz * gz > best) continue;
+            const float* b = &st[j][6];
+            if (b[3] < lx || b[0] > hx || b[4] < ly || b[1] > hy || b[5] < lz || b[2] > hz) continue;
             const float v = tri_dist2(b + 6, p.x, p.y, p.z);
             if (!(v > best)) best = v;
           }
@@ -621,7 +650,8 @@ __global__ void k_voxel_sum(const uint32_t* __restrict__ occ, const uint32_t* __
 // test and the minimum are those of k_surface_cells, so both give the same bits.
 __global__ void k_surface_xyz(const float* __restrict__ xyz, uint64_t n, const float* __restrict__ tbox,
                               const float* __restrict__ tri, const uint32_t* __restrict__ tstart,
-                              const uint32_t* __restrict__ tlist, Grid tg, float rp, float* __restrict__ out) {
+                              const uint32_t* __restrict__ tlist, Grid tg, float rp, float slack,
+                              float* __restrict__ out) {
   const float rp2 = __fmul_rn(rp, rp);
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const float px = xyz[3 * i], py = xyz[3 * i + 1], pz = xyz[3 * i + 2];
@@ -634,8 +664,12 @@ __global__ void k_surface_xyz(const float* __restrict__ xyz, uint64_t n, const f
       const float hx = __fadd_rn(px, rp), hy = __fadd_rn(py, rp), hz = __fadd_rn(pz, rp);
       const uint32_t k1 = tstart[c + 1];
       for (uint32_t k = tstart[c]; k < k1; ++k) {
-        const uint32_t t = tlist[k];
+        const uint32_t te = tlist[k], t = te & ~kTriFlat;
         const float* b = tbox + 6 * (uint64_t)t;
+        const float gx = fmaxf(fmaxf(b[0] - px, px - b[3]) - slack, 0.f),
+                    gy = fmaxf(fmaxf(b[1] - py, py - b[4]) - slack, 0.f),
+                    gz = fmaxf(fmaxf(b[2] - pz, pz - b[5]) - slack, 0.f);
+        if (gx * gx + gy * gy + gz * gz > best && !(te & kTriFlat)) continue;
         if (b[3] < lx || b[0] > hx || b[4] < ly || b[1] > hy || b[5] < lz || b[2] > hz) continue;
         const float v = tri_dist2(tri + 9 * (uint64_t)t, px, py, pz);
         if (!(v > best)) best = v;
@@ -773,8 +807,10 @@ __global__ void k_tri_count(const float* __restrict__ tbox, uint64_t ntri, Grid 
   }
 }
 
-__global__ void k_tri_fill(const float* __restrict__ tbox, uint64_t ntri, Grid tg, float grow,
-                           uint32_t* __restrict__ fill, uint32_t* __restrict__ list, uint64_t cap,
+// Entries carry kTriFlat for triangles of (nearly) no area -- two edges within
+// 0.2 degrees of one line, or lengths out of range.
+__global__ void k_tri_fill(const float* __restrict__ tri, const float* __restrict__ tbox, uint64_t ntri, Grid tg,
+                           float grow, uint32_t* __restrict__ fill, uint32_t* __restrict__ list, uint64_t cap,
                            int* __restrict__ status) {
   const int lane = threadIdx.x & 31;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -782,9 +818,16 @@ __global__ void k_tri_fill(const float* __restrict__ tbox, uint64_t ntri, Grid t
     int c0[3], c1[3];
     tri_cell_range(tbox + 6 * t, tg, grow, c0, c1);
     const uint32_t m = (uint32_t)(c1[0] - c0[0] + 1) * (uint32_t)(c1[1] - c0[1] + 1) * (uint32_t)(c1[2] - c0[2] + 1);
+    const float* v = tri + 9 * t;
+    const float e0x = v[3] - v[0], e0y = v[4] - v[1], e0z = v[5] - v[2];
+    const float e1x = v[6] - v[0], e1y = v[7] - v[1], e1z = v[8] - v[2];
+    const float a = e0x * e0x + e0y * e0y + e0z * e0z, b = e0x * e1x + e0y * e1y + e0z * e1z,
+                c = e1x * e1x + e1y * e1y + e1z * e1z;
+    const bool solid = a * c - b * b > 1e-5f * a * c && a * c > 1e-24f && a * c < 1e24f;
+    const uint32_t entry = (uint32_t)t | (solid ? 0u : kTriFlat);
     for (uint32_t i = lane; i < m; i += 32) {
       const uint32_t at = atomicAdd(&fill[tri_range_cell(tg, c0, c1, i)], 1u);
-      if (at < cap) list[at] = (uint32_t)t;
+      if (at < cap) list[at] = entry;
       else if (status) atomicOr(status, ST_LIST_OVERFLOW);
     }
   }
@@ -4252,10 +4295,16 @@ void launch_permute_labels(const uint8_t* label_by_id, const uint32_t* perm, con
 
 void launch_surface_cells(const float4* ions, const uint32_t* cell_start, Grid g, int f, const float* tri_box,
                           const float* tri, const uint32_t* tcs, const uint32_t* tct, Grid tg, float rprime,
-                          float* surf, cudaStream_t s) {
+                          float slack, double ions_per_cell, float* surf, cudaStream_t s) {
+  // About one step of 32 ions a warp: a tip's hull cells are few and a warp per
+  // cell leaves the chip idle behind the fullest (4M-ion tip 0.69 -> 0.51 ms).
+  // Large grids have cells enough, and pay for reading the empty ones again
+  // (20M ions, 0.4M cells: 1.38 ms with one warp a cell, 1.44 with three).
+  int split = ions_per_cell > 512.0 ? 16 : ions_per_cell > 32.0 ? (int)(ions_per_cell / 32.0 + 0.5) : 1;
+  while (split > 1 && tg.ncells * (uint64_t)split > 1000000ull) split /= 2;
   counted();
-  k_surface_cells<<<grid_for(tg.ncells * 32, kSurfWarps * 32), kSurfWarps * 32, 0, s>>>(ions, cell_start, g, f, tri_box,
-                                                                                     tri, tcs, tct, tg, rprime, surf);
+  k_surface_cells<<<grid_for(tg.ncells * 32 * (uint64_t)split, kSurfWarps * 32), kSurfWarps * 32, 0, s>>>(
+      ions, cell_start, g, f, tri_box, tri, tcs, tct, tg, rprime, slack, split, surf);
 }
 
 // number of cells holding at least one ion
@@ -4301,7 +4350,7 @@ const int8_t* row_table_host(int* entries) {
   return table.v;
 }
 
-int launch_tri_bins(const float* tbox, uint64_t ntri, Grid tg, float grow, uint32_t* tstart, uint32_t* tfill,
+int launch_tri_bins(const float* tri, const float* tbox, uint64_t ntri, Grid tg, float grow, uint32_t* tstart, uint32_t* tfill,
                     uint32_t* tlist, uint64_t list_cap, uint32_t* scan_tmp, uint64_t scan_tmp_elems,
                     uint64_t* total_out, cudaStream_t s) {
   if (cudaMemsetAsync(tstart, 0, (tg.ncells + 1) * 4, s) != cudaSuccess) return -1;
@@ -4315,7 +4364,7 @@ int launch_tri_bins(const float* tbox, uint64_t ntri, Grid tg, float grow, uint3
   if (total > list_cap) return 1;  // caller grows the list and calls again
   if (cudaMemcpyAsync(tfill, tstart, (tg.ncells + 1) * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return -1;
   counted();
-  k_tri_fill<<<grid_for(ntri * 32, 256), 256, 0, s>>>(tbox, ntri, tg, grow, tfill, tlist, list_cap, nullptr);
+  k_tri_fill<<<grid_for(ntri * 32, 256), 256, 0, s>>>(tri, tbox, ntri, tg, grow, tfill, tlist, list_cap, nullptr);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -4349,9 +4398,9 @@ void launch_tri_box(const float* tri, uint64_t ntri, float* box, cudaStream_t s)
 }
 
 void launch_surface_xyz(const float* xyz, uint64_t n, const float* tbox, const float* tri, const uint32_t* tstart,
-                        const uint32_t* tlist, Grid tg, float rp, float* out, cudaStream_t s) {
+                        const uint32_t* tlist, Grid tg, float rp, float slack, float* out, cudaStream_t s) {
   counted();
-  k_surface_xyz<<<grid_for(n, 256), 256, 0, s>>>(xyz, n, tbox, tri, tstart, tlist, tg, rp, out);
+  k_surface_xyz<<<grid_for(n, 256), 256, 0, s>>>(xyz, n, tbox, tri, tstart, tlist, tg, rp, slack, out);
 }
 
 void launch_select_centres(const uint8_t* labels, const float* surf, uint64_t n, float R2, const int8_t* cslot_of,

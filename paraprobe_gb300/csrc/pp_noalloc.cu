@@ -212,9 +212,9 @@ extern "C" int pp_surfdist_noalloc(const float* xyz, uint64_t n, const float* tr
   uint32_t* scan = reinterpret_cast<uint32_t*>(base + L.scan);
   uint32_t* list = reinterpret_cast<uint32_t*>(base + L.list);
   uint64_t got = 0;
-  rc = pp::launch_tri_bins(box, ntri, tg, grow, start, fill, list, L.list_cap, scan, L.scan_elems, &got, s);
+  rc = pp::launch_tri_bins(tri, box, ntri, tg, grow, start, fill, list, L.list_cap, scan, L.scan_elems, &got, s);
   if (rc) return say(err, err_cap, PP_ERR_CUDA, "triangle binning failed (%d)", rc);
-  pp::launch_surface_xyz(xyz, n, box, tri, start, list, tg, rp, d2_out, s);
+  pp::launch_surface_xyz(xyz, n, box, tri, start, list, tg, rp, slack, d2_out, s);
   NA_CK(cudaGetLastError());
 #undef NA_CK
   return PP_OK;
