@@ -3699,7 +3699,9 @@ __global__ void __launch_bounds__(512, 2) k_knn_walk(KnnArgs a) {
 // Bin: one work item = (slot t = set q * nkI + order kk, range of centres).
 // The block histograms that slot for all 32 realisations at once in shared
 // memory laid out [nC][H][32], so lane r always hits bank r; the bins go to
-// knn_core of realisation grp * 32 + r, set set_list[c][q], order kk.
+// knn_core of realisation grp * 32 + r, set set_list[c][q], order kk.  Issue
+// bound: a branch around each add cost more than adding what is not counted to
+// a row of its own (2M-ion tip, 64 shuffles, 16 regions: 9.6 -> 6.1 ms).
 __global__ void __launch_bounds__(1024, 1) k_knn_bin(KnnArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t* hist = (uint32_t*)smem;                  // [cblk][H][32]
@@ -3709,6 +3711,8 @@ __global__ void __launch_bounds__(1024, 1) k_knn_bin(KnnArgs a) {
   // nC do not fit shared memory (records are then read once per block)
   const int cblk = a.cblk, ncb = (a.nC + cblk - 1) / cblk;
   const uint32_t nh = (uint32_t)cblk * a.H * 32;
+  const uint32_t spare = nh / 32;  // one more row: what is not counted
+  const uint32_t hbase = smem_addr(hist + lane);
   __shared__ uint32_t s_item;
   for (uint32_t i = threadIdx.x; i < nh; i += blockDim.x) hist[i] = 0;
   const uint32_t nranges = (a.cn + a.tile - 1) / a.tile;
@@ -3725,23 +3729,31 @@ __global__ void __launch_bounds__(1024, 1) k_knn_bin(KnnArgs a) {
     const int c_lo = (int)(rest - (uint32_t)t * ncb) * cblk;
     const uint32_t l0 = range * a.tile, l1 = min(l0 + a.tile, a.cn);
     // 8 centres per step: their loads are in flight together
+    const uint64_t st = (uint64_t)NT * 32;
     for (uint32_t lb = l0 + warp * 8; lb < l1; lb += nwarps * 8) {
       uint32_t v8[8], c8[8];
+      const uint16_t* rp = a.rec + lb * st + (uint32_t)t * 32u + lane;
+      const uint8_t* cp = a.rec_c + (uint64_t)lb * 32 + lane;
+      if (lb + 8 <= l1) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const uint32_t li = lb + u;
-        v8[u] = 0xffff;
-        c8[u] = 0xff;
-        if (li < l1) {
-          v8[u] = a.rec[((uint64_t)li * NT + t) * 32 + lane];
-          c8[u] = a.rec_c[(uint64_t)li * 32 + lane];
+        for (int u = 0; u < 8; ++u, rp += st) {
+          v8[u] = *rp;
+          c8[u] = cp[u * 32];
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u, rp += st) {
+          const bool in = lb + u < l1;
+          v8[u] = in ? (uint32_t)*rp : 0xffffu;
+          c8[u] = in ? (uint32_t)cp[u * 32] : 0xffu;
         }
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const int cr = (int)c8[u] - c_lo;
-        if (c8[u] != 0xff && v8[u] != 0xffff && cr >= 0 && cr < cblk)
-          atomicAdd(&hist[((uint32_t)cr * a.H + v8[u]) * 32 + lane], 1u);
+        const uint32_t cr = c8[u] - (uint32_t)c_lo;  // types below c_lo wrap
+        const bool in = v8[u] != 0xffffu && cr < (uint32_t)cblk && c8[u] != 0xffu;
+        const uint32_t bin = in ? cr * (uint32_t)a.H + v8[u] : spare;
+        asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(hbase + bin * 128u) : "memory");
       }
     }
     __syncthreads();
@@ -3779,7 +3791,7 @@ __global__ void __launch_bounds__(1024, 1) k_knn_bin(KnnArgs a) {
 //   kNN  the k-th member of dom's set is the k-th zero bit; the other sets
 //        count their entries as k_knn_walk does, which takes every entry.
 // 2M-ion tip, 65 label sets (f = 4% not dom), R = 1.5 nm, 36 pairs, k = 1..8:
-// the whole call 109 -> 59 ms (k_minor_walk 25 ms where k_knn_walk and k_apply
+// the whole call 109 -> 53 ms (k_minor_walk 22 ms where k_knn_walk and k_apply
 // took 74).
 // Bins: N(dom, t) as [t][category][realisation] words (lane r hits bank r) and
 // A as [realisation][c][category] in shared memory; the rest, of centres that
@@ -3833,13 +3845,14 @@ struct MinorLayout {
     nA = a.do_rdf ? (size_t)RA * a.H * 32 : 0;
   }
   __host__ __device__ size_t warp_bytes(const KnnArgs& a) const {
-    return 128 + 64 + (a.do_knn ? (size_t)a.nsmax * 32 : 0);
+    return 64 + (a.do_knn ? (size_t)a.nsmax * 32 : 0);
   }
   __host__ __device__ size_t bytes(const KnnArgs& a, int nwarps) const {
-    return (nmiss + nN + nA) * 4 + 256 * 4 + nset + 3 * 256 + (size_t)a.nC * 4 + nwarps * warp_bytes(a);
+    return (nmiss + nN + nA) * 4 + 256 * 4 + nset + 4 * 256 + (size_t)a.nC * 4 + nwarps * warp_bytes(a);
   }
 };
 
+constexpr int kMinorChunks = 6;
 template <bool RDF, bool KNN>
 __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -3852,26 +3865,43 @@ __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
   uint32_t* sA = sN + Lo.nN;                     // [32][RA][H]
   uint32_t* sKv = sA + Lo.nA;                    // [nkI <= 256] orders
   int* sNs = (int*)(sKv + 256);                  // [nC]
-  uint32_t* wslotA = (uint32_t*)(sNs + a.nC);    // per warp: the 32 entries' slots ...
-  uint16_t* wcatA = (uint16_t*)(wslotA + nwarps * 32);  // ... and categories
+  uint16_t* wcatA = (uint16_t*)(sNs + a.nC);     // per warp: the 32 entries' categories
   uint8_t* sCnt = (uint8_t*)(wcatA + nwarps * 32);      // [nwarps][nsmax][32] members met
   int8_t* sC = (int8_t*)(sCnt + (KNN ? nwarps * a.nsmax * 32 : 0));
   int8_t* sE = sC + 256;
   int8_t* sK = sE + 256;
-  int8_t* sSet = sK + 256;                       // [nC + 1][256]
+  uint8_t* sF = (uint8_t*)(sK + 256);            // orders among the first m members
+  int8_t* sSet = (int8_t*)(sF + 256);            // [nC + 1][256]
   for (uint32_t i = threadIdx.x; i < (uint32_t)(Lo.nmiss + Lo.nN + Lo.nA); i += blockDim.x) sMiss[i] = 0;
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) { sC[i] = a.cslot_of[i]; sE[i] = a.eslot_of[i]; sK[i] = -1; }
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) { sC[i] = a.cslot_of[i]; sK[i] = -1; }
+  // rows of sN; types without an environment slot -1
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+    const int e = a.eslot_of[i];
+    sE[i] = (int8_t)(e - (a.dom_e >= 0 && e > a.dom_e ? 1 : 0));
+  }
   for (int i = threadIdx.x; i < a.nC; i += blockDim.x) sNs[i] = a.nsets[i];
+  bool holds = false;  // dom's set of a centre type holds other types too
   if (KNN)
-    for (int i = threadIdx.x; i < (a.nC + 1) * 256; i += blockDim.x) sSet[i] = i < a.nC * 256 ? a.setidx[i] : (int8_t)-1;
-  __syncthreads();
-  if (KNN)
+    for (int i = threadIdx.x; i < (a.nC + 1) * 256; i += blockDim.x) {
+      const int8_t q = i < a.nC * 256 ? a.setidx[i] : (int8_t)-1;
+      sSet[i] = q;
+      holds |= q >= 0 && (i & 255) != a.dom && q == a.setidx[(i & ~255) + a.dom];
+    }
+  // chunks of 32 entries walked before their minority entries are taken
+  const int depth = __syncthreads_or(holds) ? 1 : RDF ? kMinorChunks : kMinorChunks / 2;
+  if (KNN) {
     for (int i = threadIdx.x; i < nkI; i += blockDim.x) {
       sKv[i] = (uint32_t)a.kvals[i];
       sK[a.kvals[i]] = (int8_t)i;
     }
+    for (int m = threadIdx.x; m < 256; m += blockDim.x) {
+      int f = 0;
+      while (f < nkI && a.kvals[f] <= m) ++f;
+      sF[m] = (uint8_t)f;
+    }
+  }
+  const bool every = kmax <= 2 * nkI;  // members of dom's set one by one, or order by order
   __syncthreads();
-  uint32_t* wslot = wslotA + warp * 32;
   uint16_t* wcat = wcatA + warp * 32;
   uint8_t* cnt = sCnt + warp * a.nsmax * 32 + lane;
   const uint8_t* lab = a.labels + (uint64_t)a.grp * a.n * 32 + lane;
@@ -3907,7 +3937,7 @@ __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
       const uint32_t abits = RDF ? __ballot_sync(FULL, arow >= 0) : 0u;
       // kNN: sets with fewer than kmax members met; dom's set, its members met
       // and orders found
-      int nset = 0, unsat = 0, qd = -1, nd = 0, kd = 0;
+      int nset = 0, unsat = 0, qd = -1, nd = 0;
       const int row = (c >= 0 ? c : a.nC) * 256;
       uint16_t* out = nullptr;
       if (KNN) {
@@ -3918,24 +3948,31 @@ __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
         out = a.rec + (uint64_t)li * NT * 32 + lane;
       }
       const bool rneed = RDF && rdf_lane && c >= 0;
-      uint32_t nx_slot = 0, nx_cat = 0, nx_m = 0;
-      if (o0 + lane < o1) {
-        nx_slot = a.pair_slot[o0 + lane - a.pair_base];
-        nx_cat = a.pair_cat[o0 + lane - a.pair_base];
-        nx_m = minor[nx_slot];
+      // what is not dom in the last chunks, the newest first (b is the oldest
+      // word while they are taken)
+      uint32_t wq[kMinorChunks];
+#pragma unroll
+      for (int k = 0; k < kMinorChunks; ++k) wq[k] = 0;
+      int held = 0;
+      const uint32_t* ps = a.pair_slot + (o0 - a.pair_base);
+      const uint16_t* pc = a.pair_cat + (o0 - a.pair_base);
+      const uint32_t np = (uint32_t)(o1 - o0);
+      uint32_t nx_cat = 0, nx_m = 0;
+      if ((uint32_t)lane < np) {
+        nx_cat = pc[lane];
+        nx_m = minor[ps[lane]];
       }
-      for (unsigned long long e0 = o0; e0 < o1; e0 += 32) {
+      for (uint32_t e0 = 0; e0 < np; e0 += 32) {
         if (!RDF && !__any_sync(FULL, unsat > 0)) break;
-        const uint32_t my_slot = nx_slot, my_cat = nx_cat;
-        const uint32_t ne = (uint32_t)min(32ull, o1 - e0);
+        const uint32_t my_cat = nx_cat;
+        const uint32_t ne = min(32u, np - e0);
         const uint32_t valid = ne == 32u ? FULL : (1u << ne) - 1u;
         const uint32_t w = bits_transpose(nx_m, lane);
-        wslot[lane] = my_slot;
-        wcat[lane] = (uint16_t)my_cat;
-        if (e0 + 32 + lane < o1) {
-          nx_slot = a.pair_slot[e0 + 32 + lane - a.pair_base];
-          nx_cat = a.pair_cat[e0 + 32 + lane - a.pair_base];
-          nx_m = minor[nx_slot];
+        if (KNN) wcat[lane] = (uint16_t)my_cat;
+        const uint32_t en = e0 + 32 + lane;
+        if (en < np) {
+          nx_cat = pc[en];
+          nx_m = minor[ps[en]];
         }
         __syncwarp();
         if (RDF) {
@@ -3948,55 +3985,91 @@ __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
             }
           }
         }
-        uint32_t b = (rneed || unsat > 0) ? w & valid : 0u;
-        uint32_t z = ~w & valid;  // members of dom's set
-        while (b) {
-          // two entries at a time: their label loads are in flight together
-          const int j0 = __ffs(b) - 1;
-          b &= b - 1u;
-          const int j1 = b ? __ffs(b) - 1 : -1;
-          b &= b - 1u;  // 0 stays 0
-          uint32_t t2[2];
-          t2[0] = lab[(uint64_t)wslot[j0] << 5];
-          t2[1] = j1 >= 0 ? lab[(uint64_t)wslot[j1] << 5] : 0u;
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int j = u ? j1 : j0;
-            if (j < 0) break;
-            const uint32_t t = t2[u], cat = wcat[j];
-            if (rneed) {
-              const int e = sE[t];
-              if (e < 0) {
-                atomicAdd(&a.so[((uint64_t)real * a.nC + c) * H + cat], 1ull);
-              } else if (c == a.dom_c) {
-                atomicAdd(&sN[((uint32_t)(e - (a.dom_e >= 0 && e > a.dom_e ? 1 : 0)) * H + cat) * 32 + lane], 1u);
-              } else {
-                atomicAdd(&a.rdf_core[(((uint64_t)real * a.nC + c) * a.nE + e) * H + cat], 1ull);
-              }
+        for (int k = kMinorChunks - 1; k > 0; --k) wq[k] = wq[k - 1];
+        wq[0] = (rneed || unsat > 0) ? w & valid : 0u;
+        uint32_t z = ~w & valid;  // members of dom's set
+        if (++held >= depth || e0 + 32 >= np) {
+          // The entries of each lane one after the other, whichever chunks they
+          // lie in: the steps are those of the lane with the most of them, not the
+          // sum over chunks of the most in each (25 -> 22 ms, see above).
+          held = 0;
+          uint32_t base = e0 - 32u * (kMinorChunks - 1);  // chunk of b (wraps: no entries there)
+          uint32_t b = wq[kMinorChunks - 1];
+          auto next = [&](uint32_t& pos) -> bool {  // a lane's next entry
+            while (!b) {
+              uint32_t rest = 0;
+#pragma unroll
+              for (int k = 0; k < kMinorChunks - 1; ++k) rest |= wq[k];
+              if (!rest) return false;
+              b = wq[kMinorChunks - 2];
+#pragma unroll
+              for (int k = kMinorChunks - 2; k > 0; --k) wq[k] = wq[k - 1];
+              wq[0] = 0;
+              base += 32;
             }
-            if (KNN) {
-              const int q = sSet[row + t];
-              if (q == qd) {
-                if (q >= 0) z |= 1u << j;  // a set that holds dom too: counted with its entries below
-              } else if (q >= 0) {
-                const int m = cnt[q * 32];
-                if (m < kmax) {
-                  const int kk = sK[m + 1];
-                  if (kk >= 0) out[(q * nkI + kk) * 32] = (uint16_t)cat;
-                  cnt[q * 32] = (uint8_t)(m + 1);
-                  unsat -= (m + 1 == kmax);
+            pos = base + __ffs(b) - 1;
+            b &= b - 1u;
+            return true;
+          };
+          uint32_t p0 = 0, p1 = 0;
+          while (next(p0)) {
+            // two entries at a time: their loads are in flight together
+            const bool two = next(p1);
+            uint32_t t2[2], c2[2];
+            const uint32_t s0 = ps[p0], s1 = ps[two ? p1 : p0];
+            c2[0] = pc[p0];
+            c2[1] = pc[two ? p1 : p0];
+            t2[0] = lab[(uint64_t)s0 << 5];
+            t2[1] = lab[(uint64_t)s1 << 5];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              if (u && !two) break;
+              const uint32_t t = t2[u], cat = c2[u];
+              if (rneed) {
+                const int e = sE[t];
+                if (e >= 0 && c == a.dom_c) {
+                  atomicAdd(&sN[((uint32_t)e * H + cat) * 32 + lane], 1u);
+                } else if (e < 0) {
+                  atomicAdd(&a.so[((uint64_t)real * a.nC + c) * H + cat], 1ull);
+                } else {
+                  const int es = e + (a.dom_e >= 0 && e >= a.dom_e ? 1 : 0);
+                  atomicAdd(&a.rdf_core[(((uint64_t)real * a.nC + c) * a.nE + es) * H + cat], 1ull);
+                }
+              }
+              if (KNN) {
+                const int q = sSet[row + t];
+                if (q == qd) {
+                  if (q >= 0) z |= 1u << ((u ? p1 : p0) & 31u);  // a set that holds dom too: counted with its entries below
+                } else if (q >= 0) {
+                  const int m = cnt[q * 32];
+                  if (m < kmax) {
+                    const int kk = sK[m + 1];
+                    if (kk >= 0) out[(q * nkI + kk) * 32] = (uint16_t)cat;
+                    cnt[q * 32] = (uint8_t)(m + 1);
+                    unsat -= (m + 1 == kmax);
+                  }
                 }
               }
             }
           }
+#pragma unroll
+          for (int k = 0; k < kMinorChunks; ++k) wq[k] = 0;
         }
         if (KNN && qd >= 0 && nd < kmax) {
-          const int more = __popc(z);
-          while (kd < nkI && (int)sKv[kd] <= nd + more) {
-            out[(qd * nkI + kd) * 32] = wcat[nth_set(z, sKv[kd] - 1u - (uint32_t)nd)];
-            ++kd;
+          uint16_t* od = out + (uint32_t)qd * (uint32_t)nkI * 32u;
+          if (every) {
+            while (z && nd < kmax) {
+              const int kk = sK[++nd];
+              if (kk >= 0) od[kk * 32] = wcat[__ffs(z) - 1];
+              z &= z - 1u;
+            }
+          } else {
+            const int more = __popc(z);
+            for (int kd = sF[nd]; kd < nkI && (int)sKv[kd] <= nd + more; ++kd)
+              od[kd * 32] = wcat[nth_set(z, sKv[kd] - 1u - (uint32_t)nd)];
+            nd = min(nd + more, kmax);
           }
-          nd += more;
           unsat -= nd >= kmax;
         }
         __syncwarp();
@@ -4004,10 +4077,7 @@ __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
       if (KNN) {
         // the slots not met hold no category; orders found per set
         for (int q = 0; q < a.nsmax; ++q) {
-          int f = 0;
-          if (q == qd) f = kd;
-          else
-            while (f < nkI && (int)sKv[f] <= (int)cnt[q * 32]) ++f;
+          const int f = sF[q == qd ? nd : (int)cnt[q * 32]];
           for (int kk = f; kk < nkI; ++kk) out[(q * nkI + kk) * 32] = (uint16_t)0xffff;
           if (q < nset && f < nkI) {
             if (c == a.dom_c) atomicAdd(&sMiss[(q * (nkI + 1) + f) * 32 + lane], 1u);
@@ -4859,8 +4929,8 @@ int launch_cat_hist(const uint16_t* cat, uint64_t n, int H, unsigned long long* 
 
 int launch_knn_bin(const KnnArgs& k, int sm_count, cudaStream_t s) {
   if (k.cblk < 1) return -2;
-  const size_t smem = (size_t)k.cblk * k.H * 32 * 4;
-  if (smem > 200 * 1024) return -2;
+  const size_t smem = ((size_t)k.cblk * k.H + 1) * 32 * 4;
+  if (smem > 201 * 1024) return -2;
   if (smem > 48 * 1024 &&
       !allow_dynamic_smem((const void*)k_knn_bin, smem))
     return -1;
