@@ -2354,6 +2354,10 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
   ea.status = ctx->res.status.as<int>();
   ea.rdf_in_smem = 0;
   ea.mode = 2;
+  // balls kept in shared memory while the emit pass sorts them: some more than
+  // the mean; 1024 ions are 8 KB a warp, and beyond that few warps would be left
+  const uint64_t mean = nc ? total / nc : 0;
+  ea.pair_buf = mean <= 800 ? (int)std::min<uint64_t>((std::min<uint64_t>(mean + mean / 4 + 64, ctx->geo_maxlist) + 31) & ~31ull, 1024) : 0;
   ea.pair_slot = ctx->pair_slot.as<uint32_t>();
   ea.pair_cat = ctx->pair_cat.as<uint16_t>();
   CK(ctx->work.ensure(16));

@@ -128,6 +128,7 @@ struct ScanArgs {
   uint32_t* pair_slot;           // [total] (mode 2)
   uint16_t* pair_cat;            // [total] (mode 2)
   unsigned long long pair_cap;
+  int pair_buf;                  // mode 2: ions of a ball kept from the first walk (launch_scan: 0 where they do not fit)
   unsigned long long pair_base;  // pair_slot/pair_cat hold positions [pair_base, pair_base + pair_cap)
 };
 

@@ -939,6 +939,7 @@ struct ScanShared {
   uint32_t* rdf;
   uint32_t* cnt;
   int* hist;  // mode 2: per-warp category histogram
+  uint32_t* pbuf;  // mode 2: per warp pair_buf slots, then as many category | rank << 16
   unsigned long long* since_flush;
 };
 
@@ -1052,8 +1053,12 @@ __device__ __forceinline__ void for_each_candidate(const ScanArgs& a, const int8
   for_each_candidate_r(a, rowtab, cp, self, lane, a.R, a.Rm2, a.R2, f);
 }
 
-template <int KR, int EMAX>
-__global__ void __launch_bounds__(256) k_scan(ScanArgs a) {
+// LISTS: mode 2 (an instance of its own, which needs more registers).
+// Blocks an SM: one list in shared memory or none is faster with five than with
+// the registers of four (1M-ion cylinder, k = 10: 440 against 493 us).
+template <int KR, int EMAX, bool LISTS = false>
+__global__ void __launch_bounds__(256, LISTS ? 0 : KR == 0 || (KR == 1 && EMAX <= 1) ? 5 : EMAX == 0 || (KR == 1 && EMAX == 8) ? 3 : 0)
+k_scan(ScanArgs a) {
   // shared kNN list stride: one padding word keeps set p's k-th entry in bank
   // (p + k) % 32, so lanes testing different sets do not collide
   constexpr int LS = (KR > 0 ? KR : 1) * 32 + 1;
@@ -1073,7 +1078,8 @@ __global__ void __launch_bounds__(256) k_scan(ScanArgs a) {
     S.lst = (float*)p; p += ((KR > 0 && a.disjoint) ? nwarps * a.emax * LS * 4 : 0);
     S.rdf = (uint32_t*)p; p += (a.rdf_in_smem ? a.nC * a.nE * H * 4 : 0);
     S.cnt = (uint32_t*)p; p += ((a.flags & PP_CNTNB) ? nwarps * a.nE * 4 : 0);
-    S.hist = (int*)p; p += (a.mode == 2 ? nwarps * H * 4 : 0);
+    S.hist = (int*)p; p += (LISTS ? nwarps * H * 4 : 0);
+    S.pbuf = (uint32_t*)p; p += (LISTS ? nwarps * a.pair_buf * 8 : 0);
     S.sidx = (int8_t*)p;
   }
   for (int i = threadIdx.x; i <= H; i += blockDim.x) S.T[i] = i < H ? a.cat_T[i] : kInf();
@@ -1084,13 +1090,13 @@ __global__ void __launch_bounds__(256) k_scan(ScanArgs a) {
   if (KR > 0 && a.disjoint) for (int i = threadIdx.x; i < a.nC * 256; i += blockDim.x) S.sidx[i] = a.setidx[i];
   if (a.rdf_in_smem) for (int i = threadIdx.x; i < a.nC * a.nE * H; i += blockDim.x) S.rdf[i] = 0;
   if (a.flags & PP_CNTNB) for (int i = threadIdx.x; i < nwarps * a.nE; i += blockDim.x) S.cnt[i] = 0;
-  if (a.mode == 2) for (int i = threadIdx.x; i < nwarps * H; i += blockDim.x) S.hist[i] = 0;
+  if (LISTS) for (int i = threadIdx.x; i < nwarps * H; i += blockDim.x) S.hist[i] = 0;
   if (threadIdx.x == 0) *S.since_flush = 0ull;
   __syncthreads();
 
-  const bool doR = (a.flags & PP_RDF) && a.mode == 0;
-  const bool doC = (a.flags & PP_CNTNB) && a.mode == 0;
-  const bool doK = KR > 0 && a.mode == 0;
+  const bool doR = (a.flags & PP_RDF) && !LISTS && a.mode == 0;
+  const bool doC = (a.flags & PP_CNTNB) && !LISTS && a.mode == 0;
+  const bool doK = KR > 0 && !LISTS && a.mode == 0;
   const int krow = (a.kmax - 1) >> 5, klane = (a.kmax - 1) & 31;
   unsigned long long pairs_lane = 0, centres = 0, tests_lane = 0;
   constexpr unsigned long long FLUSH = 1ull << 30;
@@ -1116,13 +1122,13 @@ __global__ void __launch_bounds__(256) k_scan(ScanArgs a) {
       const uint32_t self = a.centres[a.sample_stride > 1 ? (uint64_t)ci * a.sample_stride : ci];
       const float4 cp = a.ions[self];
       const uint32_t ct = a.labels ? (uint32_t)a.labels[self] : __float_as_uint(cp.w);
-      const int cs = (a.mode == 0) ? S.cs[ct & 255] : 0;
+      const int cs = (!LISTS && a.mode == 0) ? S.cs[ct & 255] : 0;
       if (cs < 0) {  // selection guarantees a slot; record and skip otherwise
         if (lane == 0) atomicOr(a.status, ST_TYPE_RANGE);
         continue;
       }
       uint32_t inb = 0;
-      if (a.mode == 0) {
+      if (!LISTS && a.mode == 0) {
         // SL: shared-memory lists (disjoint environment sets, EMAX == 0);
         // otherwise register lists, one per local environment set
         constexpr bool SL = (EMAX == 0);
@@ -1260,19 +1266,35 @@ __global__ void __launch_bounds__(256) k_scan(ScanArgs a) {
           }
           __syncwarp();
         }
-      } else if (a.mode == 1) {
+      } else if (KR == 0 && !LISTS && a.mode == 1) {
         for_each_candidate(a, S.rowtab, cp, self, lane,
                            [&](bool, uint32_t, float, bool inball, uint32_t, bool) { inb += inball; });
         uint32_t tot = inb;
         for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(FULL, tot, o);
         if (lane == 0) a.pair_count[ci] = tot;
-      } else {
-        // mode 2: counting sort of the ball by category into the pair list
+      } else if constexpr (LISTS) {
+        // Mode 2: counting sort of the ball by category into the pair list.
+        // The walk that counts keeps its ions (slot, category, rank within the
+        // category) in shared memory, so that a ball of up to pair_buf ions is
+        // walked, measured and categorised once: 2M-ion tip, R = 1.5 nm, 190 ions a ball 6.5 -> 4.3 ms.  Larger
+        // balls are walked again.
         int* hist = S.hist + warp * H;
-        for_each_candidate(a, S.rowtab, cp, self, lane, [&](bool, uint32_t, float d2, bool inball, uint32_t, bool) {
-          if (inball)
-            atomicAdd(&hist[a.lut_one ? category_one(d2, S.lut, a.lut_n, a.lut_base, a.lut_shift, S.T)
-                                      : category_lut(d2, S.lut, a.lut_n, a.lut_base, a.lut_shift, S.T, H)], 1);
+        uint32_t* bslot = S.pbuf + warp * 2 * a.pair_buf;
+        uint32_t* bcr = bslot + a.pair_buf;
+        const uint32_t lt = (1u << lane) - 1u;
+        uint32_t nb = 0;
+        for_each_candidate(a, S.rowtab, cp, self, lane, [&](bool, uint32_t slot, float d2, bool inball, uint32_t, bool) {
+          const uint32_t in = __ballot_sync(FULL, inball);
+          if (inball) {
+            const int cat = a.lut_one ? category_one(d2, S.lut, a.lut_n, a.lut_base, a.lut_shift, S.T)
+                                      : category_lut(d2, S.lut, a.lut_n, a.lut_base, a.lut_shift, S.T, H);
+            const uint32_t rank = (uint32_t)atomicAdd(&hist[cat], 1), at = nb + __popc(in & lt);
+            if (at < (uint32_t)a.pair_buf) {
+              bslot[at] = slot;
+              bcr[at] = (uint32_t)cat | rank << 16;
+            }
+          }
+          nb += __popc(in);
         });
         __syncwarp();
         int run = 0;
@@ -1291,6 +1313,18 @@ __global__ void __launch_bounds__(256) k_scan(ScanArgs a) {
         __syncwarp();
         const unsigned long long off = a.pair_off[ci];
         const unsigned long long lim = a.pair_off[ci + 1];
+        if (nb <= (uint32_t)a.pair_buf) {
+          for (uint32_t e = lane; e < nb; e += 32) {
+            const uint32_t cr = bcr[e], cat = cr & 0xffffu;
+            const unsigned long long at = off + (uint32_t)hist[cat] + (cr >> 16);
+            if (at < lim && at - a.pair_base < a.pair_cap) {
+              a.pair_slot[at - a.pair_base] = bslot[e];
+              a.pair_cat[at - a.pair_base] = (uint16_t)cat;
+            }
+            else atomicOr(a.status, ST_LIST_OVERFLOW);
+            ++inb;
+          }
+        } else
         for_each_candidate(a, S.rowtab, cp, self, lane, [&](bool, uint32_t slot, float d2, bool inball, uint32_t, bool) {
           if (inball) {
             const int cat = a.lut_one ? category_one(d2, S.lut, a.lut_n, a.lut_base, a.lut_shift, S.T)
@@ -1335,7 +1369,7 @@ __global__ void __launch_bounds__(256) k_scan(ScanArgs a) {
   if (lane == 0) {
     atomicAdd(&a.counters[0], pairs_lane);
     atomicAdd(&a.counters[1], centres);
-    if (a.tests && a.mode == 0) atomicAdd(a.tests, tests_lane);
+    if (a.tests && !LISTS && a.mode == 0) atomicAdd(a.tests, tests_lane);
   }
   __syncthreads();
   if (a.rdf_in_smem && doR) {
@@ -4493,9 +4527,9 @@ void launch_select_centres(const uint8_t* labels, const float* surf, uint64_t n,
   k_select_write<<<grid_for(n, 256), 256, 0, s>>>(labels, surf, n, R2, cslot_of, extra, flags, out, count);
 }
 
-template <int KR, int EMAX>
+template <int KR, int EMAX, bool LISTS = false>
 static int launch_scan_t(const ScanArgs& a, int sm_count, size_t smem, cudaStream_t s) {
-  auto kern = k_scan<KR, EMAX>;
+  auto kern = k_scan<KR, EMAX, LISTS>;
   if (smem > 48 * 1024) {
     if (!allow_dynamic_smem((const void*)kern, smem)) return -1;
   }
@@ -4514,9 +4548,15 @@ int launch_scan(const ScanArgs& a, int kr, int emax, int sm_count, size_t* smem_
   if (kr > 0 && a.disjoint) smem += (size_t)nwarps * a.emax * (kr * 32 + 1) * 4;
   if (a.rdf_in_smem) smem += (size_t)a.nC * a.nE * a.H * 4;
   if (a.flags & PP_CNTNB) smem += (size_t)nwarps * a.nE * 4;
-  if (a.mode == 2) smem += (size_t)nwarps * a.H * 4;
+  ScanArgs b = a;
+  if (a.mode == 2) {
+    smem += (size_t)nwarps * a.H * 4;
+    if (a.H > 65535 || smem + (size_t)nwarps * a.pair_buf * 8 > 80 * 1024) b.pair_buf = 0;
+    smem += (size_t)nwarps * b.pair_buf * 8;
+  }
   if (kr > 0 && a.disjoint) smem += (size_t)a.nC * 256;
   if (smem_used) *smem_used = smem;
+  if (a.mode == 2) return kr == 0 ? launch_scan_t<0, 1, true>(b, sm_count, smem, s) : -2;
   if (kr == 0) return launch_scan_t<0, 1>(a, sm_count, smem, s);
   if (a.disjoint) {
     if (kr == 1) return launch_scan_t<1, 0>(a, sm_count, smem, s);

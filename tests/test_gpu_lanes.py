@@ -180,3 +180,26 @@ def test_inside_repeats(ctx):
     got = {tuple(sorted(ctx.inside(cid, 1.0, 1.0).items())) for _ in range(40)}
     ctx.free(cid)
     assert len(got) == 1
+
+
+@pytest.mark.parametrize("dense", [0, 500, 1500])
+def test_batched_lists_of_uneven_length(ctx, oracle, dense):
+    """Pair lists some of which are far longer than the mean: balls that the
+    first walk keeps and balls that are walked again, more than 1024 ions too."""
+    rng = np.random.default_rng(dense)
+    xyz = np.concatenate([rng.uniform(0, 11, (3000, 3)), rng.uniform(5, 5.4, (dense, 3))]).astype(np.float32)
+    n = len(xyz)
+    labels = rng.choice(np.array([1, 2], dtype=np.uint8), n, p=[0.9, 0.1])
+    sets = np.stack([rng.permutation(labels) for _ in range(2)])
+    d2, hist, ks, flags = np.full(n, 10.0, dtype=np.float32), (0.0, 0.02, 1.0), [6, 1], N.PP_RDF | N.PP_MKNN
+    trg, env = [[1], [2]], [[2], [1]]
+    cid = ctx.upload(xyz, labels)
+    ctx.surfdist(cid, d2)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.run_batched(cid, flags, ks, include_original=True, label_sets=sets)
+    got = [ctx.fetch_batched(r) for r in range(ctx.batched_count())]
+    ctx.free(cid)
+    for r, lab in enumerate([labels, sets[0], sets[1]]):
+        ref = oracle.spatstat(xyz, lab, d2, *hist, flags, trg, env, ks)
+        assert np.array_equal(got[r], ref["bins"]), r
