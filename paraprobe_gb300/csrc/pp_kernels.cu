@@ -3835,7 +3835,7 @@ __global__ void __launch_bounds__(1024, 1) k_knn_bin(KnnArgs a) {
 //   kNN  the k-th member of dom's set is the k-th zero bit; the other sets
 //        count their entries as k_knn_walk does, which takes every entry.
 // 2M-ion tip, 65 label sets (f = 4% not dom), R = 1.5 nm, 36 pairs, k = 1..8:
-// the whole call 109 -> 53 ms (k_minor_walk 22 ms where k_knn_walk and k_apply
+// the whole call 109 -> 51 ms (k_minor_walk 22 ms where k_knn_walk and k_apply
 // took 74).
 // Bins: N(dom, t) as [t][category][realisation] words (lane r hits bank r) and
 // A as [realisation][c][category] in shared memory; the rest, of centres that
@@ -4194,18 +4194,40 @@ __global__ void k_minor_fin(KnnArgs a) {
     }
 }
 
-// Realisation-major byte arrays src[rows][cols] to the group-major layout
-// k_apply reads: dst[((r / G) * cols + c) * G + r % G], rows padded to a
-// multiple of G with zeros.
-__global__ void k_interleave(const uint8_t* __restrict__ src, uint64_t rows, uint64_t cols, int G,
-                             uint8_t* __restrict__ dst) {
-  const uint64_t rows_pad = (rows + G - 1) / G * G;
-  const uint64_t total = cols * rows_pad;
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t g = t / (cols * G), rem = t - g * cols * G;
-    const uint64_t c = rem / G, r = g * G + (rem - c * G);
-    dst[t] = r < rows ? src[r * cols + c] : 0;
-  }
+// Realisation-major byte arrays src[rows][cols] to the group-major layout the
+// batched kernels read: dst[((r / G) * cols + c) * G + r % G], rows padded to a
+// multiple of G with zeros.  A thread takes the G bytes of a column and group:
+// neighbouring threads read neighbouring bytes of a row and write whole groups
+// (2M ions, 81 realisations in groups of 32: 0.68 -> 0.41 ms against a byte a
+// thread in the order written, whose reads of a warp are of 32 rows).  G is a power of two up to 32, so with dst from the allocator (256-byte
+// aligned) a group never straddles its own alignment; src needs none.
+template <int G>
+__global__ void k_interleave(const uint8_t* __restrict__ src, uint64_t rows, uint64_t cols, uint8_t* __restrict__ dst) {
+  const uint64_t ng = (rows + G - 1) / G;
+  for (uint64_t g = blockIdx.y; g < ng; g += gridDim.y)
+    for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < cols; c += (uint64_t)gridDim.x * blockDim.x) {
+      uint32_t w[(G + 3) / 4];
+#pragma unroll
+      for (int k = 0; k < (G + 3) / 4; ++k) w[k] = 0;
+#pragma unroll
+      for (int k = 0; k < G; ++k) {
+        const uint64_t r = g * G + k;
+        if (r < rows) w[k / 4] |= (uint32_t)src[r * cols + c] << (8 * (k & 3));
+      }
+      uint8_t* out = dst + (g * cols + c) * G;
+      if constexpr (G == 32) {
+        ((uint4*)out)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        ((uint4*)out)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+      } else if constexpr (G == 8) {
+        *(uint2*)out = make_uint2(w[0], w[1]);
+      } else if constexpr (G == 4) {
+        *(uint32_t*)out = w[0];
+      } else if constexpr (G == 2) {
+        *(uint16_t*)out = (uint16_t)w[0];
+      } else {
+        *out = (uint8_t)w[0];
+      }
+    }
 }
 
 // centre_ok for ROI realisations: type is a target, and r_roi - |p - c| >= R
@@ -4994,7 +5016,11 @@ int launch_knn_bin(const KnnArgs& k, int sm_count, cudaStream_t s) {
 
 void launch_interleave(const uint8_t* src, uint64_t rows, uint64_t cols, int G, uint8_t* dst, cudaStream_t s) {
   counted();
-  k_interleave<<<grid_for(cols * ((rows + G - 1) / G * G), 256), 256, 0, s>>>(src, rows, cols, G, dst);
+  const uint64_t bx = (cols + 255) / 256, by = (rows + G - 1) / G;
+  const dim3 grid((unsigned)std::min<uint64_t>(std::max<uint64_t>(bx, 1), 1u << 20),
+                  (unsigned)std::min<uint64_t>(std::max<uint64_t>(by, 1), 65535));
+  auto kern = G == 32 ? k_interleave<32> : G == 8 ? k_interleave<8> : G == 4 ? k_interleave<4> : G == 2 ? k_interleave<2> : k_interleave<1>;
+  kern<<<grid, 256, 0, s>>>(src, rows, cols, dst);
 }
 
 void launch_roi_mask(const float4* ions, const uint32_t* centres, uint32_t nc, const float* rois, int nrois, float R,
