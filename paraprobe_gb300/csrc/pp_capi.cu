@@ -1488,6 +1488,14 @@ bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long l
   return true;
 }
 
+// A buffer only the faster form of a pass needs: false when the device has no
+// room for it.
+bool scratch(DevBuf& b, size_t bytes) {
+  if (b.ensure(bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
 // The kNN part of a pass in two walks (k_lanes_near) where near_plan finds it
 // worth it, else -3.  count: the pass has no other part that counts its in-ball
 // pairs, so they are counted by a symmetric walk of their own first; the
@@ -1498,10 +1506,14 @@ int run_near(pp_ctx* ctx, Cloud& cl, const RunPlan& P, const unsigned long long*
   uint64_t sparse = 0;
   if (!near_plan(cl, P, R, type_counts, a, &sparse)) return -3;
   const uint64_t sp_words = a.sp_g.ncells + 1;
-  CK(ctx->sp_start.ensure(sp_words * 8));  // starts, then cursors
-  CK(ctx->sp_ions.ensure(std::max<uint64_t>(sparse, 1) * 16));
-  CK(ctx->sp_slot.ensure(std::max<uint64_t>(sparse, 1) * 4));
   const uint64_t tmp_elems = sp_words / 2048 + 64;
+  // shared memory before anything runs (many bins or sets leave too few
+  // warps), device memory likewise: one walk needs neither
+  if (pp::launch_lanes_near(a, ctx->sm_count, nullptr, nullptr, nullptr, nullptr, 0, nullptr, 0, nullptr, s, false)) return -3;
+  if (!scratch(ctx->sp_start, sp_words * 8) ||  // starts, then cursors
+      !scratch(ctx->sp_ions, std::max<uint64_t>(sparse, 1) * 16) ||
+      !scratch(ctx->sp_slot, std::max<uint64_t>(sparse, 1) * 4))
+    return -3;
   CK(ctx->scan_tmp.ensure(tmp_elems * 8 * 2));
   if (count) {
     pp::ScanArgs ac = a;
@@ -1652,6 +1664,8 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
       a.by = dby;
       a.bz = dbz;
     }
+    if (lanes && !a.sym && !scratch(ctx->nc_pre, (g.ncells + 1) * 4)) lanes = false;
+    if (lanes && !scratch(ctx->pass_code, std::max<uint64_t>(n, 1) * 4)) lanes = false;
     if (lanes || a.sym) {  // prefix of the non-centre ions per cell
       CK(ctx->nc_pre.ensure((g.ncells + 1) * 4));
       const uint64_t tmp_elems = (g.ncells + 1) / 2048 + 64;
@@ -1664,7 +1678,6 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
     a.brows = nullptr;
     if (lanes && (rc = ensure_block_rows(ctx, a.by, a.bz, a.bsr, s, &a.brows)) != PP_OK) return rc;
     if (lanes) {
-      CK(ctx->pass_code.ensure(std::max<uint64_t>(n, 1) * 4));
       a.pcode = ctx->pass_code.as<uint32_t>();
       a.label_sorted = labels ? labels : cl->label_sorted.as<uint8_t>();
       a.n = n;
@@ -3367,6 +3380,15 @@ int pp_server_submit(pp_server* S, int cloud, uint32_t flags, float rmin, float 
                               : (uint64_t)(13.0 * (double)cl->n + 4.0 * (double)cl->g.ncells + cores);
   q->t_submit = now_ms();
   const uint64_t need = q->footprint + (q->mergeable ? multi_base_bytes(cl->n) : 0);
+  // the centre-per-lane scans' pass codes and sparse list, which a pass does
+  // without where they do not fit: counted while the query runs, up to the
+  // budget, but no reason to refuse it
+  if (q->dense && need <= S->budget) {
+    uint64_t common = 0;
+    for (uint64_t c : cl->type_count) common = std::max<uint64_t>(common, c);
+    const uint64_t more = 4 * cl->n + 20 * (cl->n - std::min<uint64_t>(common, cl->n));
+    q->footprint = std::min<uint64_t>(q->footprint + more, S->budget);
+  }
   std::lock_guard<std::mutex> lk(S->mu);
   S->submitted++;
   if (need > S->budget) {

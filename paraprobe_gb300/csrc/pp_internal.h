@@ -289,7 +289,7 @@ int launch_lanes_knn(const ScanArgs& a, bool disjoint_sets, int sm_count, size_t
 // scratch for as many; sp_cap: ions sp_ions / sp_slot have room for
 int launch_lanes_near(const ScanArgs& a, int sm_count, uint32_t* sp_start, uint32_t* sp_cursor, float4* sp_ions,
                       uint32_t* sp_slot, uint32_t sp_cap, uint32_t* sp_tmp, uint64_t sp_tmp_elems, size_t* smem_used,
-                      cudaStream_t s);
+                      cudaStream_t s, bool launch = true);
 // the in-ball pairs (ScanArgs::counters) of a pass that need not bin them
 int launch_lanes_count(const ScanArgs& a, int sm_count, cudaStream_t s);
 void launch_type_count(const uint8_t* labels, uint64_t n, unsigned long long* out, int sm_count, cudaStream_t s);

@@ -4759,9 +4759,10 @@ void launch_type_count(const uint8_t* labels, uint64_t n, unsigned long long* ou
       labels, n, out);
 }
 
+// launch false: only whether the pass fits (0, else -3)
 int launch_lanes_near(const ScanArgs& a0, int sm_count, uint32_t* sp_start, uint32_t* sp_cursor, float4* sp_ions,
                       uint32_t* sp_slot, uint32_t sp_cap, uint32_t* sp_tmp, uint64_t sp_tmp_elems, size_t* smem_used,
-                      cudaStream_t s) {
+                      cudaStream_t s, bool launch) {
   ScanArgs a = a0;
   if (a.mode != 0 || (a.flags & (PP_CNTNB | PP_RDF)) || !a.uniform_sets || a.kmax < 1 || a.kmax > 20 || a.bx < 1 ||
       a.by < 1 || a.bz < 1 || !a.brows || a.nC > 127 || a.emax > 15 || a.near_n < 1 || a.near_n > kNearMax)
@@ -4788,6 +4789,7 @@ int launch_lanes_near(const ScanArgs& a0, int sm_count, uint32_t* sp_start, uint
   const int wd = warps(fix_d, dense_warp), ws = a.near_sp > 0 ? warps(fix_s, sparse_warp(cat)) : 4;
   if (wd < 4 || ws < 4 || (cat && a.H > 65535)) return -3;
   const size_t smem_d = fix_d + dense_warp * wd, smem_s = fix_s + sparse_warp(cat) * ws;
+  if (!launch) return 0;
   if (smem_used) *smem_used = std::max(smem_d, smem_s);
   launch_pass_codes(a, PC_NEAR, cat ? 32u : (uint32_t)a.kmax * 32u, sm_count, s);
   if (a.near_sp > 0) {

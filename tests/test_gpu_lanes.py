@@ -203,3 +203,27 @@ def test_batched_lists_of_uneven_length(ctx, oracle, dense):
     for r, lab in enumerate([labels, sets[0], sets[1]]):
         ref = oracle.spatstat(xyz, lab, d2, *hist, flags, trg, env, ks)
         assert np.array_equal(got[r], ref["bins"]), r
+
+
+@pytest.mark.parametrize("nbins", [8000, 16380])
+def test_knn_of_many_bins(ctx, oracle, nbins):
+    """Bins whose tables leave the kNN walks little shared memory, up to the most
+    that are taken."""
+    spec = synth.cylinder_specimen(n=12000, radius=2.5, height=14.0, fractions=(0.95, 0.04, 0.01), seed=3, nseg=32,
+                                   stack=4.0)
+    types = [1, 2, 3]
+    trg, env = [[a] for a in types for b in types], [[b] for a in types for b in types]
+    d2, hist, ks = np.full(len(spec.xyz), 10.0, dtype=np.float32), (0.0, 1.0 / nbins, 1.0), [20, 1]
+    cid = ctx.upload(spec.xyz, spec.labels)
+    ctx.surfdist(cid, d2)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.set_option("knn_walks", 2)
+    try:
+        ctx.run(cid, N.PP_MKNN, ks)
+        got, st = ctx.fetch(), ctx.stats()
+    finally:
+        ctx.set_option("knn_walks", 0)
+        ctx.free(cid)
+    ref = oracle.spatstat(spec.xyz, spec.labels, d2, *hist, N.PP_MKNN, trg, env, ks)
+    assert st["pairs"] == ref["pairs"] and np.array_equal(got, ref["bins"])
