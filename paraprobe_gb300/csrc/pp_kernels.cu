@@ -3025,8 +3025,7 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 1) k_lanes_knn(ScanArgs a) {
 // Bins: most centres are of one type (near_hot), and adding its categories to
 // the cores in global memory took longer than finding them.  They are counted
 // in shared memory, a dense set's below near_hd in 32 bits each, a sparse set's
-// in 16 bits each, moved to the cores every 2^15 centres of the block; the
-// other centres' go to the cores.
+// in 16 bits each (kHalfFlush); the other centres' go to the cores.
 
 // Rows (of 32 lanes) of a dense set's buffer: about 2 K and what eight tests add.
 __host__ __device__ constexpr int near_cap(int KB) { return 2 * KB + 28; }
@@ -3183,6 +3182,16 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 1) k_lanes_near(ScanArgs a) {
   nc.flush_found();
 }
 
+// Halfword bins.  A centre adds at most one count to a halfword, and `held`
+// (shared, one a block) is never less than the centres whose counts a halfword
+// may hold: a warp adds its batch's centres to it before their counts, and adds
+// the counts to the cores instead where that would take it past 2^16 - 1.  The
+// warp whose batch takes it to kHalfFlush empties every word and then takes off
+// what it was when the emptying began, less the one batch each warp may have
+// announced by then without having added it; no other warp can cross the line
+// before that.
+constexpr uint32_t kHalfFlush = 1u << 15;
+static_assert(kHalfFlush > kKnnWarps * 32u, "what an emptying takes off is positive");
 // Sparse sets together: threshold test and sorted insertion as in k_lanes_knn
 // (CAT: the lists hold categories, two ranks a word, so that an insertion into a
 // list of 20 moves 10 words: 12M-ion tip, 7 sets, k <= 20 within 2.5 nm 12.0 ->
@@ -3202,12 +3211,12 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 1) k_lanes_sparse(ScanArgs a) 
   uint32_t* skeyA = (uint32_t*)sp; sp += NW * kStageAll * 4;
   uint32_t* queueA = (uint32_t*)sp; sp += NW * 64 * 4;
   float* listA = (float*)sp; sp += (size_t)NW * lrows * 32 * 4;
-  // the hot centre slot's bins [set][order][H], halfwords; centres taken
+  // the hot centre slot's bins [set][order][H], halfwords; centres they may hold
   const uint32_t nhalf = a.near_hs ? ((uint32_t)SPN * nkI * H + 1) / 2 : 0u;
-  uint32_t* sflush = (uint32_t*)sp; sp += 16;
+  uint32_t* sheld = (uint32_t*)sp; sp += 16;
   uint32_t* shalf = (uint32_t*)sp; sp += (size_t)nhalf * 4;
   for (uint32_t i = threadIdx.x; i < nhalf; i += blockDim.x) shalf[i] = 0;
-  if (threadIdx.x == 0) *sflush = 0;
+  if (threadIdx.x == 0) *sheld = 0;
   const KnnCommon nc(a, sp);
   __syncthreads();
   float4* cand = candA + warp * kStageAll;
@@ -3305,7 +3314,26 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 1) k_lanes_sparse(ScanArgs a) 
         });
     tests += (unsigned long long)__popc(B.live) * staged;
     const int nset = cs >= 0 ? a.nsets[cs] : 0;
-    const bool hot = a.near_hs && cs == a.near_hot;
+    bool room = false;
+    if (a.near_hs) {
+      const uint32_t n = (uint32_t)__popc(B.live);
+      uint32_t held = 0;
+      if (lane == 0) held = atomicAdd(sheld, n);
+      held = __shfl_sync(FULL, held, 0);
+      room = held + n <= 0xffffu;
+      if (held < kHalfFlush && held + n >= kHalfFlush) {
+        held += n;
+        do {  // again if the other warps took as many meanwhile
+          __syncwarp();
+          flush_half(lane, 32);
+          __syncwarp();
+          const uint32_t off = held - (uint32_t)NW * 32u;
+          if (lane == 0) held = atomicSub(sheld, off) - off;
+          held = __shfl_sync(FULL, held, 0);
+        } while (held >= kHalfFlush);
+      }
+    }
+    const bool hot = room && cs == a.near_hot;
     for (int p = 0; p < nset; ++p) {
       const int m = a.near_map[p];
       if (m < 0) continue;
@@ -3330,14 +3358,6 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 1) k_lanes_sparse(ScanArgs a) 
         }
       }
       nc.found(cs, p, kk);
-    }
-    if (a.near_hs) {
-      // a halfword gains at most one count a centre: empty them before 2^16
-      const uint32_t n = (uint32_t)__popc(B.live);
-      uint32_t old = 0;
-      if (lane == 0) old = atomicAdd(sflush, n);
-      old = __shfl_sync(FULL, old, 0);
-      if ((old >> 15) != ((old + n) >> 15)) flush_half(lane, 32);
     }
     __syncwarp();
   });
