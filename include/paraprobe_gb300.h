@@ -262,6 +262,11 @@ int pp_fetch_npcorr(pp_ctx* ctx, uint32_t* counts, uint64_t cap, uint64_t* edge)
  *                       ions apart: 0 = where that is faster (default), 1 =
  *                       never, 2 = wherever the sets allow.  Results are
  *                       identical either way.
+ *   "scratch"           device buffers that only the faster form of a pass needs:
+ *                       -1 = given while there is room (default); n = a run
+ *                       gets the first n it asks for and does without the
+ *                       others, as when the device is full.  Results are
+ *                       identical either way.
  *   "box_filter"        the centre-per-lane scans test only ions within R of
  *                       the bounding box of a batch's centres (default 1);
  *                       0 tests every ion of the block's stencil rows.

@@ -238,6 +238,7 @@ struct pp_ctx {
   bool no_box = false;      // option "box_filter" = 0: the lane scans stage every candidate of the cell rows
   int knn_walks = 0;        // option "knn_walks": 0 automatic, 1 one walk, 2 two walks where the sets allow
   int knn_lists = 0;        // option "knn_lists": 0 automatic, 1 d^2 lists, 2 category lists
+  int scratch_limit = -1, scratch_taken = 0;  // option "scratch" (see scratch()); asked for by this run
   DevBuf brows;           // stencil rows of a cell block, nearest first (centre-per-lane scan)
   int brows_key[3] = {-1, -1, -1};
   pp_ctx* parent = nullptr;     // serving workers share the parent's clouds
@@ -1489,8 +1490,9 @@ bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long l
 }
 
 // A buffer only the faster form of a pass needs: false when the device has no
-// room for it.
-bool scratch(DevBuf& b, size_t bytes) {
+// room for it, or past the first scratch_limit of a run (a testing hook).
+bool scratch(pp_ctx* ctx, DevBuf& b, size_t bytes) {
+  if (ctx->scratch_limit >= 0 && ctx->scratch_taken++ >= ctx->scratch_limit) return false;
   if (b.ensure(bytes) == cudaSuccess) return true;
   cudaGetLastError();
   return false;
@@ -1510,11 +1512,11 @@ int run_near(pp_ctx* ctx, Cloud& cl, const RunPlan& P, const unsigned long long*
   // shared memory before anything runs (many bins or sets leave too few
   // warps), device memory likewise: one walk needs neither
   if (pp::launch_lanes_near(a, ctx->sm_count, nullptr, nullptr, nullptr, nullptr, 0, nullptr, 0, nullptr, s, false)) return -3;
-  if (!scratch(ctx->sp_start, sp_words * 8) ||  // starts, then cursors
-      !scratch(ctx->sp_ions, std::max<uint64_t>(sparse, 1) * 16) ||
-      !scratch(ctx->sp_slot, std::max<uint64_t>(sparse, 1) * 4))
+  if (!scratch(ctx, ctx->sp_start, sp_words * 8) ||  // starts, then cursors
+      !scratch(ctx, ctx->sp_ions, std::max<uint64_t>(sparse, 1) * 16) ||
+      !scratch(ctx, ctx->sp_slot, std::max<uint64_t>(sparse, 1) * 4) ||
+      !scratch(ctx, ctx->scan_tmp, tmp_elems * 8 * 2))
     return -3;
-  CK(ctx->scan_tmp.ensure(tmp_elems * 8 * 2));
   if (count) {
     pp::ScanArgs ac = a;
     ac.sym = ctx->no_sym ? 0 : 1;
@@ -1539,6 +1541,7 @@ int run_near(pp_ctx* ctx, Cloud& cl, const RunPlan& P, const unsigned long long*
 int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, int nk, const uint32_t* label_perm,
               cudaStream_t s, uint32_t centre_limit, const uint8_t* labels_override = nullptr,
               bool no_miss = false, const uint8_t* centre_mask = nullptr) {
+  ctx->scratch_taken = 0;
   RunPlan P;
   int rc = make_plan(ctx, flags, k_list, nk, P);
   if (rc) return rc;
@@ -1636,18 +1639,6 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
                      (block_ok || (P.disjoint && P.nC <= 8 && P.emax <= 15 && P.kmax <= 64 &&
                                    (uint64_t)ncent * std::max<uint32_t>(stride, 1) >= 4096));
   if (both && !split) lanes = false;
-  // kNN in two walks: needs the ions of each type of this run's labels
-  const bool near_ok = lanes && P.kr == 1 && P.kmax <= 20 && P.disjoint &&
-                       near_pays(ctx, *cl, R, P.kmax, (uint64_t)ncent * std::max<uint32_t>(stride, 1), !both);
-  std::vector<unsigned long long> type_counts(near_ok ? 256 : 0);
-  if (near_ok) {
-    CK(ctx->type_counts.ensure(256 * 8));
-    CK(cudaMemsetAsync(ctx->type_counts.p, 0, 256 * 8, s));
-    pp::launch_type_count(labels ? labels : cl->label_sorted.as<uint8_t>(), n, ctx->type_counts.as<unsigned long long>(),
-                          ctx->sm_count, s);
-    CK(cudaMemcpyAsync(type_counts.data(), ctx->type_counts.p, 256 * 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-  }
   // RDF / RIPK alone: each pair of two centres is computed once and credited
   // to both (the counts are the same as the per-centre ball scan's)
   a.sym = ((P.kr == 0 || split) && !(flags & PP_CNTNB) && (a.flags & PP_RDF) && !ctx->no_sym) ? 1 : 0;
@@ -1664,8 +1655,22 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
       a.by = dby;
       a.bz = dbz;
     }
-    if (lanes && !a.sym && !scratch(ctx->nc_pre, (g.ncells + 1) * 4)) lanes = false;
-    if (lanes && !scratch(ctx->pass_code, std::max<uint64_t>(n, 1) * 4)) lanes = false;
+    // the symmetric per-centre scan needs the prefix too; with kNN there is none
+    if (lanes && !(a.sym && P.kr == 0) && !scratch(ctx, ctx->nc_pre, (g.ncells + 1) * 4)) lanes = false;
+    if (lanes && !scratch(ctx, ctx->pass_code, std::max<uint64_t>(n, 1) * 4)) lanes = false;
+    if (!lanes && P.kr > 0) a.sym = 0;
+    // kNN in two walks: needs the ions of each type of this run's labels
+    const bool near_ok = lanes && P.kr == 1 && P.kmax <= 20 && P.disjoint &&
+                         near_pays(ctx, *cl, R, P.kmax, (uint64_t)ncent * std::max<uint32_t>(stride, 1), !both);
+    std::vector<unsigned long long> type_counts(near_ok ? 256 : 0);
+    if (near_ok) {
+      CK(ctx->type_counts.ensure(256 * 8));
+      CK(cudaMemsetAsync(ctx->type_counts.p, 0, 256 * 8, s));
+      pp::launch_type_count(labels ? labels : cl->label_sorted.as<uint8_t>(), n, ctx->type_counts.as<unsigned long long>(),
+                            ctx->sm_count, s);
+      CK(cudaMemcpyAsync(type_counts.data(), ctx->type_counts.p, 256 * 8, cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+    }
     if (lanes || a.sym) {  // prefix of the non-centre ions per cell
       CK(ctx->nc_pre.ensure((g.ncells + 1) * 4));
       const uint64_t tmp_elems = (g.ncells + 1) / 2048 + 64;
@@ -2111,6 +2116,11 @@ int pp_set_option(pp_ctx* ctx, const char* name, int value) {
   if (std::strcmp(name, "knn_lists") == 0) {
     if (value < 0 || value > 2) return fail(ctx, PP_ERR_INVALID, "knn_lists must be 0, 1 or 2");
     ctx->knn_lists = value;
+    return PP_OK;
+  }
+  if (std::strcmp(name, "scratch") == 0) {
+    if (value < -1) return fail(ctx, PP_ERR_INVALID, "scratch must be -1 or a number of buffers");
+    ctx->scratch_limit = value;
     return PP_OK;
   }
   if (std::strcmp(name, "knn_walks") == 0) {

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from paraprobe_gb300 import native as N
+from paraprobe_gb300 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +46,50 @@ def test_sparse_bins_of_one_lattice(ctx):
     want[:, 1] = [n - n2, n - n2, n2, n2]  # (1, 1), (1, 2), (2, 1), (2, 2)
     assert np.array_equal(one.reshape(4, 3), want)
     assert np.array_equal(two.reshape(4, 3), want)
+
+
+@pytest.mark.parametrize("flags", [N.PP_RDF, N.PP_MKNN, N.PP_RDF | N.PP_MKNN])
+@pytest.mark.parametrize("symmetric", [1, 0])
+def test_passes_without_their_scratch(ctx, oracle, flags, symmetric):
+    """A device without room for the buffers of a pass's faster form: whichever
+    of them is the first that is missing, the pass gives the same counts, and
+    one that ends up on the per-centre scan prepares nothing it does not use."""
+    spec = synth.cylinder_specimen(n=24000, radius=3.0, height=18.0, fractions=(0.95, 0.04, 0.01), seed=11, nseg=48,
+                                   stack=4.0)
+    d2 = np.where(np.arange(len(spec.xyz)) % 11 == 0, 1.0, 10.0).astype(np.float32)
+    trg, env = _pairs((1, 2, 3))
+    hist, ks = (0.0, 0.01, 1.5), [9, 1] if flags & N.PP_MKNN else []
+    cid = ctx.upload(spec.xyz, spec.labels)
+    ctx.surfdist(cid, d2)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.set_option("symmetric", symmetric)
+    ctx.set_option("knn_walks", 2)
+
+    def run():
+        before = N.kernel_launches()
+        ctx.run(cid, flags, ks)
+        return ctx.fetch(), ctx.stats(), ctx.last_kernel(), N.kernel_launches() - before, ctx.run_tests()
+
+    try:
+        run()
+        ctx.set_option("lanes", 0)
+        scan = run()
+        ctx.set_option("lanes", 1)
+        got = []
+        for limit in range(8):
+            ctx.set_option("scratch", limit)
+            got.append(run())
+        ctx.set_option("scratch", -1)
+        got.append(run())
+    finally:
+        for name, value in (("symmetric", 1), ("knn_walks", 0), ("lanes", 1), ("scratch", -1)):
+            ctx.set_option(name, value)
+        ctx.free(cid)
+    ref = oracle.spatstat(spec.xyz, spec.labels, d2, *hist, flags, trg, env, ks)
+    for bins, st, *_ in [scan] + got:
+        assert np.array_equal(bins, ref["bins"]) and st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
+    assert scan[2] == got[0][2] == "k_scan" and scan[3] == got[0][3]
+    assert got[-1][2] != "k_scan"
+    if flags & N.PP_MKNN:  # two walks, one walk without the sparse list, the per-centre scan
+        assert len({g[4] for g in got}) == 3
