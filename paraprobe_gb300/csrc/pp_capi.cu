@@ -1405,9 +1405,10 @@ bool near_pays(const pp_ctx* ctx, const Cloud& cl, float R, int kmax, uint64_t c
 
 // Dense sets of a kNN pass in two walks (k_lanes_near) for a block of a.bx x
 // a.by x a.bz cells, from the ions of each type; fills ScanArgs::near_* and
-// returns whether the pass is worth it (sparse = ions of the other sets).
-bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long long* type_counts, pp::ScanArgs& a,
-               uint64_t* sparse) {
+// returns whether the sets allow it and (unless forced) it is worth it (sparse =
+// ions of the other sets).
+bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long long* type_counts, bool forced,
+               pp::ScanArgs& a, uint64_t* sparse) {
   const uint64_t n = cl.n;
   if (!a.uniform_sets || !P.disjoint || P.kmax < 1 || P.kmax > 20 || P.emax > 15 || !cl.occupied || !n) return false;
   const double h = cl.g.h, rho = ion_density(cl);
@@ -1482,7 +1483,7 @@ bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long l
   for (int c = 1; c < P.nC; ++c)
     if (type_counts[P.ctype[c]] > type_counts[P.ctype[a.near_hot]]) a.near_hot = c;
   walk += around(R) * (double)*sparse / (double)n;
-  if (walk > 0.5 * around(R)) return false;
+  if (!forced && walk > 0.5 * around(R)) return false;
   // the dense sets' shared histograms end at the first radius
   const float d2 = a.near_r[a.near_n - 1] * a.near_r[a.near_n - 1];
   a.near_hd = (int)(std::upper_bound(P.catT.begin() + 1, P.catT.end(), d2) - P.catT.begin());
@@ -1506,7 +1507,7 @@ int run_near(pp_ctx* ctx, Cloud& cl, const RunPlan& P, const unsigned long long*
              const pp::ScanArgs& a0, bool count, size_t* smem, cudaStream_t s) {
   pp::ScanArgs a = a0;
   uint64_t sparse = 0;
-  if (!near_plan(cl, P, R, type_counts, a, &sparse)) return -3;
+  if (!near_plan(cl, P, R, type_counts, ctx->knn_walks == 2, a, &sparse)) return -3;
   const uint64_t sp_words = a.sp_g.ncells + 1;
   const uint64_t tmp_elems = sp_words / 2048 + 64;
   // shared memory before anything runs (many bins or sets leave too few

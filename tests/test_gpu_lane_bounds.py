@@ -93,3 +93,31 @@ def test_passes_without_their_scratch(ctx, oracle, flags, symmetric):
     assert got[-1][2] != "k_scan"
     if flags & N.PP_MKNN:  # two walks, one walk without the sparse list, the per-centre scan
         assert len({g[4] for g in got}) == 3
+
+
+@pytest.mark.parametrize("flags", [N.PP_MKNN, N.PP_MKNN | N.PP_RDF])
+@pytest.mark.parametrize("fractions", [(0.97, 0.02, 0.01), (0.5, 0.45, 0.05)])
+@pytest.mark.parametrize("ks", [[8, 1], [10, 1], [16, 2], [20, 19]])
+def test_two_walks_when_asked_for(ctx, oracle, flags, fractions, ks):
+    """knn_walks = 2 takes two walks wherever the sets allow, also where one walk
+    would be the cheaper: the tests it counts are others than one walk's."""
+    spec = synth.cylinder_specimen(n=24000, radius=3.0, height=18.0, fractions=fractions, seed=5, nseg=48, stack=4.0)
+    d2 = np.full(len(spec.xyz), 10.0, dtype=np.float32)
+    trg, env = _pairs((1, 2, 3))
+    hist = (0.0, 0.01, 1.5)
+    cid = ctx.upload(spec.xyz, spec.labels)
+    ctx.surfdist(cid, d2)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    try:
+        tests, bins = {}, {}
+        for walks in (1, 2):
+            ctx.set_option("knn_walks", walks)
+            ctx.run(cid, flags, ks)
+            bins[walks], tests[walks] = ctx.fetch(), ctx.run_tests()
+    finally:
+        ctx.set_option("knn_walks", 0)
+        ctx.free(cid)
+    assert tests[1] != tests[2]
+    ref = oracle.spatstat(spec.xyz, spec.labels, d2, *hist, flags, trg, env, ks)
+    assert np.array_equal(bins[1], ref["bins"]) and np.array_equal(bins[2], ref["bins"])
