@@ -2303,6 +2303,7 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
   if (flags & (PP_CNTNB | PP_NPCORR)) return fail(ctx, PP_ERR_UNSUPPORTED, "PP_CNTNB and PP_NPCORR are provided by pp_run only");
   const int nreal = (include_original ? 1 : 0) + n_label_sets + n_rois;
   if (nreal == 0) return fail(ctx, PP_ERR_INVALID, "no realisation requested");
+  ctx->scratch_taken = 0;
   CK(cudaSetDevice(ctx->device));
   cudaStream_t s = (cudaStream_t)stream;
   RunPlan P;
@@ -2601,9 +2602,32 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
             minor_knn = kq.do_knn != 0;
           }
         }
-        if (!minor_rdf && !minor_knn) kq.do_rdf = kq.do_knn = 0;
       }
     }
+    // its groups of 32 realisations and its buffers; without them the other
+    // kernels do the work.  Sums of one call: cleared, filled and read by the
+    // graph; the last group's lanes may lie past the realisations, so rows for
+    // whole groups
+    int ngm = minor_knn ? (nreal + 31) / 32 : minor_rdf ? (nlab + 31) / 32 : 0;
+    uint64_t nsa = 0, nso = 0, ntc = 0, sums_bytes = 0;
+    if (ngm) {
+      const uint64_t rr = (uint64_t)ngm * 32, H = P.H;
+      if (minor_rdf) {
+        nsa = rr * (uint64_t)(P.nC + 1) * H;
+        nso = rr * (uint64_t)P.nC * H;
+        ntc = H;
+      }
+      const uint64_t nfound = minor_knn ? rr * (uint64_t)P.nC * std::max(P.emax, 1) * (P.kvals.size() + 1) : 0;
+      sums_bytes = (nsa + nso + ntc) * 8 + nfound * 4;
+      if (!scratch(ctx, ctx->minor_masks, std::max<uint64_t>(n, 1) * 4 * ngm) || !scratch(ctx, ctx->minor_sums, sums_bytes) ||
+          (!knn32 && (!scratch(ctx, ctx->knn_labels, std::max<uint64_t>(n, 1) * 32 * ngm) ||
+                      !scratch(ctx, ctx->knn_ok, std::max<uint64_t>(nc, 1) * 32 * ngm)))) {
+        minor_rdf = minor_knn = false;
+        ngm = 0;
+        sums_bytes = 0;
+      }
+    }
+    if (!ngm) kq.do_rdf = kq.do_knn = 0;
     // the fused kernel is left with the regions of interest
     const uint8_t* RLb = RL;
     const uint8_t* OKb = OK;
@@ -2650,7 +2674,6 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
     pp::ApplyArgs bk;
     std::memset(&bk, 0, sizeof bk);
     bool knn_rest = false;
-    const int ngm = minor_knn ? (nreal + 31) / 32 : minor_rdf ? (nlab + 31) / 32 : 0;  // groups of k_minor_walk
     if (knn32) {
       const int rest = nreal % 32;
       ng32 = (nreal + 31) / 32;
@@ -2694,22 +2717,13 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
       kq.centre_ok = ctx->knn_ok.as<uint8_t>();
       kq.work = ctx->work.as<uint32_t>() + 1;
     }
-    uint64_t sums_bytes = 0;
     if (ngm) {
-      CK(ctx->minor_masks.ensure(std::max<uint64_t>(n, 1) * 4 * ngm));
       pp::launch_minor_masks(kq.labels, n * (uint64_t)ngm, kq.dom, ctx->minor_masks.as<uint32_t>(), s);
       kq.minor = ctx->minor_masks.as<uint32_t>();
-      // sums of one call: cleared, filled and read by the graph.  The last
-      // group's lanes may lie past the realisations: rows for whole groups
-      const uint64_t rr = (uint64_t)ngm * 32, H = P.H;
-      const uint64_t nsa = rr * (uint64_t)(P.nC + 1) * H, nso = rr * (uint64_t)P.nC * H;
-      const uint64_t nfound = rr * (uint64_t)P.nC * std::max(P.emax, 1) * (P.kvals.size() + 1);
-      sums_bytes = (nsa + nso + H) * 8 + nfound * 4;
-      CK(ctx->minor_sums.ensure(sums_bytes));
       kq.sa = ctx->minor_sums.as<unsigned long long>();
       kq.so = kq.sa + nsa;
       kq.tcat = kq.so + nso;
-      kq.found = (uint32_t*)(kq.tcat + H);
+      kq.found = (uint32_t*)(kq.tcat + ntc);
       if (!knn32) chunk = nc;
     }
     auto enqueue = [&](cudaStream_t st) -> int {
