@@ -279,8 +279,9 @@ int pp_fetch_npcorr(pp_ctx* ctx, uint32_t* counts, uint64_t cap, uint64_t* edge)
  *                       1 = the reference's guard loop as written (see there).
  *   "batched_minor"     pp_run_batched counts the pairs and members of the type
  *                       most ions are of by what is not of it: 0 = never, 1 =
- *                       where three quarters of the ions are (default), 2 =
- *                       always.  Results are identical either way.
+ *                       where three quarters of the ions are and the number of
+ *                       realisations and the tasks make it the faster (default),
+ *                       2 = always.  Results are identical either way.
  *   "batched_pair_cap"  most pairs pp_run_batched holds at once; larger lists
  *                       are built and applied a chunk of centres at a time
  *                       (0 = sized from free device memory, the default). */

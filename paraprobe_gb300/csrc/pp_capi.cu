@@ -2293,6 +2293,38 @@ int pp_shuffle_labels(const uint8_t* label, uint64_t n, uint64_t seed, uint8_t* 
 }
 
 // ------------------------------------------------------------- batched
+namespace {
+// Whether a group of 32 lanes of k_minor_walk pays for itself with `r`
+// realisations.  `other`: share of the ions that are not of the common type;
+// `bare`: of those in no environment, each of which costs an RDF walk an add in
+// global memory where the common type's own pairs are asked for.  Measured on
+// 50k to 1M ions of 30 to 450 a ball, 1 to 65 realisations, all pairs and eight
+// smaller task lists, as speed against the other kernels, for shares of 3, 15
+// and 23%: RDF of 8 realisations 1.02, 0.61, 0.49, of 16 1.49, 0.89, 0.72, of
+// 32 2.23, 1.36, 1.11, and with half of them bare 2.5, 0.91, 0.65; kNN of 2
+// 0.86, 0.65, 0.56, of 3 1.13, 0.85, 0.74, of 5 1.54, 1.15, 1.00, of 9 and more
+// always the faster.  RDF of a group walked for its kNN anyway costs little; not
+// so little where a set holds the common type and others (`holds`), as the walk
+// then takes its entries a chunk at a time (RDF and kNN of 16: 1.59, 0.92,
+// 0.68).  Where the common type is no centre the other kernels have few centres
+// to walk (`centres`, their share of the ions): RDF of 65 0.88, 0.79, 0.69, kNN
+// of 5 0.85 to 1.14.
+struct MinorLanes {
+  double other, bare, centres;
+  bool centre, in_env, holds, always;
+  bool knn(int r, bool with_rdf) const {
+    if (r <= 0 || always || r > 8) return r > 0;
+    return r >= (!centre ? 5.0 + 0.06 / centres : with_rdf ? 2.5 + 11.0 * other : 3.0 + 10.0 * other);
+  }
+  bool rdf(int r, bool with_knn) const {
+    const double w = other + 2.0 * bare;
+    if (r <= 0 || always) return r > 0;
+    if (!centre) return !in_env && with_knn && r >= 50.0 * w;
+    return with_knn ? w <= 0.3 && r >= (holds ? 100.0 : 20.0) * w : r >= 4.0 + 112.0 * w;
+  }
+};
+}  // namespace
+
 int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_list, int nk, int include_original,
                    const uint8_t* label_sets, int n_label_sets, const float* rois, int n_rois, void* stream) {
   if (!ctx) return PP_ERR_INVALID;
@@ -2561,10 +2593,13 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
       if (knn32) b.flags &= ~PP_MKNN;
     }
     // clouds of one common type: RDF of the label sets and kNN by what is not
-    // of it (k_minor_walk), where its bins fit.  Its work grows with the share
-    // of the other ions, and at a quarter of them is still the smaller one.
+    // of it (k_minor_walk), where its bins fit.  A group of 32 lanes costs the
+    // more, the more ions are not of that type, and little less for few
+    // realisations than for 32, so the last, partial group takes it only where
+    // enough of its lanes work: minor_knn groups of all realisations, minor_rdf
+    // label sets.
     const int nlab = nreal - n_rois;
-    bool minor_rdf = false, minor_knn = false;
+    int minor_rdf = 0, minor_knn = 0;
     {
       std::vector<unsigned long long> tc(256);
       CK(ctx->type_counts.ensure(256 * 8));
@@ -2573,7 +2608,20 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
       CK(cudaMemcpyAsync(tc.data(), ctx->type_counts.p, 256 * 8, cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
       const int dom = (int)(std::max_element(tc.begin(), tc.end()) - tc.begin());
-      if (ctx->batched_minor && (ctx->batched_minor == 2 || 4 * tc[dom] >= 3 * n)) {
+      const bool always = ctx->batched_minor == 2;
+      if (always || (ctx->batched_minor && 4 * tc[dom] >= 3 * n)) {
+        MinorLanes lanes{1.0 - (double)tc[dom] / (double)n, 0.0, 1e-6, P.cslot_of[dom] >= 0, P.eslot_of[dom] >= 0,
+                         false, always};
+        for (int t = 0; t < 256; ++t) {
+          const double share = (double)tc[t] / (double)n;
+          if (P.cslot_of[t] >= 0) lanes.centres += share;
+          if (t == dom) continue;
+          if (lanes.in_env && P.eslot_of[t] < 0) lanes.bare += share;
+          for (int c = 0; c < P.nC && P.disjoint; ++c)
+            lanes.holds |= P.setidx[c * 256 + t] >= 0 && P.setidx[c * 256 + t] == P.setidx[c * 256 + dom];
+        }
+        const bool want_knn = knn32 && P.disjoint, want_rdf = (b.flags & PP_RDF) && !(b.flags & PP_MKNN);
+        const int gk = nreal / 32 + (lanes.knn(nreal % 32, want_rdf) ? 1 : 0);
         kq.dom = dom;
         kq.dom_c = P.cslot_of[dom];
         kq.dom_e = P.eslot_of[dom];
@@ -2581,7 +2629,6 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
         kq.eslot_of = D.eslot;
         kq.rdf_core = b.rdf_core;
         kq.counters = b.counters;
-        kq.nlab = nlab;
         kq.centres = b.centres;
         kq.ncentres = nc;
         kq.pair_off = b.pair_off;
@@ -2593,13 +2640,17 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
         kq.nsets = D.nsets;
         kq.nC = P.nC;
         kq.H = P.H;
-        const int want_knn = knn32 && P.disjoint, want_rdf = nlab > 0 && (b.flags & PP_RDF) && !(b.flags & PP_MKNN);
         for (int form = 0; form < 3 && !minor_rdf && !minor_knn; ++form) {
-          kq.do_rdf = form == 1 ? 0 : want_rdf;
-          kq.do_knn = form == 2 ? 0 : want_knn;
-          if ((kq.do_rdf || kq.do_knn) && pp::minor_warps(kq)) {
-            minor_rdf = kq.do_rdf != 0;
-            minor_knn = kq.do_knn != 0;
+          const int k = want_knn && form != 2 ? gk : 0;
+          // label sets of whole groups, and of the last one where its lanes pay
+          const int last = nlab / 32, full = lanes.rdf(32, k > 0) ? 32 * last : 0;
+          const int l = !want_rdf || form == 1 ? 0 : lanes.rdf(nlab % 32, last < k) ? nlab : full;
+          kq.do_rdf = l > 0;
+          kq.do_knn = k > 0;
+          kq.nlab = l;
+          if ((k || l) && pp::minor_warps(kq)) {
+            minor_rdf = l;
+            minor_knn = k;
           }
         }
       }
@@ -2608,11 +2659,11 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
     // kernels do the work.  Sums of one call: cleared, filled and read by the
     // graph; the last group's lanes may lie past the realisations, so rows for
     // whole groups
-    int ngm = minor_knn ? (nreal + 31) / 32 : minor_rdf ? (nlab + 31) / 32 : 0;
+    int ngm = std::max(minor_knn, (minor_rdf + 31) / 32);
     uint64_t nsa = 0, nso = 0, ntc = 0, sums_bytes = 0;
     if (ngm) {
       const uint64_t rr = (uint64_t)ngm * 32, H = P.H;
-      if (minor_rdf) {
+      if (minor_rdf && kq.dom_e >= 0) {
         nsa = rr * (uint64_t)(P.nC + 1) * H;
         nso = rr * (uint64_t)P.nC * H;
         ntc = H;
@@ -2622,21 +2673,21 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
       if (!scratch(ctx, ctx->minor_masks, std::max<uint64_t>(n, 1) * 4 * ngm) || !scratch(ctx, ctx->minor_sums, sums_bytes) ||
           (!knn32 && (!scratch(ctx, ctx->knn_labels, std::max<uint64_t>(n, 1) * 32 * ngm) ||
                       !scratch(ctx, ctx->knn_ok, std::max<uint64_t>(nc, 1) * 32 * ngm)))) {
-        minor_rdf = minor_knn = false;
-        ngm = 0;
-        sums_bytes = 0;
+        minor_rdf = minor_knn = ngm = 0;
+        ntc = sums_bytes = 0;
       }
     }
-    if (!ngm) kq.do_rdf = kq.do_knn = 0;
-    // the fused kernel is left with the regions of interest
+    if (!ngm) kq.do_rdf = kq.do_knn = kq.nlab = 0;
+    kq.nwalk = std::min(nreal, 32 * ngm);
+    // the fused kernel is left with the other label sets and the regions of interest
     const uint8_t* RLb = RL;
     const uint8_t* OKb = OK;
     int nrb = nreal;
     if (minor_rdf) {
-      b.rbase = nlab;
-      b.nreal = nrb = n_rois;
-      RLb = RL + (uint64_t)nlab * n;
-      OKb = OK + (uint64_t)nlab * nc;
+      b.rbase = minor_rdf;
+      b.nreal = nrb = nreal - minor_rdf;
+      RLb = RL + (uint64_t)minor_rdf * n;
+      OKb = OK + (uint64_t)minor_rdf * nc;
     }
     if (pp::apply_configure(b)) return fail(ctx, PP_ERR_UNSUPPORTED, "RDF bins of one realisation exceed shared memory");
     b.ngroups = std::max(1, (nrb + b.group - 1) / b.group);
@@ -2677,7 +2728,7 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
     if (knn32) {
       const int rest = nreal % 32;
       ng32 = (nreal + 31) / 32;
-      if (rest > 0 && rest <= 8 && !minor_knn) {
+      if (rest > 0 && rest <= 8 && 32 * minor_knn < nreal) {
         bk = b;
         bk.flags = PP_MKNN;
         bk.count = 0;
@@ -2743,7 +2794,7 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
         bc.pair_base = ch.p0;
         if (cudaMemsetAsync(ctx->work.p, 0, 8, st) != cudaSuccess) return fail(ctx, PP_ERR_CUDA, "memset failed");
         if (nrb && pp::launch_apply(bc, ctx->sm_count, st)) return fail(ctx, PP_ERR_CUDA, "apply launch failed");
-        if (minor_rdf &&
+        if (ntc &&
             pp::launch_cat_hist(b.pair_cat, ch.p1 - ch.p0, P.H, kq.tcat, ctx->sm_count, st))
           return fail(ctx, PP_ERR_CUDA, "pair sum launch failed");
         if (knn_rest) {
@@ -2766,11 +2817,13 @@ int pp_run_batched(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_lis
             k.cn = std::min(chunk, ch.c1 - c0);
             k.tile = 4;  // centres per warp work item
             if (g < ngm) {
+              k.do_rdf = 32 * g < minor_rdf;
+              k.do_knn = g < minor_knn;
               if (cudaMemsetAsync(k.work, 0, 4, st) != cudaSuccess) return fail(ctx, PP_ERR_CUDA, "memset failed");
               if (pp::launch_minor_walk(k, ctx->sm_count, st)) return fail(ctx, PP_ERR_CUDA, "minor walk launch failed");
             }
             if (g >= ng32) continue;
-            if (!minor_knn) {
+            if (g >= minor_knn) {
               if (cudaMemsetAsync(k.work, 0, 4, st) != cudaSuccess) return fail(ctx, PP_ERR_CUDA, "memset failed");
               if (pp::launch_knn_walk(k, ctx->sm_count, st)) return fail(ctx, PP_ERR_CUDA, "kNN walk launch failed");
             }

@@ -326,10 +326,10 @@ struct KnnArgs {
   int cblk;                         // centre types per bin histogram (set by knn32_check)
   unsigned long long* knn_core;     // [nreal][nC][nS][nkI][H]
   // k_minor_walk: the type most ions are of, its centre and environment slot
-  // (-1: none), what the walk does, and for RDF the realisations that are whole
-  // label sets (the first nlab)
+  // (-1: none), what the walk does, and for RDF the realisations it counts (the
+  // first nlab, whole label sets); those of its groups (nwalk)
   int dom, dom_c, dom_e;
-  int do_rdf, do_knn, nlab, nE;
+  int do_rdf, do_knn, nlab, nwalk, nE;
   const uint32_t* minor;            // [ngroups][n] bit r: not dom in realisation r of the group
   const int8_t* eslot_of;
   unsigned long long* rdf_core;     // [nreal][nC][nE][H]

@@ -3851,7 +3851,8 @@ __global__ void __launch_bounds__(1024, 1) k_knn_bin(KnnArgs a) {
 //        centres of type c, for c != dom (few lanes hold such a centre: the
 //        warp adds the list for them); then with T, all pairs by category,
 //        A(dom) = T - sum A(c) and N(c, dom) = A(c) - sum N(c, t): whole
-//        numbers, exactly what counting every pair gives (k_minor_fin).
+//        numbers, exactly what counting every pair gives (k_minor_fin).  The
+//        sums are left out where dom is in no environment.
 //   kNN  the k-th member of dom's set is the k-th zero bit; the other sets
 //        count their entries as k_knn_walk does, which takes every entry.
 // 2M-ion tip, 65 label sets (f = 4% not dom), R = 1.5 nm, 36 pairs, k = 1..8:
@@ -3906,7 +3907,7 @@ struct MinorLayout {
     nset = a.do_knn ? (size_t)(a.nC + 1) * 256 : 0;
     nmiss = a.do_knn ? (size_t)a.nsmax * (a.nkI + 1) * 32 : 0;
     nN = a.do_rdf && a.dom_c >= 0 ? (size_t)RN * a.H * 32 : 0;
-    nA = a.do_rdf ? (size_t)RA * a.H * 32 : 0;
+    nA = a.do_rdf && a.dom_e >= 0 ? (size_t)RA * a.H * 32 : 0;
   }
   __host__ __device__ size_t warp_bytes(const KnnArgs& a) const {
     return 64 + (a.do_knn ? (size_t)a.nsmax * 32 : 0);
@@ -3973,6 +3974,7 @@ __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
   const uint32_t* minor = a.minor + (uint64_t)a.grp * a.n;
   const int real = a.grp * 32 + lane;
   const bool rdf_lane = RDF && real < a.nlab;
+  const bool sums = a.dom_e >= 0;  // N(c, dom) is asked for
   unsigned long long pairs = 0, centres = 0;
   const uint32_t ntiles = (a.cn + a.tile - 1) / a.tile;
   for (;;) {
@@ -3993,8 +3995,8 @@ __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
         if (c >= 0) {
           pairs += o1 - o0;
           ++centres;
-          if (c != a.dom_c) arow = c - (a.dom_c >= 0 && c > a.dom_c ? 1 : 0);
-        } else if (a.dom_c >= 0) {
+          if (sums && c != a.dom_c) arow = c - (a.dom_c >= 0 && c > a.dom_c ? 1 : 0);
+        } else if (sums && a.dom_c >= 0) {
           arow = RA;
         }
       }
@@ -4095,7 +4097,7 @@ __global__ void __launch_bounds__(1024, 1) k_minor_walk(KnnArgs a) {
                 if (e >= 0 && c == a.dom_c) {
                   atomicAdd(&sN[((uint32_t)e * H + cat) * 32 + lane], 1u);
                 } else if (e < 0) {
-                  atomicAdd(&a.so[((uint64_t)real * a.nC + c) * H + cat], 1ull);
+                  if (sums) atomicAdd(&a.so[((uint64_t)real * a.nC + c) * H + cat], 1ull);
                 } else {
                   const int es = e + (a.dom_e >= 0 && e >= a.dom_e ? 1 : 0);
                   atomicAdd(&a.rdf_core[(((uint64_t)real * a.nC + c) * a.nE + es) * H + cat], 1ull);
@@ -5004,7 +5006,7 @@ int launch_minor_walk(const KnnArgs& k, int sm_count, cudaStream_t s) {
 
 int launch_minor_fin(const KnnArgs& k, cudaStream_t s) {
   counted();
-  k_minor_fin<<<dim3(8, (unsigned)k.nreal), 256, 0, s>>>(k);
+  k_minor_fin<<<dim3(8, (unsigned)k.nwalk), 256, 0, s>>>(k);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

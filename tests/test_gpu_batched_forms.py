@@ -88,3 +88,41 @@ def test_knn_by_common_type_holds_no_rdf_sums(native_lib):
         assert used[0] - used[1] < 24 << 20
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("flags,ks", [(N.PP_RDF, []), (N.PP_MKNN, [5, 1]), (N.PP_RDF | N.PP_MKNN, [5, 1])])
+@pytest.mark.parametrize("share", [0.97, 0.85, 0.77])
+def test_groups_by_number_of_realisations(ctx, flags, ks, share):
+    """The last, partial group of 32 realisations is counted by the common type
+    only where enough of its lanes work, a share of it on either side of the
+    line; regions of interest share its groups.  Counts are those of the other
+    kernels, one realisation never pays, and a full group always does."""
+    hist = (0.0, 0.02, 0.9)
+    spec, d2, trg, env, cid = _setup(ctx, (share, 0.6 * (1 - share), 0.4 * (1 - share)), hist, n=3000)
+    rng = np.random.default_rng(3)
+    sets = np.stack([rng.permutation(spec.labels) for _ in range(65)])
+    roi = np.array([[0.1 * q, 0.0, 4.5, 2.3] for q in range(5)], dtype=np.float32)
+
+    def run(minor, nsets, rois):
+        ctx.set_option("batched_minor", minor)
+        ctx.run_batched(cid, flags, ks, include_original=False, label_sets=sets[:nsets] if nsets else None,
+                        rois=roi[:rois] if rois else None)
+        count = ctx.batched_count()
+        return (ctx.batched_graph()["nodes"], [ctx.fetch_batched(r) for r in range(count)],
+                [ctx.batched_stats(r) for r in range(count)])
+
+    try:
+        for nsets, rois in [(1, 0), (2, 0), (3, 0), (5, 0), (8, 0), (9, 2), (20, 0), (29, 5), (31, 1), (32, 0), (33, 0),
+                            (37, 0), (40, 3), (64, 0), (65, 2), (0, 5)]:
+            nodes = {}
+            nodes[0], base, stats = run(0, nsets, rois)
+            for minor in (1, 2):
+                nodes[minor], got, st = run(minor, nsets, rois)
+                assert st == stats and np.array_equal(got, base), (nsets, rois, minor)
+            if (nsets, rois) == (1, 0) or (nsets == 0 and flags == N.PP_RDF):
+                assert nodes[1] == nodes[0]
+            if nsets >= 32:
+                assert nodes[1] != nodes[0] and nodes[2] != nodes[0]
+    finally:
+        _reset(ctx)
+        ctx.free(cid)
