@@ -108,6 +108,7 @@ struct Cloud {
   // (0 = the defaults below)
   uint32_t lanes_bx = 0, lanes_by = 0, lanes_bz = 0;
   uint64_t occupied = 0;  // non-empty cells of the grid
+  uint64_t fullest = 0, fullest_cell = 0;  // most ions of one of its 4 x 4 x 4 cell tiles, of a cell
   // the cell block was set by pp_cloud_prepare rather than by tuning: passes
   // take it only where centres are dense enough to fill a warp (default_block)
   bool lanes_auto = false;
@@ -199,6 +200,7 @@ struct pp_ctx {
   DevBuf tmp_cell_of, tmp_rank, scan_tmp, bbox, centres, centre_count, work, tables_dev, sel_flags, sel_tmp;
   DevBuf tri_fill, cflag, rowtab, nc_pre, pass_code;
   DevBuf type_counts, sp_start, sp_ions, sp_slot;  // kNN passes in two walks
+  DevBuf heavy;    // chunks of the lane scans that several warps share: count, then items
   DevBuf labels_run, perm_dev, gather_src;
   DevBuf vox;      // pp_cloud_inside: sums, ions per voxel, union-find parents
   DevBuf neigh;    // pp_neighbors: count and records
@@ -476,15 +478,17 @@ int build_grid(pp_ctx* ctx, Cloud& cl, float R, cudaStream_t s) {
                      ctx->tmp_rank.as<uint32_t>(), cl.cell_start.as<uint32_t>(), cl.ions.as<float4>(),
                      cl.slot_of_id.as<uint32_t>(), cl.id_of_slot.as<uint32_t>(), cl.label_sorted.as<uint8_t>(), s);
   CK(cudaGetLastError());
-  // non-empty cells: the default cell block of the centre-per-lane scans
-  unsigned long long occ = 0;
-  CK(ctx->work.ensure(16));
-  CK(cudaMemsetAsync(ctx->work.p, 0, 8, s));
-  pp::launch_count_occupied(cl.cell_start.as<uint32_t>(), g.ncells, ctx->work.as<unsigned long long>(),
-                            ctx->sm_count, s);
-  CK(cudaMemcpyAsync(&occ, ctx->work.p, 8, cudaMemcpyDeviceToHost, s));
+  // non-empty cells and the fullest tile: the default cell block and the work
+  // items of the centre-per-lane scans
+  unsigned long long occ[3] = {0, 0, 0};
+  CK(ctx->work.ensure(32));
+  CK(cudaMemsetAsync(ctx->work.p, 0, 24, s));
+  pp::launch_count_occupied(cl.cell_start.as<uint32_t>(), g, ctx->work.as<unsigned long long>(), ctx->sm_count, s);
+  CK(cudaMemcpyAsync(occ, ctx->work.p, 24, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  cl.occupied = occ;
+  cl.occupied = occ[0];
+  cl.fullest = occ[1];
+  cl.fullest_cell = occ[2];
   cl.g = g;
   cl.grid_ok = true;
   cl.grid_version = ctx->grid_counter++;
@@ -518,16 +522,46 @@ bool default_block(const Cloud& cl, uint64_t ncent, int* bx, int* by, int* bz) {
   return true;
 }
 
+// A buffer only the faster form of a pass needs: false when the device has no
+// room for it, or past the first scratch_limit of a run (a testing hook).
+bool scratch(pp_ctx* ctx, DevBuf& b, size_t bytes) {
+  if (ctx->scratch_limit >= 0 && ctx->scratch_taken++ >= ctx->scratch_limit) return false;
+  if (b.ensure(bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
+// What a batch of centres costs the centre-per-lane scans, in ions met: those of
+// some 8 R^3 and about 500 ions' worth of rows and set-up; on average, and where
+// the cloud is fullest (less what chance makes of the fullest tile).
+struct LaneCost {
+  double mean, most;
+  LaneCost(const Cloud& cl, float R) {
+    const double tile_nm3 = std::pow(4.0 * cl.g.h, 3), tile = ion_density(cl) * tile_nm3, near = 8.0 * std::pow((double)R, 3);
+    const double full = std::max(tile, (double)cl.fullest - 4.0 * std::sqrt(tile));
+    mean = tile / tile_nm3 * near + 500.0;
+    most = std::min(full / tile_nm3 * near + 500.0, 2.0 * full + mean);
+  }
+};
+
 // Work items of the centre-per-lane scans: chunks of columns of blocks, as long
 // as leaves every warp of the device (32 an SM) 8 of them that hold ions, since
 // the last block of a chunk is cut short; but no shorter than holds 10 centres,
 // unless not every warp would have one then.  False when they cannot be counted
 // in 32 bits.
-bool lane_items(const pp_ctx* ctx, const Cloud& cl, uint64_t ncent, pp::ScanArgs& a) {
+//
+// That makes items alike where ions lie evenly.  A small ball of very many ions
+// is a few chunks of thousands of centres, each a warp's alone, and the device
+// waits for them (300k ions, 3,000 of them within 0.4 nm, R = 1 nm: RDF 3.2 ms,
+// kNN 6.7; now 0.63 and 1.0): where the fullest chunk could hold many times the
+// mean and keep a warp busy for as long as the whole pass should take, chunks of
+// more than heavy_lim centres are listed first (launch_lane_heavy) and shared by
+// kHeavyParts warps each.
+bool lane_items(pp_ctx* ctx, const Cloud& cl, uint64_t ncent, pp::ScanArgs& a, cudaStream_t s) {
   const Grid& g = cl.g;
   const uint64_t cols = (((uint64_t)g.ny + a.by - 1) / a.by) * (((uint64_t)g.nz + a.bz - 1) / a.bz);
-  const double h = g.h, density = ion_density(cl);
-  const double column = density * h * h * h * a.by * a.bz * (double)ncent / (double)cl.n;  // centres per cell of length
+  const double h = g.h, density = ion_density(cl), share = (double)ncent / (double)cl.n;
+  const double column = density * h * h * h * a.by * a.bz * share;  // centres per cell of length
   const double held = density > 0.0 ? (double)cl.n / (density * h * h * h * (double)g.ncells) : 1.0;
   auto items = [&](int ch) { return cols * (((uint64_t)g.nx + ch - 1) / ch); };
   const double warps = 32.0 * ctx->sm_count;
@@ -537,6 +571,16 @@ bool lane_items(const pp_ctx* ctx, const Cloud& cl, uint64_t ncent, pp::ScanArgs
   if (nb >= (1ull << 32)) return false;
   if (a.sample_stride > 1) nb = std::max<uint64_t>(1, nb / a.sample_stride);
   a.nbricks = (uint32_t)nb;
+  a.heavy = nullptr;
+  const double cells = (double)a.by * a.bz * a.chunk;
+  const double most = share * std::min((double)cl.fullest_cell * cells, (double)cl.fullest * std::max(1.0, cells / 64.0));
+  const LaneCost cost(cl, a.R);
+  a.heavy_lim = (uint32_t)std::max(64.0, std::min(8.0 * column * a.chunk, 1e9));
+  if (most > (double)a.heavy_lim && nb < (1ull << 31) && most * cost.most > (double)ncent * cost.mean / warps &&
+      scratch(ctx, ctx->heavy, (cl.n / a.heavy_lim + 2) * 4)) {  // more than heavy_lim centres each
+    a.heavy = ctx->heavy.as<uint32_t>();
+    if (pp::launch_lane_heavy(a, ctx->heavy.as<uint32_t>(), s)) a.heavy = nullptr;
+  }
   return true;
 }
 
@@ -1490,15 +1534,6 @@ bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long l
   return true;
 }
 
-// A buffer only the faster form of a pass needs: false when the device has no
-// room for it, or past the first scratch_limit of a run (a testing hook).
-bool scratch(pp_ctx* ctx, DevBuf& b, size_t bytes) {
-  if (ctx->scratch_limit >= 0 && ctx->scratch_taken++ >= ctx->scratch_limit) return false;
-  if (b.ensure(bytes) == cudaSuccess) return true;
-  cudaGetLastError();
-  return false;
-}
-
 // The kNN part of a pass in two walks (k_lanes_near) where near_plan finds it
 // worth it, else -3.  count: the pass has no other part that counts its in-ball
 // pairs, so they are counted by a symmetric walk of their own first; the
@@ -1633,12 +1668,18 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
   // stream, takes 2291 us against 1884 on a 1M-ion tip at R = 1 nm (56 ions a
   // ball, k <= 10), 5530 against 1578 at R = 2 nm, and 481 against 303 at 20k
   // ions.  It keeps the passes whose kNN no lane scan takes (overlapping sets,
-  // more than 8 centre types) and those of too few centres to give the lanes of
+  // more than 8 centre types), those of too few centres to give the lanes of
   // two passes work (2191 against 2698 us at 3.3k centres of 1000 neighbours),
-  // unless the cloud is tuned to a block.
+  // and small ones of clouds with places so full that a batch there lasts as
+  // long as the rest of the pass (100k ions, a fifth of them in 30 balls of 0.8
+  // nm, R = 1 nm: 505 against 865 us; at R = 2 nm, 400 ions a ball, 1200 against
+  // 1050), unless the cloud is tuned to a block.
+  const LaneCost cost(*cl, R);
+  const double batches = (double)ncent * std::max<uint32_t>(stride, 1) / (28.0 * 32.0 * ctx->sm_count);  // a warp
+  const bool even = batches > 3.0 || cost.mean > 1000.0 || cost.most <= cost.mean * (1.0 + 0.5 * batches);
   const bool split = both && lanes &&
                      (block_ok || (P.disjoint && P.nC <= 8 && P.emax <= 15 && P.kmax <= 64 &&
-                                   (uint64_t)ncent * std::max<uint32_t>(stride, 1) >= 4096));
+                                   (uint64_t)ncent * std::max<uint32_t>(stride, 1) >= 4096 && even));
   if (both && !split) lanes = false;
   // RDF / RIPK alone: each pair of two centres is computed once and credited
   // to both (the counts are the same as the per-centre ball scan's)
@@ -1694,7 +1735,7 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
     // RDF / RIPK and kNN: the second pass on fresh work counters and with its
     // pair and centre counts dropped (the first counted them)
     if (rc == -3 && a.brows && split) {
-      if (lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a)) {
+      if (lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a, s)) {
         pp::ScanArgs ar = a;
         rc = pp::launch_lanes(ar, 0, ctx->sm_count, &smem, s);
         if (rc == 0) {
@@ -1715,11 +1756,11 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
       }
     }
     if (P.kr > 0) a.sym = 0;  // the per-centre scans need every centre's whole ball
-    if (rc == -3 && a.brows && P.kr == 0 && (a.flags & PP_RDF) && lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a)) {
+    if (rc == -3 && a.brows && P.kr == 0 && (a.flags & PP_RDF) && lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a, s)) {
       rc = pp::launch_lanes(a, P.kr, ctx->sm_count, &smem, s);
       if (rc == 0) ctx->last_kind = 2;
     }
-    if (rc == -3 && a.brows && P.kr > 0 && !(a.flags & PP_RDF) && lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a)) {
+    if (rc == -3 && a.brows && P.kr > 0 && !(a.flags & PP_RDF) && lane_items(ctx, *cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), a, s)) {
       rc = near_ok ? run_near(ctx, *cl, P, type_counts.data(), R, a, true, &smem, s) : -3;
       if (rc == -3) rc = pp::launch_lanes_knn(a, P.disjoint != 0, ctx->sm_count, &smem, s);
       if (rc == 0) ctx->last_kind = 3;

@@ -60,6 +60,8 @@ struct ScanArgs {
   int by, bz;
   uint32_t nbricks;
   int chunk;
+  const uint32_t* heavy;         // chunks of more than heavy_lim centres: their number, then which (null: none)
+  uint32_t heavy_lim;
   // centre-per-lane scans: per-slot pass codes (written by the pass, n words),
   // the labels they are made from, and 1.f (see dist2_x2)
   uint32_t* pcode;
@@ -277,9 +279,12 @@ int launch_scan(const ScanArgs& a, int kr, int emax, int sm_count, size_t* smem_
 int launch_brick(const ScanArgs& a, int kr, int sm_count, size_t* smem_used, cudaStream_t s);
 // centre-per-lane brick scan of RDF / RIPK passes (k_lanes); -3 = not applicable
 int launch_lanes(const ScanArgs& a, int kr, int sm_count, size_t* smem_used, cudaStream_t s);
-// *out += the number of non-empty cells (cell_start has ncells + 1 entries)
-void launch_count_occupied(const uint32_t* cell_start, uint64_t ncells, unsigned long long* out, int sm_count,
-                           cudaStream_t s);
+// out[0] += the number of non-empty cells; out[1], out[2] at least the ions of
+// any 4 x 4 x 4 cells at a multiple of 4 and of any cell (cell_start has ncells
+// + 1 entries)
+void launch_count_occupied(const uint32_t* cell_start, Grid g, unsigned long long* out, int sm_count, cudaStream_t s);
+// lists the chunks of more than a.heavy_lim centres: out[0] = their number
+int launch_lane_heavy(const ScanArgs& a, uint32_t* out, cudaStream_t s);
 // centre-per-lane block scan of kNN-only passes (k_lanes_knn); disjoint_sets:
 // every type in at most one environment set of each centre type
 // (ScanArgs::setidx valid); -3 = not applicable

@@ -2118,7 +2118,8 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
 // fourth word; in symmetric mode its lowest bit says that it is a centre and
 // is staged as 0.
 // Warps fetch chunks of `chunk` cells of a column of blocks from the global
-// work counter, without block barriers.  lanes_blocks calls, warp-uniformly,
+// work counter, without block barriers (ScanArgs::heavy: very full ones first,
+// shared by several warps).  lanes_blocks calls, warp-uniformly,
 //   start(self)                a new batch; self = this lane's centre slot or
 //                              0xffffffff; returns the lane's centre position
 //                              (at infinity for no centre)
@@ -2329,27 +2330,73 @@ __device__ __forceinline__ uint32_t stage_rows(const ScanArgs& a, const LaneBatc
   return staged;
 }
 
+// Chunk w of the columns of blocks: cells [x0, x1) of the rows of its blocks;
+// number of its centres in rows r, r + step, ...
+struct LaneChunk {
+  int x0, x1, yb, ye, zb, ze;
+  __device__ __forceinline__ LaneChunk(const ScanArgs& a, uint32_t w) {
+    const Grid& g = a.g;
+    const int BY = max(a.by, 1), BZ = max(a.bz, 1), CH = a.chunk;
+    const uint32_t nch = (uint32_t)((g.nx + CH - 1) / CH), nby = (uint32_t)((g.ny + BY - 1) / BY);
+    if (a.sample_stride > 1) w *= a.sample_stride;
+    const uint32_t col = w / nch, bz_i = col / nby;
+    yb = (int)(col - bz_i * nby) * BY;
+    zb = (int)bz_i * BZ;
+    ye = min(yb + BY, g.ny);
+    ze = min(zb + BZ, g.nz);
+    x0 = (int)(w - col * nch) * CH;
+    x1 = min(x0 + CH, g.nx);
+  }
+  __device__ __forceinline__ uint32_t centres(const ScanArgs& a, int r, int step) const {
+    uint32_t n = 0;
+    for (; r < (ye - yb) * (ze - zb); r += step) {
+      const uint32_t row = ((uint32_t)(zb + r / (ye - yb)) * (uint32_t)a.g.ny + (uint32_t)(yb + r % (ye - yb))) * (uint32_t)a.g.nx;
+      n += (a.cell_start[row + x1] - a.cell_start[row + x0]) - (a.nc_pre[row + x1] - a.nc_pre[row + x0]);
+    }
+    return n;
+  }
+};
+
+// Chunks of very many centres are shared: their batches go round kHeavyParts
+// warps, which take them from a list before all other chunks.
+constexpr uint32_t kHeavyParts = 32;
+__global__ void k_lane_heavy(ScanArgs a, uint32_t* out) {
+  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < a.nbricks; w += (uint64_t)gridDim.x * blockDim.x)
+    if (LaneChunk(a, (uint32_t)w).centres(a, 0, 1) > a.heavy_lim) out[1 + atomicAdd(out, 1u)] = (uint32_t)w;
+}
+
 template <class Start, class Body>
 __device__ __forceinline__ void lanes_blocks(const ScanArgs& a, float4* sbox, uint32_t* queue, Start start, Body body) {
   const Grid& g = a.g;
   const int lane = threadIdx.x & 31;
   const uint32_t ltmask = (1u << lane) - 1u;
-  const int BY = max(a.by, 1), BZ = max(a.bz, 1), CH = a.chunk;
-  const uint32_t nch = (uint32_t)((g.nx + CH - 1) / CH), nby = (uint32_t)((g.ny + BY - 1) / BY);
   for (;;) {
     uint32_t w = 0;
     if (lane == 0) w = atomicAdd(a.work, 1u);
     w = __shfl_sync(FULL, w, 0);
+    uint32_t turn = 0, every = 0;  // batches until this warp's next one, and between them
+    bool light = false;            // heavy chunks are not this warp's alone
+    if (a.heavy) {
+      const uint32_t shared = a.heavy[0] * kHeavyParts;
+      light = w >= shared;
+      if (light) {
+        w -= shared;
+      } else {
+        turn = w % kHeavyParts;
+        every = kHeavyParts - 1u;
+        w = a.heavy[1 + w / kHeavyParts];
+      }
+    }
     if (w >= a.nbricks) break;
-    if (a.sample_stride > 1) w *= a.sample_stride;
-    const uint32_t col = w / nch, bz_i = col / nby;
+    const LaneChunk K(a, w);
+    if (light && __reduce_add_sync(FULL, K.centres(a, lane, 32)) > a.heavy_lim) continue;
     LaneBatch B;
-    B.yb = (int)(col - bz_i * nby) * BY;
-    B.zb = (int)bz_i * BZ;
-    B.ye = min(B.yb + BY, g.ny);
-    B.ze = min(B.zb + BZ, g.nz);
-    const int X1 = min((int)(w - col * nch) * CH + CH, g.nx);
-    for (B.xb = (int)(w - col * nch) * CH; B.xb < X1; B.xb = B.xe) {
+    B.yb = K.yb;
+    B.zb = K.zb;
+    B.ye = K.ye;
+    B.ze = K.ze;
+    const int X1 = K.x1;
+    for (B.xb = K.x0; B.xb < X1; B.xb = B.xe) {
       // the block's length: as many columns, up to 32, as hold at most 32
       // centres; cum = centres of the columns up to this lane's
       const int x = min(B.xb + lane, X1 - 1);
@@ -2401,6 +2448,11 @@ __device__ __forceinline__ void lanes_blocks(const ScanArgs& a, float4* sbox, ui
         have -= take;
         head += take;
         __syncwarp();
+        if (turn > 0u) {  // another warp's batch
+          --turn;
+          continue;
+        }
+        turn = every;
         const float4 cp = start(self);
         const bool lv = cp.x != kInf();
         B.live = __ballot_sync(FULL, lv);
@@ -4465,19 +4517,45 @@ void launch_surface_cells(const float4* ions, const uint32_t* cell_start, Grid g
       ions, cell_start, g, f, tri_box, tri, tcs, tct, tg, rprime, slack, split, surf);
 }
 
-// number of cells holding at least one ion
-__global__ void k_count_occupied(const uint32_t* __restrict__ cell_start, uint64_t ncells, unsigned long long* out) {
-  unsigned long long c = 0;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < ncells; i += (uint64_t)gridDim.x * blockDim.x)
-    c += cell_start[i + 1] > cell_start[i] ? 1ull : 0ull;
-  for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(FULL, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
+// number of cells holding at least one ion; the fullest 4 x 4 x 4 cells; the
+// fullest cell
+__global__ void k_count_occupied(const uint32_t* __restrict__ cell_start, Grid g, unsigned long long* out) {
+  unsigned long long c = 0, m = 0;
+  uint32_t cell = 0;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < g.ncells; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t k = cell_start[i + 1] - cell_start[i];
+    c += k > 0u ? 1ull : 0ull;
+    cell = max(cell, k);
+  }
+  const uint32_t tx = (uint32_t)(g.nx + 3) / 4, ty = (uint32_t)(g.ny + 3) / 4, tz = (uint32_t)(g.nz + 3) / 4;
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < (uint64_t)tx * ty * tz;
+       t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t r = t / tx;
+    const int x0 = (int)(t - r * tx) * 4, x1 = min(x0 + 4, g.nx), y0 = (int)(r % ty) * 4, z0 = (int)(r / ty) * 4;
+    unsigned long long k = 0;
+    for (int z = z0; z < min(z0 + 4, g.nz); ++z)
+      for (int y = y0; y < min(y0 + 4, g.ny); ++y) {
+        const uint64_t row = ((uint64_t)z * g.ny + y) * g.nx;
+        k += cell_start[row + x1] - cell_start[row + x0];
+      }
+    m = k > m ? k : m;
+  }
+  cell = __reduce_max_sync(FULL, cell);
+  for (int o = 16; o; o >>= 1) {
+    c += __shfl_xor_sync(FULL, c, o);
+    const unsigned long long k = __shfl_xor_sync(FULL, m, o);
+    m = k > m ? k : m;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (c) atomicAdd(&out[0], c);
+    if (m) atomicMax(&out[1], m);
+    if (cell) atomicMax(&out[2], (unsigned long long)cell);
+  }
 }
 
-void launch_count_occupied(const uint32_t* cell_start, uint64_t ncells, unsigned long long* out, int sm_count,
-                           cudaStream_t s) {
+void launch_count_occupied(const uint32_t* cell_start, Grid g, unsigned long long* out, int sm_count, cudaStream_t s) {
   counted();
-  k_count_occupied<<<sm_count * 4, 256, 0, s>>>(cell_start, ncells, out);
+  k_count_occupied<<<sm_count * 4, 256, 0, s>>>(cell_start, g, out);
 }
 
 void launch_nc_prefix(const uint32_t* cell_start, uint64_t ncells, const uint8_t* cflag, uint32_t* out,
@@ -4771,6 +4849,13 @@ int launch_lanes_count(const ScanArgs& a, int sm_count, cudaStream_t s) {
   launch_pass_codes(a, PC_COUNT, 0, sm_count, s);
   counted();
   kern<<<sm_count, kLanesWarps * 32, smem, s>>>(a);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_lane_heavy(const ScanArgs& a, uint32_t* out, cudaStream_t s) {
+  if (cudaMemsetAsync(out, 0, 4, s) != cudaSuccess) return -1;
+  counted();
+  k_lane_heavy<<<grid_for(a.nbricks, 256), 256, 0, s>>>(a, out);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -121,3 +121,50 @@ def test_two_walks_when_asked_for(ctx, oracle, flags, fractions, ks):
     assert tests[1] != tests[2]
     ref = oracle.spatstat(spec.xyz, spec.labels, d2, *hist, flags, trg, env, ks)
     assert np.array_equal(bins[1], ref["bins"]) and np.array_equal(bins[2], ref["bins"])
+
+
+@pytest.mark.parametrize("flags,ks", [(N.PP_RDF, []), (N.PP_MKNN, [10, 1]), (N.PP_RDF | N.PP_MKNN, [20, 2])])
+@pytest.mark.parametrize("symmetric,walks", [(1, 2), (0, 1)])
+@pytest.mark.parametrize("sigma", [0.05, 0.3, 0.8])
+def test_chunks_shared_by_warps(ctx, oracle, flags, ks, symmetric, walks, sigma):
+    """A ball of very many ions in a thin cloud, down to one cell of them: its
+    chunks are listed and shared, and every batch is taken once."""
+    rng = np.random.default_rng(8)
+    xyz = rng.uniform(0, 14, (20000, 3))
+    xyz[:4000] = [7.1, 6.9, 7.0] + sigma * rng.normal(size=(4000, 3))
+    xyz = rng.permutation(xyz).astype(np.float32)
+    n = len(xyz)
+    labels = rng.choice(np.array([1, 2, 3], dtype=np.uint8), n, p=[0.9, 0.07, 0.03])
+    d2 = np.where(np.arange(n) % 13 == 0, 0.1, 50.0).astype(np.float32)
+    trg, env = _pairs((1, 2, 3))
+    hist = (0.0, 0.01, 1.0)
+    cid = ctx.upload(xyz, labels)
+    ctx.surfdist(cid, d2)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.set_option("symmetric", symmetric)
+    ctx.set_option("knn_walks", walks)
+    try:
+        if flags == N.PP_RDF | N.PP_MKNN:  # a place so full keeps an untuned pass of both on the per-centre scan
+            ctx.run(cid, flags, ks)
+            assert ctx.last_kernel() == "k_scan"
+            ctx.tuning(cid, 4.0, ((2 | 2 << 8 | 2 << 12) << 16) | N.PP_TILE_LANES)
+        launches, got = {}, {}
+        without = 1 if symmetric and flags == N.PP_RDF else 2  # the buffers asked for before the list
+        for limit in (without, -1):
+            ctx.set_option("scratch", limit)
+            ctx.run(cid, flags, ks)
+            before = N.kernel_launches()
+            ctx.run(cid, flags, ks)
+            got[limit], launches[limit] = (ctx.fetch(), ctx.stats(), ctx.run_tests()), N.kernel_launches() - before
+            assert ctx.last_kernel() != "k_scan"
+    finally:
+        for name, value in (("symmetric", 1), ("knn_walks", 0), ("scratch", -1)):
+            ctx.set_option(name, value)
+        ctx.free(cid)
+    if flags == N.PP_RDF and sigma < 0.1:
+        assert launches[-1] == launches[without] + 1
+        assert got[without][2] == got[-1][2]  # the same tests
+    ref = oracle.spatstat(xyz, labels, d2, *hist, flags, trg, env, ks)
+    for bins, st, _ in got.values():
+        assert np.array_equal(bins, ref["bins"]) and st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
