@@ -1661,6 +1661,7 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
   const bool both = P.kr > 0 && (a.flags & PP_RDF);
   int dbx = 0, dby = 0, dbz = 0;
   const bool dense = default_block(*cl, (uint64_t)ncent * std::max<uint32_t>(stride, 1), &dbx, &dby, &dbz);
+  a.sparse_centres = dense ? 0 : 1;
   const bool block_ok = cl->lanes_bx != 0 && (!cl->lanes_auto || dense);
   bool lanes = rows_fit && !ctx->no_lanes && !(flags & (PP_CNTNB | PP_NPCORR)) && (block_ok || dense);
   // RDF / RIPK and kNN in one pass run as two centre-per-lane passes, RDF /

@@ -38,6 +38,7 @@ struct ScanArgs {
   const uint8_t* labels;       // type per sorted slot (plain or permuted)
   const uint32_t* centres;     // sorted slots of the centres
   uint32_t ncentres;
+  int sparse_centres;          // fewer than 0.35 per non-empty cell (see k_scan)
   // geometry of the query
   float R, R2;                 // SpatStatRadiusMax and float(R*R)
   float Rm2;                   // (R + margin)^2 for conservative row trimming

@@ -1006,7 +1006,7 @@ __device__ __forceinline__ void for_each_candidate_r(const ScanArgs& a, const in
     const uint32_t ne = __ballot_sync(FULL, len > 0);
     const int cnt = __popc(ne);
     if (cnt == 0) continue;
-    const int src = (lane < cnt) ? (int)__fns(ne, 0, lane + 1) : 0;
+    const int src = (lane < cnt) ? (int)nth_set(ne, (uint32_t)lane) : 0;
     const uint32_t rst = __shfl_sync(FULL, st, src);
     uint32_t rlen = __shfl_sync(FULL, len, src);
     if (lane >= cnt) rlen = 0;
@@ -1054,10 +1054,16 @@ __device__ __forceinline__ void for_each_candidate(const ScanArgs& a, const int8
 }
 
 // LISTS: mode 2 (an instance of its own, which needs more registers).
-// Blocks an SM: one list in shared memory or none is faster with five than with
-// the registers of four (1M-ion cylinder, k = 10: 440 against 493 us).
-template <int KR, int EMAX, bool LISTS = false>
-__global__ void __launch_bounds__(256, LISTS ? 0 : KR == 0 || (KR == 1 && EMAX <= 1) ? 5 : EMAX == 0 || (KR == 1 && EMAX == 8) ? 3 : 0)
+// MINB: least blocks an SM.  One kNN list in shared memory or in registers takes
+// 62 registers left alone and spills with the 48 of five blocks: passes of dense
+// centres, whose neighbours find their ions in L1, are the faster without
+// spills (1M ions, every one a centre, counts and k = 4, R = 1.5 nm: 3.65 against
+// 3.83 ms; overlapping sets 3.76 against 4.60), those of sparse centres, which wait
+// for memory, with five blocks (1M-ion cylinder, 6% of them, k = 10: 440 against
+// 493 us).  Without lists 55 registers are the faster for both (2.00 against 2.16
+// ms and 62 against 64 us).
+template <int KR, int EMAX, bool LISTS = false, int MINB = 0>
+__global__ void __launch_bounds__(256, MINB)
 k_scan(ScanArgs a) {
   // shared kNN list stride: one padding word keeps set p's k-th entry in bank
   // (p + k) % 32, so lanes testing different sets do not collide
@@ -4649,9 +4655,9 @@ void launch_select_centres(const uint8_t* labels, const float* surf, uint64_t n,
   k_select_write<<<grid_for(n, 256), 256, 0, s>>>(labels, surf, n, R2, cslot_of, extra, flags, out, count);
 }
 
-template <int KR, int EMAX, bool LISTS = false>
+template <int KR, int EMAX, bool LISTS = false, int MINB = 0>
 static int launch_scan_t(const ScanArgs& a, int sm_count, size_t smem, cudaStream_t s) {
-  auto kern = k_scan<KR, EMAX, LISTS>;
+  auto kern = k_scan<KR, EMAX, LISTS, MINB>;
   if (smem > 48 * 1024) {
     if (!allow_dynamic_smem((const void*)kern, smem)) return -1;
   }
@@ -4681,11 +4687,13 @@ int launch_scan(const ScanArgs& a, int kr, int emax, int sm_count, size_t* smem_
   if (a.mode == 2) return kr == 0 ? launch_scan_t<0, 1, true>(b, sm_count, smem, s) : -2;
   if (kr == 0) return launch_scan_t<0, 1>(a, sm_count, smem, s);
   if (a.disjoint) {
-    if (kr == 1) return launch_scan_t<1, 0>(a, sm_count, smem, s);
+    if (kr == 1)
+      return a.sparse_centres ? launch_scan_t<1, 0, false, 5>(a, sm_count, smem, s) : launch_scan_t<1, 0>(a, sm_count, smem, s);
     if (kr <= 4) return launch_scan_t<4, 0>(a, sm_count, smem, s);
   }
   if (kr == 1) {
-    if (emax <= 1) return launch_scan_t<1, 1>(a, sm_count, smem, s);
+    if (emax <= 1)
+      return a.sparse_centres ? launch_scan_t<1, 1, false, 5>(a, sm_count, smem, s) : launch_scan_t<1, 1>(a, sm_count, smem, s);
     if (emax <= 8) return launch_scan_t<1, 8>(a, sm_count, smem, s);
     return launch_scan_t<1, 32>(a, sm_count, smem, s);
   }

@@ -168,3 +168,28 @@ def test_chunks_shared_by_warps(ctx, oracle, flags, ks, symmetric, walks, sigma)
     ref = oracle.spatstat(xyz, labels, d2, *hist, flags, trg, env, ks)
     for bins, st, _ in got.values():
         assert np.array_equal(bins, ref["bins"]) and st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
+
+
+@pytest.mark.parametrize("targets", [[[1], [2], [1, 3]], [[2], [3], [2, 3]], [[3]]])
+@pytest.mark.parametrize("env", [[[1], [2, 3], [1]], [[1, 2, 3], [1, 2], [3]]])
+def test_scan_of_dense_and_sparse_centres(ctx, oracle, targets, env):
+    """The per-centre scan with counts, RDF and kNN at once, one list or several,
+    for centres in most cells and in few."""
+    env = env[: len(targets)]
+    spec = synth.cylinder_specimen(n=16000, radius=3.0, height=12.0, fractions=(0.9, 0.07, 0.03), seed=23, nseg=48,
+                                   stack=4.0)
+    d2 = np.where(np.arange(len(spec.xyz)) % 7 == 0, 0.5, 10.0).astype(np.float32)
+    hist, ks, flags = (0.0, 0.02, 1.0), [31, 4, 1], N.PP_RDF | N.PP_MKNN | N.PP_CNTNB
+    cid = ctx.upload(spec.xyz, spec.labels)
+    ctx.surfdist(cid, d2)
+    ctx.tasks(targets, env)
+    ctx.hist(*hist)
+    try:
+        ctx.run(cid, flags, ks)
+        bins, counts, st = ctx.fetch(), ctx.fetch_cntnb(), ctx.stats()
+        assert ctx.last_kernel() == "k_scan"
+    finally:
+        ctx.free(cid)
+    ref = oracle.spatstat(spec.xyz, spec.labels, d2, *hist, flags, targets, env, ks)
+    assert np.array_equal(bins, ref["bins"]) and st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
+    assert np.array_equal(counts, ref["cntnb"][:, : counts.shape[1]]) and ref["cntnb"][:, counts.shape[1]:].sum() == 0
