@@ -200,6 +200,7 @@ struct pp_ctx {
   DevBuf tmp_cell_of, tmp_rank, scan_tmp, bbox, centres, centre_count, work, tables_dev, sel_flags, sel_tmp;
   DevBuf tri_fill, cflag, rowtab, nc_pre, pass_code;
   DevBuf type_counts, sp_start, sp_ions, sp_slot;  // kNN passes in two walks
+  DevBuf row_map;  // rows of the RDF cores in shared memory (hold_rows)
   DevBuf heavy;    // chunks of the lane scans that several warps share: count, then items
   DevBuf labels_run, perm_dev, gather_src;
   DevBuf vox;      // pp_cloud_inside: sums, ions per voxel, union-find parents
@@ -1534,6 +1535,25 @@ bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long l
   return true;
 }
 
+// Rows of the RDF cores that k_lanes keeps in shared memory where it has room for
+// `rows` of them: those of the most pairs by the ions of each type.
+int hold_rows(pp_ctx* ctx, const RunPlan& P, const unsigned long long* type_counts, int rows, pp::ScanArgs& a,
+              cudaStream_t s) {
+  std::vector<std::pair<double, int>> order((size_t)P.nC * P.nE);
+  for (int c = 0; c < P.nC; ++c)
+    for (int e = 0; e < P.nE; ++e)
+      order[(size_t)c * P.nE + e] = {-(double)type_counts[P.ctype[c]] * (double)type_counts[P.etype[e]], c * P.nE + e};
+  std::sort(order.begin(), order.end());
+  std::vector<int16_t> map(order.size(), -1);
+  rows = std::min(rows, (int)order.size());
+  for (int r = 0; r < rows; ++r) map[order[r].second] = (int16_t)r;
+  if (!scratch(ctx, ctx->row_map, map.size() * 2)) return PP_OK;
+  CK(cudaMemcpyAsync(ctx->row_map.p, map.data(), map.size() * 2, cudaMemcpyHostToDevice, s));
+  a.row_of = ctx->row_map.as<int16_t>();
+  a.rows_held = rows;
+  return PP_OK;
+}
+
 // The kNN part of a pass in two walks (k_lanes_near) where near_plan finds it
 // worth it, else -3.  count: the pass has no other part that counts its in-ball
 // pairs, so they are counted by a symmetric walk of their own first; the
@@ -1702,11 +1722,13 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
     if (lanes && !(a.sym && P.kr == 0) && !scratch(ctx, ctx->nc_pre, (g.ncells + 1) * 4)) lanes = false;
     if (lanes && !scratch(ctx, ctx->pass_code, std::max<uint64_t>(n, 1) * 4)) lanes = false;
     if (!lanes && P.kr > 0) a.sym = 0;
-    // kNN in two walks: needs the ions of each type of this run's labels
+    // kNN in two walks and RDF bins that do not fit need the ions of each type
+    // of this run's labels
     const bool near_ok = lanes && P.kr == 1 && P.kmax <= 20 && P.disjoint &&
                          near_pays(ctx, *cl, R, P.kmax, (uint64_t)ncent * std::max<uint32_t>(stride, 1), !both);
-    std::vector<unsigned long long> type_counts(near_ok ? 256 : 0);
-    if (near_ok) {
+    const int rows = lanes && (a.flags & PP_RDF) ? pp::lanes_rows(a) : 0;
+    std::vector<unsigned long long> type_counts(near_ok || rows > 0 ? 256 : 0);
+    if (!type_counts.empty()) {
       CK(ctx->type_counts.ensure(256 * 8));
       CK(cudaMemsetAsync(ctx->type_counts.p, 0, 256 * 8, s));
       pp::launch_type_count(labels ? labels : cl->label_sorted.as<uint8_t>(), n, ctx->type_counts.as<unsigned long long>(),
@@ -1714,6 +1736,7 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
       CK(cudaMemcpyAsync(type_counts.data(), ctx->type_counts.p, 256 * 8, cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
     }
+    if (rows > 0 && (rc = hold_rows(ctx, P, type_counts.data(), rows, a, s)) != PP_OK) return rc;
     if (lanes || a.sym) {  // prefix of the non-centre ions per cell
       CK(ctx->nc_pre.ensure((g.ncells + 1) * 4));
       const uint64_t tmp_elems = (g.ncells + 1) / 2048 + 64;

@@ -69,6 +69,10 @@ struct ScanArgs {
   const uint8_t* label_sorted;
   uint64_t n;
   float one;
+  // k_lanes whose bins do not fit: the rows of the cores (centre slot, environment
+  // slot) kept in shared memory
+  const int16_t* row_of;         // [nC * nE] which one, -1 = none
+  int rows_held;
   // kNN passes in two walks (k_lanes_near): the dense sets, each with the
   // radius its k-th neighbours are looked for in first and the stencil rows
   // within it; near_map[set] = row of a sparse set's list, or ~(index) of a
@@ -280,6 +284,8 @@ int launch_scan(const ScanArgs& a, int kr, int emax, int sm_count, size_t* smem_
 int launch_brick(const ScanArgs& a, int kr, int sm_count, size_t* smem_used, cudaStream_t s);
 // centre-per-lane brick scan of RDF / RIPK passes (k_lanes); -3 = not applicable
 int launch_lanes(const ScanArgs& a, int kr, int sm_count, size_t* smem_used, cudaStream_t s);
+// rows of the cores it can keep in shared memory where not all bins fit, else 0
+int lanes_rows(const ScanArgs& a);
 // out[0] += the number of non-empty cells; out[1], out[2] at least the ions of
 // any 4 x 4 x 4 cells at a multiple of 4 and of any cell (cell_start has ncells
 // + 1 entries)

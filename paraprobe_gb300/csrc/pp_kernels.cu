@@ -2533,8 +2533,11 @@ struct FastCat {
 // ions without one.  A pair is one atomic, whatever it is credited to; the
 // credits and the pair count are worked out once per bin when the bins are
 // added to the global cores.  BINS = 1: shared bins in the layout of the
-// cores, up to two atomics a pair (where the kinds do not fit); BINS = 0:
-// atomics on the cores; BINS = 3: no bins, the pass counts the in-ball pairs
+// cores, up to two atomics a pair (where the kinds do not fit); BINS = 0: as
+// many rows of the cores as fit in shared memory, those of the commonest types
+// (ScanArgs::row_of), and atomics on the cores for the others: a common pair's
+// atomics on few global words take longer than everything else (1M ions, R = 2
+// nm, 36 pairs of 2,000 bins: 20.0 ms with no row held, 2.1 with 20); BINS = 3: no bins, the pass counts the in-ball pairs
 // of a kNN pass whose own walk does not meet them all (k_lanes_near).
 // Pass code of an ion: BINS 2 the byte offset of its row, others (env slot +
 // 1) << 1 | (centre slot + 1) << 9; the lowest bit set for centres in
@@ -2550,7 +2553,8 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
   const int H = a.H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t RW = (SYM ? (uint32_t)a.nC : 0u) + (uint32_t)a.nE + 1u;  // BINS 2: rows per centre slot
-  const uint32_t nbin = BINS == 2 ? (uint32_t)a.nC * RW * (uint32_t)H : BINS == 1 ? (uint32_t)a.nC * a.nE * H : 0u;
+  const uint32_t nbin = BINS == 2 ? (uint32_t)a.nC * RW * (uint32_t)H
+                                  : BINS == 1 ? (uint32_t)a.nC * a.nE * H : BINS == 0 ? (uint32_t)a.rows_held * H : 0u;
   unsigned char* sp = smem;
   unsigned long long* since_flush = (unsigned long long*)sp; sp += 16;
   float4* candA = (float4*)sp; sp += NW * kStageAll * 16;
@@ -2563,7 +2567,9 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
   int8_t* scs = (int8_t*)sp; sp += 256;
   int8_t* ses = (int8_t*)sp; sp += 256;
   int8_t* sce = (int8_t*)sp; sp += 256;  // environment slot of a centre slot's type
-  uint16_t* slut = (uint16_t*)sp;        // not FAST
+  uint16_t* slut = (uint16_t*)sp; sp += FAST ? 0 : ((a.lut_n + 7) & ~7) * 2;
+  int16_t* sheld = (int16_t*)sp;         // BINS 0, any row held: [nC * nE] shared row of a core row (-1: none) ...
+  int16_t* sback = sheld + a.nC * a.nE;  // ... and [rows_held] the other way
   for (int i = threadIdx.x; i <= H; i += blockDim.x) sT[i] = i < H ? a.cat_T[i] : kInf();
   if (!FAST)
     for (int i = threadIdx.x; i < a.lut_n; i += blockDim.x) slut[i] = a.cat_lut[i];
@@ -2573,8 +2579,14 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
     ses[i] = e;
     if (c >= 0) sce[c] = e;  // slots and types are one to one
   }
-  if constexpr (BINS == 1 || BINS == 2)
+  if constexpr (BINS != 3)
     for (uint32_t i = threadIdx.x; i < nbin; i += blockDim.x) srdf[i] = 0;
+  if (BINS == 0 && a.rows_held > 0)
+    for (int i = threadIdx.x; i < a.nC * a.nE; i += blockDim.x) {
+      const int16_t r = a.row_of[i];
+      sheld[i] = r;
+      if (r >= 0) sback[r] = (int16_t)i;
+    }
   if (threadIdx.x == 0) *since_flush = 0ull;
   __syncthreads();
 
@@ -2600,6 +2612,9 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
         const uint32_t e = row - (SYM ? (uint32_t)a.nC : 0u);
         if (e < (uint32_t)a.nE) atomicAdd(&a.rdf_core[((uint64_t)c * a.nE + e) * H + b], (unsigned long long)v);
       }
+    } else if constexpr (BINS == 0) {
+      const uint32_t r = i / (uint32_t)H;
+      atomicAdd(&a.rdf_core[(uint32_t)sback[r] * (uint32_t)H + (i - r * (uint32_t)H)], (unsigned long long)v);
     } else {
       atomicAdd(&a.rdf_core[i], (unsigned long long)v);
     }
@@ -2734,16 +2749,21 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
           cat += sT[cat + 1] <= d[u] ? 1u : 0u;
           const uint32_t cj = __float_as_uint(u ? c1.w : c1.z);
           const int esj = (int)((cj >> 1) & 255u) - 1, csj = (int)((cj >> 9) & 255u) - 1;
-          auto add = [&](uint32_t i) {
-            if constexpr (BINS == 1) atomicAdd(&srdf[i], 1u);
-            else atomicAdd(&a.rdf_core[i], 1ull);
+          auto add = [&](uint32_t row) {
+            if constexpr (BINS == 1) {
+              atomicAdd(&srdf[row * (uint32_t)H + cat], 1u);
+            } else {
+              const int held = a.rows_held > 0 ? (int)sheld[row] : -1;
+              if (held >= 0) atomicAdd(&srdf[(uint32_t)held * (uint32_t)H + cat], 1u);
+              else atomicAdd(&a.rdf_core[row * (uint32_t)H + cat], 1ull);
+            }
           };
           ++inb;
-          if (esj >= 0) add(((uint32_t)cs * a.nE + (uint32_t)esj) * (uint32_t)H + cat);
+          if (esj >= 0) add((uint32_t)cs * a.nE + (uint32_t)esj);
           if (SYM && csj >= 0) {
             // the same pair seen from the staged ion, a centre too
             ++inb;
-            if (esc >= 0) add(((uint32_t)csj * a.nE + (uint32_t)esc) * (uint32_t)H + cat);
+            if (esc >= 0) add((uint32_t)csj * a.nE + (uint32_t)esc);
           }
         }
       }
@@ -2752,7 +2772,7 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
   auto finish = [&](uint32_t live, uint32_t btests) {
     pairs_lane += BINS == 3 ? inb >> 1 : inb;
     if (lane == 0) centres += (unsigned long long)__popc(live);
-    if constexpr (BINS == 1 || BINS == 2) {
+    if constexpr (BINS != 3) {
       // keep every shared bin below 2^32: a bin gains at most one count per
       // credit of a test; each time the block's tests cross a multiple of 2^30
       // the warp that crossed it moves all bins to the global uint64 cores
@@ -2781,7 +2801,7 @@ __global__ void __launch_bounds__(kLanesWarps * 32, 1) k_lanes(ScanArgs a) {
   });
   if (lane == 0 && a.tests) atomicAdd(a.tests, tests);
   __syncthreads();
-  if constexpr (BINS == 1 || BINS == 2)
+  if constexpr (BINS != 3)
     for (uint32_t i = threadIdx.x; i < nbin; i += blockDim.x) {
       const uint32_t v = srdf[i];
       if (v) flush_bin(i, v);
@@ -4822,19 +4842,41 @@ static size_t lanes_smem(const ScanArgs& a, size_t bins, bool fast) {
          (fast ? 0 : (size_t)((a.lut_n + 7) & ~7) * 2);
 }
 
+// Where k_lanes keeps its bins: by kind of pair while they fit beside the
+// staging buffers (2), then in the cores' layout (1), then some rows of the cores
+// (0; rows: how many fit).
+static constexpr size_t kLanesSmem = 224 * 1024;
+static int lanes_bins(const ScanArgs& a, size_t* words, int* rows) {
+  const bool fast = a.cat_fast != 0;
+  const size_t kinds = (size_t)a.nC * ((a.sym ? a.nC : 0) + a.nE + 1) * a.H, cores = (size_t)a.nC * a.nE * a.H;
+  const int bins = lanes_smem(a, kinds, fast) <= kLanesSmem ? 2 : lanes_smem(a, cores, fast) <= kLanesSmem ? 1 : 0;
+  *words = bins == 2 ? kinds : bins == 1 ? cores : 0;
+  // the map of the rows, both ways (at most as many as the cores have)
+  const size_t fixed = lanes_smem(a, 0, fast) + (size_t)a.nC * a.nE * 4;
+  *rows = bins || a.nC * a.nE > 4096 || fixed > kLanesSmem ? 0 : (int)((kLanesSmem - fixed) / ((size_t)a.H * 4));
+  return bins;
+}
+
+int lanes_rows(const ScanArgs& a) {
+  size_t words;
+  int rows;
+  lanes_bins(a, &words, &rows);
+  return rows;
+}
+
 int launch_lanes(const ScanArgs& a, int kr, int sm_count, size_t* smem_used, cudaStream_t s) {
   if (a.mode != 0 || kr > 0 || (a.flags & PP_CNTNB) || !(a.flags & PP_RDF) || a.bx < 1 || a.by < 1 || a.bz < 1 ||
       a.nC > 254 || a.nE > 254 || !a.brows)
     return -3;
-  // bins by kind of pair while they fit beside the staging buffers, then in
-  // the cores' layout, then none in shared memory
-  constexpr size_t cap = 224 * 1024;
   const bool fast = a.cat_fast != 0;
-  const size_t kinds = (size_t)a.nC * ((a.sym ? a.nC : 0) + a.nE + 1) * a.H, cores = (size_t)a.nC * a.nE * a.H;
-  const int bins = lanes_smem(a, kinds, fast) <= cap ? 2 : lanes_smem(a, cores, fast) <= cap ? 1 : 0;
-  const size_t smem = lanes_smem(a, bins == 2 ? kinds : bins == 1 ? cores : 0, fast);
+  size_t words;
+  int rows;
+  const int bins = lanes_bins(a, &words, &rows);
+  if (a.rows_held > rows) return -1;  // the caller asked lanes_rows
+  const size_t smem = a.rows_held > 0 ? lanes_smem(a, (size_t)a.rows_held * a.H, fast) + (size_t)a.nC * a.nE * 4
+                                      : lanes_smem(a, words, fast);
   if (smem_used) *smem_used = smem;
-  if (smem > cap) return -3;
+  if (smem > kLanesSmem) return -3;
 #define PP_LANES_KERN(SYMV, FASTV) \
   (bins == 2 ? k_lanes<SYMV, 2, FASTV> : bins == 1 ? k_lanes<SYMV, 1, FASTV> : k_lanes<SYMV, 0, FASTV>)
   auto kern = a.sym ? (fast ? PP_LANES_KERN(true, true) : PP_LANES_KERN(true, false))

@@ -193,3 +193,40 @@ def test_scan_of_dense_and_sparse_centres(ctx, oracle, targets, env):
     ref = oracle.spatstat(spec.xyz, spec.labels, d2, *hist, flags, targets, env, ks)
     assert np.array_equal(bins, ref["bins"]) and st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
     assert np.array_equal(counts, ref["cntnb"][:, : counts.shape[1]]) and ref["cntnb"][:, counts.shape[1]:].sum() == 0
+
+
+@pytest.mark.parametrize("nbins", [2500, 6000, 16380])
+@pytest.mark.parametrize("symmetric", [1, 0])
+@pytest.mark.parametrize("tasks", ["pairs", "matrix only around others", "matrix in no environment"])
+def test_rdf_rows_in_shared_memory(ctx, oracle, nbins, symmetric, tasks):
+    """Bins of which some rows fit in shared memory, one row or none: those of
+    the commonest types there, the others in global memory; more than half of
+    the ions are centres, some are not."""
+    spec = synth.cone_specimen(n=14000, r_apex=4.0, half_angle_deg=10.0, length=14.0, n_clusters=20, members=40,
+                               nspecies=6, seed=31, nseg=48, stack=4.0)
+    trg, env = {"pairs": _pairs(range(1, 7)),
+                "matrix only around others": ([[2], [3], [4, 5, 6]], [[1], [1, 2], [1]]),
+                "matrix in no environment": ([[t] for t in range(1, 7)], [[2, 3], [4], [5], [6], [2], [3]])}[tasks]
+    d2 = np.where(np.arange(len(spec.xyz)) % 5 == 0, 0.1, 10.0).astype(np.float32)
+    hist = (0.0, 0.9 / nbins, 0.9)
+    cid = ctx.upload(spec.xyz, spec.labels)
+    ctx.surfdist(cid, d2)
+    ctx.tasks(trg, env)
+    ctx.hist(*hist)
+    ctx.tuning(cid, 4.0, ((3 | 2 << 8 | 2 << 12) << 16) | N.PP_TILE_LANES)
+    ctx.set_option("symmetric", symmetric)
+    try:
+        got = []
+        for limit in (-1, 1 if symmetric else 2):  # with the map of the rows, and without it
+            ctx.set_option("scratch", limit)
+            ctx.run(cid, N.PP_RDF)
+            got.append((ctx.fetch(), ctx.stats()))
+            assert ctx.last_kernel() == "k_lanes"
+    finally:
+        ctx.set_option("scratch", -1)
+        ctx.set_option("symmetric", 1)
+        ctx.free(cid)
+    ref = oracle.spatstat(spec.xyz, spec.labels, d2, *hist, N.PP_RDF, trg, env, [])
+    for bins, st in got:
+        assert st["pairs"] == ref["pairs"] and st["centres"] == ref["centres"]
+        assert np.array_equal(bins, ref["bins"])
