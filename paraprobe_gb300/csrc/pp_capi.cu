@@ -1299,12 +1299,12 @@ int pp_cloud_inside(pp_ctx* ctx, int cloud, float bin_width_min, float bin_width
   // sums and status, then the ions per voxel and the union-find parents
   const size_t vox_bytes = 64 + (size_t)nxyz * 8;
   CK(ctx->vox.ensure(vox_bytes));
-  CK(cudaMemsetAsync(ctx->vox.p, 0, 64 + nxyz * 4, s));
+  CK(cudaMemsetAsync(ctx->vox.p, 0, vox_bytes, s));
   unsigned long long* sums = ctx->vox.as<unsigned long long>();
   uint32_t* occ = ctx->vox.as<uint32_t>() + 16;
   const uint32_t nv32[3] = {(uint32_t)nx, (uint32_t)ny, (uint32_t)nz};
   pp::launch_voxel_count(cl->xyz.as<float>(), n, lo, w, nv32, occ, (int*)(sums + 5), s);
-  pp::launch_voxel_classes(occ, nv32, occ + nxyz, (uint32_t*)(sums + 4), sums, s);
+  pp::launch_voxel_classes(occ, nv32, occ + nxyz, sums, s);
   CK(cudaGetLastError());
   unsigned long long got[6];
   CK(cudaMemcpyAsync(got, sums, sizeof got, cudaMemcpyDeviceToHost, s));

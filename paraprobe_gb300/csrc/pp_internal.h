@@ -257,9 +257,8 @@ void launch_tri_box(const float* tri, uint64_t ntri, float* box, cudaStream_t s)
 void launch_voxel_count(const float* xyz, uint64_t n, const float* lo, float w, const uint32_t* nv, uint32_t* occ,
                         int* status, cudaStream_t s);
 // vacuum, surface and inside voxels and the ions of the latter (sums[0..3],
-// zeroed by the caller); parent holds a word per voxel
-void launch_voxel_classes(const uint32_t* occ, const uint32_t* nv, uint32_t* parent, uint32_t* corner_root,
-                          unsigned long long* sums, cudaStream_t s);
+// zeroed by the caller, like up, a word per voxel); marks occ
+void launch_voxel_classes(uint32_t* occ, const uint32_t* nv, uint32_t* up, unsigned long long* sums, cudaStream_t s);
 // adds the list entries binning into tg makes to *total (caller zeroes it)
 void launch_tri_entries(const float* tbox, uint64_t ntri, Grid tg, float grow, unsigned long long* total,
                         cudaStream_t s);

@@ -548,101 +548,128 @@ __global__ void k_voxel_count(const float* __restrict__ xyz, uint64_t n, float l
 // labelled -y and -z alone), so the raster pass's clusters are the components
 // of a fixed graph and can be joined in any order: union-find in global memory,
 // a root hooked under a smaller root by compare-and-swap (parents only ever
-// fall, so every walk ends).  Bound by the latency of the walks; a 4M-ion tip's
-// 0.6M voxels take 0.15 ms where the host's raster pass took 8 ms.
-__device__ __forceinline__ uint32_t vox_root(uint32_t* parent, uint32_t a) {
+// fall, so every walk ends), as the concurrent disjoint sets of Anderson and
+// Woll (1991).  up[v] = v - parent of v, 0 for a root, so that cleared memory
+// holds single voxels.  Bound by the latency of the walks; a 4M-ion tip's 0.6M
+// voxels take 0.15 ms where the host's raster pass took 8 ms.  Vacuum voxels are
+// marked in occ (they hold no ion).  Grids that fit take one block, in shared
+// memory: three launches and walks in global memory cost clouds of 100 to 2,000
+// ions more than the host's pass did (a call 53 to 66 us -> 67 to 76; now 48 to 52).
+constexpr uint32_t kVacuum = 0xffffffffu;
+constexpr uint64_t kVoxelBlock = 4096;  // most voxels of a one-block grid
+__device__ __forceinline__ uint32_t vox_root(uint32_t* up, uint32_t a) {
   for (;;) {
-    const uint32_t p = *(volatile uint32_t*)&parent[a];
+    const uint32_t p = a - *(volatile uint32_t*)&up[a];
     if (p == a) return a;
-    const uint32_t g = *(volatile uint32_t*)&parent[p];
-    if (g != p) parent[a] = g;  // an ancestor still: shortens later walks
+    const uint32_t g = p - *(volatile uint32_t*)&up[p];
+    if (g != p) up[a] = a - g;  // an ancestor still: shortens later walks
     a = g;
   }
 }
-__device__ __forceinline__ void vox_join(uint32_t* parent, uint32_t a, uint32_t b) {
+__device__ __forceinline__ void vox_join(uint32_t* up, uint32_t a, uint32_t b) {
   for (;;) {
-    a = vox_root(parent, a);
-    b = vox_root(parent, b);
+    a = vox_root(up, a);
+    b = vox_root(up, b);
     if (a == b) return;
     if (a < b) {
       const uint32_t t = a;
       a = b;
       b = t;
     }
-    if (atomicCAS(&parent[a], a, b) == a) return;
+    if (atomicCAS(&up[a], 0u, a - b) == 0u) return;
   }
 }
-__global__ void k_voxel_init(uint64_t nv, uint32_t* parent) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x)
-    parent[v] = (uint32_t)v;
-}
-__global__ void k_voxel_join(const uint32_t* __restrict__ occ, uint32_t nx, uint32_t ny, uint64_t nv, uint32_t* parent) {
-  const uint64_t nxy = (uint64_t)nx * ny;
-  auto labelled = [&](uint64_t b) { return b != 0 && occ[b] == 0; };
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x) {
-    if (!labelled(v)) continue;
-    const uint64_t z = v / nxy, r = v - z * nxy, y = r / nx, x = r - y * nx;
-    const bool lx = x > 0 && labelled(v - 1), ly = y > 0 && labelled(v - nx), lz = z > 0 && labelled(v - nxy);
-    if (lx && !(ly && lz)) vox_join(parent, (uint32_t)v, (uint32_t)(v - 1));
-    if (ly) vox_join(parent, (uint32_t)v, (uint32_t)(v - nx));
-    if (lz) vox_join(parent, (uint32_t)v, (uint32_t)(v - nxy));
-  }
-}
-// parent[v] becomes 1 for the voxels of the guard corner's cluster (vacuum), 0
-// for the others; needs the roots first (k_voxel_roots).
-__global__ void k_voxel_roots(uint64_t nv, uint32_t* parent, uint32_t corner, uint32_t* corner_root) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x) {
-    // walks that shorten nothing: the roots written here must stay
-    uint32_t r = (uint32_t)v;
-    for (uint32_t p = *(volatile uint32_t*)&parent[r]; p != r; p = *(volatile uint32_t*)&parent[r]) r = p;
-    if (v == corner) *corner_root = r;
-    parent[v] = r;
-  }
-}
-__global__ void k_voxel_vacuum(const uint32_t* __restrict__ occ, uint64_t nv, uint32_t* root, uint32_t corner,
-                               const uint32_t* corner_root) {
-  const bool any = corner != 0 && occ[corner] == 0;
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x)
-    root[v] = any && v != 0 && occ[v] == 0 && root[v] == *corner_root ? 1u : 0u;
-}
-// Vacuum, surface (a Moore neighbour off the border is vacuum,
-// src/PARAPROBE_SolverHdl.cpp:5132-5194) and inside voxels, and the ions of the
-// latter: out[0..3].
-__global__ void k_voxel_sum(const uint32_t* __restrict__ occ, const uint32_t* __restrict__ vac, uint32_t nx, uint32_t ny,
-                            uint32_t nz, unsigned long long* __restrict__ out) {
-  const uint64_t nxy = (uint64_t)nx * ny, nv = nxy * nz;
-  unsigned long long cnt[4] = {0, 0, 0, 0};
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x) {
-    if (vac[v]) {
-      ++cnt[0];
-      continue;
+struct VoxelGrid {
+  uint32_t nx, ny, nz;
+  uint32_t* occ;
+  uint32_t* up;
+  __device__ __forceinline__ uint64_t nxy() const { return (uint64_t)nx * ny; }
+  // voxels first, first + step, ... of each pass; all of one before the next
+  __device__ __forceinline__ void join(uint64_t first, uint64_t step) const {
+    auto labelled = [&](uint64_t b) { return b != 0 && occ[b] == 0; };
+    for (uint64_t v = first; v < nxy() * nz; v += step) {
+      if (!labelled(v)) continue;
+      const uint64_t z = v / nxy(), r = v - z * nxy(), y = r / nx, x = r - y * nx;
+      const bool lx = x > 0 && labelled(v - 1), ly = y > 0 && labelled(v - nx), lz = z > 0 && labelled(v - nxy());
+      if (lx && !(ly && lz)) vox_join(up, (uint32_t)v, (uint32_t)(v - 1));
+      if (ly) vox_join(up, (uint32_t)v, (uint32_t)(v - nx));
+      if (lz) vox_join(up, (uint32_t)v, (uint32_t)(v - nxy()));
     }
-    const int z = (int)(v / nxy);
-    const uint64_t r = v - (uint64_t)z * nxy;
-    const int y = (int)(r / nx), x = (int)(r - (uint64_t)y * nx);
-    bool srf = false;
-    for (int dz = -1; dz <= 1 && !srf; ++dz)
-      for (int dy = -1; dy <= 1 && !srf; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int64_t X = (int64_t)x + dx, Y = (int64_t)y + dy, Z = (int64_t)z + dz;
-          if (X < 1 || Y < 1 || Z < 1 || X + 1 >= nx || Y + 1 >= ny || Z + 1 >= nz) continue;
-          if (vac[(uint64_t)Z * nxy + (uint64_t)Y * nx + (uint64_t)X]) {
-            srf = true;
-            break;
+  }
+  // marks the cluster of the guard corner (0, 0, nz - 1); walks that shorten nothing
+  __device__ __forceinline__ void mark(uint64_t first, uint64_t step) const {
+    auto root = [&](uint32_t a) {
+      for (uint32_t d = up[a]; d; d = up[a]) a -= d;
+      return a;
+    };
+    const uint64_t corner = (nz - 1) * nxy();
+    const uint32_t o = *(volatile uint32_t*)&occ[corner];
+    if (corner == 0 || (o != 0 && o != kVacuum)) return;
+    const uint32_t rc = root((uint32_t)corner);
+    for (uint64_t v = first; v < nxy() * nz; v += step)
+      if (v != 0 && *(volatile uint32_t*)&occ[v] == 0 && root((uint32_t)v) == rc) occ[v] = kVacuum;
+  }
+  // vacuum, surface (a Moore neighbour off the border is vacuum,
+  // src/PARAPROBE_SolverHdl.cpp:5132-5194) and inside voxels, and the ions of the
+  // latter, added to out[0..3]
+  __device__ __forceinline__ void sum(uint64_t first, uint64_t step, unsigned long long* __restrict__ out) const {
+    unsigned long long cnt[4] = {0, 0, 0, 0};
+    for (uint64_t v = first; v < nxy() * nz; v += step) {
+      if (occ[v] == kVacuum) {
+        ++cnt[0];
+        continue;
+      }
+      const int z = (int)(v / nxy());
+      const uint64_t r = v - (uint64_t)z * nxy();
+      const int y = (int)(r / nx), x = (int)(r - (uint64_t)y * nx);
+      bool srf = false;
+      for (int dz = -1; dz <= 1 && !srf; ++dz)
+        for (int dy = -1; dy <= 1 && !srf; ++dy)
+          for (int dx = -1; dx <= 1; ++dx) {
+            const int64_t X = (int64_t)x + dx, Y = (int64_t)y + dy, Z = (int64_t)z + dz;
+            if (X < 1 || Y < 1 || Z < 1 || X + 1 >= nx || Y + 1 >= ny || Z + 1 >= nz) continue;
+            if (occ[(uint64_t)Z * nxy() + (uint64_t)Y * nx + (uint64_t)X] == kVacuum) {
+              srf = true;
+              break;
+            }
           }
-        }
-    if (srf) {
-      ++cnt[1];
-    } else {
-      ++cnt[2];
-      cnt[3] += occ[v];
+      if (srf) {
+        ++cnt[1];
+      } else {
+        ++cnt[2];
+        cnt[3] += occ[v];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      for (int o = 16; o; o >>= 1) cnt[k] += __shfl_xor_sync(FULL, cnt[k], o);
+      if ((threadIdx.x & 31) == 0 && cnt[k]) atomicAdd(&out[k], cnt[k]);
     }
   }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    for (int o = 16; o; o >>= 1) cnt[k] += __shfl_xor_sync(FULL, cnt[k], o);
-    if ((threadIdx.x & 31) == 0 && cnt[k]) atomicAdd(&out[k], cnt[k]);
+};
+__global__ void k_voxel_join(VoxelGrid V) {
+  V.join(blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x);
+}
+__global__ void k_voxel_mark(VoxelGrid V) {
+  V.mark(blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x);
+}
+__global__ void k_voxel_sum(VoxelGrid V, unsigned long long* __restrict__ out) {
+  V.sum(blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x, out);
+}
+__global__ void __launch_bounds__(1024) k_voxel_block(VoxelGrid V, unsigned long long* __restrict__ out) {
+  __shared__ uint32_t occ[kVoxelBlock], up[kVoxelBlock];
+  for (uint32_t v = threadIdx.x; v < V.nxy() * V.nz; v += blockDim.x) {
+    occ[v] = V.occ[v];
+    up[v] = 0;
   }
+  V.occ = occ;
+  V.up = up;
+  __syncthreads();
+  V.join(threadIdx.x, blockDim.x);
+  __syncthreads();
+  V.mark(threadIdx.x, blockDim.x);
+  __syncthreads();
+  V.sum(threadIdx.x, blockDim.x, out);
 }
 
 // Caller-order variant for the entry point without allocations: positions as
@@ -4642,16 +4669,18 @@ void launch_voxel_count(const float* xyz, uint64_t n, const float* lo, float w, 
   k_voxel_count<<<grid_for(n, 256), 256, 0, s>>>(xyz, n, lo[0], lo[1], lo[2], w, nv[0], nv[1], nv[2], occ, status);
 }
 
-void launch_voxel_classes(const uint32_t* occ, const uint32_t* nv3, uint32_t* parent, uint32_t* corner_root,
-                          unsigned long long* sums, cudaStream_t s) {
-  const uint64_t nxy = (uint64_t)nv3[0] * nv3[1], nv = nxy * nv3[2];
-  const uint32_t corner = (uint32_t)((nv3[2] - 1) * nxy);
-  for (int k = 0; k < 5; ++k) counted();
-  k_voxel_init<<<grid_for(nv, 256), 256, 0, s>>>(nv, parent);
-  k_voxel_join<<<grid_for(nv, 256), 256, 0, s>>>(occ, nv3[0], nv3[1], nv, parent);
-  k_voxel_roots<<<grid_for(nv, 256), 256, 0, s>>>(nv, parent, corner, corner_root);
-  k_voxel_vacuum<<<grid_for(nv, 256), 256, 0, s>>>(occ, nv, parent, corner, corner_root);
-  k_voxel_sum<<<grid_for(nv, 256), 256, 0, s>>>(occ, parent, nv3[0], nv3[1], nv3[2], sums);
+void launch_voxel_classes(uint32_t* occ, const uint32_t* nv3, uint32_t* up, unsigned long long* sums, cudaStream_t s) {
+  const VoxelGrid V{nv3[0], nv3[1], nv3[2], occ, up};
+  const uint64_t nv = (uint64_t)nv3[0] * nv3[1] * nv3[2];
+  if (nv <= kVoxelBlock) {
+    counted();
+    k_voxel_block<<<1, 1024, 0, s>>>(V, sums);
+    return;
+  }
+  for (int k = 0; k < 3; ++k) counted();
+  k_voxel_join<<<grid_for(nv, 256), 256, 0, s>>>(V);
+  k_voxel_mark<<<grid_for(nv, 256), 256, 0, s>>>(V);
+  k_voxel_sum<<<grid_for(nv, 256), 256, 0, s>>>(V, sums);
 }
 
 void launch_tri_box(const float* tri, uint64_t ntri, float* box, cudaStream_t s) {
