@@ -110,6 +110,7 @@ struct Cloud {
   // (0 = the defaults below)
   uint32_t lanes_bx = 0, lanes_by = 0, lanes_bz = 0;
   uint64_t occupied = 0;  // non-empty cells of the grid
+  double density = 0.0;   // ions per nm^3 inside the specimen
   uint64_t fullest = 0, fullest_cell = 0;  // most ions of one of its 4 x 4 x 4 cell tiles, of a cell
   // the cell block was set by pp_cloud_prepare rather than by tuning: passes
   // take it only where centres are dense enough to fill a warp (default_block)
@@ -280,6 +281,16 @@ int fail(pp_ctx* c, int code, const char* fmt, ...) {
 inline bool has_type(const uint32_t* m, int t) { return (m[t >> 5] >> (t & 31)) & 1u; }
 
 // --------------------------------------------------------------------- grid
+// Ions per nm^3 inside the specimen: the mean m of a grid cell from the share
+// of cells that hold any, n / occupied = m / (1 - exp(-m)).
+double ion_density(uint64_t n, uint64_t occupied, double h) {
+  if (!occupied || !n) return 0.0;
+  const double per = (double)n / (double)occupied;
+  double m = per;
+  for (int i = 0; i < 30; ++i) m = per * (1.0 - std::exp(-m));
+  return m > 1e-3 ? m / (h * h * h) : 0.0;
+}
+
 int build_grid(pp_ctx* ctx, Cloud& cl, float R, cudaStream_t s) {
   const uint64_t n = cl.n;
   CK(ctx->bbox.ensure(8 * sizeof(uint32_t)));
@@ -353,21 +364,11 @@ int build_grid(pp_ctx* ctx, Cloud& cl, float R, cudaStream_t s) {
   cl.occupied = occ[0];
   cl.fullest = occ[1];
   cl.fullest_cell = occ[2];
+  cl.density = ion_density(n, occ[0], g.h);
   cl.g = g;
   cl.grid_ok = true;
   cl.grid_version = ctx->grid_counter++;
   return PP_OK;
-}
-
-// Ions per nm^3 inside the specimen: the mean m of a grid cell from the share
-// of cells that hold any, n / occupied = m / (1 - exp(-m)).
-double ion_density(const Cloud& cl) {
-  if (!cl.occupied || !cl.n) return 0.0;
-  const double per = (double)cl.n / (double)cl.occupied;
-  double m = per;
-  for (int i = 0; i < 30; ++i) m = per * (1.0 - std::exp(-m));
-  const double h = cl.g.h;
-  return m > 1e-3 ? m / (h * h * h) : 0.0;
 }
 
 // Default cell block of the centre-per-lane scans: about 28 centres (most of a
@@ -378,7 +379,7 @@ double ion_density(const Cloud& cl) {
 bool default_block(const Cloud& cl, uint64_t ncent, int* bx, int* by, int* bz) {
   const double per_cell = cl.occupied ? (double)ncent / (double)cl.occupied : 0.0;
   if (per_cell < 0.35) return false;
-  const double h = cl.g.h, mean = ion_density(cl) * h * h * h * (double)ncent / (double)cl.n;
+  const double h = cl.g.h, mean = cl.density * h * h * h * (double)ncent / (double)cl.n;
   const double cells = std::max(1.0, 28.0 / std::max(mean, 1e-3));
   const int side = (int)std::lround(std::cbrt(cells / 2.0));
   *by = *bz = std::min(15, std::max(1, side));
@@ -401,7 +402,7 @@ bool scratch(pp_ctx* ctx, DevBuf& b, size_t bytes) {
 struct LaneCost {
   double mean, most;
   LaneCost(const Cloud& cl, float R) {
-    const double tile_nm3 = std::pow(4.0 * cl.g.h, 3), tile = ion_density(cl) * tile_nm3, near = 8.0 * std::pow((double)R, 3);
+    const double tile_nm3 = std::pow(4.0 * cl.g.h, 3), tile = cl.density * tile_nm3, near = 8.0 * std::pow((double)R, 3);
     const double full = std::max(tile, (double)cl.fullest - 4.0 * std::sqrt(tile));
     mean = tile / tile_nm3 * near + 500.0;
     most = std::min(full / tile_nm3 * near + 500.0, 2.0 * full + mean);
@@ -424,7 +425,7 @@ struct LaneCost {
 bool lane_items(pp_ctx* ctx, const Cloud& cl, uint64_t ncent, pp::ScanArgs& a, cudaStream_t s) {
   const Grid& g = cl.g;
   const uint64_t cols = (((uint64_t)g.ny + a.by - 1) / a.by) * (((uint64_t)g.nz + a.bz - 1) / a.bz);
-  const double h = g.h, density = ion_density(cl), share = (double)ncent / (double)cl.n;
+  const double h = g.h, density = cl.density, share = (double)ncent / (double)cl.n;
   const double column = density * h * h * h * a.by * a.bz * share;  // centres per cell of length
   const double held = density > 0.0 ? (double)cl.n / (density * h * h * h * (double)g.ncells) : 1.0;
   auto items = [&](int ch) { return cols * (((uint64_t)g.nx + ch - 1) / ch); };
@@ -437,13 +438,20 @@ bool lane_items(pp_ctx* ctx, const Cloud& cl, uint64_t ncent, pp::ScanArgs& a, c
   a.nbricks = (uint32_t)nb;
   a.heavy = nullptr;
   const double cells = (double)a.by * a.bz * a.chunk;
-  const double most = share * std::min((double)cl.fullest_cell * cells, (double)cl.fullest * std::max(1.0, cells / 64.0));
+  // up to eight tiles as full as the fullest, the rest as full as the mean
+  const double most = share * (std::min((double)cl.fullest_cell * std::min(cells, 512.0),
+                                        (double)cl.fullest * std::min(std::max(1.0, cells / 64.0), 8.0)) +
+                               density * h * h * h * std::max(cells - 512.0, 0.0));
   const LaneCost cost(cl, a.R);
   a.heavy_lim = (uint32_t)std::max(64.0, std::min(8.0 * column * a.chunk, 1e9));
+  const uint64_t cap = cl.n / a.heavy_lim + 2;  // their number, and more than there can be of them
   if (most > (double)a.heavy_lim && nb < (1ull << 31) && most * cost.most > (double)ncent * cost.mean / warps &&
-      scratch(ctx, ctx->heavy, (cl.n / a.heavy_lim + 2) * 4)) {  // more than heavy_lim centres each
-    a.heavy = ctx->heavy.as<uint32_t>();
-    if (pp::launch_lane_heavy(a, ctx->heavy.as<uint32_t>(), s)) a.heavy = nullptr;
+      scratch(ctx, ctx->heavy, (cap + (nb + 31) / 32) * 4)) {
+    uint32_t* list = ctx->heavy.as<uint32_t>();
+    if (!pp::launch_lane_heavy(a, list, list + cap, s)) {
+      a.heavy = list;
+      a.heavy_bits = list + cap;
+    }
   }
   return true;
 }
@@ -559,7 +567,7 @@ int ensure_surface(pp_ctx* ctx, Cloud& cl, float R, cudaStream_t s, const float*
     pp::launch_surface_cells(cl.ions.as<float4>(), cl.cell_start.as<uint32_t>(), cl.g, cl.tri_f,
                              cl.tri_box.as<float>(), cl.tri_dev.as<float>(), cl.tcell_start.as<uint32_t>(),
                              cl.tcell_list.as<uint32_t>(), cl.tg, rp, cl.tri_slack,
-                             ion_density(cl) * cl.tg.h * cl.tg.h * cl.tg.h, dst->as<float>(), s);
+                             cl.density * cl.tg.h * cl.tg.h * cl.tg.h, dst->as<float>(), s);
     CK(cudaGetLastError());
   }
   if (!ctx->readonly_clouds) {
@@ -1306,7 +1314,7 @@ constexpr double kNearDenseR = 0.6;  // dense: first radius up to this share of 
 // RDF part 983 -> 817 us from 1e7 pairs on; with a count of their own even at
 // 9e7 (1108 / 1152 us) and 1775 -> 1442 us at 3.3e8.
 bool near_pays(const pp_ctx* ctx, const Cloud& cl, float R, int kmax, uint64_t centres, bool count) {
-  const double rho = ion_density(cl);
+  const double rho = cl.density;
   if (ctx->knn_walks == 1 || !(rho > 0.0) || near_radius(rho, 1.0, kmax) > kNearDenseR * R) return false;
   return ctx->knn_walks == 2 || (double)centres * rho * 4.18879 * R * R * R >= (count ? 1.5e8 : 1e7);
 }
@@ -1319,7 +1327,7 @@ bool near_plan(const Cloud& cl, const RunPlan& P, float R, const unsigned long l
                pp::ScanArgs& a, uint64_t* sparse) {
   const uint64_t n = cl.n;
   if (!a.uniform_sets || !P.disjoint || P.kmax < 1 || P.kmax > 20 || P.emax > 15 || !cl.occupied || !n) return false;
-  const double h = cl.g.h, rho = ion_density(cl);
+  const double h = cl.g.h, rho = cl.density;
   if (!(rho > 0.0)) return false;
   std::vector<uint64_t> ions(16, 0);
   for (int ty = 0; ty < 256; ++ty) {

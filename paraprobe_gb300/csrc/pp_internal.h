@@ -62,6 +62,7 @@ struct ScanArgs {
   uint32_t nbricks;
   int chunk;
   const uint32_t* heavy;         // chunks of more than heavy_lim centres: their number, then which (null: none)
+  const uint32_t* heavy_bits;    // a bit per chunk
   uint32_t heavy_lim;
   // centre-per-lane scans: per-slot pass codes (written by the pass, n words),
   // the labels they are made from, and 1.f (see dist2_x2)
@@ -289,8 +290,9 @@ int lanes_rows(const ScanArgs& a);
 // any 4 x 4 x 4 cells at a multiple of 4 and of any cell (cell_start has ncells
 // + 1 entries)
 void launch_count_occupied(const uint32_t* cell_start, Grid g, unsigned long long* out, int sm_count, cudaStream_t s);
-// lists the chunks of more than a.heavy_lim centres: out[0] = their number
-int launch_lane_heavy(const ScanArgs& a, uint32_t* out, cudaStream_t s);
+// lists the chunks of more than a.heavy_lim centres (list[0] = their number) and
+// sets their bits
+int launch_lane_heavy(const ScanArgs& a, uint32_t* list, uint32_t* bits, cudaStream_t s);
 // centre-per-lane block scan of kNN-only passes (k_lanes_knn); disjoint_sets:
 // every type in at most one environment set of each centre type
 // (ScanArgs::setidx valid); -3 = not applicable

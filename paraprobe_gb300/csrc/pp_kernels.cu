@@ -2363,39 +2363,29 @@ __device__ __forceinline__ uint32_t stage_rows(const ScanArgs& a, const LaneBatc
   return staged;
 }
 
-// Chunk w of the columns of blocks: cells [x0, x1) of the rows of its blocks;
-// number of its centres in rows r, r + step, ...
-struct LaneChunk {
-  int x0, x1, yb, ye, zb, ze;
-  __device__ __forceinline__ LaneChunk(const ScanArgs& a, uint32_t w) {
-    const Grid& g = a.g;
-    const int BY = max(a.by, 1), BZ = max(a.bz, 1), CH = a.chunk;
-    const uint32_t nch = (uint32_t)((g.nx + CH - 1) / CH), nby = (uint32_t)((g.ny + BY - 1) / BY);
-    if (a.sample_stride > 1) w *= a.sample_stride;
+// Chunks of more than heavy_lim centres are shared: their batches go round
+// kHeavyParts warps, which take them from a list before all other chunks (bits:
+// which those are).
+constexpr uint32_t kHeavyParts = 32, kShared = 1u << 31;
+__global__ void k_lane_heavy(ScanArgs a, uint32_t* list, uint32_t* bits) {
+  const Grid& g = a.g;
+  const int BY = max(a.by, 1), BZ = max(a.bz, 1), CH = a.chunk;
+  const uint32_t nch = (uint32_t)((g.nx + CH - 1) / CH), nby = (uint32_t)((g.ny + BY - 1) / BY);
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < a.nbricks; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t w = (uint32_t)i * (a.sample_stride > 1 ? a.sample_stride : 1u);
     const uint32_t col = w / nch, bz_i = col / nby;
-    yb = (int)(col - bz_i * nby) * BY;
-    zb = (int)bz_i * BZ;
-    ye = min(yb + BY, g.ny);
-    ze = min(zb + BZ, g.nz);
-    x0 = (int)(w - col * nch) * CH;
-    x1 = min(x0 + CH, g.nx);
-  }
-  __device__ __forceinline__ uint32_t centres(const ScanArgs& a, int r, int step) const {
+    const int y0 = (int)(col - bz_i * nby) * BY, z0 = (int)bz_i * BZ, x0 = (int)(w - col * nch) * CH, x1 = min(x0 + CH, g.nx);
     uint32_t n = 0;
-    for (; r < (ye - yb) * (ze - zb); r += step) {
-      const uint32_t row = ((uint32_t)(zb + r / (ye - yb)) * (uint32_t)a.g.ny + (uint32_t)(yb + r % (ye - yb))) * (uint32_t)a.g.nx;
-      n += (a.cell_start[row + x1] - a.cell_start[row + x0]) - (a.nc_pre[row + x1] - a.nc_pre[row + x0]);
+    for (int z = z0; z < min(z0 + BZ, g.nz); ++z)
+      for (int y = y0; y < min(y0 + BY, g.ny); ++y) {
+        const uint32_t row = ((uint32_t)z * (uint32_t)g.ny + (uint32_t)y) * (uint32_t)g.nx;
+        n += (a.cell_start[row + x1] - a.cell_start[row + x0]) - (a.nc_pre[row + x1] - a.nc_pre[row + x0]);
+      }
+    if (n > a.heavy_lim) {
+      list[1 + atomicAdd(list, 1u)] = (uint32_t)i;
+      atomicOr(&bits[i >> 5], 1u << (i & 31u));
     }
-    return n;
   }
-};
-
-// Chunks of very many centres are shared: their batches go round kHeavyParts
-// warps, which take them from a list before all other chunks.
-constexpr uint32_t kHeavyParts = 32;
-__global__ void k_lane_heavy(ScanArgs a, uint32_t* out) {
-  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < a.nbricks; w += (uint64_t)gridDim.x * blockDim.x)
-    if (LaneChunk(a, (uint32_t)w).centres(a, 0, 1) > a.heavy_lim) out[1 + atomicAdd(out, 1u)] = (uint32_t)w;
 }
 
 template <class Start, class Body>
@@ -2404,32 +2394,34 @@ __device__ __forceinline__ void lanes_blocks(const ScanArgs& a, float4* sbox, ui
   const int lane = threadIdx.x & 31;
   const uint32_t ltmask = (1u << lane) - 1u;
   for (;;) {
+    // found anew for every chunk: kept, they cost k_lanes registers it has not
+    // (104 bytes of spills a thread against 64; 2% of the 20M-ion tip's RDF pass)
+    const int BY = max(a.by, 1), BZ = max(a.bz, 1), CH = a.chunk;
+    const uint32_t nch = (uint32_t)((g.nx + CH - 1) / CH), nby = (uint32_t)((g.ny + BY - 1) / BY);
     uint32_t w = 0;
     if (lane == 0) w = atomicAdd(a.work, 1u);
     w = __shfl_sync(FULL, w, 0);
-    uint32_t turn = 0, every = 0;  // batches until this warp's next one, and between them
-    bool light = false;            // heavy chunks are not this warp's alone
+    uint32_t turn = 0;  // batches until this warp's next one; kShared: the chunk is shared
     if (a.heavy) {
       const uint32_t shared = a.heavy[0] * kHeavyParts;
-      light = w >= shared;
-      if (light) {
-        w -= shared;
-      } else {
-        turn = w % kHeavyParts;
-        every = kHeavyParts - 1u;
+      if (w < shared) {
+        turn = kShared | (w % kHeavyParts);
         w = a.heavy[1 + w / kHeavyParts];
+      } else {
+        w -= shared;
+        if (w < a.nbricks && (a.heavy_bits[w >> 5] >> (w & 31u)) & 1u) continue;  // taken from the list
       }
     }
     if (w >= a.nbricks) break;
-    const LaneChunk K(a, w);
-    if (light && __reduce_add_sync(FULL, K.centres(a, lane, 32)) > a.heavy_lim) continue;
+    if (a.sample_stride > 1) w *= a.sample_stride;
+    const uint32_t col = w / nch, bz_i = col / nby;
     LaneBatch B;
-    B.yb = K.yb;
-    B.zb = K.zb;
-    B.ye = K.ye;
-    B.ze = K.ze;
-    const int X1 = K.x1;
-    for (B.xb = K.x0; B.xb < X1; B.xb = B.xe) {
+    B.yb = (int)(col - bz_i * nby) * BY;
+    B.zb = (int)bz_i * BZ;
+    B.ye = min(B.yb + BY, g.ny);
+    B.ze = min(B.zb + BZ, g.nz);
+    const int X1 = min((int)(w - col * nch) * CH + CH, g.nx);
+    for (B.xb = (int)(w - col * nch) * CH; B.xb < X1; B.xb = B.xe) {
       // the block's length: as many columns, up to 32, as hold at most 32
       // centres; cum = centres of the columns up to this lane's
       const int x = min(B.xb + lane, X1 - 1);
@@ -2481,11 +2473,11 @@ __device__ __forceinline__ void lanes_blocks(const ScanArgs& a, float4* sbox, ui
         have -= take;
         head += take;
         __syncwarp();
-        if (turn > 0u) {  // another warp's batch
+        if (turn & (kShared - 1u)) {  // another warp's batch
           --turn;
           continue;
         }
-        turn = every;
+        if (turn) turn += kHeavyParts - 1u;
         const float4 cp = start(self);
         const bool lv = cp.x != kInf();
         B.live = __ballot_sync(FULL, lv);
@@ -4738,7 +4730,7 @@ int launch_scan(const ScanArgs& a, int kr, int emax, int sm_count, size_t* smem_
   if (a.disjoint) {
     if (kr == 1)
       return a.sparse_centres ? launch_scan_t<1, 0, false, 5>(a, sm_count, smem, s) : launch_scan_t<1, 0>(a, sm_count, smem, s);
-    if (kr <= 4) return launch_scan_t<4, 0>(a, sm_count, smem, s);
+    if (kr <= 4) return launch_scan_t<4, 0, false, 3>(a, sm_count, smem, s);
   }
   if (kr == 1) {
     if (emax <= 1)
@@ -4931,10 +4923,12 @@ int launch_lanes_count(const ScanArgs& a, int sm_count, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_lane_heavy(const ScanArgs& a, uint32_t* out, cudaStream_t s) {
-  if (cudaMemsetAsync(out, 0, 4, s) != cudaSuccess) return -1;
+int launch_lane_heavy(const ScanArgs& a, uint32_t* list, uint32_t* bits, cudaStream_t s) {
+  if (cudaMemsetAsync(list, 0, 4, s) != cudaSuccess ||
+      cudaMemsetAsync(bits, 0, ((uint64_t)a.nbricks + 31) / 32 * 4, s) != cudaSuccess)
+    return -1;
   counted();
-  k_lane_heavy<<<grid_for(a.nbricks, 256), 256, 0, s>>>(a, out);
+  k_lane_heavy<<<grid_for(a.nbricks, 256), 256, 0, s>>>(a, list, bits);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
