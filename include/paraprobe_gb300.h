@@ -116,7 +116,8 @@ int pp_surfdist_fetch(pp_ctx* ctx, int cloud, float* d2_out, uint64_t n);
  * bin_width_max) (Settings AdvIonPruneBinWidthMin/Max), its Hoshen-Kopelman
  * vacuum, surface and inside voxels (:5059-5270,
  * src/PARAPROBE_HoshenKopelman.cpp).  voxels (nullable) receives 6 counts:
- * vacuum, surface and inside voxels, then nx, ny, nz. */
+ * vacuum, surface and inside voxels, then nx, ny, nz.  Takes 8 bytes of device
+ * memory a voxel, which the context keeps up to 256 MiB. */
 int pp_cloud_inside(pp_ctx* ctx, int cloud, float bin_width_min, float bin_width_max, uint64_t* nions_inside,
                     float* volume_inside, uint64_t* voxels);
 
@@ -246,15 +247,15 @@ int pp_fetch_npcorr(pp_ctx* ctx, uint32_t* counts, uint64_t cap, uint64_t* edge)
  *   "symmetric"         RDF/RIPK-only passes take each pair of two centres
  *                       once and credit both (default 1); 0 scans every
  *                       centre's full ball.  Results are identical either way.
- *   "lanes"             RDF/RIPK-only passes take the centre-per-lane brick
- *                       scan (default 1); 0 = the per-centre or brick scan.
+ *   "lanes"             passes of dense centres take the centre-per-lane scans
+ *                       (default 1); 0 = the per-centre or brick scan.
  *                       Results are identical either way.
  *   "uniform_sets"      the kNN centre-per-lane scan stages one set row per ion
  *                       when every centre type maps types to sets alike
  *                       (default 1); 0 decodes the set per centre slot.
  *                       Results are identical either way.
- *   "knn_lists"         lists of the kNN centre-per-lane scan: 0 = distances
- *                       while they fit two blocks per SM, bin categories
+ *   "knn_lists"         lists of the kNN centre-per-lane scans: 0 = distances
+ *                       while they leave 16 warps an SM, bin categories
  *                       beyond (default); 1 = distances; 2 = categories.
  *                       Results are identical either way.
  *   "knn_walks"         the kNN centre-per-lane scan walks dense sets only as
@@ -321,7 +322,8 @@ int pp_batched_graph(pp_ctx* ctx, uint64_t* nodes, uint64_t* captures, uint64_t*
 
 /* Neighbour set of one ion (input index): every other ion with float
  * d^2 <= r^2, d^2 = (xi-xj)^2 + (yi-yj)^2 + (zi-zj)^2 evaluated left to right
- * without contraction (src/PARAPROBE_KDTree.h:55-58), sorted by (d^2, id). */
+ * without contraction (src/PARAPROBE_KDTree.h:55-58), sorted by (d^2, id).
+ * The context keeps the 32 MiB the first call allocates. */
 int pp_neighbors(pp_ctx* ctx, int cloud, uint64_t ion, float r, uint64_t* ids,
                  float* d2, uint64_t cap, uint64_t* count);
 
@@ -356,8 +358,8 @@ int pp_run_tests(pp_ctx* ctx, uint64_t* tests);
  * builds its cell grid with edge r_lo, the hull lists for R' up to
  * max(r_hi, carve radius) and the cached ion2surf for R' = max(r_lo, carve);
  * unless the cloud was tuned, passes of dense centres then take the
- * centre-per-lane scans at a 4 x 2 x 2 cell block.  Required before a cloud
- * is served. */
+ * centre-per-lane scans with blocks of 2 x 2 cells across.  Required before a
+ * cloud is served. */
 int pp_cloud_prepare(pp_ctx* ctx, int cloud, float r_lo, float r_hi);
 
 /* ---- serving loop (no counterpart in the reference, which runs one task per

@@ -1513,8 +1513,8 @@ int run_plain(pp_ctx* ctx, Cloud* cl, uint32_t flags, const uint32_t* k_list, in
   }
   ctx->res.ncentres_total = ncent;
   ctx->res.n_ions = n;
-  // work counters of up to two launches, then pair / centre counters for a
-  // second launch that must not count them again
+  // work counters of up to three launches, then pair / centre counters for the
+  // launches that must not count them again
   CK(ctx->work.ensure(32));
   CK(cudaMemsetAsync(ctx->work.p, 0, 32, s));
   pp::ScanArgs a{};
@@ -1874,10 +1874,9 @@ int pp_autotune(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_list, 
   CK(cudaSetDevice(ctx->device));
   if (sample == 0) sample = 200000;
   // The sample must fill the GPU several times over, or kernels whose work
-  // items hold many centres (the centre-per-lane scans: a warp takes four cell
-  // blocks of about a warp of centres at once) run partly idle and rank below
-  // the per-centre scan although they win on the whole cloud: at least 8192
-  // centres per SM (four work items for each of 64 warps).
+  // items hold many centres (the centre-per-lane scans: a warp takes a chunk of
+  // a column of cells at once) run partly idle and rank below the per-centre
+  // scan although they win on the whole cloud: at least 8192 centres per SM.
   sample = std::max<uint32_t>(sample, (uint32_t)ctx->sm_count * 8192u);
   const float R = ctx->tab.rmax;
   const float ratios[] = {2.0f, 3.0f, 4.0f, 5.0f};
@@ -1924,9 +1923,10 @@ int pp_autotune(pp_ctx* ctx, int cloud, uint32_t flags, const uint32_t* k_list, 
     const bool lanes = ctx->last_kind >= 2;
     // two fixed cell-block shapes; for RDF / RIPK with kNN also the default
     // block at this cell edge (about a warp of centres), as the fixed shapes
-    // are sized for R = 2 nm at atom-probe densities.  (Offered to single
-    // passes too, the default block won on the tuning sample but lost on the
-    // whole 20M-ion tip, so they keep the two shapes.)
+    // are sized for R = 2 nm at atom-probe densities.  Single passes are not
+    // offered the default block; untuned, which is that block on cells of R/4,
+    // the 20M-ion tip is the faster now (RDF 13.1 against 13.6 ms, kNN 18.8
+    // against 20.6).
     int dbx = 0, dby = 0, dbz = 0;
     const bool dense = lanes && combined && default_block(*cl, ctx->last_centres_all, &dbx, &dby, &dbz);
     uint32_t tiles[sizeof scan_tiles / sizeof scan_tiles[0] + 3];
@@ -3299,8 +3299,8 @@ int pp_cloud_prepare(pp_ctx* ctx, int cloud, float r_lo, float r_hi) {
   }
   const float* surf = nullptr;
   if ((rc = ensure_surface(ctx, *cl, r_lo, 0, &surf))) return rc;
-  // passes of dense centres take the centre-per-lane scans at a 4 x 2 x 2 cell
-  // block (cells of r_lo), unless the cloud was tuned already
+  // passes of dense centres take the centre-per-lane scans with blocks of 2 x 2
+  // cells across (cells of r_lo), unless the cloud was tuned already
   if (!cl->lanes_bx) {
     cl->lanes_bx = 4;
     cl->lanes_by = 2;

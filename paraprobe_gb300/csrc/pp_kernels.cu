@@ -2142,10 +2142,11 @@ __device__ __forceinline__ void block_row_range(const ScanArgs& a, int r, int nr
 // never exceeds a centre's distance), so no ion an exact test would take is
 // dropped.  Survivors are packed into the staging buffer in stencil order (a
 // ring of two halves of 32); a batch of tests runs each time a half is full,
-// and once more for the rest after the last row.  On the 20M-ion tip (cells of R/4, 4 x 2 x 2 blocks) this took
+// and once more for the rest after the last row.  On the 20M-ion tip this took
 // the distance tests per pair from 2.66 to 1.78 (RDF) and from 4.43 to 2.92
-// (kNN).  An infinite ScanArgs::box_R2 stages every candidate, as an A/B
-// switch.
+// (kNN) when blocks were 4 x 2 x 2 cells; cut at 32 centres they take 1.47 in
+// symmetric passes.  An infinite ScanArgs::box_R2 stages every candidate, as an
+// A/B switch.
 //
 // An ion's pass code (ScanArgs::pcode, k_pass_codes) is staged as its record's
 // fourth word; in symmetric mode its lowest bit says that it is a centre and
@@ -2532,12 +2533,12 @@ struct FastCat {
 // RDF / RIPK pass.  Every lane bins its in-ball pairs inside the test loop:
 // d^2, the category and one shared-memory atomic per test, eight tests in
 // flight, no lists and no further warp synchronisation.  On the tips about a
-// fifth of the lanes hold an in-ball pair at a test, so four categories out of
-// five are computed for nothing; still this takes 20 instructions a test,
-// where a bit mask per test, a list of the taken pairs and their binning by
-// full warps (this kernel before) took 45.  Issue slots bound it (87% busy;
-// DRAM 0.3%): a third of its instructions stage the ions, two thirds test and
-// bin them.  All 36 pair RDFs of the 20M-ion tip (R = 2 nm, 0.01 nm bins): 32.1
+// third of the lanes hold an in-ball pair at a test (1.47 tests a pair, a pair
+// of two centres tested once), so two categories out of three are computed for
+// nothing; still this takes 20 instructions a test, where a bit mask per test, a
+// list of the taken pairs and their binning by full warps (this kernel before)
+// took 45.  Issue slots bound it (80% busy; DRAM 0.3%): a third of its
+// instructions stage the ions, two thirds test and bin them.  All 36 pair RDFs of the 20M-ion tip (R = 2 nm, 0.01 nm bins): 32.1
 // ms with lists, 23.3 ms binning in the loop, 19.1 ms with pairs of blocks met
 // once and the ring buffer, 15.6 ms with pass codes, packed sums, the
 // unpredicated atomic and the branch-free staging, 13.2 ms with blocks cut at
@@ -4451,13 +4452,13 @@ void launch_audit(const ScanArgs& a, double start, double scale, double end, dou
   k_audit<<<sm_count * 4, 256, smem, s>>>(a, x);
 }
 
-// all ions j != self with d^2 <= R^2 in the full 3-D stencil (debug / parity)
-// Neighbours of one ion (input index), as (bits of d^2, input index) in any
+// Neighbours of one ion (input index): all j != self with d^2 <= R^2 in the full
+// 3-D stencil, as (bits of d^2, input index) in any
 // order: out[0].x counts them, out[1 + i] holds the first `cap`.  Latency bound
 // (one ball): a block per few stencil rows, the ion's slot and the neighbours'
 // indices looked up here, so that the call needs one launch and one small
 // download (it used to allocate, and to download the whole index table: 380 us
-// a call on a 1M-ion cloud, now 22).
+// a call on a 1M-ion cloud, now 32).
 __global__ void k_neighbors(const float4* __restrict__ ions, const uint32_t* __restrict__ cell_start, Grid g,
                             const uint32_t* __restrict__ slot_of_id, const uint32_t* __restrict__ id_of_slot,
                             uint32_t ion, float R, uint2* out, uint32_t cap) {
